@@ -101,7 +101,6 @@ struct GemmParams {
   int tma_epi;                 // 1: bf16 outputs leave (and auxiliary inputs arrive) by TMA; 0: register/shared-memory epilogue
   int bias_vec;                // bias pointer is 16-byte aligned (vector loads)
   float* colsum;               // EPI_DGELU, TMA epilogue: colsum[n] += sum over rows of the (bf16) result, i.e. the bias gradient of the layer below
-  int dbg;                     // measurement switches: 1 = drain accumulators without storing, 2 = always fetch tile (0,0), 8 = skip the GELU math
   int* status;
 };
 
@@ -181,8 +180,7 @@ __device__ __forceinline__ void epi4(const GemmParams& p, float (&v)[4], int row
     for (int k = 0; k < 4; ++k) v[k] += x[k];
   }
   const uint2 o = pack4(v);
-  if (p.dbg & 4) asm volatile("st.global.cs.v2.b32 [%0], {%1, %2};" ::"l"(dp), "r"(o.x), "r"(o.y) : "memory");   // streaming store (measurement switch)
-  else *reinterpret_cast<uint2*>(dp) = o;
+  *reinterpret_cast<uint2*>(dp) = o;
 }
 
 // One epilogue warp drains its 32 rows x NCOLS columns of accumulator `tacc` (TMEM address incl. lane quarter).
@@ -204,21 +202,19 @@ __device__ __forceinline__ void epilogue_warp(const GemmParams& p, uint32_t tacc
       *reinterpret_cast<uint4*>(myrow + (((c + 8) ^ (lane & 15)) << 4)) = make_uint4(r1[4 * c], r1[4 * c + 1], r1[4 * c + 2], r1[4 * c + 3]);
     }
     __syncwarp();
-    if (!(p.dbg & 1)) {
 #pragma unroll
-      for (int it = 0; it < 8; ++it) {
-        const int rr = it * 4 + rsub;
-        const int row = row_base + rr;
-        const unsigned char* src = stage + rr * 256;
+    for (int it = 0; it < 8; ++it) {
+      const int rr = it * 4 + rsub;
+      const int row = row_base + rr;
+      const unsigned char* src = stage + rr * 256;
 #pragma unroll
-        for (int half = 0; half < 2; ++half) {
-          const int chunk = cl + half * 8;
-          const float4 f = *reinterpret_cast<const float4*>(src + ((chunk ^ (rr & 15)) << 4));
-          const int col = n0 + s * 64 + chunk * 4;
-          if (row < p.M && col < p.N) {
-            float v[4] = {f.x, f.y, f.z, f.w};
-            epi4<EPI>(p, v, row, col, alpha);
-          }
+      for (int half = 0; half < 2; ++half) {
+        const int chunk = cl + half * 8;
+        const float4 f = *reinterpret_cast<const float4*>(src + ((chunk ^ (rr & 15)) << 4));
+        const int col = n0 + s * 64 + chunk * 4;
+        if (row < p.M && col < p.N) {
+          float v[4] = {f.x, f.y, f.z, f.w};
+          epi4<EPI>(p, v, row, col, alpha);
         }
       }
     }
@@ -436,7 +432,7 @@ __device__ __forceinline__ void epi_slab_bf16(const GemmParams& p, const uint32_
       float x[8]; unpack8(pre, x);
 #pragma unroll
       for (int j = 0; j < 8; j += 2) {
-        const float2 y = (p.dbg & 8) ? make_float2(x[j], x[j + 1]) : gelu_fast2(make_float2(x[j], x[j + 1]));
+        const float2 y = gelu_fast2(make_float2(x[j], x[j + 1]));
         v[j] = y.x; v[j + 1] = y.y;
       }
       *reinterpret_cast<uint4*>(slot + SLAB_BYTES) = pack8(v);
@@ -493,7 +489,7 @@ __device__ __forceinline__ void epi_slab_gelu(const GemmParams& p, const uint4 (
     float x[8]; unpack8(pre[c], x);
 #pragma unroll
     for (int j = 0; j < 8; j += 2) {
-      const float2 y = (p.dbg & 8) ? make_float2(x[j], x[j + 1]) : gelu_fast2(make_float2(x[j], x[j + 1]));
+      const float2 y = gelu_fast2(make_float2(x[j], x[j + 1]));
       x[j] = y.x; x[j + 1] = y.y;
     }
     *reinterpret_cast<uint4*>(myrow + ((c ^ (lane & 7)) << 4)) = pack8(x);
@@ -590,8 +586,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       if (!ok && lane == 0) { *abort_flag = 1; atomicExch(p.status, LLMB_ERR_TIMEOUT); }
       for (int unit = cluster_id; unit < total_units && ok && !*abort_flag; unit += num_clusters) {
         int m_blk, n_blk, kb0, kb1; unit_coords(unit, m_blk, n_blk, kb0, kb1);
-        int m0 = m_blk * 2 * BM + (int)cta * BM, n0 = n_blk * BN + (int)cta * 128;
-        if (p.dbg & 2) { m0 = (int)cta * BM; n0 = (int)cta * 128; }
+        const int m0 = m_blk * 2 * BM + (int)cta * BM, n0 = n_blk * BN + (int)cta * 128;
         if (p.g.W > 1) {                                 // gathered A: this tile's chunk must have landed in local memory
           const int chunk = m_blk / p.g.tiles_per_chunk;
           if (chunk != p.g.me && chunk != landed) {
@@ -610,7 +605,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           unsigned char* sa = smem + stage * STAGE2_BYTES;
           unsigned char* sb = sa + A_STAGE;
           const uint32_t lead_full = lead_full0 + stage * 8;
-          const int k0 = (p.dbg & 2) ? 0 : kb * p.bke;
+          const int k0 = kb * p.bke;
           if (elect_one()) {
             if (leader) mbar_expect_tx(&full_bar[stage], 2 * STAGE2_BYTES);     // bytes of both CTAs
             if (!p.a_mn) tma_load_2d_pair(sa, &tmA, lead_full, k0, m0);
@@ -836,7 +831,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             }
             fence_proxy_async();
             __syncwarp();
-            if (lane == 0 && !(p.dbg & 1)) {
+            if (lane == 0) {
               if (EPI == EPI_ACC_F32) {
                 tma_reduce_add_2d(&tmD, buf, col0, row0);
                 if (col0 + 32 < p.N) tma_reduce_add_2d(&tmD, buf + SLAB_BYTES, col0 + 32, row0);
@@ -862,11 +857,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             epi_slab_pre(p, r0, r1, buf, col0, alpha, lane, pre);
             fence_proxy_async();
             __syncwarp();
-            if (lane == 0 && !(p.dbg & 1)) { tma_store_2d(&tmAux, buf, col0, row0); bulk_commit(); }
+            if (lane == 0) { tma_store_2d(&tmAux, buf, col0, row0); bulk_commit(); }
             epi_slab_gelu(p, pre, buf + SLAB_BYTES, lane);
             fence_proxy_async();
             __syncwarp();
-            if (lane == 0 && !(p.dbg & 1)) { tma_store_2d(&tmD, buf + SLAB_BYTES, col0, row0); bulk_commit(); }
+            if (lane == 0) { tma_store_2d(&tmD, buf + SLAB_BYTES, col0, row0); bulk_commit(); }
             continue;
           }
           epi_slab_bf16<EPI>(p, r0, r1, buf, col0, alpha, lane);
@@ -888,7 +883,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
               asm volatile("red.global.add.f32 [%0], %1;" ::"l"(p.colsum + col + 1), "f"(s1) : "memory");
             }
           }
-          if (lane == 0 && !(p.dbg & 1)) {
+          if (lane == 0) {
             if (Cfg::TWO_OUT) {
               tma_store_2d(&tmAux, buf, col0, row0);
               tma_store_2d(&tmD, buf + SLAB_BYTES, col0, row0);
@@ -1046,7 +1041,6 @@ int gemm_dispatch(void* D, const void* A, const void* B, const void* bias, void*
   p.io_f32 = (KIND == KIND_TF32) ? 1 : 0;
   p.bias_vec = (reinterpret_cast<uintptr_t>(bias) & 15) == 0;
   p.tma_epi = 0;
-  { static int dbg = -1; if (dbg < 0) { const char* e = getenv("LLMB_GEMM_DBG"); dbg = e ? atoi(e) : 0; } p.dbg = dbg; }
   if (pair) {
     const long long units2 = (long long)ceil_div(M, 2 * BM) * p.n_tiles * p.splits;
     const int max_clusters = sm_count() / 2;

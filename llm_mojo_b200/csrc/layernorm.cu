@@ -4,8 +4,8 @@
 // Reference behaviour: llmm/layernorm.mojo:197-331 (fwd, mean/rstd saved fp32), :651-1096 (fused
 // residual fwd), :1582-1895 (bwd with register-accumulated dgamma/dbeta partials + finalize),
 // :2426-2614 (fused residual bwd).  B200 design: one warp per row, the row lives in registers
-// (single HBM read), 16-byte accesses; backward is a persistent grid whose blocks write one
-// dgamma/dbeta partial row each into scratch, summed in block order by a finalize kernel so
+// (single HBM read), 16-byte accesses; backward is a persistent grid whose CTAs write one
+// dgamma/dbeta partial row each into scratch, summed in fixed order by a finalize kernel so
 // the result does not depend on scheduling.
 #include "common.cuh"
 using namespace llmb;
@@ -13,6 +13,7 @@ using namespace llmb;
 namespace {
 constexpr int LN_MAX_VEC = 16;  // 16-byte vectors per lane: C <= 32*16*8 = 4096 for bf16
 constexpr float LN_EPS = 1e-5f;
+constexpr int LN_BWD_ROWS = 3;    // rows a group of the backward kernel has in flight
 
 template <typename T, bool RESID, int PER_LANE>
 __global__ void __launch_bounds__(256) ln_fwd_kernel(T* __restrict__ out, float* __restrict__ mean_o, float* __restrict__ rstd_o,
@@ -75,117 +76,145 @@ __global__ void __launch_bounds__(256) ln_fwd_kernel(T* __restrict__ out, float*
   }
 }
 
-// Backward.  dres[row] (+)= LN'(dout[row]); partial dgamma/dbeta per block into scratch.
-// Each warp walks rows grid-stride and keeps dgamma/dbeta partials for its lanes' channels in
-// registers; warps of a block are then combined in fixed order through shared memory.
-// SUMOUT: the column sums of the values written to dres are a third per-block partial (the bias gradient of the
-// linear layer whose output gradient dres is), taken from the values as stored (after rounding to T).
-template <typename T, int PER_LANE, bool ACCUM, bool SUMOUT = false>
-__global__ void __launch_bounds__(256) ln_bwd_kernel(T* __restrict__ dres, float* __restrict__ partial,
-                                                    const T* __restrict__ dout, const T* __restrict__ inp,
-                                                    const T* __restrict__ w, const float* __restrict__ mean_i,
-                                                    const float* __restrict__ rstd_i, int rows, int C) {
+// Backward.  dres[row] (+)= LN'(dout[row]); partial dgamma / dbeta of every CTA into scratch.
+//
+// Bound by memory: three row reads and one row write.  A row belongs to a GROUP of ceil(C / N) threads rounded up to a warp, one
+// 16-byte vector per thread, so that a thread's dgamma / dbeta sums are 2 N registers whatever C is (with a warp per row they are
+// 2 C / 32 and leave one CTA of 256 threads per SM at C = 1280).  A group takes ROWS rows at a time: all their loads are in flight
+// before the first use, and their 2 ROWS dot products share one exchange through shared memory.  Several groups fill a CTA (one
+// CTA per SM), meet only at named barriers of their own, and add their sums up in group order at the end, which leaves
+// 148 partial rows for the finalize kernel instead of 296.
+// Measured on a B200, both kernels of a call, warp-per-row form -> this one: 4096 x 1280 25.2 -> 15.5 us, 8192 x 1280 32.1 -> 21.4,
+// 4096 x 1600 31.8 -> 18.5, 12288 x 1024 34.9 -> 23.5, 4096 x 768 14.5 -> 12.8, 65536 x 768 82.9 -> 81.8 (403 MB: 4.9 TB/s).
+// ROWS = 2 is within 1 us of 3 up to 12288 rows and 9 % slower at 65536; 4 spills and is 10 - 30 % slower everywhere.
+// SUMOUT: the column sums of the values written to dres are a third partial (the bias gradient of the linear layer whose output
+// gradient dres is), taken from the values as stored (after rounding to T).
+template <typename T, int ROWS, bool ACCUM, bool SUMOUT>
+__global__ void __launch_bounds__(640) ln_bwd_kernel(T* __restrict__ dres, float* __restrict__ partial, const T* __restrict__ dout,
+                                                    const T* __restrict__ inp, const T* __restrict__ w,
+                                                    const float* __restrict__ mean_i, const float* __restrict__ rstd_i, int rows,
+                                                    int C, int gthreads, int groups) {
   constexpr int N = Pack<T>::N;
   constexpr int NS = SUMOUT ? 3 : 2;
-  extern __shared__ float sm[];  // [warps][NS][C]
-  const int lane = threadIdx.x % 32, wid = threadIdx.x / 32, nwarps = blockDim.x / 32;
+  extern __shared__ float sm[];                        // [NS][C] column sums
+  __shared__ float2 xch[2][20][ROWS];                  // [parity][warp of the CTA][row]
+  const int group = threadIdx.x / gthreads, t = threadIdx.x - group * gthreads;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, gwarps = gthreads >> 5, gw0 = group * gwarps;
   const int nvec = C / N;
-  float dg[PER_LANE][N], db[PER_LANE][N], ds[SUMOUT ? PER_LANE : 1][N];
+  const bool act = t < nvec;
+  float dg[N], db[N], ds[SUMOUT ? N : 1];
 #pragma unroll
-  for (int i = 0; i < PER_LANE; ++i) {
+  for (int k = 0; k < N; ++k) { dg[k] = 0.f; db[k] = 0.f; if (SUMOUT) ds[k] = 0.f; }
+  uint4 wr = make_uint4(0, 0, 0, 0);                   // gamma of this thread's channels (raw: unpacked where it is used)
+  if (act) wr = *reinterpret_cast<const uint4*>(w + t * N);
+  const float inv_c = 1.f / C;
+  int par = 0;
+  const int stride = gridDim.x * groups * ROWS;
+  for (int row0 = (group * gridDim.x + blockIdx.x) * ROWS; row0 < rows; row0 += stride, par ^= 1) {
+    uint4 xr[ROWS], dr[ROWS], ar[ROWS];
 #pragma unroll
-    for (int k = 0; k < N; ++k) { dg[i][k] = 0.f; db[i][k] = 0.f; if (SUMOUT) ds[i][k] = 0.f; }
-  }
-  for (int row = blockIdx.x * nwarps + wid; row < rows; row += gridDim.x * nwarps) {
-    float mean = mean_i[row], rstd = rstd_i[row];
-    uint4 xr[PER_LANE], dr[PER_LANE], ar[PER_LANE];   // raw 16-byte vectors: the row stays in registers
-    float s1 = 0.f, s2 = 0.f;
-    // all global loads of the row (input, upstream gradient and the gradient accumulated so far) are issued
-    // before the first use, so the row costs one memory round trip instead of two
-#pragma unroll
-    for (int i = 0; i < PER_LANE; ++i) {
-      int vc = i * 32 + lane;
-      if (vc < nvec) {
-        xr[i] = *reinterpret_cast<const uint4*>(inp + (size_t)row * C + vc * N);
-        dr[i] = *reinterpret_cast<const uint4*>(dout + (size_t)row * C + vc * N);
-        if (ACCUM) ar[i] = *reinterpret_cast<const uint4*>(dres + (size_t)row * C + vc * N);
-      }
-    }
-#pragma unroll
-    for (int i = 0; i < PER_LANE; ++i) {
-      int vc = i * 32 + lane;
-      if (vc < nvec) {
-        Pack<T> x, d, ww; x.load(reinterpret_cast<const T*>(&xr[i])); d.load(reinterpret_cast<const T*>(&dr[i]));
-        ww.load(w + vc * N);
-#pragma unroll
-        for (int k = 0; k < N; ++k) {
-          float n_ = (x.v[k] - mean) * rstd;
-          float dn_ = d.v[k] * ww.v[k];
-          s1 += dn_; s2 += dn_ * n_;
-          dg[i][k] += d.v[k] * n_; db[i][k] += d.v[k];
+    for (int r = 0; r < ROWS; ++r) {
+      const int row = row0 + r;
+      if (row < rows) {
+        if (act) {
+          const size_t o = (size_t)row * C + t * N;
+          xr[r] = *reinterpret_cast<const uint4*>(inp + o);
+          dr[r] = *reinterpret_cast<const uint4*>(dout + o);
+          if (ACCUM) ar[r] = *reinterpret_cast<const uint4*>(dres + o);
         }
       }
+      if (row >= rows || !act) { xr[r] = make_uint4(0, 0, 0, 0); dr[r] = make_uint4(0, 0, 0, 0); }
     }
-    s1 = warp_sum(s1) / C; s2 = warp_sum(s2) / C;
+    float s1[ROWS], s2[ROWS];
 #pragma unroll
-    for (int i = 0; i < PER_LANE; ++i) {
-      int vc = i * 32 + lane;
-      if (vc < nvec) {
-        Pack<T> x, d, ww, o; x.load(reinterpret_cast<const T*>(&xr[i])); d.load(reinterpret_cast<const T*>(&dr[i]));
-        ww.load(w + vc * N);
-        if (ACCUM) o.load(reinterpret_cast<const T*>(&ar[i]));
-#pragma unroll
-        for (int k = 0; k < N; ++k) {
-          float n_ = (x.v[k] - mean) * rstd;
-          float g = (d.v[k] * ww.v[k] - s1 - n_ * s2) * rstd;
-          o.v[k] = ACCUM ? o.v[k] + g : g;
-          if (SUMOUT) ds[i][k] += round_to<T>(o.v[k]);
-        }
-        o.store(dres + (size_t)row * C + vc * N);
-      }
-    }
-  }
-  // block combine (fixed warp order)
-#pragma unroll
-  for (int i = 0; i < PER_LANE; ++i) {
-    int vc = i * 32 + lane;
-    if (vc < nvec) {
+    for (int r = 0; r < ROWS; ++r) {
+      Pack<T> x, d, ww; x.load(reinterpret_cast<const T*>(&xr[r])); d.load(reinterpret_cast<const T*>(&dr[r]));
+      ww.load(reinterpret_cast<const T*>(&wr));
+      const int row = min(row0 + r, rows - 1);
+      const float mean = mean_i[row], rstd = rstd_i[row];
+      s1[r] = 0.f; s2[r] = 0.f;
 #pragma unroll
       for (int k = 0; k < N; ++k) {
-        sm[(wid * NS + 0) * C + vc * N + k] = dg[i][k];
-        sm[(wid * NS + 1) * C + vc * N + k] = db[i][k];
-        if (SUMOUT) sm[(wid * NS + 2) * C + vc * N + k] = ds[i][k];
+        const float n_ = (x.v[k] - mean) * rstd;
+        const float dn_ = d.v[k] * ww.v[k];
+        s1[r] += dn_; s2[r] += dn_ * n_;
+        dg[k] += d.v[k] * n_; db[k] += d.v[k];
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r) { s1[r] = warp_sum(s1[r]); s2[r] = warp_sum(s2[r]); }
+    if (gwarps > 1) {                                  // alternating buffers: one barrier per exchange
+      if (lane == 0) {
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r) xch[par][wid][r] = make_float2(s1[r], s2[r]);
+      }
+      asm volatile("bar.sync %0, %1;" ::"r"(group + 1), "r"(gthreads) : "memory");
+#pragma unroll
+      for (int r = 0; r < ROWS; ++r) { s1[r] = 0.f; s2[r] = 0.f; }
+      for (int j = 0; j < gwarps; ++j) {
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r) { const float2 v = xch[par][gw0 + j][r]; s1[r] += v.x; s2[r] += v.y; }
+      }
+    }
+    if (act) {
+#pragma unroll
+      for (int r = 0; r < ROWS; ++r) {
+        const int row = row0 + r;
+        if (row >= rows) break;
+        // opaque to the compiler: otherwise it keeps the unpacked values of the first pass (64 registers) across the exchange
+        asm volatile("" : "+r"(xr[r].x), "+r"(xr[r].y), "+r"(xr[r].z), "+r"(xr[r].w), "+r"(dr[r].x), "+r"(dr[r].y), "+r"(dr[r].z), "+r"(dr[r].w));
+        asm volatile("" : "+r"(wr.x), "+r"(wr.y), "+r"(wr.z), "+r"(wr.w));
+        const float mean = mean_i[row], rstd = rstd_i[row];
+        Pack<T> ww; ww.load(reinterpret_cast<const T*>(&wr));
+        Pack<T> x, d, o; x.load(reinterpret_cast<const T*>(&xr[r])); d.load(reinterpret_cast<const T*>(&dr[r]));
+        if (ACCUM) o.load(reinterpret_cast<const T*>(&ar[r]));
+        const float m1 = s1[r] * inv_c, m2 = s2[r] * inv_c;
+#pragma unroll
+        for (int k = 0; k < N; ++k) {
+          const float n_ = (x.v[k] - mean) * rstd;
+          const float g = (d.v[k] * ww.v[k] - m1 - n_ * m2) * rstd;
+          o.v[k] = ACCUM ? o.v[k] + g : g;
+          if (SUMOUT) ds[k] += round_to<T>(o.v[k]);
+        }
+        o.store(dres + (size_t)row * C + t * N);
       }
     }
   }
-  __syncthreads();
-  for (int c = threadIdx.x; c < NS * C; c += blockDim.x) {
-    int which = c / C, cc = c % C;
-    float s = 0.f;
-    for (int wdx = 0; wdx < nwarps; ++wdx) s += sm[(wdx * NS + which) * C + cc];
-    partial[(size_t)blockIdx.x * NS * C + c] = s;
+  // the groups of the CTA in fixed order
+  for (int g = 0; g < groups; ++g) {
+    if (group == g && act) {
+#pragma unroll
+      for (int k = 0; k < N; ++k) {
+        const int c = t * N + k;
+        if (g == 0) { sm[c] = dg[k]; sm[C + c] = db[k]; if (SUMOUT) sm[2 * C + c] = ds[k]; }
+        else { sm[c] += dg[k]; sm[C + c] += db[k]; if (SUMOUT) sm[2 * C + c] += ds[k]; }
+      }
+    }
+    __syncthreads();
   }
+  for (int c = threadIdx.x; c < NS * C; c += blockDim.x) partial[(size_t)blockIdx.x * NS * C + c] = sm[c];
 }
 
-// dw[c] += sum_i partial[i][c], db[c] += sum_i partial[i][C + c] over the per-block partial rows.  A block of
-// 32 x 8 threads owns 32 adjacent columns of the 2C-wide partial matrix: 8 row groups walk the rows in parallel
-// (coalesced 128-byte reads) and are combined in fixed order through shared memory.
-__global__ void __launch_bounds__(256) ln_bwd_final_kernel(float* __restrict__ dw, float* __restrict__ db, float* __restrict__ dsum,
-                                                          const float* __restrict__ partial, int C, int nblocks) {
-  __shared__ float red[8][33];
+// dw[c] += sum_i partial[i][c], db[c] += sum_i partial[i][C + c] over the per-CTA partial rows.  A block of
+// 32 x 32 threads owns 32 adjacent columns of the partial matrix: 32 row groups walk the rows in parallel (coalesced
+// 128-byte reads, at most five dependent steps for 148 rows) and are combined in fixed order through shared memory.
+__global__ void __launch_bounds__(1024) ln_bwd_final_kernel(float* __restrict__ dw, float* __restrict__ db, float* __restrict__ dsum,
+                                                           const float* __restrict__ partial, int C, int nblocks) {
+  __shared__ float red[32][33];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int c = blockIdx.x * 32 + tx;
   const int NS = dsum ? 3 : 2;                           // dsum: third partial = column sums of the stored dres
   float s = 0.f;
-  if (c < NS * C)
-    for (int i = ty; i < nblocks; i += 8) s += partial[(size_t)i * NS * C + c];
+  if (c < NS * C) {
+#pragma unroll 5
+    for (int i = ty; i < nblocks; i += 32) s += partial[(size_t)i * NS * C + c];
+  }
   red[ty][tx] = s;
   __syncthreads();
-  if (ty == 0 && c < NS * C) {
-    float t = 0.f;
-#pragma unroll
-    for (int k = 0; k < 8; ++k) t += red[k][tx];
-    if (c < C) dw[c] += t; else if (c < 2 * C) db[c - C] += t; else dsum[c - 2 * C] += t;
+  const float v = warp_sum(red[tx][ty]);                 // warp ty adds up column ty
+  const int cc = blockIdx.x * 32 + ty;
+  if (tx == 0 && cc < NS * C) {
+    if (cc < C) dw[cc] += v; else if (cc < 2 * C) db[cc - C] += v; else dsum[cc - 2 * C] += v;
   }
 }
 
@@ -213,23 +242,36 @@ int ln_fwd_launch(void* out, float* mean, float* rstd, void* resid_out, const vo
 #undef LNF
 }
 
-template <typename T, int PER_LANE>
-int ln_bwd_launch_n(void* dres, float* partial, const void* dout, const void* inp, const void* w, const float* mean,
-                    const float* rstd, int rows, int C, int accumulate, int grid, cudaStream_t st, bool sumout = false) {
-  size_t smem = (size_t)8 * (sumout ? 3 : 2) * C * sizeof(float);
-  if (smem > 220 * 1024) return LLMB_ERR_BAD_ARG;
-  auto kern_a = ln_bwd_kernel<T, PER_LANE, true>;
-  auto kern_n = ln_bwd_kernel<T, PER_LANE, false>;
-  auto kern_as = ln_bwd_kernel<T, PER_LANE, true, true>;
-  auto kern_ns = ln_bwd_kernel<T, PER_LANE, false, true>;
-  if (smem > 48 * 1024) {
-    cudaFuncSetAttribute(kern_a, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    cudaFuncSetAttribute(kern_n, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    cudaFuncSetAttribute(kern_as, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    cudaFuncSetAttribute(kern_ns, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+// Threads per row group, groups per CTA and CTAs of the backward kernel: as many groups as fill 640 threads (96 registers each),
+// but no more than there are chunks of rows for (every group costs a step of the final combination).
+struct LnBwdPlan { int gthreads, groups, grid; };
+inline LnBwdPlan ln_bwd_plan(int rows, int C, int elems_per_vec) {
+  LnBwdPlan p;
+  p.gthreads = ceil_div(ceil_div(C, elems_per_vec), 32) * 32;
+  const int chunks = ceil_div(rows, LN_BWD_ROWS);
+  p.grid = chunks < sm_count() ? chunks : sm_count();
+  p.groups = 640 / p.gthreads;
+  if (p.groups > ceil_div(chunks, p.grid)) p.groups = ceil_div(chunks, p.grid);
+  if (p.groups < 1) p.groups = 1;
+  if (p.groups > 15) p.groups = 15;                      // named barriers 1 .. 15
+  return p;
+}
+
+template <typename T>
+int ln_bwd_launch(void* dres, float* partial, const void* dout, const void* inp, const void* w, const float* mean, const float* rstd,
+                  int rows, int C, int accumulate, bool sumout, cudaStream_t st) {
+  constexpr int N = Pack<T>::N;
+  if (C % N || C / N > 512) return LLMB_ERR_BAD_ARG;
+  const LnBwdPlan p = ln_bwd_plan(rows, C, N);
+  const size_t smem = (size_t)(sumout ? 3 : 2) * C * sizeof(float);
+  auto kern = sumout ? (accumulate ? ln_bwd_kernel<T, LN_BWD_ROWS, true, true> : ln_bwd_kernel<T, LN_BWD_ROWS, false, true>)
+                     : (accumulate ? ln_bwd_kernel<T, LN_BWD_ROWS, true, false> : ln_bwd_kernel<T, LN_BWD_ROWS, false, false>);
+  if (smem > 40 * 1024) {
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return (int)e;
   }
-  auto kern = sumout ? (accumulate ? kern_as : kern_ns) : (accumulate ? kern_a : kern_n);
-  kern<<<grid, 256, smem, st>>>((T*)dres, partial, (const T*)dout, (const T*)inp, (const T*)w, mean, rstd, rows, C);
+  kern<<<p.grid, p.gthreads * p.groups, smem, st>>>((T*)dres, partial, (const T*)dout, (const T*)inp, (const T*)w, mean, rstd, rows, C,
+                                                    p.gthreads, p.groups);
   return (int)cudaGetLastError();
 }
 }  // namespace
@@ -241,9 +283,9 @@ LLMB_API int llmb_layernorm_fwd(void* out, float* mean, float* rstd, void* resid
                             : ln_fwd_launch<float>(out, mean, rstd, resid_out, inp1, inp2, w, b, rows, C, st);
 }
 
-LLMB_API int llmb_layernorm_bwd_blocks(int rows) { int g = sm_count() * 2; int need = ceil_div(rows, 8); return need < g ? need : g; }
 LLMB_API long long llmb_layernorm_bwd_scratch_bytes(int rows, int C) {
-  return (long long)llmb_layernorm_bwd_blocks(rows) * 3 * C * sizeof(float);      // room for the optional column-sum partial
+  const int need = ceil_div(rows, LN_BWD_ROWS);
+  return (long long)(need < sm_count() ? need : sm_count()) * 3 * C * sizeof(float);      // room for the optional column-sum partial
 }
 
 // dres (+)= LN-backward(dout); dw += ..., db += ...  (dw/db fp32).  accumulate=1 adds into dres.
@@ -260,28 +302,12 @@ LLMB_API int llmb_layernorm_bwd(void* dres, float* dw, float* db, float* scratch
 LLMB_API int llmb_layernorm_bwd_colsum(void* dres, float* dw, float* db, float* dsum, float* scratch, long long scratch_bytes,
                                        const void* dout, const void* inp, const void* w, const float* mean,
                                        const float* rstd, int rows, int C, int accumulate, int dtype, cudaStream_t st) {
-  int grid = llmb_layernorm_bwd_blocks(rows);
   const bool sumout = dsum != nullptr;
-  if (scratch_bytes < (long long)grid * (sumout ? 3 : 2) * C * (long long)sizeof(float)) return LLMB_ERR_BAD_ARG;
-  int rc;
-  if (dtype == LLMB_BF16) {
-    int per = ceil_div(C / 8, 32);
-    if (C % 8) return LLMB_ERR_BAD_ARG;
-#define LN_CASE(P) rc = ln_bwd_launch_n<__nv_bfloat16, P>(dres, scratch, dout, inp, w, mean, rstd, rows, C, accumulate, grid, st, sumout)
-    if (per <= 2) LN_CASE(2); else if (per <= 3) LN_CASE(3); else if (per <= 4) LN_CASE(4); else if (per <= 5) LN_CASE(5);
-    else if (per <= 7) LN_CASE(7); else if (per <= 8) LN_CASE(8); else if (per <= 12) LN_CASE(12); else if (per <= 16) LN_CASE(16);
-    else return LLMB_ERR_BAD_ARG;
-#undef LN_CASE
-  } else {
-    int per = ceil_div(C / 4, 32);
-    if (C % 4) return LLMB_ERR_BAD_ARG;
-#define LN_CASE(P) rc = ln_bwd_launch_n<float, P>(dres, scratch, dout, inp, w, mean, rstd, rows, C, accumulate, grid, st, sumout)
-    if (per <= 2) LN_CASE(2); else if (per <= 4) LN_CASE(4); else if (per <= 6) LN_CASE(6); else if (per <= 8) LN_CASE(8);
-    else if (per <= 10) LN_CASE(10); else if (per <= 13) LN_CASE(13); else if (per <= 16) LN_CASE(16);
-    else return LLMB_ERR_BAD_ARG;
-#undef LN_CASE
-  }
+  const int grid = ln_bwd_plan(rows, C, 8).grid;
+  if (rows <= 0 || scratch_bytes < (long long)grid * (sumout ? 3 : 2) * C * (long long)sizeof(float)) return LLMB_ERR_BAD_ARG;
+  const int rc = dtype == LLMB_BF16 ? ln_bwd_launch<__nv_bfloat16>(dres, scratch, dout, inp, w, mean, rstd, rows, C, accumulate, sumout, st)
+                                    : ln_bwd_launch<float>(dres, scratch, dout, inp, w, mean, rstd, rows, C, accumulate, sumout, st);
   if (rc) return rc;
-  ln_bwd_final_kernel<<<ceil_div((sumout ? 3 : 2) * C, 32), 256, 0, st>>>(dw, db, dsum, scratch, C, grid);
+  ln_bwd_final_kernel<<<ceil_div((sumout ? 3 : 2) * C, 32), 1024, 0, st>>>(dw, db, dsum, scratch, C, grid);
   return (int)cudaGetLastError();
 }

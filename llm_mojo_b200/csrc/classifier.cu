@@ -320,22 +320,90 @@ __global__ void __launch_bounds__(1024, 1) classifier_stream2_kernel(__nv_bfloat
   }
 }
 
-template <typename T>
-__global__ void softmax_rows_kernel(float* __restrict__ out, const T* __restrict__ inp, int V, int ld, float inv_temp) {
-  __shared__ float red[32];
-  __shared__ float bc;
-  const int row = blockIdx.x, tid = threadIdx.x, lane = tid % 32, wid = tid / 32, nw = blockDim.x / 32;
+// Natural exponential of a difference to a row maximum: ex2.approx for values that came from bf16 (as in the fused classifier),
+// the library function for fp32 rows.
+template <typename T> __device__ __forceinline__ float exp_row(float d);
+template <> __device__ __forceinline__ float exp_row<float>(float d) { return expf(d); }
+template <> __device__ __forceinline__ float exp_row<__nv_bfloat16>(float d) { return ex2_fast(d * 1.4426950408889634f); }
+
+// (max, sum of exp(x - max)) of two disjoint sets of values
+__device__ __forceinline__ float2 merge_ms(float2 a, float2 b) {
+  const float m = fmaxf(a.x, b.x);
+  if (m == -INFINITY) return make_float2(m, 0.f);
+  return make_float2(m, a.y * expf(a.x - m) + b.y * expf(b.x - m));
+}
+__device__ __forceinline__ float2 warp_merge_ms(float2 v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v = merge_ms(v, make_float2(__shfl_xor_sync(0xffffffffu, v.x, o), __shfl_xor_sync(0xffffffffu, v.y, o)));
+  return v;
+}
+
+// Row softmax to fp32 with a cluster of CL CTAs per row.  A single row of a 50k vocabulary (one sampling step) is bound by one
+// SM's latency and load rate: spread over eight SMs, whose (max, sum) pairs meet through distributed shared memory, each thread
+// reads a couple of 16-byte vectors once for the statistics and once (from L1 / L2) for the result.  1 x 50257 bf16, one B200:
+// 74 us with one CTA and scalar loads.  From SM_CLUSTER_ROWS rows on one CTA per row fills the chip.
+template <typename T, int CL>
+__global__ void __launch_bounds__(512) softmax_rows_kernel(float* __restrict__ out, const T* __restrict__ inp, int V, int ld, float inv_temp) {
+  constexpr int N = Pack<T>::N;
+  __shared__ float2 red[16];
+  __shared__ float2 part[8];                              // written by every CTA of the cluster
+  const int tid = threadIdx.x, lane = tid % 32, wid = tid / 32;
+  const int row = blockIdx.x / CL, rank = CL > 1 ? (int)cluster_ctarank() : 0;
   const T* g = inp + (size_t)row * ld;
-  float mx = -INFINITY;
-  for (int i = tid; i < V; i += blockDim.x) mx = fmaxf(mx, to_f<T>(g[i]) * inv_temp);
-  mx = warp_max(mx); if (lane == 0) red[wid] = mx; __syncthreads();
-  if (wid == 0) { float m = lane < nw ? red[lane] : -INFINITY; m = warp_max(m); if (lane == 0) bc = m; } __syncthreads();
-  mx = bc; float s = 0.f;
-  for (int i = tid; i < V; i += blockDim.x) s += expf(to_f<T>(g[i]) * inv_temp - mx);
-  s = warp_sum(s); __syncthreads(); if (lane == 0) red[wid] = s; __syncthreads();
-  if (wid == 0) { float t = lane < nw ? red[lane] : 0.f; t = warp_sum(t); if (lane == 0) bc = t; } __syncthreads();
-  float inv = 1.f / bc;
-  for (int i = tid; i < V; i += blockDim.x) out[(size_t)row * V + i] = expf(to_f<T>(g[i]) * inv_temp - mx) * inv;
+  if (CL > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");   // the peers have started before anything is written to them
+  const bool vec = (reinterpret_cast<uintptr_t>(g) & 15) == 0;
+  const int chunk = ceil_div(ceil_div(V, CL), N) * N;     // columns per CTA, a whole number of vectors
+  const int c0 = min(rank * chunk, V), c1 = min(c0 + chunk, V);
+  float2 ms = make_float2(-INFINITY, 0.f);
+  for (int i = c0 + tid * N; i < c1; i += blockDim.x * N) {
+    float x[N], m = -INFINITY, sum = 0.f;
+    if (vec && i + N <= c1) { Pack<T> p; p.load(g + i);
+#pragma unroll
+      for (int k = 0; k < N; ++k) x[k] = p.v[k] * inv_temp;
+    } else {
+#pragma unroll
+      for (int k = 0; k < N; ++k) x[k] = i + k < c1 ? to_f<T>(g[i + k]) * inv_temp : -INFINITY;
+    }
+#pragma unroll
+    for (int k = 0; k < N; ++k) m = fmaxf(m, x[k]);
+    if (m == -INFINITY) continue;
+#pragma unroll
+    for (int k = 0; k < N; ++k) sum += expf(x[k] - m);
+    ms = merge_ms(ms, make_float2(m, sum));
+  }
+  ms = warp_merge_ms(ms);
+  if (lane == 0) red[wid] = ms;
+  __syncthreads();
+  if (CL > 1) asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+  if (wid == 0) {
+    ms = warp_merge_ms(lane < (int)blockDim.x / 32 ? red[lane] : make_float2(-INFINITY, 0.f));
+    if (CL == 1) { if (lane == 0) part[0] = ms; }
+    else if (lane < CL) {
+      const uint32_t a = mapa_u32(smem_u32(&part[rank]), lane);
+      asm volatile("st.shared::cluster.v2.f32 [%0], {%1, %2};" ::"r"(a), "f"(ms.x), "f"(ms.y) : "memory");
+    }
+  }
+  if (CL > 1) cluster_sync_all(); else __syncthreads();
+  ms = part[0];
+#pragma unroll
+  for (int j = 1; j < CL; ++j) ms = merge_ms(ms, part[j]);
+  const float inv = 1.f / ms.y;
+  for (int i = c0 + tid; i < c1; i += blockDim.x) out[(size_t)row * V + i] = expf(to_f<T>(g[i]) * inv_temp - ms.x) * inv;
+}
+constexpr int SM_CLUSTER_ROWS = 64;
+template <typename T>
+int softmax_rows_launch(float* out, const void* inp, int rows, int V, int ld, float inv_temp, cudaStream_t st) {
+  if (rows >= SM_CLUSTER_ROWS) {
+    softmax_rows_kernel<T, 1><<<rows, 512, 0, st>>>(out, (const T*)inp, V, ld, inv_temp);
+    return (int)cudaGetLastError();
+  }
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(rows * 8); cfg.blockDim = dim3(512); cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = 8; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+  cfg.attrs = at; cfg.numAttrs = 1;
+  return (int)cudaLaunchKernelEx(&cfg, softmax_rows_kernel<T, 8>, out, (const T*)inp, V, ld, inv_temp);
 }
 
 // dlogits = probs * (dprobs - sum_k dprobs[k] * probs[k]) over the first V columns of a row (one block per row);
@@ -426,42 +494,63 @@ LLMB_API int llmb_fused_classifier(void* logits, float* losses, const int* targe
 
 LLMB_API int llmb_softmax_rows(float* out, const void* inp, int rows, int V, int ld, float inv_temp, int dtype,
                                cudaStream_t st) {
-  if (dtype == LLMB_BF16) softmax_rows_kernel<__nv_bfloat16><<<rows, 256, 0, st>>>(out, (const __nv_bfloat16*)inp, V, ld, inv_temp);
-  else softmax_rows_kernel<float><<<rows, 256, 0, st>>>(out, (const float*)inp, V, ld, inv_temp);
-  return (int)cudaGetLastError();
+  return dtype == LLMB_BF16 ? softmax_rows_launch<__nv_bfloat16>(out, inp, rows, V, ld, inv_temp, st)
+                            : softmax_rows_launch<float>(out, inp, rows, V, ld, inv_temp, st);
 }
 
 // ---------------------------------------------------------------- chunked cross-entropy
 // Two-pass online-softmax CE over vocabulary tiles, so the full [rows, Vp] logits never exist
 // (llmm/fused_classifier.mojo:503-841).  stats[row] = {running max, running sum-exp, target logit, -}.
 namespace {
+// Both passes are bound by memory: pass 1 reads the tile once, pass 2 reads and writes it.  One CTA per row; a thread issues up to
+// four 16-byte loads before it uses the first.  Pass 1 keeps a running (max, sum of exponentials) per thread, so the tile is read
+// once (the maximum and the exponentials were separate sweeps of 2-byte loads before).
 template <typename T>
 __global__ void __launch_bounds__(256) ce_pass1_kernel(float4* __restrict__ stats, const T* __restrict__ tile, const int* __restrict__ targets,
                                                       int ld, int col0, int width, int V, int first) {
-  __shared__ float red[32];
-  __shared__ float bc;
-  const int row = blockIdx.x, tid = threadIdx.x, lane = tid % 32, wid = tid / 32, nw = blockDim.x / 32;
+  constexpr int N = Pack<T>::N, U = 4;
+  __shared__ float2 red[8];
+  const int row = blockIdx.x, tid = threadIdx.x, lane = tid % 32, wid = tid / 32;
   const T* g = tile + (size_t)row * ld;
   const int valid = min(width, V - col0);           // columns of this tile that are real vocabulary
-  float mx = -INFINITY;
-  for (int i = tid; i < valid; i += blockDim.x) mx = fmaxf(mx, to_f<T>(g[i]));
-  mx = warp_max(mx); if (lane == 0) red[wid] = mx; __syncthreads();
-  if (wid == 0) { float m = lane < nw ? red[lane] : -INFINITY; m = warp_max(m); if (lane == 0) bc = m; } __syncthreads();
-  mx = bc;
-  float s = 0.f;
-  for (int i = tid; i < valid; i += blockDim.x) s += expf(to_f<T>(g[i]) - mx);
-  s = warp_sum(s); __syncthreads(); if (lane == 0) red[wid] = s; __syncthreads();
-  if (wid == 0) { float t = lane < nw ? red[lane] : 0.f; t = warp_sum(t); if (lane == 0) bc = t; } __syncthreads();
-  if (tid == 0) {
-    float4 st = first ? make_float4(-INFINITY, 0.f, 0.f, 0.f) : stats[row];
-    if (valid > 0) {
-      const float m_new = fmaxf(st.x, mx);
-      st.y = st.y * expf(st.x - m_new) + bc * expf(mx - m_new);
-      st.x = m_new;
+  const int nvec = (reinterpret_cast<uintptr_t>(g) & 15) == 0 && valid > 0 ? valid / N : 0;
+  float2 ms = make_float2(-INFINITY, 0.f);
+  for (int v0 = tid; v0 < nvec; v0 += 256 * U) {
+    uint4 raw[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) if (v0 + u * 256 < nvec) raw[u] = *reinterpret_cast<const uint4*>(g + (size_t)(v0 + u * 256) * N);
+    float m = ms.x;
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (v0 + u * 256 < nvec) {
+        Pack<T> p; p.load(reinterpret_cast<const T*>(&raw[u]));
+#pragma unroll
+        for (int k = 0; k < N; ++k) m = fmaxf(m, p.v[k]);
+      }
+    if (m == -INFINITY) continue;
+    float s = ms.x == m ? ms.y : ms.y * exp_row<T>(ms.x - m);
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (v0 + u * 256 < nvec) {
+        Pack<T> p; p.load(reinterpret_cast<const T*>(&raw[u]));
+#pragma unroll
+        for (int k = 0; k < N; ++k) s += exp_row<T>(p.v[k] - m);
+      }
+    ms = make_float2(m, s);
+  }
+  for (int i = nvec * N + tid; i < valid; i += 256) ms = merge_ms(ms, make_float2(to_f<T>(g[i]), 1.f));
+  ms = warp_merge_ms(ms);
+  if (lane == 0) red[wid] = ms;
+  __syncthreads();
+  if (wid == 0) {
+    ms = warp_merge_ms(lane < 8 ? red[lane] : make_float2(-INFINITY, 0.f));
+    if (lane == 0) {
+      float4 st = first ? make_float4(-INFINITY, 0.f, 0.f, 0.f) : stats[row];
+      if (valid > 0) { const float2 n = merge_ms(make_float2(st.x, st.y), ms); st.x = n.x; st.y = n.y; }
+      const int tgt = targets[row];
+      if (tgt >= col0 && tgt < col0 + valid) st.z = to_f<T>(g[tgt - col0]);
+      stats[row] = st;
     }
-    const int tgt = targets[row];
-    if (tgt >= col0 && tgt < col0 + valid) st.z = to_f<T>(g[tgt - col0]);
-    stats[row] = st;
   }
 }
 __global__ void ce_loss_kernel(float* __restrict__ losses, const float4* __restrict__ stats, int rows) {
@@ -471,16 +560,30 @@ __global__ void ce_loss_kernel(float* __restrict__ losses, const float4* __restr
 template <typename T>
 __global__ void __launch_bounds__(256) ce_pass2_kernel(T* __restrict__ tile, const float4* __restrict__ stats, const int* __restrict__ targets,
                                                       int ld, int col0, int width, int V, float dloss) {
-  const int row = blockIdx.x;
+  constexpr int N = Pack<T>::N, U = 4;
+  const int row = blockIdx.x, tid = threadIdx.x;
   T* g = tile + (size_t)row * ld;
   const float4 st = stats[row];
   const float lse = st.x + logf(st.y);
   const int tgt = targets[row] - col0;
-  for (int i = threadIdx.x; i < width; i += blockDim.x) {
-    float v = 0.f;
-    if (col0 + i < V) v = (expf(to_f<T>(g[i]) - lse) - (i == tgt ? 1.f : 0.f)) * dloss;
-    g[i] = from_f<T>(v);
+  const int nvec = (reinterpret_cast<uintptr_t>(g) & 15) == 0 ? width / N : 0;
+  auto value = [&](float x, int i) { return col0 + i < V ? (exp_row<T>(x - lse) - (i == tgt ? 1.f : 0.f)) * dloss : 0.f; };
+  for (int v0 = tid; v0 < nvec; v0 += 256 * U) {
+    uint4 raw[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) if (v0 + u * 256 < nvec) raw[u] = *reinterpret_cast<const uint4*>(g + (size_t)(v0 + u * 256) * N);
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int v = v0 + u * 256;
+      if (v < nvec) {
+        Pack<T> p; p.load(reinterpret_cast<const T*>(&raw[u]));
+#pragma unroll
+        for (int k = 0; k < N; ++k) p.v[k] = value(p.v[k], v * N + k);
+        p.store(g + (size_t)v * N);
+      }
+    }
   }
+  for (int i = nvec * N + tid; i < width; i += 256) g[i] = from_f<T>(value(to_f<T>(g[i]), i));
 }
 }  // namespace
 

@@ -47,3 +47,39 @@ def test_layernorm_bwd_edges(rows, C, dtype):
     assert_close(got[0][1], rw, 1e-5 * math.sqrt(rows) + 1e-4, 1e-4, "dgamma")
     assert_close(got[0][2], rb, 1e-5 * math.sqrt(rows) + 1e-4, 1e-4, "dbeta")
     assert all(torch.equal(a, b) for a, b in zip(*got)), "LayerNorm backward must be bitwise repeatable"
+
+
+# whole vectors, a straddling last vector, a tile that ends beyond the vocabulary, a tile without any real column
+@pytest.mark.parametrize("rows,width,col0", [(1, 1024, 0), (37, 1000, 128), (5, 517, 3), (64, 1024, 29990), (3, 256, 30016)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_chunked_ce_edges(rows, width, col0, dtype):
+    V, ld = 30011, 1024
+    x = rnd(rows, ld, dtype=dtype, scale=3.0)
+    t = torch.randint(0, V, (rows,), dtype=torch.int32, generator=torch.Generator().manual_seed(1))
+    t[0] = col0 if col0 < V else 0
+    st0 = torch.tensor([2.0, 5.0, 0.5, 0.0]).repeat(rows, 1)
+    for first in (True, False):
+        ref, got = st0.clone(), st0.to(DEV)
+        ops.chunked_ce_pass1(ref, x[:, :width].float(), t, col0, width, V, first)
+        ops.chunked_ce_pass1(got, x.to(DEV)[:, :width], t.to(DEV), col0, width, V, first)
+        if first and col0 >= V:
+            assert bool((got[:, 1] == 0).all())
+            continue
+        assert_close(got[:, :3], ref[:, :3], 1e-6, 1e-5, f"statistics first={first}")
+    tile = x.to(DEV)
+    ops.chunked_ce_pass2(tile[:, :width], got, t.to(DEV), col0, width, V, 0.125)
+    ref_tile = x.float()[:, :width].clone()
+    ops.chunked_ce_pass2(ref_tile, ref, t, col0, width, V, 0.125)
+    eps = 2.0 ** -8 if dtype == torch.bfloat16 else 1e-5
+    assert_close(tile[:, :width], ref_tile, 1e-7, eps, "dlogits")
+    assert torch.equal(tile[:, width:].cpu(), x[:, width:]), "columns beyond the tile must stay"
+
+
+@pytest.mark.parametrize("rows", [1, 63, 64])          # a cluster of CTAs per row / one CTA per row
+@pytest.mark.parametrize("V", [1, 9, 4097, 50257])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_softmax_rows_edges(rows, V, dtype):
+    x = rnd(rows, (V + 15) // 8 * 8, dtype=dtype, scale=4.0)
+    got = ops.softmax_rows(x.to(DEV), V, 0.7)
+    assert_close(got, ops.softmax_rows(x, V, 0.7), 1e-7, 2e-5, "softmax")
+    assert _lib.read_status() == 0

@@ -895,7 +895,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         }
         if (!ok) { *abort_flag = 1; atomicExch(p.status, LLMB_ERR_TIMEOUT); break; }
         if (Cfg::AUX_IN && has_next) {                    // refill each buffer once its store has been read
-          if (lane == 0) bulk_wait_read<1>();
+          // (a unit at the right edge may have stored its last slab from buffer 0: then both stores must have been read)
+          if (lane == 0) { if (slab_valid(row0, n0, 1)) bulk_wait_read<1>(); else bulk_wait_read<0>(); }
           __syncwarp();
           aux_issue(nrow0, nn0, 0);
           if (lane == 0) bulk_wait_read<0>();

@@ -83,3 +83,16 @@ def test_softmax_rows_edges(rows, V, dtype):
     got = ops.softmax_rows(x.to(DEV), V, 0.7)
     assert_close(got, ops.softmax_rows(x, V, 0.7), 1e-7, 2e-5, "softmax")
     assert _lib.read_status() == 0
+
+
+def test_gemm_residual_right_edge_many_tiles():
+    """Several tiles per CTA pair with a right edge that leaves one 64-column slab in a warp's half of the tile: the slab's buffer is
+    refilled with the next tile's residual, which must wait for the store that still reads it."""
+    M, N, K = 256 * 74 * 3 + 40, 320, 64
+    x, w, r = rnd(M, K), rnd(N, K, scale=0.1, seed=1), rnd(M, N, seed=2)
+    ref = x.float() @ w.float().t() + r.float()
+    X, W, Rs = x.to(DEV), w.to(DEV), r.to(DEV)
+    for _ in range(5):
+        out = torch.empty(M, N, dtype=torch.bfloat16, device=DEV)
+        ops.matmul_fwd(out, X, W, torch.zeros(N, dtype=torch.bfloat16, device=DEV), residual=Rs)
+        assert_close(out, ref, 2.0 ** -6, 2.0 ** -8, "residual at the right edge")

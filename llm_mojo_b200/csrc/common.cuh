@@ -148,6 +148,13 @@ __device__ __forceinline__ float2 gelu_grad_fast2(float2 x) {
   return __ffma2_rn(__fmul2_rn(__fmul2_rn(x, half), d), u, s);
 }
 
+// Programmatic dependent launch.  A kernel launched with the attribute may start while the kernel before it in the stream is still
+// running: pdl_wait() returns once that kernel has completed and its writes are visible (and so, since every kernel here waits before
+// it touches anything, everything before it too); pdl_trigger() lets the kernel after this one be scheduled once all CTAs of this
+// one have called it or exited.  Both do nothing in an ordinary launch.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 inline int sm_count() {
   static int n = 0;
   if (n == 0) { int dev = 0; cudaGetDevice(&dev); cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev); if (n <= 0) n = 148; }

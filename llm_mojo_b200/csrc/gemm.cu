@@ -4,498 +4,19 @@
 // forward + bias / bias+GELU epilogues, :2789-2938 dinp with the dGELU epilogue, :3231-3509 dW
 // with beta=1 accumulate, :3671-3908 LM head; all of them cuBLASLt calls in the reference).
 //
-// Design (one CTA per SM, 192 threads):
-//   warp 0   TMA producer: streams 128x(128 B) A tiles and 256x(128 B) B tiles through a
-//            4-stage shared-memory ring (cp.async.bulk.tensor, 128-byte swizzle, no multicast)
-//   warp 1   MMA issuer: one elected lane issues tcgen05.mma 128x256xK_mma into one of two
-//            256-column TMEM accumulators and commits stage / accumulator mbarriers
-//   warps 2-5 epilogue: tcgen05.ld the finished accumulator (each warp its own 32-lane TMEM
-//            quarter), apply bias / GELU / dGELU / fp32 accumulate, store 16-byte vectors
-// so the epilogue of tile i overlaps the main loop of tile i+1.  Operands may be K-major or
-// MN-major (the UMMA descriptor and the TMA box change, not the data), which is how dinp
-// (B = W as stored) and dW (A = dout^T, B = inp^T as stored) run without any transposes.
-// Split-K work units reduce through fp32 red.global.add into the (fp32) gradient buffer.
+// Design: warp-specialised kernels in which a TMA producer streams 128-byte-swizzled operand tiles through a shared-memory ring
+// (cp.async.bulk.tensor, no multicast), one elected lane issues tcgen05.mma into TMEM accumulators, and epilogue warps read a
+// finished accumulator back, apply bias / GELU / dGELU / residual / fp32 accumulate and store through TMA.  Operands may be K-major or
+// MN-major (the UMMA descriptor and the TMA box change, not the data), which is how dinp (B = W as stored) and dW (A = dout^T,
+// B = inp^T as stored) run without any transposes.  Split-K work units add into the (fp32) gradient buffer.
 //
-// Three kernels share these parts: gemm_kernel (the design above, kept as the single-CTA comparator),
-// gemm_pair_kernel (the default: two CTAs per 256 x 256 tile with cta_group::2 MMAs, eight epilogue warps, TMA-store
-// epilogue, optional all-gather of A from peer GPUs and optional column sums of the result) and gemm_nvfp4_kernel
-// (block-scaled NVFP4 / MXFP8 operands with their scales in tensor memory, 128 x 256 tiles); each is described where
-// it is defined.
-#include <stdlib.h>
-#include "tc05.cuh"
-using namespace llmb;
-using namespace tc05;
+// gemm_pair_kernel (two CTAs per 256 x 256 tile with cta_group::2 MMAs, persistent, eight epilogue warps, optional all-gather of A
+// from peer GPUs and optional column sums of the result) runs what fills the chip with such tiles; gemm_small.cu runs the rest on
+// 128-row tiles; gemm_nvfp4_kernel has block-scaled NVFP4 / MXFP8 operands with their scales in tensor memory.  pick_tile() chooses.
+#include <math.h>
+#include "gemm_common.cuh"
 
 namespace {
-__device__ __forceinline__ unsigned ld_acquire_gpu(const unsigned* p) {
-  unsigned v; asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory"); return v;
-}
-__device__ __forceinline__ unsigned ld_acquire_sys(const unsigned* p) {
-  unsigned v; asm volatile("ld.acquire.sys.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory"); return v;
-}
-__device__ __forceinline__ uint4 ld_nc_v4(const uint4* p) {     // streaming 16-byte load (peer memory: read once)
-  uint4 v; asm volatile("ld.global.cg.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory"); return v;
-}
-__device__ __forceinline__ void fence_proxy_async_all() { asm volatile("fence.proxy.async;" ::: "memory"); }
-constexpr int BM = 128, BN = 256;
-constexpr int STAGES = 4;
-constexpr int ROW_BYTES = 128;                       // one swizzled row
-constexpr int A_STAGE = BM * ROW_BYTES;              // 16 KB
-constexpr int B_STAGE = BN * ROW_BYTES;              // 32 KB
-constexpr int STAGE_BYTES = A_STAGE + B_STAGE;
-constexpr int NUM_THREADS = 192;
-constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 4 * 32 * 256 /*epilogue transpose*/ + 1024 /*align*/ + 256 /*barriers*/;
-constexpr int BAND = 16;                             // m-tiles per rasterisation band
-
-enum { EPI_NONE = 0, EPI_BIAS = 1, EPI_BIAS_GELU = 2, EPI_DGELU = 3, EPI_ACC_F32 = 4, EPI_BIAS_RESID = 5, EPI_STORE_F32 = 6 };
-
-// All-gather fused into the GEMM: the A matrix [W*n, K] is the concatenation of W row chunks, chunk r produced by
-// rank r.  Every rank holds a full-size local buffer whose own chunk is already in place; two copier warps per
-// CTA pull the other chunks out of the peers' buffers (plain 16-byte peer loads over NVLink, each byte crosses
-// once) into the local buffer WHILE the tile loop runs, starting with the tiles of the local chunk and taking the
-// remote chunks in ring order.  A chunk's tiles are fetched (TMA, local memory) once every CTA's copiers have
-// counted it complete.
-struct GatherArgs {
-  const void* peer_src[8];     // [r]: start of chunk r inside rank r's buffer
-  void* local;                 // start of this rank's [W*n, K] buffer
-  const void* flags;           // this rank's flag words: peers announce "my chunk is written" (kind ROWS_READY)
-  unsigned* counts;            // [16] local counters, zeroed before the launch: [r] = slices of chunk r copied, [8 + r] = slice tickets
-  long long chunk_vecs;        // 16-byte vectors per chunk
-  unsigned seq, target;        // announce sequence number to wait for; slices per chunk (counts[r] == target: chunk landed)
-  int W, me, tiles_per_chunk;  // W = 0: no gather
-};
-
-// Parameter pull fused into a GEMM (ZeRO-3): the kernel's copier warps copy up to 8 segments of weights out of their
-// owners' parameter shards (plain 16-byte loads over NVLink, or local memory for the rank's own part) into this
-// rank's layer window while the tensor-core tile loop of the SAME kernel runs.  The segments may belong to the B
-// operand of this GEMM (then its TMA producer waits for them) or to the operand of a later GEMM of the layer, which
-// only checks the counters: every weight then arrives under the math of a tile loop.  Owners announce "my shard
-// holds the parameters of optimizer step seq" at flag kind PARAM; all waits are bounded.
-struct PullArgs {
-  const void* src[8];          // segment source (peer or local shard memory), 16-byte aligned
-  void* dst[8];                // segment destination inside the local window
-  long long vecs[8];           // 16-byte vectors per segment
-  const void* flags;           // this rank's flag words
-  unsigned* counts;            // [16] zeroed before the launch: [s] = slices of segment s landed, [8 + s] = slice tickets
-  const unsigned* wait_counts[8];   // counters this GEMM's B operand depends on ...
-  unsigned wait_target[8];          // ... and the value each must reach
-  unsigned seq;                // parameter sequence number the owners must have announced (0: none yet, no wait)
-  int owner[8];
-  int nseg, nwait, W;          // nseg = 0: nothing to pull; nwait = 0: nothing to wait for
-};
-
-struct GemmParams {
-  GatherArgs g;
-  PullArgs pull;
-  void* D; const void* bias; void* aux; const float* alpha;
-  int M, N, K;                 // K in elements
-  long long ldd, ldaux;
-  int a_mn, b_mn;              // operand majorness (0 = K-major)
-  int a_3d, b_3d;              // MN-major operand fetched with ONE 3-D box (chunk, k, chunk index) per stage
-  uint32_t a_lbo, a_sbo, a_kstep, b_lbo, b_sbo, b_kstep;   // bytes
-  uint32_t a_layout, b_layout; // UMMA layout type: 2 = SWIZZLE_128B, 1 = SWIZZLE_128B with 32-byte base (fp32 MN-major)
-  uint32_t idesc;
-  int bke;                     // K elements per stage
-  int m_tiles, n_tiles, splits, kb_per_split, kb_total;
-  int io_f32;                  // 1: D, bias and aux are fp32 (tf32 kind); 0: bf16
-  int tma_epi;                 // 1: bf16 outputs leave (and auxiliary inputs arrive) by TMA; 0: register/shared-memory epilogue
-  int bias_vec;                // bias pointer is 16-byte aligned (vector loads)
-  float* colsum;               // EPI_DGELU, TMA epilogue: colsum[n] += sum over rows of the (bf16) result, i.e. the bias gradient of the layer below
-  int* status;
-};
-
-// ------------------------------------------------------------------------------------------------
-// Coalesced epilogue.  tcgen05.ld hands each thread one accumulator ROW; stored directly, a warp
-// would touch 32 different rows per instruction.  Instead every 64-column slab of the warp's
-// 32 x 256 block goes through an 8 KB shared-memory transpose (XOR-swizzled 16-byte chunks, conflict
-// free in both directions) so that 8 consecutive lanes cover 64 contiguous bytes of one output row
-// and all global traffic of the epilogue (output, bias, GELU aux, residual) is sector-aligned.
-constexpr int EPI_STAGE_BYTES = 32 * 256;             // per epilogue warp: 32 rows x 64 fp32
-
-template <int EPI>
-__device__ __forceinline__ void epi4(const GemmParams& p, float (&v)[4], int row, int col, float alpha) {
-#pragma unroll
-  for (int k = 0; k < 4; ++k) v[k] *= alpha;
-  if (EPI == EPI_BIAS || EPI == EPI_BIAS_GELU || EPI == EPI_BIAS_RESID) {
-    if (p.bias && p.io_f32) {
-      const float4 b = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(p.bias) + col);
-      v[0] += b.x; v[1] += b.y; v[2] += b.z; v[3] += b.w;
-    } else if (p.bias) {
-      const uint2 braw = *reinterpret_cast<const uint2*>(reinterpret_cast<const __nv_bfloat16*>(p.bias) + col);
-      const __nv_bfloat162* bh = reinterpret_cast<const __nv_bfloat162*>(&braw);
-      const float2 b0 = __bfloat1622float2(bh[0]), b1 = __bfloat1622float2(bh[1]);
-      v[0] += b0.x; v[1] += b0.y; v[2] += b1.x; v[3] += b1.y;
-    }
-  }
-  if (EPI == EPI_ACC_F32 || EPI == EPI_STORE_F32) {
-    float* dp = reinterpret_cast<float*>(p.D) + (size_t)row * p.ldd + col;
-    if (EPI == EPI_ACC_F32)
-      asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dp), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]) : "memory");
-    else
-      *reinterpret_cast<float4*>(dp) = make_float4(v[0], v[1], v[2], v[3]);
-    return;
-  }
-  if (p.io_f32) {                                       // fp32 storage (tf32 tensor path)
-    float* dp = reinterpret_cast<float*>(p.D) + (size_t)row * p.ldd + col;
-    float* ap = reinterpret_cast<float*>(p.aux) + (size_t)row * p.ldaux + col;
-    if (EPI == EPI_BIAS_GELU) {
-      *reinterpret_cast<float4*>(ap) = make_float4(v[0], v[1], v[2], v[3]);
-#pragma unroll
-      for (int k = 0; k < 4; ++k) v[k] = gelu_f(v[k]);
-    } else if (EPI == EPI_DGELU) {
-      const float4 x = *reinterpret_cast<const float4*>(ap);
-      v[0] *= gelu_grad_f(x.x); v[1] *= gelu_grad_f(x.y); v[2] *= gelu_grad_f(x.z); v[3] *= gelu_grad_f(x.w);
-    } else if (EPI == EPI_BIAS_RESID) {
-      const float4 x = *reinterpret_cast<const float4*>(ap);
-      v[0] += x.x; v[1] += x.y; v[2] += x.z; v[3] += x.w;
-    }
-    *reinterpret_cast<float4*>(dp) = make_float4(v[0], v[1], v[2], v[3]);
-    return;
-  }
-  __nv_bfloat16* dp = reinterpret_cast<__nv_bfloat16*>(p.D) + (size_t)row * p.ldd + col;
-  __nv_bfloat16* ap = reinterpret_cast<__nv_bfloat16*>(p.aux) + (size_t)row * p.ldaux + col;
-  auto pack4 = [](const float (&x)[4]) {
-    uint2 u; __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&u);
-    h[0] = __floats2bfloat162_rn(x[0], x[1]); h[1] = __floats2bfloat162_rn(x[2], x[3]);
-    return u;
-  };
-  auto unpack4 = [](uint2 u, float (&x)[4]) {
-    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&u);
-    const float2 a = __bfloat1622float2(h[0]), b = __bfloat1622float2(h[1]);
-    x[0] = a.x; x[1] = a.y; x[2] = b.x; x[3] = b.y;
-  };
-  if (EPI == EPI_BIAS_GELU) {
-    const uint2 pre = pack4(v);
-    *reinterpret_cast<uint2*>(ap) = pre;               // pre-GELU activations (bf16)
-    float x[4]; unpack4(pre, x);
-#pragma unroll
-    for (int k = 0; k < 4; ++k) v[k] = gelu_f(x[k]);
-  } else if (EPI == EPI_DGELU) {
-    float x[4]; unpack4(*reinterpret_cast<const uint2*>(ap), x);
-#pragma unroll
-    for (int k = 0; k < 4; ++k) v[k] *= gelu_grad_f(x[k]);
-  } else if (EPI == EPI_BIAS_RESID) {
-    float x[4]; unpack4(*reinterpret_cast<const uint2*>(ap), x);
-#pragma unroll
-    for (int k = 0; k < 4; ++k) v[k] += x[k];
-  }
-  const uint2 o = pack4(v);
-  *reinterpret_cast<uint2*>(dp) = o;
-}
-
-// One epilogue warp drains its 32 rows x NCOLS columns of accumulator `tacc` (TMEM address incl. lane quarter).
-template <int EPI, int NCOLS = BN>
-__device__ __forceinline__ void epilogue_warp(const GemmParams& p, uint32_t tacc, unsigned char* stage, int row_base, int n0,
-                                              float alpha, int lane) {
-  const int rsub = lane >> 3, cl = lane & 7;
-#pragma unroll 1
-  for (int s = 0; s < NCOLS / 64; ++s) {
-    if (n0 + s * 64 >= p.N) break;                      // warp-uniform
-    uint32_t r0[32], r1[32];
-    tmem_ld32(tacc + s * 64, r0);
-    tmem_ld32(tacc + s * 64 + 32, r1);
-    tmem_wait_ld();
-    unsigned char* myrow = stage + lane * 256;
-#pragma unroll
-    for (int c = 0; c < 8; ++c) {
-      *reinterpret_cast<uint4*>(myrow + ((c ^ (lane & 15)) << 4)) = make_uint4(r0[4 * c], r0[4 * c + 1], r0[4 * c + 2], r0[4 * c + 3]);
-      *reinterpret_cast<uint4*>(myrow + (((c + 8) ^ (lane & 15)) << 4)) = make_uint4(r1[4 * c], r1[4 * c + 1], r1[4 * c + 2], r1[4 * c + 3]);
-    }
-    __syncwarp();
-#pragma unroll
-    for (int it = 0; it < 8; ++it) {
-      const int rr = it * 4 + rsub;
-      const int row = row_base + rr;
-      const unsigned char* src = stage + rr * 256;
-#pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        const int chunk = cl + half * 8;
-        const float4 f = *reinterpret_cast<const float4*>(src + ((chunk ^ (rr & 15)) << 4));
-        const int col = n0 + s * 64 + chunk * 4;
-        if (row < p.M && col < p.N) {
-          float v[4] = {f.x, f.y, f.z, f.w};
-          epi4<EPI>(p, v, row, col, alpha);
-        }
-      }
-    }
-    __syncwarp();
-  }
-}
-
-template <int KIND, int EPI>
-__global__ void __launch_bounds__(NUM_THREADS, 1)
-gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, const GemmParams p) {
-  extern __shared__ unsigned char smem_raw[];
-  unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  unsigned char* epi_stage = smem + STAGES * STAGE_BYTES;
-  uint64_t* full_bar = reinterpret_cast<uint64_t*>(epi_stage + 4 * 32 * 256);
-  uint64_t* empty_bar = full_bar + STAGES;
-  uint64_t* tfull_bar = empty_bar + STAGES;      // [2] accumulator ready
-  uint64_t* tempty_bar = tfull_bar + 2;          // [2] accumulator drained
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty_bar + 2);
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-
-  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < STAGES; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
-    for (int a = 0; a < 2; ++a) { mbar_init(&tfull_bar[a], 1); mbar_init(&tempty_bar[a], 4); }
-    *abort_flag = 0;
-    fence_barrier_init();
-    prefetch_tmap(&tmA); prefetch_tmap(&tmB);
-  }
-  if (warp == 1) tmem_alloc<512>(tmem_slot);
-  fence_before_sync();
-  __syncthreads();
-  fence_after_sync();
-  const uint32_t tmem_base = *tmem_slot;
-
-  const int tiles_per_split = p.m_tiles * p.n_tiles;
-  const int total_units = tiles_per_split * p.splits;
-
-  auto unit_coords = [&](int unit, int& m_blk, int& n_blk, int& kb0, int& kb1) {
-    int split = unit / tiles_per_split, t = unit % tiles_per_split;
-    int band_sz = BAND * p.n_tiles;
-    int b = t / band_sz, r = t % band_sz;
-    int m_in_band = min(BAND, p.m_tiles - b * BAND);
-    m_blk = b * BAND + r % m_in_band;
-    n_blk = r / m_in_band;
-    kb0 = split * p.kb_per_split;
-    kb1 = min(p.kb_total, kb0 + p.kb_per_split);
-  };
-
-  if (warp == 0) {
-    // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
-      int stage = 0; uint32_t phase = 0;
-      for (int unit = blockIdx.x; unit < total_units && !*abort_flag; unit += gridDim.x) {
-        int m_blk, n_blk, kb0, kb1; unit_coords(unit, m_blk, n_blk, kb0, kb1);
-        const int m0 = m_blk * BM, n0 = n_blk * BN;
-        for (int kb = kb0; kb < kb1; ++kb) {
-          if (!mbar_wait(&empty_bar[stage], phase ^ 1)) { *abort_flag = 1; atomicExch(p.status, LLMB_ERR_TIMEOUT); break; }
-          unsigned char* sa = smem + stage * STAGE_BYTES;
-          unsigned char* sb = sa + A_STAGE;
-          mbar_expect_tx(&full_bar[stage], STAGE_BYTES);
-          const int k0 = kb * p.bke;
-          if (!p.a_mn) tma_load_2d(sa, &tmA, &full_bar[stage], k0, m0);
-          else if (p.a_3d) tma_load_3d(sa, &tmA, &full_bar[stage], 0, k0, m0 / p.bke);
-          else {
-            const int chunk_elems = p.bke;   // elements per 128-byte row
-            const int nchunk = BM / chunk_elems;
-            for (int c = 0; c < nchunk; ++c) tma_load_2d(sa + c * p.bke * ROW_BYTES, &tmA, &full_bar[stage], m0 + c * chunk_elems, k0);
-          }
-          if (!p.b_mn) tma_load_2d(sb, &tmB, &full_bar[stage], k0, n0);
-          else if (p.b_3d) tma_load_3d(sb, &tmB, &full_bar[stage], 0, k0, n0 / p.bke);
-          else {
-            const int chunk_elems = p.bke;
-            const int nchunk = BN / chunk_elems;
-            for (int c = 0; c < nchunk; ++c) tma_load_2d(sb + c * p.bke * ROW_BYTES, &tmB, &full_bar[stage], n0 + c * chunk_elems, k0);
-          }
-          if (++stage == STAGES) { stage = 0; phase ^= 1; }
-        }
-      }
-    }
-  } else if (warp == 1) {
-    // ------------------------------------------------------------ MMA issuer
-    // warp-uniform loop, one elected lane issues; descriptors of stage 0 and the per-MMA increments are hoisted
-    {
-      int stage = 0; uint32_t phase = 0;
-      int it = 0;
-      const uint64_t adesc0 = make_smem_desc(smem_u32(smem), p.a_lbo, p.a_sbo, p.a_layout);
-      const uint64_t bdesc0 = make_smem_desc(smem_u32(smem) + A_STAGE, p.b_lbo, p.b_sbo, p.b_layout);
-      const uint64_t a_inc = (uint64_t)(p.a_kstep >> 4), b_inc = (uint64_t)(p.b_kstep >> 4);
-      const uint32_t idesc = p.idesc;
-      bool ok = true;
-      for (int unit = blockIdx.x; unit < total_units && !*abort_flag; unit += gridDim.x, ++it) {
-        int m_blk, n_blk, kb0, kb1; unit_coords(unit, m_blk, n_blk, kb0, kb1);
-        const int acc = it & 1;
-        const uint32_t acc_phase = (it >> 1) & 1;
-        if (!mbar_wait(&tempty_bar[acc], acc_phase ^ 1)) { ok = false; break; }
-        fence_after_sync();
-        const uint32_t d_tmem = tmem_base + acc * BN;
-        for (int kb = kb0; kb < kb1; ++kb) {
-          if (!mbar_wait(&full_bar[stage], phase)) { ok = false; break; }
-          fence_after_sync();
-          const uint64_t adesc = adesc0 + (uint64_t)(stage * (STAGE_BYTES >> 4));
-          const uint64_t bdesc = bdesc0 + (uint64_t)(stage * (STAGE_BYTES >> 4));
-          if (elect_one()) {
-            umma_ss<KIND>(d_tmem, adesc, bdesc, idesc, kb > kb0 ? 1u : 0u);
-#pragma unroll
-            for (int k = 1; k < 4; ++k) umma_ss<KIND>(d_tmem, adesc + k * a_inc, bdesc + k * b_inc, idesc, 1u);
-            umma_commit(&empty_bar[stage]);   // stage reusable once these MMAs have read it
-          }
-          __syncwarp();
-          if (++stage == STAGES) { stage = 0; phase ^= 1; }
-        }
-        if (!ok) break;
-        if (elect_one()) umma_commit(&tfull_bar[acc]);
-        __syncwarp();
-      }
-      if (!ok && lane == 0) { *abort_flag = 1; atomicExch(p.status, LLMB_ERR_TIMEOUT); }
-    }
-  } else {
-    // ------------------------------------------------------------ epilogue (warps 2..5)
-    const int q = warp & 3;                 // TMEM lane quarter this warp may access
-    int it = 0;
-    for (int unit = blockIdx.x; unit < total_units && !*abort_flag; unit += gridDim.x, ++it) {
-      int m_blk, n_blk, kb0, kb1; unit_coords(unit, m_blk, n_blk, kb0, kb1);
-      const int acc = it & 1;
-      const uint32_t acc_phase = (it >> 1) & 1;
-      if (!mbar_wait(&tfull_bar[acc], acc_phase)) { *abort_flag = 1; atomicExch(p.status, LLMB_ERR_TIMEOUT); break; }
-      fence_after_sync();
-      const int n0 = n_blk * BN;
-      const float alpha = p.alpha ? *p.alpha : 1.0f;
-      epilogue_warp<EPI>(p, tmem_base + ((uint32_t)(q * 32) << 16) + acc * BN, epi_stage + (warp - 2) * EPI_STAGE_BYTES,
-                         m_blk * BM + q * 32, n0, alpha, lane);
-      fence_before_sync();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&tempty_bar[acc]);
-    }
-  }
-
-  fence_before_sync();
-  __syncthreads();
-  if (warp == 1) { fence_after_sync(); tmem_dealloc<512>(tmem_base); }
-}
-
-
-// ------------------------------------------------------------------------------------------------
-// Epilogue through TMA (bf16 outputs of the CTA-pair kernel).  Each of the eight epilogue warps owns
-// 32 rows x 128 columns of the accumulator and moves them as two slabs of 64 columns = one
-// 128-byte-swizzled box of 32 rows x 128 B (4 KB) each:
-//   * tcgen05.ld gives each lane one row of the slab; bias, GELU, dGELU and the residual add happen in
-//     registers in that layout;
-//   * the auxiliary INPUT (residual stream, pre-GELU activations) arrives by TMA loads that are issued a
-//     whole tile ahead - while the tensor core is still busy with that tile - into the buffer the
-//     result is then written to in place;
-//   * results leave by TMA stores (bulk groups), so no lane ever waits on global memory and every
-//     global access of the epilogue is a full 128-byte row segment; out-of-range rows and columns are
-//     clipped by the tensor maps.
-// Epilogues with an auxiliary input or a second output (BIAS_GELU stores the pre-activation too) get
-// two 4 KB buffers per warp and a 5-deep operand ring, and so do the fp32 outputs (two 32-column boxes of a 64-column slab,
-// added into or stored to global memory by TMA); the others one buffer and a 6-deep ring.
-template <int EPI> struct EpiCfg {
-  static constexpr bool AUX_IN = EPI == EPI_DGELU || EPI == EPI_BIAS_RESID;
-  static constexpr bool TWO_OUT = EPI == EPI_BIAS_GELU;
-  static constexpr bool F32_OUT = EPI == EPI_ACC_F32 || EPI == EPI_STORE_F32;
-  static constexpr int STAGES = (F32_OUT || AUX_IN || TWO_OUT) ? 5 : 6;
-  static constexpr int WARP_STAGE = STAGES == 5 ? 16384 : 8192;     // staging bytes per warp of the 4-warp register epilogue (half that per warp of the 8-warp TMA epilogue)
-};
-constexpr int SLAB_BYTES = 32 * 128;
-
-__device__ __forceinline__ uint4 pack8(const float (&x)[8]) {
-  uint4 u; __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&u);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) h[i] = __floats2bfloat162_rn(x[2 * i], x[2 * i + 1]);
-  return u;
-}
-__device__ __forceinline__ void unpack8(const uint4& u, float (&x)[8]) {
-  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&u);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) { const float2 f = __bfloat1622float2(h[i]); x[2 * i] = f.x; x[2 * i + 1] = f.y; }
-}
-
-// One slab (this lane's row, 64 columns) from registers to the swizzled staging buffer.  With an
-// auxiliary input the buffer holds it on entry and the result replaces it; BIAS_GELU writes the
-// pre-activation to `buf` and the activation to `buf + SLAB_BYTES`.
-template <int EPI>
-__device__ __forceinline__ void epi_slab_bf16(const GemmParams& p, const uint32_t (&r0)[32], const uint32_t (&r1)[32],
-                                              unsigned char* buf, int col0, float alpha, int lane) {
-  unsigned char* myrow = buf + lane * 128;
-  const __nv_bfloat16* bias = reinterpret_cast<const __nv_bfloat16*>(p.bias);
-#pragma unroll
-  for (int c = 0; c < 8; ++c) {
-    float v[8], b[8];
-    const int col = col0 + c * 8;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) b[j] = 0.f;
-    if (EPI == EPI_BIAS || EPI == EPI_BIAS_GELU || EPI == EPI_BIAS_RESID) {
-      if (bias && col < p.N) {
-        if (p.bias_vec) unpack8(__ldg(reinterpret_cast<const uint4*>(bias + col)), b);
-        else {
-#pragma unroll
-          for (int j = 0; j < 8; ++j) b[j] = __bfloat162float(bias[col + j]);
-        }
-      }
-    }
-#pragma unroll
-    for (int j = 0; j < 8; j += 2) {
-      const uint32_t (&r)[32] = c < 4 ? r0 : r1;
-      const float2 y = __ffma2_rn(make_float2(__uint_as_float(r[(c & 3) * 8 + j]), __uint_as_float(r[(c & 3) * 8 + j + 1])),
-                                  make_float2(alpha, alpha), make_float2(b[j], b[j + 1]));
-      v[j] = y.x; v[j + 1] = y.y;
-    }
-    unsigned char* slot = myrow + ((c ^ (lane & 7)) << 4);
-    if (EPI == EPI_BIAS_GELU) {
-      const uint4 pre = pack8(v);
-      *reinterpret_cast<uint4*>(slot) = pre;
-      float x[8]; unpack8(pre, x);
-#pragma unroll
-      for (int j = 0; j < 8; j += 2) {
-        const float2 y = gelu_fast2(make_float2(x[j], x[j + 1]));
-        v[j] = y.x; v[j + 1] = y.y;
-      }
-      *reinterpret_cast<uint4*>(slot + SLAB_BYTES) = pack8(v);
-    } else {
-      if (EPI == EPI_DGELU || EPI == EPI_BIAS_RESID) {
-        float x[8]; unpack8(*reinterpret_cast<const uint4*>(slot), x);
-#pragma unroll
-        for (int j = 0; j < 8; j += 2) {
-          const float2 xx = make_float2(x[j], x[j + 1]), vv = make_float2(v[j], v[j + 1]);
-          const float2 y = (EPI == EPI_DGELU) ? __fmul2_rn(vv, gelu_grad_fast2(xx)) : __fadd2_rn(vv, xx);
-          v[j] = y.x; v[j + 1] = y.y;
-        }
-      }
-      *reinterpret_cast<uint4*>(slot) = pack8(v);
-    }
-  }
-}
-
-// The two halves of the bias + GELU epilogue, so that the pre-activation box can start leaving by TMA while the GELU of the
-// same slab is still being computed: first alpha, bias and the bf16 pre-activations (kept in registers as well) ...
-__device__ __forceinline__ void epi_slab_pre(const GemmParams& p, const uint32_t (&r0)[32], const uint32_t (&r1)[32],
-                                             unsigned char* buf, int col0, float alpha, int lane, uint4 (&pre)[8]) {
-  unsigned char* myrow = buf + lane * 128;
-  const __nv_bfloat16* bias = reinterpret_cast<const __nv_bfloat16*>(p.bias);
-#pragma unroll
-  for (int c = 0; c < 8; ++c) {
-    float v[8], b[8];
-    const int col = col0 + c * 8;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) b[j] = 0.f;
-    if (bias && col < p.N) {
-      if (p.bias_vec) unpack8(__ldg(reinterpret_cast<const uint4*>(bias + col)), b);
-      else {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) b[j] = __bfloat162float(bias[col + j]);
-      }
-    }
-#pragma unroll
-    for (int j = 0; j < 8; j += 2) {
-      const uint32_t (&r)[32] = c < 4 ? r0 : r1;
-      const float2 y = __ffma2_rn(make_float2(__uint_as_float(r[(c & 3) * 8 + j]), __uint_as_float(r[(c & 3) * 8 + j + 1])),
-                                  make_float2(alpha, alpha), make_float2(b[j], b[j + 1]));
-      v[j] = y.x; v[j + 1] = y.y;
-    }
-    pre[c] = pack8(v);
-    *reinterpret_cast<uint4*>(myrow + ((c ^ (lane & 7)) << 4)) = pre[c];
-  }
-}
-// ... then GELU of those bf16 values into the second box.
-__device__ __forceinline__ void epi_slab_gelu(const GemmParams& p, const uint4 (&pre)[8], unsigned char* buf, int lane) {
-  unsigned char* myrow = buf + lane * 128;
-#pragma unroll
-  for (int c = 0; c < 8; ++c) {
-    float x[8]; unpack8(pre[c], x);
-#pragma unroll
-    for (int j = 0; j < 8; j += 2) {
-      const float2 y = gelu_fast2(make_float2(x[j], x[j + 1]));
-      x[j] = y.x; x[j + 1] = y.y;
-    }
-    *reinterpret_cast<uint4*>(myrow + ((c ^ (lane & 7)) << 4)) = pack8(x);
-  }
-}
-
 // ------------------------------------------------------------------------------------------------
 // CTA-pair variant: a cluster of two CTAs computes a 256 x 256 tile with cta_group::2 MMAs.  Each
 // CTA stages its own 128 rows of A and its own 128-row half of B (half the B traffic per SM, and
@@ -765,20 +286,24 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     // Eight warps: warp % 4 selects the 32-row band (the TMEM lane quarter a warp may read), (warp - 2) / 4 the
     // 128-column half of the tile, i.e. two 64-column slabs per warp and tile.  The register epilogue (fp32
     // outputs, layouts without a tensor map) keeps four working warps with all four slabs of a band each.
+    // An fp32-storage problem (tf32) moves its 128 columns as four 32-column boxes through the same buffers.
+    constexpr bool F32_IO = KIND == KIND_TF32 && !Cfg::F32_OUT;
+    constexpr int NBOX = F32_IO ? 4 : 2, BOXC = F32_IO ? 32 : 64;
     const int q = warp & 3, e = warp - 2, hcol = e >> 2;
     const bool tma_epi = p.tma_epi;                       // warp-uniform
     unsigned char* wstage = epi_stage + e * (tma_epi ? WSB / 2 : WSB);
     uint64_t* abar = aux_bar + e * 2;
     const int band_off = (int)cta * BM + q * 32;
     uint32_t aux_phase = 0, aux_pending = 0;              // per-slab-buffer phase bits / loads in flight (warp-uniform)
-    // auxiliary-input tiles of a work unit: one box per 64-column slab that lies inside the matrix (ls = 0, 1)
-    auto slab_valid = [&](int row0, int n0, int ls) { return row0 < p.M && n0 + (hcol * 2 + ls) * 64 < p.N; };
+    // auxiliary-input tiles of a work unit: one box per slab that lies inside the matrix (ls < NBOX), in buffer ls & 1
+    auto slab_valid = [&](int row0, int n0, int ls) { return row0 < p.M && n0 + hcol * 128 + ls * BOXC < p.N; };
     auto aux_issue = [&](int row0, int n0, int ls) {      // all lanes keep the books, lane 0 issues
       if (!slab_valid(row0, n0, ls)) return;
-      aux_pending |= 1u << ls;
+      const int b = ls & 1;
+      aux_pending |= 1u << b;
       if (lane == 0) {
-        mbar_expect_tx(&abar[ls], SLAB_BYTES);
-        tma_load_2d(wstage + ls * SLAB_BYTES, &tmAux, &abar[ls], n0 + (hcol * 2 + ls) * 64, row0);
+        mbar_expect_tx(&abar[b], SLAB_BYTES);
+        tma_load_2d(wstage + b * SLAB_BYTES, &tmAux, &abar[b], n0 + hcol * 128 + ls * BOXC, row0);
       }
     };
     if (Cfg::AUX_IN && tma_epi && cluster_id < total_units) {
@@ -805,12 +330,12 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         if (has_next) { int mb, nb, k0, k1; unit_coords(nunit, mb, nb, k0, k1); nrow0 = mb * 2 * BM + band_off; nn0 = nb * BN; }
         bool ok = true;
 #pragma unroll 1
-        for (int ls = 0; ls < 2; ++ls) {
+        for (int ls = 0; ls < NBOX; ++ls) {
           if (!slab_valid(row0, n0, ls)) break;            // warp-uniform
-          const int col0 = n0 + (hcol * 2 + ls) * 64;
+          const int col0 = n0 + hcol * 128 + ls * BOXC;
           uint32_t r0[32], r1[32];
-          tmem_ld32(tacc + (hcol * 2 + ls) * 64, r0);
-          tmem_ld32(tacc + (hcol * 2 + ls) * 64 + 32, r1);
+          tmem_ld32(tacc + hcol * 128 + ls * BOXC, r0);
+          if (!F32_IO) tmem_ld32(tacc + hcol * 128 + ls * BOXC + 32, r1);
           tmem_wait_ld();
           unsigned char* buf;
           if (Cfg::F32_OUT) {
@@ -844,13 +369,30 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             continue;
           }
           if (Cfg::AUX_IN) {
-            buf = wstage + ls * SLAB_BYTES;
-            if (!mbar_wait(&abar[ls], (aux_phase >> ls) & 1)) { ok = false; break; }
-            aux_phase ^= 1u << ls; aux_pending &= ~(1u << ls);
+            const int b = ls & 1;
+            buf = wstage + b * SLAB_BYTES;
+            if (!mbar_wait(&abar[b], (aux_phase >> b) & 1)) { ok = false; break; }
+            aux_phase ^= 1u << b; aux_pending &= ~(1u << b);
           } else {
             buf = wstage;
             if (lane == 0) bulk_wait_read<0>();           // the previous slab's stores have read the buffer
             __syncwarp();
+          }
+          if (F32_IO) {
+            epi_box_f32<EPI>(p, r0, buf, buf + SLAB_BYTES, col0, alpha, lane);
+            fence_proxy_async();
+            __syncwarp();
+            if (lane == 0) {
+              if (Cfg::TWO_OUT) { tma_store_2d(&tmAux, buf, col0, row0); tma_store_2d(&tmD, buf + SLAB_BYTES, col0, row0); }
+              else tma_store_2d(&tmD, buf, col0, row0);
+              bulk_commit();
+            }
+            if (Cfg::AUX_IN && ls + 2 < NBOX && slab_valid(row0, n0, ls + 2)) {   // this buffer's next box, once the store has read it
+              if (lane == 0) bulk_wait_read<0>();
+              __syncwarp();
+              aux_issue(row0, n0, ls + 2);
+            }
+            continue;
           }
           if (Cfg::TWO_OUT) {
             uint4 pre[8];
@@ -867,22 +409,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           epi_slab_bf16<EPI>(p, r0, r1, buf, col0, alpha, lane);
           fence_proxy_async();
           __syncwarp();
-          if (EPI == EPI_DGELU && p.colsum) {
-            // column sums of the slab as stored (bf16): lane l adds up columns 2l and 2l + 1 of the warp's rows out of the
-            // swizzled box (conflict-free: the 32 lanes read the 128 bytes of one row) and adds them to colsum
-            float s0 = 0.f, s1 = 0.f;
-            const int nrows = min(32, p.M - row0);
-#pragma unroll 8
-            for (int r = 0; r < nrows; ++r) {
-              const uint32_t w = *reinterpret_cast<const uint32_t*>(buf + r * 128 + ((((lane >> 2) ^ (r & 7))) << 4) + (lane & 3) * 4);
-              s0 += __uint_as_float(w << 16); s1 += __uint_as_float(w & 0xffff0000u);
-            }
-            const int col = col0 + 2 * lane;
-            if (col < p.N) {
-              asm volatile("red.global.add.f32 [%0], %1;" ::"l"(p.colsum + col), "f"(s0) : "memory");
-              asm volatile("red.global.add.f32 [%0], %1;" ::"l"(p.colsum + col + 1), "f"(s1) : "memory");
-            }
-          }
+          if (EPI == EPI_DGELU && p.colsum) epi_slab_colsum(p, buf, row0, col0, lane);
           if (lane == 0) {
             if (Cfg::TWO_OUT) {
               tma_store_2d(&tmAux, buf, col0, row0);
@@ -896,7 +423,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         if (!ok) { *abort_flag = 1; atomicExch(p.status, LLMB_ERR_TIMEOUT); break; }
         if (Cfg::AUX_IN && has_next) {                    // refill each buffer once its store has been read
           // (a unit at the right edge may have stored its last slab from buffer 0: then both stores must have been read)
-          if (lane == 0) { if (slab_valid(row0, n0, 1)) bulk_wait_read<1>(); else bulk_wait_read<0>(); }
+          if (lane == 0) { if (slab_valid(row0, n0, NBOX - 1)) bulk_wait_read<1>(); else bulk_wait_read<0>(); }
           __syncwarp();
           aux_issue(nrow0, nn0, 0);
           if (lane == 0) bulk_wait_read<0>();
@@ -923,17 +450,12 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   if (warp == 1) { fence_after_sync(); tmem_dealloc_pair<512>(tmem_base); }
 }
 
-template <int KIND> struct KindTraits;
-template <> struct KindTraits<KIND_F16> { static constexpr int ESZ = 2; static constexpr CUtensorMapDataType DT = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16; };
-template <> struct KindTraits<KIND_TF32> { static constexpr int ESZ = 4; static constexpr CUtensorMapDataType DT = CU_TENSOR_MAP_DATA_TYPE_FLOAT32; };
-template <> struct KindTraits<KIND_F8F6F4> { static constexpr int ESZ = 1; static constexpr CUtensorMapDataType DT = CU_TENSOR_MAP_DATA_TYPE_UINT8; };
-
 int g_dbg_mn_lbo = -1, g_dbg_mn_sbo = -1;   // test hooks: override the MN-major descriptor strides
 thread_local float* g_pending_colsum = nullptr;   // armed by llmb_gemm_set_colsum, consumed by the calling thread's next llmb_gemm
 thread_local GatherArgs g_pending_gather{};   // armed by llmb_gemm_set_gather, consumed (and cleared) by the calling thread's next llmb_gemm
 thread_local PullArgs g_pending_pull{};       // armed by llmb_gemm_set_pull, consumed (and cleared) the same way
-int g_pair_mode = -1;                         // -1: read LLMB_GEMM_PAIR once; 0: single-CTA tiles; 1: CTA-pair tiles
-
+// LLMB_GEMM_PAIR=0 / llmb_gemm_set_pair_mode(0): 128 x 128 tiles on single CTAs wherever the layout allows (a comparator)
+int g_pair_mode = -1;
 bool pair_mode() {
   if (g_pair_mode < 0) { const char* e = getenv("LLMB_GEMM_PAIR"); g_pair_mode = (e && e[0] == '0') ? 0 : 1; }
   return g_pair_mode == 1;
@@ -953,16 +475,45 @@ int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap&
   return (int)cudaGetLastError();
 }
 
-template <int KIND, int EPI>
-int launch(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, int grid, cudaStream_t st) {
-  static bool attr_done = false;
-  if (!attr_done) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_kernel<KIND, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
-    if (e != cudaSuccess) return (int)e;
-    attr_done = true;
+// Tile configuration of one problem: bn = 256 is the CTA-pair kernel, 64 / 128 the kernel of gemm_small.cu with cl CTAs per tile.
+struct Tile { int bn, cl, splits; };
+int g_force_bn = 0, g_force_cl = 1;                       // test hook (llmb_gemm_force_tile): 0 = the rule decides
+
+// The configuration with the smallest estimated time, in microseconds on a B200 from linear fits over M = 64 ... 5439, K and N =
+// 384 ... 5120 (the fits are within 15 %; the small kernel must win by 5 %): a fixed part (launch, set-up, epilogue) plus a cost per
+// 128-byte k-block, bounded by what one SM can fetch (24 / 32 KB per k-block) in the small kernel and by the 256-row MMAs in the pair
+// kernel; MN-major operands cost more per k-block; more CTAs than SMs run side by side at the cost of each other's k-blocks; a
+// further round of pair tiles costs its epilogue if that is longer than its k-loop.  Clusters only while they fit in one round:
+// beyond it they were 1.5 - 4 times slower than one CTA per tile.  Measured, bias + residual: M 64, K 3072, N 768: pair 22.4 us,
+// 128 x 128 17.8, 64 x 4 CTAs 8.7; M 776, K 1024, N 1024: 14.3 / 10.7 / (64 x 1) 8.8; M 4096, K 768, N 3072: 27.1 / 50.6 / 44.8.
+Tile pick_tile(int kind, int epi, int M, int N, int kb_total, int splits, int a_mn, int b_mn) {
+  if (g_force_bn) return {kind == KIND_F8F6F4 && g_force_bn == 64 ? 128 : g_force_bn, g_force_cl, splits};
+  if (!pair_mode()) return {128, 1, splits};
+  const bool aux = epi == EPI_BIAS_GELU || epi == EPI_DGELU || epi == EPI_BIAS_RESID, acc = epi == EPI_ACC_F32;
+  const int sms = sm_count();
+  const float mn = a_mn ? 1.8f : b_mn ? 1.4f : 1.0f, f32 = kind == KIND_TF32 ? 2.0f : 0.0f;
+  const long long pt = (long long)ceil_div(M, 256) * ceil_div(N, 256) * splits;
+  const int rounds = (int)((pt + sms / 2 - 1) / (sms / 2));
+  const float pair_kb = 0.285f * ceil_div(kb_total, splits) * (a_mn ? 1.4f : b_mn ? 1.12f : 1.0f);
+  const float pair_epi = aux ? 6.0f + f32 : 4.8f;
+  float best = 0.95f * ((aux ? 9.3f : acc ? 8.0f : 6.7f) + f32 + pair_kb + (rounds - 1) * (pair_kb > pair_epi ? pair_kb : pair_epi));
+  Tile t{256, 1, splits};
+  for (int bn = 64; bn <= 128; bn += 64) {
+    if (bn == 64 && kind == KIND_F8F6F4) continue;        // an fp8 row of an MN-major operand is 128 columns
+    const long long tiles = (long long)ceil_div(M, BM) * ceil_div(N, bn);
+    for (int cl = 1; cl <= (bn == 64 ? 4 : 2); cl *= 2) {
+      if (cl > 1 && (acc || kind == KIND_TF32 || tiles * cl > sms || cl > kb_total)) break;
+      int sp = 1;
+      if (acc)                                            // one round of CTAs, at least four k-blocks each
+        while (sp < 16 && tiles * (sp + 1) <= sms && kb_total / (sp + 1) >= 4) ++sp;
+      const float per_sm = (float)(tiles * cl * sp) / sms;
+      const float w = per_sm <= 1.f ? 1.f : 0.5f * (per_sm + ceilf(per_sm));
+      const float fixed = (cl == 1 ? (bn == 64 ? 4.2f : 5.0f) : cl == 2 ? 5.6f : 6.2f) + (aux ? (bn == 64 ? 0.3f : 1.2f) : 0.f) + f32;
+      const float est = fixed + w * ceil_div(kb_total, cl * sp) * 0.24f * mn + (w - 1.f) * (aux ? 3.0f : 0.7f) * (bn / 64);
+      if (est < best) { best = est; t = {bn, cl, sp}; }
+    }
   }
-  gemm_kernel<KIND, EPI><<<grid, NUM_THREADS, SMEM_BYTES, st>>>(ta, tb, p);
-  return (int)cudaGetLastError();
+  return t;
 }
 
 template <int KIND>
@@ -977,11 +528,51 @@ int gemm_dispatch(void* D, const void* A, const void* B, const void* bias, void*
   if ((lda * ESZ) % 16 || (ldb * ESZ) % 16 || N % 8) return LLMB_ERR_BAD_ARG;
   if ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B) | reinterpret_cast<uintptr_t>(D)) & 15) return LLMB_ERR_BAD_ARG;
 
-  const bool pair = pair_mode();
-  CUtensorMap ta, tb;
+  GemmParams p;
+  p.g = g_pending_gather;
+  g_pending_gather.W = 0;
+  p.pull = g_pending_pull;
+  g_pending_pull.nseg = 0; g_pending_pull.nwait = 0;
+  p.colsum = g_pending_colsum;
+  g_pending_colsum = nullptr;
+  if ((p.pull.nseg > 0 || p.pull.nwait > 0) && p.g.W > 1) return LLMB_ERR_BAD_ARG;
+  if (p.colsum && !(epi == EPI_DGELU && (KIND == KIND_F16 || KIND == KIND_F8F6F4))) return LLMB_ERR_BAD_ARG;   // bf16 output, TMA epilogue
+  if (p.g.W > 1) {
+    // gathered A: K-major bf16 rows, CTA-pair kernel, whole 256-row tiles per chunk, no split-K
+    if (a_mn || KIND != KIND_F16 || p.g.tiles_per_chunk <= 0 || M != p.g.W * p.g.tiles_per_chunk * 2 * BM || epi == EPI_ACC_F32)
+      return LLMB_ERR_BAD_ARG;
+  }
+  // outputs (and auxiliary tensors) travel by TMA when their layout allows a tensor map
+  const bool needs_aux = epi == EPI_BIAS_GELU || epi == EPI_DGELU || epi == EPI_BIAS_RESID;
+  const bool out_f32 = KIND == KIND_TF32 || epi == EPI_ACC_F32 || epi == EPI_STORE_F32;
+  const int osz = out_f32 ? 4 : 2;
+  static int tma_epi_on = -1;
+  if (tma_epi_on < 0) { const char* e = getenv("LLMB_GEMM_TMA_EPI"); tma_epi_on = (e && e[0] == '0') ? 0 : 1; }
+  CUtensorMap ta, tb, td, taux;
+  p.tma_epi = 0;
+  if (tma_epi_on && (ldd * osz) % 16 == 0 && (!needs_aux || (aux && (reinterpret_cast<uintptr_t>(aux) & 15) == 0 && (ldaux * osz) % 16 == 0))) {
+    const CUtensorMapDataType odt = out_f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
+    const uint32_t box_cols = out_f32 ? 32 : 64;
+    int ok = make_tmap_2d(&td, D, odt, osz, (uint64_t)M, (uint64_t)N, (uint64_t)ldd, 32, box_cols) == 0;
+    if (ok && needs_aux) ok = make_tmap_2d(&taux, aux, odt, osz, (uint64_t)M, (uint64_t)N, (uint64_t)ldaux, 32, box_cols) == 0;
+    p.tma_epi = ok;
+  }
+  if (p.colsum && !p.tma_epi) return LLMB_ERR_BAD_ARG;    // the column sums are taken in the TMA epilogue only
+  const int kb_total = ceil_div(K, BKE);
+  if (splits < 1 || epi != EPI_ACC_F32) splits = 1;
+  if (splits > kb_total) splits = kb_total;
+  Tile tile{256, 1, splits};
+  if (p.tma_epi && p.g.W <= 1 && p.pull.nseg == 0 && p.pull.nwait == 0) tile = pick_tile(KIND, epi, M, N, kb_total, splits, a_mn, b_mn);
+  while (tile.cl > 1 && tile.cl > kb_total) tile.cl >>= 1;
+  splits = tile.splits;
+  const bool pair = tile.bn == 256;
+  // weight gradients of fp32 operands: vector reductions from registers; adding boxes by TMA took the LM head's from 263 to 299 us
+  // (2048 x 768 x 50304) and left the layers' as they were
+  if (pair && KIND == KIND_TF32 && epi == EPI_ACC_F32) p.tma_epi = 0;
+  const int b_rows = pair ? 128 : tile.bn;                // rows of B per load (in the pair kernel each CTA fetches half of the tile)
+
   int rc;
   // K-major: global [MN rows, K cols], box [tile rows, ROW_ELEMS]; MN-major: global [K rows, MN cols], box [BKE, ROW_ELEMS]
-  // (in pair mode each CTA fetches a 128-row half of the B tile)
   const bool base32 = (KIND == KIND_TF32);            // fp32 operands stored MN-major need the 32-byte-base swizzle
   const CUtensorMapSwizzle mn_swz = base32 ? CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B : CU_TENSOR_MAP_SWIZZLE_128B;
   rc = a_mn ? make_tmap_2d(&ta, A, KindTraits<KIND>::DT, ESZ, (uint64_t)K, (uint64_t)M, (uint64_t)lda, BKE, ROW_ELEMS, mn_swz)
@@ -997,28 +588,16 @@ int gemm_dispatch(void* D, const void* A, const void* B, const void* bias, void*
                      ROW_ELEMS, BKE, BM / ROW_ELEMS, mn_swz) == 0) { ta = t3; a_3d = 1; }
   }
   rc = b_mn ? make_tmap_2d(&tb, B, KindTraits<KIND>::DT, ESZ, (uint64_t)K, (uint64_t)N, (uint64_t)ldb, BKE, ROW_ELEMS, mn_swz)
-            : make_tmap_2d(&tb, B, KindTraits<KIND>::DT, ESZ, (uint64_t)N, (uint64_t)K, (uint64_t)ldb, pair ? 128 : BN, ROW_ELEMS);
+            : make_tmap_2d(&tb, B, KindTraits<KIND>::DT, ESZ, (uint64_t)N, (uint64_t)K, (uint64_t)ldb, b_rows, ROW_ELEMS);
   if (rc) return 1000 + rc;
 
   if (b_mn && use3d && N % ROW_ELEMS == 0) {
     CUtensorMap t3;
     if (make_tmap_3d(&t3, B, KindTraits<KIND>::DT, ESZ, ROW_ELEMS, (uint64_t)K, (uint64_t)(N / ROW_ELEMS), (uint64_t)ldb, ROW_ELEMS,
-                     ROW_ELEMS, BKE, (pair ? 128 : BN) / ROW_ELEMS, mn_swz) == 0) { tb = t3; b_3d = 1; }
+                     ROW_ELEMS, BKE, b_rows / ROW_ELEMS, mn_swz) == 0) { tb = t3; b_3d = 1; }
   }
-  GemmParams p;
-  p.g = g_pending_gather;
-  g_pending_gather.W = 0;
-  p.pull = g_pending_pull;
-  g_pending_pull.nseg = 0; g_pending_pull.nwait = 0;
-  if ((p.pull.nseg > 0 || p.pull.nwait > 0) && (!pair || p.g.W > 1)) return LLMB_ERR_BAD_ARG;   // copier warps exist in the pair kernel only
-  p.colsum = g_pending_colsum;
-  g_pending_colsum = nullptr;
-  if (p.colsum && !(pair && epi == EPI_DGELU && (KIND == KIND_F16 || KIND == KIND_F8F6F4))) return LLMB_ERR_BAD_ARG;   // bf16 output, TMA epilogue
-  if (p.g.W > 1) {
-    // gathered A: K-major bf16 rows, CTA-pair kernel, whole 256-row tiles per chunk, no split-K
-    if (!pair || a_mn || KIND != KIND_F16 || p.g.tiles_per_chunk <= 0 || M != p.g.W * p.g.tiles_per_chunk * 2 * BM || epi == EPI_ACC_F32)
-      return LLMB_ERR_BAD_ARG;
-  }
+  if (!p.tma_epi) td = ta;                                // placeholders
+  if (!p.tma_epi || !needs_aux) taux = ta;
   p.a_3d = a_3d; p.b_3d = b_3d;
   p.D = D; p.bias = bias; p.aux = aux; p.alpha = alpha;
   p.M = M; p.N = N; p.K = K; p.ldd = ldd; p.ldaux = ldaux;
@@ -1029,61 +608,28 @@ int gemm_dispatch(void* D, const void* A, const void* B, const void* bias, void*
   p.b_layout = (b_mn && base32) ? 1u : 2u;
   p.a_lbo = a_mn ? mn_lbo : 16; p.a_sbo = a_mn ? mn_sbo : 1024; p.a_kstep = a_mn ? MMA_K * ROW_BYTES : 32;
   p.b_lbo = b_mn ? mn_lbo : 16; p.b_sbo = b_mn ? mn_sbo : 1024; p.b_kstep = b_mn ? MMA_K * ROW_BYTES : 32;
-  p.idesc = make_idesc((uint32_t)a_fmt, (uint32_t)b_fmt, (uint32_t)a_mn, (uint32_t)b_mn, pair ? 2 * BM : BM, BN);
+  p.idesc = make_idesc((uint32_t)a_fmt, (uint32_t)b_fmt, (uint32_t)a_mn, (uint32_t)b_mn, pair ? 2 * BM : BM, (uint32_t)tile.bn);
   p.bke = BKE;                                          // a 128-byte stage row holds BKE / MMA_K = 4 MMA k-steps for every kind
-  p.m_tiles = ceil_div(M, BM); p.n_tiles = ceil_div(N, BN);
-  p.kb_total = ceil_div(K, BKE);
-  if (splits < 1) splits = 1;
-  if (splits > p.kb_total) splits = p.kb_total;
-  if (epi != EPI_ACC_F32) splits = 1;
-  p.kb_per_split = ceil_div(p.kb_total, splits);
-  p.splits = ceil_div(p.kb_total, p.kb_per_split);
+  p.m_tiles = ceil_div(M, BM); p.n_tiles = ceil_div(N, tile.bn);
+  p.kb_total = kb_total;
+  p.kb_per_split = ceil_div(kb_total, splits);
+  p.splits = pair ? ceil_div(kb_total, p.kb_per_split) : splits;
   p.status = status;
   p.io_f32 = (KIND == KIND_TF32) ? 1 : 0;
   p.bias_vec = (reinterpret_cast<uintptr_t>(bias) & 15) == 0;
-  p.tma_epi = 0;
-  if (pair) {
-    const long long units2 = (long long)ceil_div(M, 2 * BM) * p.n_tiles * p.splits;
-    const int max_clusters = sm_count() / 2;
-    const int grid2 = 2 * (int)(units2 < max_clusters ? units2 : max_clusters);
-    // bf16 outputs (and bf16 auxiliary tensors) travel by TMA when their layout allows a tensor map
-    CUtensorMap td = ta, taux = ta;                       // placeholders when the register epilogue runs
-    static int tma_epi_on = -1;
-    if (tma_epi_on < 0) { const char* e = getenv("LLMB_GEMM_TMA_EPI"); tma_epi_on = (e && e[0] == '0') ? 0 : 1; }
-    const bool needs_aux = epi == EPI_BIAS_GELU || epi == EPI_DGELU || epi == EPI_BIAS_RESID;
-    if (tma_epi_on && !p.io_f32 && epi != EPI_ACC_F32 && epi != EPI_STORE_F32 && (ldd * 2) % 16 == 0 &&
-        (!needs_aux || (aux && (reinterpret_cast<uintptr_t>(aux) & 15) == 0 && (ldaux * 2) % 16 == 0))) {
-      int ok = make_tmap_2d(&td, D, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)M, (uint64_t)N, (uint64_t)ldd, 32, 64) == 0;
-      if (ok && needs_aux)
-        ok = make_tmap_2d(&taux, aux, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)M, (uint64_t)N, (uint64_t)ldaux, 32, 64) == 0;
-      p.tma_epi = ok;
-    }
-    if (tma_epi_on && !p.io_f32 && (epi == EPI_ACC_F32 || epi == EPI_STORE_F32) && (ldd * 4) % 16 == 0 &&
-        (reinterpret_cast<uintptr_t>(D) & 15) == 0)
-      p.tma_epi = make_tmap_2d(&td, D, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, (uint64_t)M, (uint64_t)N, (uint64_t)ldd, 32, 32) == 0;
-    if (p.colsum && !p.tma_epi) return LLMB_ERR_BAD_ARG;   // the column sums are taken in the TMA epilogue only
-    switch (epi) {
-      case EPI_NONE: return launch_pair<KIND, EPI_NONE>(ta, tb, td, taux, p, grid2, st);
-      case EPI_BIAS: return launch_pair<KIND, EPI_BIAS>(ta, tb, td, taux, p, grid2, st);
-      case EPI_BIAS_GELU: return launch_pair<KIND, EPI_BIAS_GELU>(ta, tb, td, taux, p, grid2, st);
-      case EPI_DGELU: return launch_pair<KIND, EPI_DGELU>(ta, tb, td, taux, p, grid2, st);
-      case EPI_ACC_F32: return launch_pair<KIND, EPI_ACC_F32>(ta, tb, td, taux, p, grid2, st);
-      case EPI_BIAS_RESID: return launch_pair<KIND, EPI_BIAS_RESID>(ta, tb, td, taux, p, grid2, st);
-      case EPI_STORE_F32: return launch_pair<KIND, EPI_STORE_F32>(ta, tb, td, taux, p, grid2, st);
-    }
-    return LLMB_ERR_BAD_ARG;
-  }
-  long long units = (long long)p.m_tiles * p.n_tiles * p.splits;
-  int grid = (int)(units < sm_count() ? units : sm_count());
+  if (!pair) return llmb_gemm_small_launch(KIND, epi, tile.bn, tile.cl, ta, tb, td, taux, p, st);
 
+  const long long units2 = (long long)ceil_div(M, 2 * BM) * p.n_tiles * p.splits;
+  const int max_clusters = sm_count() / 2;
+  const int grid2 = 2 * (int)(units2 < max_clusters ? units2 : max_clusters);
   switch (epi) {
-    case EPI_NONE: return launch<KIND, EPI_NONE>(ta, tb, p, grid, st);
-    case EPI_BIAS: return launch<KIND, EPI_BIAS>(ta, tb, p, grid, st);
-    case EPI_BIAS_GELU: return launch<KIND, EPI_BIAS_GELU>(ta, tb, p, grid, st);
-    case EPI_DGELU: return launch<KIND, EPI_DGELU>(ta, tb, p, grid, st);
-    case EPI_ACC_F32: return launch<KIND, EPI_ACC_F32>(ta, tb, p, grid, st);
-    case EPI_BIAS_RESID: return launch<KIND, EPI_BIAS_RESID>(ta, tb, p, grid, st);
-    case EPI_STORE_F32: return launch<KIND, EPI_STORE_F32>(ta, tb, p, grid, st);
+    case EPI_NONE: return launch_pair<KIND, EPI_NONE>(ta, tb, td, taux, p, grid2, st);
+    case EPI_BIAS: return launch_pair<KIND, EPI_BIAS>(ta, tb, td, taux, p, grid2, st);
+    case EPI_BIAS_GELU: return launch_pair<KIND, EPI_BIAS_GELU>(ta, tb, td, taux, p, grid2, st);
+    case EPI_DGELU: return launch_pair<KIND, EPI_DGELU>(ta, tb, td, taux, p, grid2, st);
+    case EPI_ACC_F32: return launch_pair<KIND, EPI_ACC_F32>(ta, tb, td, taux, p, grid2, st);
+    case EPI_BIAS_RESID: return launch_pair<KIND, EPI_BIAS_RESID>(ta, tb, td, taux, p, grid2, st);
+    case EPI_STORE_F32: return launch_pair<KIND, EPI_STORE_F32>(ta, tb, td, taux, p, grid2, st);
   }
   return LLMB_ERR_BAD_ARG;
 }
@@ -1431,8 +977,11 @@ LLMB_API int llmb_gemm_set_pull(const void* const* src, void* const* dst, const 
 // sums of its result to colsum[N] (fp32, red.add): the bias gradient of the layer that produced the pre-activations.
 LLMB_API void llmb_gemm_set_colsum(float* colsum) { g_pending_colsum = colsum; }
 LLMB_API void llmb_gemm_debug_mn_strides(int lbo_bytes, int sbo_bytes) { g_dbg_mn_lbo = lbo_bytes; g_dbg_mn_sbo = sbo_bytes; }
-// 0: single-CTA 128x256 tiles, 1: CTA-pair 256x256 tiles (default; env LLMB_GEMM_PAIR=0 selects the former)
+// 0: single-CTA 128x128 tiles, 1: the rule of pick_tile() (default; env LLMB_GEMM_PAIR=0 selects the former)
 LLMB_API void llmb_gemm_set_pair_mode(int on) { g_pair_mode = on ? 1 : 0; }
+// Test hook: every following llmb_gemm call uses tiles of bn columns (256: CTA pair; 64 / 128: gemm_small.cu with cl = 1, 2 or 4 CTAs
+// per tile); bn = 0 gives the choice back to pick_tile().
+LLMB_API void llmb_gemm_force_tile(int bn, int cl) { g_force_bn = bn; g_force_cl = cl; }
 
 // D[M,N] = epi(alpha * (A sfa)(B sfb)^T) on the NVFP4 tensor path (`kind::mxf4nvf4`, 16-value blocks, ue4m3 scales).
 // A [M, K/2] and B [N, K/2]: packed e2m1 bytes as llmb_nvfp4_quantize writes them (K % 32 == 0); sfa / sfb: its

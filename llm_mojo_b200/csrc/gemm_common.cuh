@@ -1,0 +1,396 @@
+// Parts shared by the GEMM kernels: parameters, epilogue arithmetic and staging.
+#pragma once
+#include <stdlib.h>
+#include "tc05.cuh"
+using namespace llmb;
+using namespace tc05;
+
+namespace lgemm {
+__device__ __forceinline__ unsigned ld_acquire_gpu(const unsigned* p) {
+  unsigned v; asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory"); return v;
+}
+__device__ __forceinline__ unsigned ld_acquire_sys(const unsigned* p) {
+  unsigned v; asm volatile("ld.acquire.sys.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory"); return v;
+}
+__device__ __forceinline__ uint4 ld_nc_v4(const uint4* p) {     // streaming 16-byte load (peer memory: read once)
+  uint4 v; asm volatile("ld.global.cg.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory"); return v;
+}
+__device__ __forceinline__ void fence_proxy_async_all() { asm volatile("fence.proxy.async;" ::: "memory"); }
+constexpr int BM = 128, BN = 256;
+constexpr int ROW_BYTES = 128;                       // one swizzled row
+constexpr int A_STAGE = BM * ROW_BYTES;              // 16 KB
+constexpr int BAND = 16;                             // m-tiles per rasterisation band
+
+enum { EPI_NONE = 0, EPI_BIAS = 1, EPI_BIAS_GELU = 2, EPI_DGELU = 3, EPI_ACC_F32 = 4, EPI_BIAS_RESID = 5, EPI_STORE_F32 = 6 };
+
+// All-gather fused into the GEMM: the A matrix [W*n, K] is the concatenation of W row chunks, chunk r produced by
+// rank r.  Every rank holds a full-size local buffer whose own chunk is already in place; two copier warps per
+// CTA pull the other chunks out of the peers' buffers (plain 16-byte peer loads over NVLink, each byte crosses
+// once) into the local buffer WHILE the tile loop runs, starting with the tiles of the local chunk and taking the
+// remote chunks in ring order.  A chunk's tiles are fetched (TMA, local memory) once every CTA's copiers have
+// counted it complete.
+struct GatherArgs {
+  const void* peer_src[8];     // [r]: start of chunk r inside rank r's buffer
+  void* local;                 // start of this rank's [W*n, K] buffer
+  const void* flags;           // this rank's flag words: peers announce "my chunk is written" (kind ROWS_READY)
+  unsigned* counts;            // [16] local counters, zeroed before the launch: [r] = slices of chunk r copied, [8 + r] = slice tickets
+  long long chunk_vecs;        // 16-byte vectors per chunk
+  unsigned seq, target;        // announce sequence number to wait for; slices per chunk (counts[r] == target: chunk landed)
+  int W, me, tiles_per_chunk;  // W = 0: no gather
+};
+
+// Parameter pull fused into a GEMM (ZeRO-3): the kernel's copier warps copy up to 8 segments of weights out of their
+// owners' parameter shards (plain 16-byte loads over NVLink, or local memory for the rank's own part) into this
+// rank's layer window while the tensor-core tile loop of the SAME kernel runs.  The segments may belong to the B
+// operand of this GEMM (then its TMA producer waits for them) or to the operand of a later GEMM of the layer, which
+// only checks the counters: every weight then arrives under the math of a tile loop.  Owners announce "my shard
+// holds the parameters of optimizer step seq" at flag kind PARAM; all waits are bounded.
+struct PullArgs {
+  const void* src[8];          // segment source (peer or local shard memory), 16-byte aligned
+  void* dst[8];                // segment destination inside the local window
+  long long vecs[8];           // 16-byte vectors per segment
+  const void* flags;           // this rank's flag words
+  unsigned* counts;            // [16] zeroed before the launch: [s] = slices of segment s landed, [8 + s] = slice tickets
+  const unsigned* wait_counts[8];   // counters this GEMM's B operand depends on ...
+  unsigned wait_target[8];          // ... and the value each must reach
+  unsigned seq;                // parameter sequence number the owners must have announced (0: none yet, no wait)
+  int owner[8];
+  int nseg, nwait, W;          // nseg = 0: nothing to pull; nwait = 0: nothing to wait for
+};
+
+struct GemmParams {
+  GatherArgs g;
+  PullArgs pull;
+  void* D; const void* bias; void* aux; const float* alpha;
+  int M, N, K;                 // K in elements
+  long long ldd, ldaux;
+  int a_mn, b_mn;              // operand majorness (0 = K-major)
+  int a_3d, b_3d;              // MN-major operand fetched with ONE 3-D box (chunk, k, chunk index) per stage
+  uint32_t a_lbo, a_sbo, a_kstep, b_lbo, b_sbo, b_kstep;   // bytes
+  uint32_t a_layout, b_layout; // UMMA layout type: 2 = SWIZZLE_128B, 1 = SWIZZLE_128B with 32-byte base (fp32 MN-major)
+  uint32_t idesc;
+  int bke;                     // K elements per stage
+  int m_tiles, n_tiles, splits, kb_per_split, kb_total;
+  int io_f32;                  // 1: D, bias and aux are fp32 (tf32 kind); 0: bf16
+  int tma_epi;                 // 1: bf16 outputs leave (and auxiliary inputs arrive) by TMA; 0: register/shared-memory epilogue
+  int bias_vec;                // bias pointer is 16-byte aligned (vector loads)
+  float* colsum;               // EPI_DGELU, TMA epilogue: colsum[n] += sum over rows of the (bf16) result, i.e. the bias gradient of the layer below
+  int* status;
+};
+
+// ------------------------------------------------------------------------------------------------
+// Coalesced epilogue.  tcgen05.ld hands each thread one accumulator ROW; stored directly, a warp
+// would touch 32 different rows per instruction.  Instead every 64-column slab of the warp's
+// 32 x 256 block goes through an 8 KB shared-memory transpose (XOR-swizzled 16-byte chunks, conflict
+// free in both directions) so that 8 consecutive lanes cover 64 contiguous bytes of one output row
+// and all global traffic of the epilogue (output, bias, GELU aux, residual) is sector-aligned.
+constexpr int EPI_STAGE_BYTES = 32 * 256;             // per epilogue warp: 32 rows x 64 fp32
+
+template <int EPI>
+__device__ __forceinline__ void epi4(const GemmParams& p, float (&v)[4], int row, int col, float alpha) {
+#pragma unroll
+  for (int k = 0; k < 4; ++k) v[k] *= alpha;
+  if (EPI == EPI_BIAS || EPI == EPI_BIAS_GELU || EPI == EPI_BIAS_RESID) {
+    if (p.bias && p.io_f32) {
+      const float4 b = *reinterpret_cast<const float4*>(reinterpret_cast<const float*>(p.bias) + col);
+      v[0] += b.x; v[1] += b.y; v[2] += b.z; v[3] += b.w;
+    } else if (p.bias) {
+      const uint2 braw = *reinterpret_cast<const uint2*>(reinterpret_cast<const __nv_bfloat16*>(p.bias) + col);
+      const __nv_bfloat162* bh = reinterpret_cast<const __nv_bfloat162*>(&braw);
+      const float2 b0 = __bfloat1622float2(bh[0]), b1 = __bfloat1622float2(bh[1]);
+      v[0] += b0.x; v[1] += b0.y; v[2] += b1.x; v[3] += b1.y;
+    }
+  }
+  if (EPI == EPI_ACC_F32 || EPI == EPI_STORE_F32) {
+    float* dp = reinterpret_cast<float*>(p.D) + (size_t)row * p.ldd + col;
+    if (EPI == EPI_ACC_F32)
+      asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dp), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]) : "memory");
+    else
+      *reinterpret_cast<float4*>(dp) = make_float4(v[0], v[1], v[2], v[3]);
+    return;
+  }
+  if (p.io_f32) {                                       // fp32 storage (tf32 tensor path)
+    float* dp = reinterpret_cast<float*>(p.D) + (size_t)row * p.ldd + col;
+    float* ap = reinterpret_cast<float*>(p.aux) + (size_t)row * p.ldaux + col;
+    if (EPI == EPI_BIAS_GELU) {
+      *reinterpret_cast<float4*>(ap) = make_float4(v[0], v[1], v[2], v[3]);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) v[k] = gelu_f(v[k]);
+    } else if (EPI == EPI_DGELU) {
+      const float4 x = *reinterpret_cast<const float4*>(ap);
+      v[0] *= gelu_grad_f(x.x); v[1] *= gelu_grad_f(x.y); v[2] *= gelu_grad_f(x.z); v[3] *= gelu_grad_f(x.w);
+    } else if (EPI == EPI_BIAS_RESID) {
+      const float4 x = *reinterpret_cast<const float4*>(ap);
+      v[0] += x.x; v[1] += x.y; v[2] += x.z; v[3] += x.w;
+    }
+    *reinterpret_cast<float4*>(dp) = make_float4(v[0], v[1], v[2], v[3]);
+    return;
+  }
+  __nv_bfloat16* dp = reinterpret_cast<__nv_bfloat16*>(p.D) + (size_t)row * p.ldd + col;
+  __nv_bfloat16* ap = reinterpret_cast<__nv_bfloat16*>(p.aux) + (size_t)row * p.ldaux + col;
+  auto pack4 = [](const float (&x)[4]) {
+    uint2 u; __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&u);
+    h[0] = __floats2bfloat162_rn(x[0], x[1]); h[1] = __floats2bfloat162_rn(x[2], x[3]);
+    return u;
+  };
+  auto unpack4 = [](uint2 u, float (&x)[4]) {
+    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&u);
+    const float2 a = __bfloat1622float2(h[0]), b = __bfloat1622float2(h[1]);
+    x[0] = a.x; x[1] = a.y; x[2] = b.x; x[3] = b.y;
+  };
+  if (EPI == EPI_BIAS_GELU) {
+    const uint2 pre = pack4(v);
+    *reinterpret_cast<uint2*>(ap) = pre;               // pre-GELU activations (bf16)
+    float x[4]; unpack4(pre, x);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) v[k] = gelu_f(x[k]);
+  } else if (EPI == EPI_DGELU) {
+    float x[4]; unpack4(*reinterpret_cast<const uint2*>(ap), x);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) v[k] *= gelu_grad_f(x[k]);
+  } else if (EPI == EPI_BIAS_RESID) {
+    float x[4]; unpack4(*reinterpret_cast<const uint2*>(ap), x);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) v[k] += x[k];
+  }
+  const uint2 o = pack4(v);
+  *reinterpret_cast<uint2*>(dp) = o;
+}
+
+// One epilogue warp drains its 32 rows x NCOLS columns of accumulator `tacc` (TMEM address incl. lane quarter).
+template <int EPI, int NCOLS = BN>
+__device__ __forceinline__ void epilogue_warp(const GemmParams& p, uint32_t tacc, unsigned char* stage, int row_base, int n0,
+                                              float alpha, int lane) {
+  const int rsub = lane >> 3, cl = lane & 7;
+#pragma unroll 1
+  for (int s = 0; s < NCOLS / 64; ++s) {
+    if (n0 + s * 64 >= p.N) break;                      // warp-uniform
+    uint32_t r0[32], r1[32];
+    tmem_ld32(tacc + s * 64, r0);
+    tmem_ld32(tacc + s * 64 + 32, r1);
+    tmem_wait_ld();
+    unsigned char* myrow = stage + lane * 256;
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      *reinterpret_cast<uint4*>(myrow + ((c ^ (lane & 15)) << 4)) = make_uint4(r0[4 * c], r0[4 * c + 1], r0[4 * c + 2], r0[4 * c + 3]);
+      *reinterpret_cast<uint4*>(myrow + (((c + 8) ^ (lane & 15)) << 4)) = make_uint4(r1[4 * c], r1[4 * c + 1], r1[4 * c + 2], r1[4 * c + 3]);
+    }
+    __syncwarp();
+#pragma unroll
+    for (int it = 0; it < 8; ++it) {
+      const int rr = it * 4 + rsub;
+      const int row = row_base + rr;
+      const unsigned char* src = stage + rr * 256;
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        const int chunk = cl + half * 8;
+        const float4 f = *reinterpret_cast<const float4*>(src + ((chunk ^ (rr & 15)) << 4));
+        const int col = n0 + s * 64 + chunk * 4;
+        if (row < p.M && col < p.N) {
+          float v[4] = {f.x, f.y, f.z, f.w};
+          epi4<EPI>(p, v, row, col, alpha);
+        }
+      }
+    }
+    __syncwarp();
+  }
+}
+
+// ------------------------------------------------------------------------------------------------
+// Epilogue through TMA (bf16 outputs of the CTA-pair kernel).  Each of the eight epilogue warps owns
+// 32 rows x 128 columns of the accumulator and moves them as two slabs of 64 columns = one
+// 128-byte-swizzled box of 32 rows x 128 B (4 KB) each:
+//   * tcgen05.ld gives each lane one row of the slab; bias, GELU, dGELU and the residual add happen in
+//     registers in that layout;
+//   * the auxiliary INPUT (residual stream, pre-GELU activations) arrives by TMA loads that are issued a
+//     whole tile ahead - while the tensor core is still busy with that tile - into the buffer the
+//     result is then written to in place;
+//   * results leave by TMA stores (bulk groups), so no lane ever waits on global memory and every
+//     global access of the epilogue is a full 128-byte row segment; out-of-range rows and columns are
+//     clipped by the tensor maps.
+// Epilogues with an auxiliary input or a second output (BIAS_GELU stores the pre-activation too) get
+// two 4 KB buffers per warp and a 5-deep operand ring, and so do the fp32 outputs (two 32-column boxes of a 64-column slab,
+// added into or stored to global memory by TMA); the others one buffer and a 6-deep ring.
+template <int EPI> struct EpiCfg {
+  static constexpr bool AUX_IN = EPI == EPI_DGELU || EPI == EPI_BIAS_RESID;
+  static constexpr bool TWO_OUT = EPI == EPI_BIAS_GELU;
+  static constexpr bool F32_OUT = EPI == EPI_ACC_F32 || EPI == EPI_STORE_F32;
+  static constexpr int STAGES = (F32_OUT || AUX_IN || TWO_OUT) ? 5 : 6;
+  static constexpr int WARP_STAGE = STAGES == 5 ? 16384 : 8192;     // staging bytes per warp of the 4-warp register epilogue (half that per warp of the 8-warp TMA epilogue)
+};
+constexpr int SLAB_BYTES = 32 * 128;
+
+__device__ __forceinline__ uint4 pack8(const float (&x)[8]) {
+  uint4 u; __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&u);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) h[i] = __floats2bfloat162_rn(x[2 * i], x[2 * i + 1]);
+  return u;
+}
+__device__ __forceinline__ void unpack8(const uint4& u, float (&x)[8]) {
+  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&u);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) { const float2 f = __bfloat1622float2(h[i]); x[2 * i] = f.x; x[2 * i + 1] = f.y; }
+}
+
+// One slab (this lane's row, 64 columns) from registers to the swizzled staging buffer.  With an
+// auxiliary input the buffer holds it on entry and the result replaces it; BIAS_GELU writes the
+// pre-activation to `buf` and the activation to `buf + SLAB_BYTES`.
+template <int EPI>
+__device__ __forceinline__ void epi_slab_bf16(const GemmParams& p, const uint32_t (&r0)[32], const uint32_t (&r1)[32],
+                                              unsigned char* buf, int col0, float alpha, int lane) {
+  unsigned char* myrow = buf + lane * 128;
+  const __nv_bfloat16* bias = reinterpret_cast<const __nv_bfloat16*>(p.bias);
+#pragma unroll
+  for (int c = 0; c < 8; ++c) {
+    float v[8], b[8];
+    const int col = col0 + c * 8;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) b[j] = 0.f;
+    if (EPI == EPI_BIAS || EPI == EPI_BIAS_GELU || EPI == EPI_BIAS_RESID) {
+      if (bias && col < p.N) {
+        if (p.bias_vec) unpack8(__ldg(reinterpret_cast<const uint4*>(bias + col)), b);
+        else {
+#pragma unroll
+          for (int j = 0; j < 8; ++j) b[j] = __bfloat162float(bias[col + j]);
+        }
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 8; j += 2) {
+      const uint32_t (&r)[32] = c < 4 ? r0 : r1;
+      const float2 y = __ffma2_rn(make_float2(__uint_as_float(r[(c & 3) * 8 + j]), __uint_as_float(r[(c & 3) * 8 + j + 1])),
+                                  make_float2(alpha, alpha), make_float2(b[j], b[j + 1]));
+      v[j] = y.x; v[j + 1] = y.y;
+    }
+    unsigned char* slot = myrow + ((c ^ (lane & 7)) << 4);
+    if (EPI == EPI_BIAS_GELU) {
+      const uint4 pre = pack8(v);
+      *reinterpret_cast<uint4*>(slot) = pre;
+      float x[8]; unpack8(pre, x);
+#pragma unroll
+      for (int j = 0; j < 8; j += 2) {
+        const float2 y = gelu_fast2(make_float2(x[j], x[j + 1]));
+        v[j] = y.x; v[j + 1] = y.y;
+      }
+      *reinterpret_cast<uint4*>(slot + SLAB_BYTES) = pack8(v);
+    } else {
+      if (EPI == EPI_DGELU || EPI == EPI_BIAS_RESID) {
+        float x[8]; unpack8(*reinterpret_cast<const uint4*>(slot), x);
+#pragma unroll
+        for (int j = 0; j < 8; j += 2) {
+          const float2 xx = make_float2(x[j], x[j + 1]), vv = make_float2(v[j], v[j + 1]);
+          const float2 y = (EPI == EPI_DGELU) ? __fmul2_rn(vv, gelu_grad_fast2(xx)) : __fadd2_rn(vv, xx);
+          v[j] = y.x; v[j + 1] = y.y;
+        }
+      }
+      *reinterpret_cast<uint4*>(slot) = pack8(v);
+    }
+  }
+}
+
+// Column sums of a 32 x 64 slab as stored (bf16): lane l adds up columns 2l and 2l + 1 of the warp's rows out of the swizzled box
+// (conflict-free: the 32 lanes read the 128 bytes of one row) and adds them to colsum.
+__device__ __forceinline__ void epi_slab_colsum(const GemmParams& p, const unsigned char* buf, int row0, int col0, int lane) {
+  float s0 = 0.f, s1 = 0.f;
+  const int nrows = min(32, p.M - row0);
+#pragma unroll 8
+  for (int r = 0; r < nrows; ++r) {
+    const uint32_t w = *reinterpret_cast<const uint32_t*>(buf + r * 128 + ((((lane >> 2) ^ (r & 7))) << 4) + (lane & 3) * 4);
+    s0 += __uint_as_float(w << 16); s1 += __uint_as_float(w & 0xffff0000u);
+  }
+  const int col = col0 + 2 * lane;
+  if (col < p.N) {
+    asm volatile("red.global.add.f32 [%0], %1;" ::"l"(p.colsum + col), "f"(s0) : "memory");
+    asm volatile("red.global.add.f32 [%0], %1;" ::"l"(p.colsum + col + 1), "f"(s1) : "memory");
+  }
+}
+
+// The two halves of the bias + GELU epilogue, so that the pre-activation box can start leaving by TMA while the GELU of the
+// same slab is still being computed: first alpha, bias and the bf16 pre-activations (kept in registers as well) ...
+__device__ __forceinline__ void epi_slab_pre(const GemmParams& p, const uint32_t (&r0)[32], const uint32_t (&r1)[32],
+                                             unsigned char* buf, int col0, float alpha, int lane, uint4 (&pre)[8]) {
+  unsigned char* myrow = buf + lane * 128;
+  const __nv_bfloat16* bias = reinterpret_cast<const __nv_bfloat16*>(p.bias);
+#pragma unroll
+  for (int c = 0; c < 8; ++c) {
+    float v[8], b[8];
+    const int col = col0 + c * 8;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) b[j] = 0.f;
+    if (bias && col < p.N) {
+      if (p.bias_vec) unpack8(__ldg(reinterpret_cast<const uint4*>(bias + col)), b);
+      else {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) b[j] = __bfloat162float(bias[col + j]);
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 8; j += 2) {
+      const uint32_t (&r)[32] = c < 4 ? r0 : r1;
+      const float2 y = __ffma2_rn(make_float2(__uint_as_float(r[(c & 3) * 8 + j]), __uint_as_float(r[(c & 3) * 8 + j + 1])),
+                                  make_float2(alpha, alpha), make_float2(b[j], b[j + 1]));
+      v[j] = y.x; v[j + 1] = y.y;
+    }
+    pre[c] = pack8(v);
+    *reinterpret_cast<uint4*>(myrow + ((c ^ (lane & 7)) << 4)) = pre[c];
+  }
+}
+// ... then GELU of those bf16 values into the second box.
+__device__ __forceinline__ void epi_slab_gelu(const GemmParams& p, const uint4 (&pre)[8], unsigned char* buf, int lane) {
+  unsigned char* myrow = buf + lane * 128;
+#pragma unroll
+  for (int c = 0; c < 8; ++c) {
+    float x[8]; unpack8(pre[c], x);
+#pragma unroll
+    for (int j = 0; j < 8; j += 2) {
+      const float2 y = gelu_fast2(make_float2(x[j], x[j + 1]));
+      x[j] = y.x; x[j + 1] = y.y;
+    }
+    *reinterpret_cast<uint4*>(myrow + ((c ^ (lane & 7)) << 4)) = pack8(x);
+  }
+}
+
+
+// fp32 storage (tf32 kind): one box of 32 rows x 32 columns (this lane's row) from registers to the swizzled staging box; with an
+// auxiliary input the box holds it on entry, BIAS_GELU writes the activation to `act` and the pre-activation to `buf`.
+template <int EPI>
+__device__ __forceinline__ void epi_box_f32(const GemmParams& p, const uint32_t (&r)[32], unsigned char* buf, unsigned char* act, int col0,
+                                            float alpha, int lane) {
+  const float* bias = reinterpret_cast<const float*>(p.bias);
+#pragma unroll
+  for (int c = 0; c < 8; ++c) {
+    const int col = col0 + c * 4;
+    float4 v = make_float4(__uint_as_float(r[4 * c]) * alpha, __uint_as_float(r[4 * c + 1]) * alpha, __uint_as_float(r[4 * c + 2]) * alpha,
+                           __uint_as_float(r[4 * c + 3]) * alpha);
+    if ((EPI == EPI_BIAS || EPI == EPI_BIAS_GELU || EPI == EPI_BIAS_RESID) && bias && col < p.N) {
+      float4 b;
+      if (p.bias_vec) b = __ldg(reinterpret_cast<const float4*>(bias + col));
+      else b = make_float4(bias[col], bias[col + 1], bias[col + 2], bias[col + 3]);
+      v.x += b.x; v.y += b.y; v.z += b.z; v.w += b.w;
+    }
+    const int off = lane * 128 + ((c ^ (lane & 7)) << 4);
+    if (EPI == EPI_BIAS_GELU) {
+      *reinterpret_cast<float4*>(buf + off) = v;
+      v = make_float4(gelu_f(v.x), gelu_f(v.y), gelu_f(v.z), gelu_f(v.w));
+      *reinterpret_cast<float4*>(act + off) = v;
+      continue;
+    }
+    if (EPI == EPI_DGELU || EPI == EPI_BIAS_RESID) {
+      const float4 x = *reinterpret_cast<const float4*>(buf + off);
+      if (EPI == EPI_DGELU) { v.x *= gelu_grad_f(x.x); v.y *= gelu_grad_f(x.y); v.z *= gelu_grad_f(x.z); v.w *= gelu_grad_f(x.w); }
+      else { v.x += x.x; v.y += x.y; v.z += x.z; v.w += x.w; }
+    }
+    *reinterpret_cast<float4*>(buf + off) = v;
+  }
+}
+
+template <int KIND> struct KindTraits;
+template <> struct KindTraits<KIND_F16> { static constexpr int ESZ = 2; static constexpr CUtensorMapDataType DT = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16; };
+template <> struct KindTraits<KIND_TF32> { static constexpr int ESZ = 4; static constexpr CUtensorMapDataType DT = CU_TENSOR_MAP_DATA_TYPE_FLOAT32; };
+template <> struct KindTraits<KIND_F8F6F4> { static constexpr int ESZ = 1; static constexpr CUtensorMapDataType DT = CU_TENSOR_MAP_DATA_TYPE_UINT8; };
+}  // namespace lgemm
+using namespace lgemm;
+
+// gemm_small.cu: 128 x bn tiles, one per CTA, `cl` CTAs sharing the contraction of a tile (see there)
+int llmb_gemm_small_launch(int kind, int epi, int bn, int cl, const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td,
+                           const CUtensorMap& taux, const GemmParams& p, cudaStream_t st);

@@ -56,6 +56,7 @@ _SIGS = {
     "llmb_gemm_set_colsum": [c_p],
     "llmb_gemm_debug_mn_strides": [c_int, c_int],
     "llmb_gemm_set_pair_mode": [c_int],
+    "llmb_gemm_force_tile": [c_int, c_int],
     "llmb_amax": [c_p, c_p, c_ll, c_int, c_p],
     "llmb_amax_rht": [c_p, c_p, c_int, c_int, c_int, c_int, c_p],
     "llmb_fp8_block_fake_quant": [c_p, c_p, c_int, c_int, c_int, c_int, c_p],

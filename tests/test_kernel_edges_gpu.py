@@ -85,6 +85,81 @@ def test_softmax_rows_edges(rows, V, dtype):
     assert _lib.read_status() == 0
 
 
+@pytest.fixture
+def force_tile():
+    yield lambda bn, cl: _lib.lib().llmb_gemm_force_tile(bn, cl)
+    _lib.lib().llmb_gemm_force_tile(0, 1)
+
+
+# 256: CTA-pair kernel; 64 / 128: one tile per CTA, with 1, 2 or 4 CTAs sharing the contraction
+@pytest.mark.parametrize("bn,cl", [(256, 1), (128, 1), (128, 2), (64, 1), (64, 2), (64, 4)])
+# one row, a partial band, a partial tile; column counts that end inside a slab / inside a pair of slabs; odd numbers of k-blocks
+@pytest.mark.parametrize("M,N,K", [(1, 64, 320), (37, 200, 264), (300, 1608, 456), (129, 320, 1288)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_gemm_tile_configurations(bn, cl, M, N, K, dtype, force_tile):
+    """Every epilogue and operand layout on every tile configuration, at sizes that leave partial tiles, slabs and k-blocks."""
+    force_tile(bn, cl)
+    x, w, b, r = rnd(M, K, dtype=dtype), rnd(N, K, dtype=dtype, scale=0.05, seed=1), rnd(N, dtype=dtype, seed=2), rnd(M, N, dtype=dtype, seed=3)
+    X, W, Bi, Rs = (t.to(DEV) for t in (x, w, b, r))
+    # operands: bf16 exact, fp32 rounded to tf32 (2^-11 each, K terms of size ~0.05); results rounded once to the storage type
+    eps = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -10
+    tol = dict(atol=eps * 4, rtol=eps)
+    y = x.float() @ w.float().t()
+    out, pre = torch.full((M, N), 7.0, dtype=dtype, device=DEV), torch.full((M, N), 7.0, dtype=dtype, device=DEV)
+    ops.matmul_fwd(out, X, W)
+    assert_close(out, y, what="none", **tol)
+    ops.matmul_fwd(out, X, W, Bi)
+    assert_close(out, y + b.float(), what="bias", **tol)
+    ops.matmul_fwd(out, X, W, Bi, residual=Rs)
+    assert_close(out, y + b.float() + r.float(), what="residual", **tol)
+    ops.matmul_fwd(out, X, W, Bi, pre_gelu=pre)
+    assert_close(pre, y + b.float(), what="pre-GELU", **tol)
+    assert_close(out, torch.nn.functional.gelu(pre.float(), approximate="tanh"), 2 * eps, eps, "GELU")
+    # backward: dinp [M, K] contracted over N, dW [N, K] contracted over M (added to what is there), column sums of dinp
+    d = rnd(M, N, dtype=dtype, seed=4)
+    D = d.to(DEV)
+    g = d.float() @ w.float()
+    tol_b = dict(atol=eps * 8, rtol=eps)
+    dinp = torch.empty(M, K, dtype=dtype, device=DEV)
+    ops.matmul_bwd(dinp, None, None, D, X, W)
+    assert_close(dinp, g, what="dinp", **tol_b)
+    cs = torch.full((K,), 0.5, device=DEV)
+    ops.matmul_bwd(dinp, None, None, D, X, W, gelu_pre=X, dinp_colsum=cs)
+    xg = x.float().requires_grad_(True)
+    torch.nn.functional.gelu(xg, approximate="tanh").backward(g)
+    assert_close(dinp, xg.grad, eps * 16, 2 * eps, "dGELU")
+    assert_close(cs, 0.5 + dinp.float().sum(0).cpu(), 1e-4 * math.sqrt(M), 1e-4, "column sums")
+    dw = torch.full((N, K), 0.25, device=DEV)
+    ops.matmul_bwd(None, dw, None, D, X, W)
+    assert_close(dw, 0.25 + d.float().t() @ x.float(), (1e-4 if dtype == torch.bfloat16 else 4 * eps) * math.sqrt(M), 1e-4 if dtype == torch.bfloat16 else eps, "dW")
+    f32 = torch.empty(M, K, device=DEV)
+    ops.gemm(f32, D, W, b_mn=True, epi=ops.EPI_STORE_F32, kind=0 if dtype == torch.bfloat16 else 1)
+    assert_close(f32, g, 1e-4 if dtype == torch.bfloat16 else eps * 8, 1e-4 if dtype == torch.bfloat16 else eps, "fp32 store")
+    torch.cuda.synchronize()
+    assert _lib.read_status() == 0
+
+
+@pytest.mark.parametrize("bn,cl", [(256, 1), (128, 1), (128, 2)])
+def test_gemm_fp8_tile_configurations(bn, cl, force_tile):
+    force_tile(bn, cl)
+    M, N, K = 200, 336, 272
+    a = rnd(M, K, dtype=torch.float32).to(torch.float8_e4m3fn)
+    w = rnd(N, K, dtype=torch.float32, seed=1).to(torch.float8_e4m3fn)
+    d = rnd(M, N, dtype=torch.float32, seed=2).to(torch.float8_e5m2)
+    A, W, D = (t.view(torch.uint8).to(DEV) for t in (a, w, d))
+    alpha = torch.full((1,), 0.125, device=DEV)
+    out = torch.empty(M, N, dtype=torch.bfloat16, device=DEV)
+    ops.gemm(out, A, W, kind=2, alpha=alpha)
+    assert_close(out, 0.125 * a.float() @ w.float().t(), 2.0 ** -7, 2.0 ** -8, "fp8 forward")
+    dinp = torch.empty(M, K, dtype=torch.bfloat16, device=DEV)
+    ops.gemm(dinp, D, W, b_mn=True, kind=2, a_fmt=1, alpha=alpha)
+    assert_close(dinp, 0.125 * d.float() @ w.float(), 2.0 ** -7, 2.0 ** -8, "fp8 dinp")
+    dw = torch.zeros(N, K, device=DEV)
+    ops.gemm(dw, D, A, a_mn=True, b_mn=True, epi=ops.EPI_ACC_F32, splits=2, kind=2, a_fmt=1, alpha=alpha)
+    assert_close(dw, 0.125 * d.float().t() @ a.float(), 2e-3, 1e-4, "fp8 dW")
+    assert _lib.read_status() == 0
+
+
 def test_gemm_residual_right_edge_many_tiles():
     """Several tiles per CTA pair with a right edge that leaves one 64-column slab in a warp's half of the tile: the slab's buffer is
     refilled with the next tile's residual, which must wait for the store that still reads it."""

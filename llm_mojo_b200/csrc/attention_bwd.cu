@@ -54,6 +54,8 @@ struct B3Params {
 // so that a warp reads four whole 128-byte rows per instruction.
 __global__ void attn_bwd3_prep_kernel(float* __restrict__ stats, const float* __restrict__ lse, const __nv_bfloat16* __restrict__ dout,
                                       const __nv_bfloat16* __restrict__ out, int B, int T, int NH, int C) {
+  pdl_trigger();
+  pdl_wait();
   const int n_t = ceil_div(T, TILE), Tp = n_t * TILE;
   const long long idx = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 3;   // (b * NH + h) * Tp + t
   const int part = threadIdx.x & 7;
@@ -172,6 +174,8 @@ __global__ void __launch_bounds__(B3_THREADS, 1) attn_bwd3_kernel(const __grid_c
   const uint32_t tmem = *tmem_slot;
   const uint32_t tS = tmem, tDP = tmem + 128, tDV = tmem + 256, tDK = tmem + 320, tDQ = tmem + 384, tP = tmem + 448;
   bool failed = false;
+  pdl_trigger();
+  pdl_wait();
 
   // Registers move from the dQ warpgroup and the producer / issuer warpgroup to the two compute warpgroups:
   // 2 x 128 x 176 + 2 x 128 x 80 = 65536 = the registers of the launch (512 x 128).
@@ -471,6 +475,8 @@ __global__ void __launch_bounds__(B3_THREADS, 1) attn_bwd3_kernel(const __grid_c
 // rounded rows cross a swizzled shared-memory tile, and every warp then writes four whole 128-byte rows per instruction.
 __global__ void __launch_bounds__(128) attn_bwd3_dq_kernel(__nv_bfloat16* __restrict__ dqkv, float* __restrict__ dbias, float* __restrict__ dq_acc,
                                                            int T, int NH, int C, float scale) {
+  pdl_trigger();
+  pdl_wait();
   __shared__ float part[4][HS];
   __shared__ __align__(16) unsigned char tile_s[TILE * ROWB];
   const int n_t = ceil_div(T, TILE);
@@ -539,10 +545,10 @@ LLMB_API int llmb_attention_bwd_fused(void* dqkv, float* dbias, float* stats, fl
   }
   const int n_t = ceil_div(T, TILE);
   const long long rows = (long long)B * NH * n_t * TILE;
-  attn_bwd3_prep_kernel<<<(unsigned)ceil_div_ll(rows * 8, 256), 256, 0, st>>>(stats, lse, (const __nv_bfloat16*)dout, (const __nv_bfloat16*)out, B, T, NH, C);
+  launch_pdl(attn_bwd3_prep_kernel, (unsigned)ceil_div_ll(rows * 8, 256), 256, 0, st, stats, lse, (const __nv_bfloat16*)dout, (const __nv_bfloat16*)out, B, T, NH, C);
   const long long n_items = (long long)((n_t + 1) / 2) * B * NH;
   const int grid = (int)(n_items < sm_count() ? n_items : sm_count());          // persistent: one CTA per SM
-  attn_bwd3_kernel<<<grid, B3_THREADS, B3_SMEM, st>>>(tq, td, to, p);
-  attn_bwd3_dq_kernel<<<(unsigned)(B * NH * n_t), 128, 0, st>>>((__nv_bfloat16*)dqkv, dbias, dq_acc, T, NH, C, p.scale);
+  launch_pdl(attn_bwd3_kernel, grid, B3_THREADS, B3_SMEM, st, tq, td, to, p);
+  launch_pdl(attn_bwd3_dq_kernel, (unsigned)(B * NH * n_t), 128, 0, st, (__nv_bfloat16*)dqkv, dbias, dq_acc, T, NH, C, p.scale);
   return (int)cudaGetLastError();
 }

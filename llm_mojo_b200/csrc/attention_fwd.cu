@@ -108,6 +108,8 @@ __global__ void __launch_bounds__(F3_THREADS, 1) attn_fwd3_kernel(const __grid_c
   fence_after_sync();
   const uint32_t tmem = *tmem_slot;
   bool failed = false;
+  pdl_trigger();
+  pdl_wait();
   // Registers move from the output and producer / issuer warpgroups to the two softmax warpgroups:
   // 2 x 128 x 176 + 2 x 128 x 80 = 65536 = the 512 x 128 registers the CTA was launched with.  A warpgroup can only
   // grow into registers that warpgroups of the same CTA have released: asking for more than that would block
@@ -416,6 +418,5 @@ LLMB_API int llmb_attention_fwd_pair(void* out, float* lse, const void* qkv, int
   int grid = sm_count();
   if (n_items < grid) grid = (int)n_items;
   if (grid < n_pairs) grid = n_pairs;                     // one (batch, head) needs n_pairs CTAs side by side
-  attn_fwd3_kernel<<<grid, F3_THREADS, F3_SMEM, st>>>(tm, tmo, p);
-  return (int)cudaGetLastError();
+  return launch_pdl(attn_fwd3_kernel, grid, F3_THREADS, F3_SMEM, st, tm, tmo, p);
 }

@@ -16,6 +16,8 @@ template <typename T>
 __global__ void __launch_bounds__(1024) classifier_kernel(T* __restrict__ logits, float* __restrict__ losses,
                                                          const int* __restrict__ targets, float dloss, int V, int Vp,
                                                          int write_dlogits) {
+  pdl_trigger();
+  pdl_wait();
   constexpr int N = Pack<T>::N;
   extern __shared__ __align__(16) unsigned char smraw[];
   T* row_s = reinterpret_cast<T*>(smraw);
@@ -87,6 +89,8 @@ __device__ __forceinline__ void bulk_store_1d(void* gdst, const void* ssrc, uint
 __global__ void __launch_bounds__(1024, 1) classifier_stream_kernel(__nv_bfloat16* __restrict__ logits, float* __restrict__ losses,
                                                                    const int* __restrict__ targets, float dloss, int rows, int V,
                                                                    int Vp, int write_dlogits, int buf_bytes, int* status) {
+  pdl_trigger();
+  pdl_wait();
   using T = __nv_bfloat16;
   constexpr int N = 8;
   extern __shared__ __align__(128) unsigned char smraw[];
@@ -198,6 +202,8 @@ __global__ void __launch_bounds__(1024, 1) classifier_stream_kernel(__nv_bfloat1
 __global__ void __launch_bounds__(1024, 1) classifier_stream2_kernel(__nv_bfloat16* __restrict__ logits, float* __restrict__ losses,
                                                                      const int* __restrict__ targets, float dloss, int rows, int V,
                                                                      int Vp, int write_dlogits, int buf_bytes, int* status) {
+  pdl_trigger();
+  pdl_wait();
   using T = __nv_bfloat16;
   constexpr int N = 8;
   constexpr int NC = 992, NCW = 31;                       // compute threads / warps
@@ -344,6 +350,8 @@ __device__ __forceinline__ float2 warp_merge_ms(float2 v) {
 // 74 us with one CTA and scalar loads.  From SM_CLUSTER_ROWS rows on one CTA per row fills the chip.
 template <typename T, int CL>
 __global__ void __launch_bounds__(512) softmax_rows_kernel(float* __restrict__ out, const T* __restrict__ inp, int V, int ld, float inv_temp) {
+  pdl_trigger();
+  pdl_wait();
   constexpr int N = Pack<T>::N;
   __shared__ float2 red[16];
   __shared__ float2 part[8];                              // written by every CTA of the cluster
@@ -394,16 +402,9 @@ constexpr int SM_CLUSTER_ROWS = 64;
 template <typename T>
 int softmax_rows_launch(float* out, const void* inp, int rows, int V, int ld, float inv_temp, cudaStream_t st) {
   if (rows >= SM_CLUSTER_ROWS) {
-    softmax_rows_kernel<T, 1><<<rows, 512, 0, st>>>(out, (const T*)inp, V, ld, inv_temp);
-    return (int)cudaGetLastError();
+    return launch_pdl(softmax_rows_kernel<T, 1>, rows, 512, 0, st, out, (const T*)inp, V, ld, inv_temp);
   }
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(rows * 8); cfg.blockDim = dim3(512); cfg.stream = st;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = 8; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
-  cfg.attrs = at; cfg.numAttrs = 1;
-  return (int)cudaLaunchKernelEx(&cfg, softmax_rows_kernel<T, 8>, out, (const T*)inp, V, ld, inv_temp);
+  return launch_pdl_cluster(8, softmax_rows_kernel<T, 8>, rows * 8, 512, 0, st, out, (const T*)inp, V, ld, inv_temp);
 }
 
 // dlogits = probs * (dprobs - sum_k dprobs[k] * probs[k]) over the first V columns of a row (one block per row);
@@ -469,11 +470,11 @@ LLMB_API int llmb_fused_classifier(void* logits, float* losses, const int* targe
       const int grid = rows < sm_count() ? rows : sm_count();
       if (stream_on == 2) {                               // LLMB_CLASSIFIER_STREAM=2: row traffic on thread 0 of the compute block
         cudaFuncSetAttribute(classifier_stream_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * buf_bytes);
-        classifier_stream_kernel<<<grid, 1024, 2 * buf_bytes, st>>>((__nv_bfloat16*)logits, losses, targets, dloss, rows, V, Vp,
+        launch_pdl(classifier_stream_kernel, grid, 1024, 2 * buf_bytes, st, (__nv_bfloat16*)logits, losses, targets, dloss, rows, V, Vp,
                                                                    write_dlogits, buf_bytes, status);
       } else {
         cudaFuncSetAttribute(classifier_stream2_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * buf_bytes);
-        classifier_stream2_kernel<<<grid, 1024, 2 * buf_bytes, st>>>((__nv_bfloat16*)logits, losses, targets, dloss, rows, V, Vp,
+        launch_pdl(classifier_stream2_kernel, grid, 1024, 2 * buf_bytes, st, (__nv_bfloat16*)logits, losses, targets, dloss, rows, V, Vp,
                                                                     write_dlogits, buf_bytes, status);
       }
       return (int)cudaGetLastError();
@@ -481,13 +482,13 @@ LLMB_API int llmb_fused_classifier(void* logits, float* losses, const int* targe
     size_t smem = (size_t)Vp * 2;
     if (smem > 200 * 1024) return LLMB_ERR_BAD_ARG;
     cudaFuncSetAttribute(classifier_kernel<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    classifier_kernel<__nv_bfloat16><<<rows, 1024, smem, st>>>((__nv_bfloat16*)logits, losses, targets, dloss, V, Vp, write_dlogits);
+    launch_pdl(classifier_kernel<__nv_bfloat16>, rows, 1024, smem, st, (__nv_bfloat16*)logits, losses, targets, dloss, V, Vp, write_dlogits);
   } else {
     if (Vp % 4) return LLMB_ERR_BAD_ARG;
     size_t smem = (size_t)Vp * 4;
     if (smem > 220 * 1024) return LLMB_ERR_BAD_ARG;
     cudaFuncSetAttribute(classifier_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    classifier_kernel<float><<<rows, 1024, smem, st>>>((float*)logits, losses, targets, dloss, V, Vp, write_dlogits);
+    launch_pdl(classifier_kernel<float>, rows, 1024, smem, st, (float*)logits, losses, targets, dloss, V, Vp, write_dlogits);
   }
   return (int)cudaGetLastError();
 }
@@ -508,6 +509,8 @@ namespace {
 template <typename T>
 __global__ void __launch_bounds__(256) ce_pass1_kernel(float4* __restrict__ stats, const T* __restrict__ tile, const int* __restrict__ targets,
                                                       int ld, int col0, int width, int V, int first) {
+  pdl_trigger();
+  pdl_wait();
   constexpr int N = Pack<T>::N, U = 4;
   __shared__ float2 red[8];
   const int row = blockIdx.x, tid = threadIdx.x, lane = tid % 32, wid = tid / 32;
@@ -554,12 +557,16 @@ __global__ void __launch_bounds__(256) ce_pass1_kernel(float4* __restrict__ stat
   }
 }
 __global__ void ce_loss_kernel(float* __restrict__ losses, const float4* __restrict__ stats, int rows) {
+  pdl_trigger();
+  pdl_wait();
   int r = blockIdx.x * blockDim.x + threadIdx.x;
   if (r < rows) { float4 st = stats[r]; losses[r] = -(st.z - st.x - logf(st.y)); }
 }
 template <typename T>
 __global__ void __launch_bounds__(256) ce_pass2_kernel(T* __restrict__ tile, const float4* __restrict__ stats, const int* __restrict__ targets,
                                                       int ld, int col0, int width, int V, float dloss) {
+  pdl_trigger();
+  pdl_wait();
   constexpr int N = Pack<T>::N, U = 4;
   const int row = blockIdx.x, tid = threadIdx.x;
   T* g = tile + (size_t)row * ld;
@@ -589,17 +596,17 @@ __global__ void __launch_bounds__(256) ce_pass2_kernel(T* __restrict__ tile, con
 
 LLMB_API int llmb_ce_pass1(float* stats, const void* tile, const int* targets, int rows, int ld, int col0, int width, int V,
                            int first, int dtype, cudaStream_t st) {
-  if (dtype == LLMB_BF16) ce_pass1_kernel<__nv_bfloat16><<<rows, 256, 0, st>>>((float4*)stats, (const __nv_bfloat16*)tile, targets, ld, col0, width, V, first);
-  else ce_pass1_kernel<float><<<rows, 256, 0, st>>>((float4*)stats, (const float*)tile, targets, ld, col0, width, V, first);
+  if (dtype == LLMB_BF16) launch_pdl(ce_pass1_kernel<__nv_bfloat16>, rows, 256, 0, st, (float4*)stats, (const __nv_bfloat16*)tile, targets, ld, col0, width, V, first);
+  else launch_pdl(ce_pass1_kernel<float>, rows, 256, 0, st, (float4*)stats, (const float*)tile, targets, ld, col0, width, V, first);
   return (int)cudaGetLastError();
 }
 LLMB_API int llmb_ce_loss(float* losses, const float* stats, int rows, cudaStream_t st) {
-  ce_loss_kernel<<<ceil_div(rows, 256), 256, 0, st>>>(losses, (const float4*)stats, rows);
+  launch_pdl(ce_loss_kernel, ceil_div(rows, 256), 256, 0, st, losses, (const float4*)stats, rows);
   return (int)cudaGetLastError();
 }
 LLMB_API int llmb_ce_pass2(void* tile, const float* stats, const int* targets, int rows, int ld, int col0, int width, int V,
                            float dloss, int dtype, cudaStream_t st) {
-  if (dtype == LLMB_BF16) ce_pass2_kernel<__nv_bfloat16><<<rows, 256, 0, st>>>((__nv_bfloat16*)tile, (const float4*)stats, targets, ld, col0, width, V, dloss);
-  else ce_pass2_kernel<float><<<rows, 256, 0, st>>>((float*)tile, (const float4*)stats, targets, ld, col0, width, V, dloss);
+  if (dtype == LLMB_BF16) launch_pdl(ce_pass2_kernel<__nv_bfloat16>, rows, 256, 0, st, (__nv_bfloat16*)tile, (const float4*)stats, targets, ld, col0, width, V, dloss);
+  else launch_pdl(ce_pass2_kernel<float>, rows, 256, 0, st, (float*)tile, (const float4*)stats, targets, ld, col0, width, V, dloss);
   return (int)cudaGetLastError();
 }

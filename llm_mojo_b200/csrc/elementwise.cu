@@ -15,6 +15,8 @@ using namespace llmb;
 template <typename T>
 __global__ void encoder_fwd_kernel(T* __restrict__ out, const int* __restrict__ tok, const T* __restrict__ wte,
                                    const T* __restrict__ wpe, int BT, int Tlen, int C, int V) {
+  pdl_trigger();
+  pdl_wait();
   constexpr int N = Pack<T>::N;
   const int vec_per_row = C / N;
   long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -41,12 +43,12 @@ LLMB_API int llmb_encoder_fwd(void* out, const int* tok, const void* wte, const 
   if (dtype == LLMB_BF16) {
     if (C % 8) return LLMB_ERR_BAD_ARG;
     long long total = (long long)BT * (C / 8);
-    encoder_fwd_kernel<__nv_bfloat16><<<(unsigned)ceil_div_ll(total, 256), 256, 0, st>>>(
+    launch_pdl(encoder_fwd_kernel<__nv_bfloat16>, (unsigned)ceil_div_ll(total, 256), 256, 0, st,
         (__nv_bfloat16*)out, tok, (const __nv_bfloat16*)wte, (const __nv_bfloat16*)wpe, BT, T, C, V);
   } else {
     if (C % 4) return LLMB_ERR_BAD_ARG;
     long long total = (long long)BT * (C / 4);
-    encoder_fwd_kernel<float><<<(unsigned)ceil_div_ll(total, 256), 256, 0, st>>>(
+    launch_pdl(encoder_fwd_kernel<float>, (unsigned)ceil_div_ll(total, 256), 256, 0, st,
         (float*)out, tok, (const float*)wte, (const float*)wpe, BT, T, C, V);
   }
   return (int)cudaGetLastError();
@@ -54,6 +56,8 @@ LLMB_API int llmb_encoder_fwd(void* out, const int* tok, const void* wte, const 
 
 // ---------------------------------------------------------------- encoder backward
 __global__ void make_keys_kernel(unsigned long long* keys, const int* tok, int BT) {
+  pdl_trigger();
+  pdl_wait();
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < BT) keys[i] = ((unsigned long long)(unsigned)tok[i] << 32) | (unsigned)i;
 }
@@ -68,6 +72,8 @@ constexpr int WTE_SEG = 16;
 template <typename T>
 __global__ void __launch_bounds__(256) wte_bwd_kernel(float* __restrict__ dwte, float* __restrict__ partial, const T* __restrict__ dout,
                                                       const unsigned long long* __restrict__ keys, int BT, int C, int V) {
+  pdl_trigger();
+  pdl_wait();
   constexpr int N = Pack<T>::N;
   const int lane = threadIdx.x % 32, seg = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
   const int j0 = seg * WTE_SEG;
@@ -118,6 +124,8 @@ __global__ void __launch_bounds__(256) wte_bwd_kernel(float* __restrict__ dwte, 
 // is where the run's first piece lives), its pieces are summed in segment order and added to dwte.
 __global__ void __launch_bounds__(256) wte_bwd_combine_kernel(float* __restrict__ dwte, const float* __restrict__ partial,
                                                               const unsigned long long* __restrict__ keys, int BT, int C, int V) {
+  pdl_trigger();
+  pdl_wait();
   const int seg = blockIdx.x, j0 = seg * WTE_SEG, cnt = min(WTE_SEG, BT - j0);
   const unsigned tokv = (unsigned)(keys[j0 + cnt - 1] >> 32);
   if (j0 + cnt >= BT || (unsigned)(keys[j0 + cnt] >> 32) != tokv) return;            // nothing leaves through the end
@@ -146,6 +154,8 @@ __global__ void __launch_bounds__(256) wte_bwd_combine_kernel(float* __restrict_
 
 template <typename T>
 __global__ void wpe_bwd_kernel(float* __restrict__ dwpe, const T* __restrict__ dout, int B, int Tlen, int C) {
+  pdl_trigger();
+  pdl_wait();
   constexpr int N = Pack<T>::N;
   const int vec_per_row = C / N;
   int idx = blockIdx.x * blockDim.x + threadIdx.x;
@@ -184,21 +194,21 @@ LLMB_API int llmb_encoder_bwd(float* dwte, float* dwpe, const void* dout, const 
   const size_t sort_bytes = encoder_bwd_sort_bytes(BT);
   size_t temp_bytes = sort_bytes - 2 * (size_t)BT * sizeof(unsigned long long);
   float* partial = reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(scratch) + sort_bytes);
-  make_keys_kernel<<<ceil_div(BT, 256), 256, 0, st>>>(kin, tok, BT);
+  launch_pdl(make_keys_kernel, ceil_div(BT, 256), 256, 0, st, kin, tok, BT);
   // position bits live in [0, 32); token bits in [32, 32 + vocab_bits). Sort only the used bits.
   cudaError_t e = cub::DeviceRadixSort::SortKeys(temp, temp_bytes, kin, kout, BT, 0, 32 + vocab_bits, st);
   if (e != cudaSuccess) return (int)e;
   const int nseg = ceil_div(BT, WTE_SEG);
   if (dtype == LLMB_BF16) {
     if (C % 8) return LLMB_ERR_BAD_ARG;
-    wte_bwd_kernel<__nv_bfloat16><<<ceil_div(nseg, 8), 256, 0, st>>>(dwte, partial, (const __nv_bfloat16*)dout, kout, BT, C, V);
-    wte_bwd_combine_kernel<<<nseg, 256, 0, st>>>(dwte, partial, kout, BT, C, V);
-    wpe_bwd_kernel<__nv_bfloat16><<<ceil_div(T * (C / 8), 256), 256, 0, st>>>(dwpe, (const __nv_bfloat16*)dout, B, T, C);
+    launch_pdl(wte_bwd_kernel<__nv_bfloat16>, ceil_div(nseg, 8), 256, 0, st, dwte, partial, (const __nv_bfloat16*)dout, kout, BT, C, V);
+    launch_pdl(wte_bwd_combine_kernel, nseg, 256, 0, st, dwte, partial, kout, BT, C, V);
+    launch_pdl(wpe_bwd_kernel<__nv_bfloat16>, ceil_div(T * (C / 8), 256), 256, 0, st, dwpe, (const __nv_bfloat16*)dout, B, T, C);
   } else {
     if (C % 4) return LLMB_ERR_BAD_ARG;
-    wte_bwd_kernel<float><<<ceil_div(nseg, 8), 256, 0, st>>>(dwte, partial, (const float*)dout, kout, BT, C, V);
-    wte_bwd_combine_kernel<<<nseg, 256, 0, st>>>(dwte, partial, kout, BT, C, V);
-    wpe_bwd_kernel<float><<<ceil_div(T * (C / 4), 256), 256, 0, st>>>(dwpe, (const float*)dout, B, T, C);
+    launch_pdl(wte_bwd_kernel<float>, ceil_div(nseg, 8), 256, 0, st, dwte, partial, (const float*)dout, kout, BT, C, V);
+    launch_pdl(wte_bwd_combine_kernel, nseg, 256, 0, st, dwte, partial, kout, BT, C, V);
+    launch_pdl(wpe_bwd_kernel<float>, ceil_div(T * (C / 4), 256), 256, 0, st, dwpe, (const float*)dout, B, T, C);
   }
   return (int)cudaGetLastError();
 }
@@ -206,6 +216,8 @@ LLMB_API int llmb_encoder_bwd(float* dwte, float* dwpe, const void* dout, const 
 // ---------------------------------------------------------------- GELU
 template <typename T>
 __global__ void gelu_fwd_kernel(T* __restrict__ out, const T* __restrict__ inp, long long nvec) {
+  pdl_trigger();
+  pdl_wait();
   constexpr int N = Pack<T>::N;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < nvec; i += (long long)gridDim.x * blockDim.x) {
     Pack<T> p; p.load(inp + i * N);
@@ -216,6 +228,8 @@ __global__ void gelu_fwd_kernel(T* __restrict__ out, const T* __restrict__ inp, 
 }
 template <typename T>
 __global__ void gelu_bwd_kernel(T* __restrict__ dinp, const T* __restrict__ inp, const T* __restrict__ dout, long long nvec) {
+  pdl_trigger();
+  pdl_wait();
   constexpr int N = Pack<T>::N;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < nvec; i += (long long)gridDim.x * blockDim.x) {
     Pack<T> x, d; x.load(inp + i * N); d.load(dout + i * N);
@@ -226,14 +240,14 @@ __global__ void gelu_bwd_kernel(T* __restrict__ dinp, const T* __restrict__ inp,
 }
 LLMB_API int llmb_gelu_fwd(void* out, const void* inp, long long n, int dtype, cudaStream_t st) {
   int grid = sm_count() * 8;
-  if (dtype == LLMB_BF16) { if (n % 8) return LLMB_ERR_BAD_ARG; gelu_fwd_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>((__nv_bfloat16*)out, (const __nv_bfloat16*)inp, n / 8); }
-  else { if (n % 4) return LLMB_ERR_BAD_ARG; gelu_fwd_kernel<float><<<grid, 256, 0, st>>>((float*)out, (const float*)inp, n / 4); }
+  if (dtype == LLMB_BF16) { if (n % 8) return LLMB_ERR_BAD_ARG; launch_pdl(gelu_fwd_kernel<__nv_bfloat16>, grid, 256, 0, st, (__nv_bfloat16*)out, (const __nv_bfloat16*)inp, n / 8); }
+  else { if (n % 4) return LLMB_ERR_BAD_ARG; launch_pdl(gelu_fwd_kernel<float>, grid, 256, 0, st, (float*)out, (const float*)inp, n / 4); }
   return (int)cudaGetLastError();
 }
 LLMB_API int llmb_gelu_bwd(void* dinp, const void* inp, const void* dout, long long n, int dtype, cudaStream_t st) {
   int grid = sm_count() * 8;
-  if (dtype == LLMB_BF16) { if (n % 8) return LLMB_ERR_BAD_ARG; gelu_bwd_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>((__nv_bfloat16*)dinp, (const __nv_bfloat16*)inp, (const __nv_bfloat16*)dout, n / 8); }
-  else { if (n % 4) return LLMB_ERR_BAD_ARG; gelu_bwd_kernel<float><<<grid, 256, 0, st>>>((float*)dinp, (const float*)inp, (const float*)dout, n / 4); }
+  if (dtype == LLMB_BF16) { if (n % 8) return LLMB_ERR_BAD_ARG; launch_pdl(gelu_bwd_kernel<__nv_bfloat16>, grid, 256, 0, st, (__nv_bfloat16*)dinp, (const __nv_bfloat16*)inp, (const __nv_bfloat16*)dout, n / 8); }
+  else { if (n % 4) return LLMB_ERR_BAD_ARG; launch_pdl(gelu_bwd_kernel<float>, grid, 256, 0, st, (float*)dinp, (const float*)inp, (const float*)dout, n / 4); }
   return (int)cudaGetLastError();
 }
 
@@ -242,6 +256,8 @@ LLMB_API int llmb_gelu_bwd(void* dinp, const void* inp, const void* dout, long l
 // partial[slab][c] written to scratch; stage 2 sums slabs in order (deterministic) and accumulates.
 template <typename T, int RL>
 __global__ void __launch_bounds__(256) dbias_partial_kernel(float* __restrict__ partial, const T* __restrict__ dout, int rows, int OC, int rows_per_slab) {
+  pdl_trigger();
+  pdl_wait();
   constexpr int N = Pack<T>::N;
   constexpr int CV = 256 / RL;                           // column vectors per block; RL row lanes
   __shared__ float sm[RL][CV * N + 1];
@@ -285,15 +301,17 @@ void dbias_partial_launch(float* partial, const T* dout, int rows, int OC, int r
   constexpr int N = Pack<T>::N;
   const int want = 6 * sm_count();
   if (ceil_div(OC, 32 * N) * slabs >= want)
-    dbias_partial_kernel<T, 8><<<dim3(ceil_div(OC, 32 * N), slabs), 256, 0, st>>>(partial, dout, rows, OC, rows_per_slab);
+    launch_pdl(dbias_partial_kernel<T, 8>, dim3(ceil_div(OC, 32 * N), slabs), 256, 0, st, partial, dout, rows, OC, rows_per_slab);
   else if (ceil_div(OC, 16 * N) * slabs >= want)
-    dbias_partial_kernel<T, 16><<<dim3(ceil_div(OC, 16 * N), slabs), 256, 0, st>>>(partial, dout, rows, OC, rows_per_slab);
+    launch_pdl(dbias_partial_kernel<T, 16>, dim3(ceil_div(OC, 16 * N), slabs), 256, 0, st, partial, dout, rows, OC, rows_per_slab);
   else
-    dbias_partial_kernel<T, 32><<<dim3(ceil_div(OC, 8 * N), slabs), 256, 0, st>>>(partial, dout, rows, OC, rows_per_slab);
+    launch_pdl(dbias_partial_kernel<T, 32>, dim3(ceil_div(OC, 8 * N), slabs), 256, 0, st, partial, dout, rows, OC, rows_per_slab);
 }
 // Stage 2: 32 columns per block, eight threads per column each summing every eighth slab (independent loads in flight
 // instead of one thread walking all slabs), then a fixed-order sum of the eight: deterministic.
 __global__ void __launch_bounds__(256) dbias_final_kernel(float* __restrict__ dbias, const float* __restrict__ partial, int OC, int slabs) {
+  pdl_trigger();
+  pdl_wait();
   __shared__ float sm[8][33];
   const int cl = threadIdx.x % 32, sl = threadIdx.x / 32;
   const int c = blockIdx.x * 32 + cl;
@@ -325,7 +343,7 @@ LLMB_API int llmb_dbias(float* dbias, const void* dout, float* scratch, long lon
     if (OC % 4) return LLMB_ERR_BAD_ARG;
     dbias_partial_launch<float>(scratch, (const float*)dout, rows, OC, rows_per_slab, slabs, st);
   }
-  dbias_final_kernel<<<ceil_div(OC, 32), 256, 0, st>>>(dbias, scratch, OC, slabs);
+  launch_pdl(dbias_final_kernel, ceil_div(OC, 32), 256, 0, st, dbias, scratch, OC, slabs);
   return (int)cudaGetLastError();
 }
 
@@ -411,6 +429,6 @@ LLMB_API int llmb_dbias_noalloc(float* dbias, const void* dout, int rows, int OC
   } else {
     return LLMB_ERR_BAD_ARG;
   }
-  dbias_final_kernel<<<ceil_div(OC, 32), 256, 0, st>>>(dbias, scratch, OC, slabs);
+  launch_pdl(dbias_final_kernel, ceil_div(OC, 32), 256, 0, st, dbias, scratch, OC, slabs);
   return (int)cudaGetLastError();
 }

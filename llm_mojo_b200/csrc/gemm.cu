@@ -68,6 +68,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   cluster_sync_all();                                   // both CTAs' barriers exist before any remote signal
   fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  if (p.g.W <= 1 && p.pull.nseg == 0 && p.pull.nwait == 0) pdl_trigger();   // else this kernel waits for other GPUs or streams
+  pdl_wait();
 
   const int m_tiles = ceil_div(p.M, 2 * BM);            // cluster tiles of 256 rows
   const int tiles_per_split = m_tiles * p.n_tiles;
@@ -471,8 +473,7 @@ int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap&
     if (e != cudaSuccess) return (int)e;
     attr_done = true;
   }
-  gemm_pair_kernel<KIND, EPI><<<grid, PAIR_THREADS, SMEM, st>>>(ta, tb, td, taux, p);
-  return (int)cudaGetLastError();
+  return launch_pdl(gemm_pair_kernel<KIND, EPI>, grid, PAIR_THREADS, SMEM, st, ta, tb, td, taux, p);
 }
 
 // Tile configuration of one problem: bn = 256 is the CTA-pair kernel, 64 / 128 the kernel of gemm_small.cu with cl CTAs per tile.
@@ -713,6 +714,8 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   __syncthreads();
   fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_trigger();
+  pdl_wait();
 
   const int tiles_per_split = p.m_tiles * p.n_tiles;
   const int total_units = tiles_per_split * p.splits;
@@ -923,8 +926,7 @@ int launch_nvfp4(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap
     if (e != cudaSuccess) return (int)e;
     attr_done = true;
   }
-  gemm_nvfp4_kernel<MX, EPI><<<grid, NV_THREADS, NV_SMEM_BYTES, st>>>(ta, tb, td, taux, q);
-  return (int)cudaGetLastError();
+  return launch_pdl(gemm_nvfp4_kernel<MX, EPI>, grid, NV_THREADS, NV_SMEM_BYTES, st, ta, tb, td, taux, q);
 }
 }  // namespace
 

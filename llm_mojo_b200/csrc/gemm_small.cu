@@ -70,8 +70,8 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   __syncthreads();
   fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
-  pdl_wait();
   pdl_trigger();
+  pdl_wait();
 
   // the 32-row band this warp runs the epilogue of: its own quarter, or one of the 4 / CL bands that this CTA collects
   constexpr int NB = 4 / CL;
@@ -252,17 +252,7 @@ int launch_small(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap
     if (e != cudaSuccess) return (int)e;
     attr_done = true;
   }
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(p.m_tiles * p.n_tiles * CL, CL > 1 ? 1 : p.splits);
-  cfg.blockDim = dim3(SM_THREADS);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = CL; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = CL > 1 ? 1 : 0;
-  return (int)cudaLaunchKernelEx(&cfg, kern, ta, tb, td, taux, p, stages);
+  return launch_pdl_cluster(CL, kern, dim3(p.m_tiles * p.n_tiles * CL, CL > 1 ? 1 : p.splits), SM_THREADS, smem, st, ta, tb, td, taux, p, stages);
 }
 
 template <int KIND, int EPI>

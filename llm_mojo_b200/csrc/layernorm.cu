@@ -20,6 +20,8 @@ __global__ void __launch_bounds__(256) ln_fwd_kernel(T* __restrict__ out, float*
                                                     T* __restrict__ resid_out, const T* __restrict__ inp1,
                                                     const T* __restrict__ inp2, const T* __restrict__ w,
                                                     const T* __restrict__ b, int rows, int C) {
+  pdl_trigger();
+  pdl_wait();
   constexpr int N = Pack<T>::N;
   const int lane = threadIdx.x % 32, wid = threadIdx.x / 32;
   const int nvec = C / N;                       // vectors per row
@@ -94,6 +96,8 @@ __global__ void __launch_bounds__(640) ln_bwd_kernel(T* __restrict__ dres, float
                                                     const T* __restrict__ inp, const T* __restrict__ w,
                                                     const float* __restrict__ mean_i, const float* __restrict__ rstd_i, int rows,
                                                     int C, int gthreads, int groups) {
+  pdl_trigger();
+  pdl_wait();
   constexpr int N = Pack<T>::N;
   constexpr int NS = SUMOUT ? 3 : 2;
   extern __shared__ float sm[];                        // [NS][C] column sums
@@ -200,6 +204,8 @@ __global__ void __launch_bounds__(640) ln_bwd_kernel(T* __restrict__ dres, float
 // 128-byte reads, at most five dependent steps for 148 rows) and are combined in fixed order through shared memory.
 __global__ void __launch_bounds__(1024) ln_bwd_final_kernel(float* __restrict__ dw, float* __restrict__ db, float* __restrict__ dsum,
                                                            const float* __restrict__ partial, int C, int nblocks) {
+  pdl_trigger();
+  pdl_wait();
   __shared__ float red[32][33];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int c = blockIdx.x * 32 + tx;
@@ -223,9 +229,9 @@ int ln_fwd_launch_n(void* out, float* mean, float* rstd, void* resid_out, const 
                     const void* w, const void* b, int rows, int C, cudaStream_t st) {
   int grid = ceil_div(rows, 8);
   if (inp2)
-    ln_fwd_kernel<T, true, PER_LANE><<<grid, 256, 0, st>>>((T*)out, mean, rstd, (T*)resid_out, (const T*)inp1, (const T*)inp2, (const T*)w, (const T*)b, rows, C);
+    launch_pdl(ln_fwd_kernel<T, true, PER_LANE>, grid, 256, 0, st, (T*)out, mean, rstd, (T*)resid_out, (const T*)inp1, (const T*)inp2, (const T*)w, (const T*)b, rows, C);
   else
-    ln_fwd_kernel<T, false, PER_LANE><<<grid, 256, 0, st>>>((T*)out, mean, rstd, nullptr, (const T*)inp1, nullptr, (const T*)w, (const T*)b, rows, C);
+    launch_pdl(ln_fwd_kernel<T, false, PER_LANE>, grid, 256, 0, st, (T*)out, mean, rstd, nullptr, (const T*)inp1, nullptr, (const T*)w, (const T*)b, rows, C);
   return (int)cudaGetLastError();
 }
 
@@ -270,7 +276,7 @@ int ln_bwd_launch(void* dres, float* partial, const void* dout, const void* inp,
     const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
   }
-  kern<<<p.grid, p.gthreads * p.groups, smem, st>>>((T*)dres, partial, (const T*)dout, (const T*)inp, (const T*)w, mean, rstd, rows, C,
+  launch_pdl(kern, p.grid, p.gthreads * p.groups, smem, st, (T*)dres, partial, (const T*)dout, (const T*)inp, (const T*)w, mean, rstd, rows, C,
                                                     p.gthreads, p.groups);
   return (int)cudaGetLastError();
 }
@@ -308,6 +314,6 @@ LLMB_API int llmb_layernorm_bwd_colsum(void* dres, float* dw, float* db, float* 
   const int rc = dtype == LLMB_BF16 ? ln_bwd_launch<__nv_bfloat16>(dres, scratch, dout, inp, w, mean, rstd, rows, C, accumulate, sumout, st)
                                     : ln_bwd_launch<float>(dres, scratch, dout, inp, w, mean, rstd, rows, C, accumulate, sumout, st);
   if (rc) return rc;
-  ln_bwd_final_kernel<<<ceil_div((sumout ? 3 : 2) * C, 32), 1024, 0, st>>>(dw, db, dsum, scratch, C, grid);
+  launch_pdl(ln_bwd_final_kernel, ceil_div((sumout ? 3 : 2) * C, 32), 1024, 0, st, dw, db, dsum, scratch, C, grid);
   return (int)cudaGetLastError();
 }

@@ -39,6 +39,8 @@ __global__ void adamw_kernel(TP* __restrict__ params, float* __restrict__ master
                              float* __restrict__ m, float* __restrict__ v, long long n, float lr, float beta1,
                              float beta2, float bc1, float bc2, float eps, float wd, float grad_scale,
                              const float* __restrict__ dev_scale, unsigned long long seed, int use_sr) {
+  pdl_trigger();
+  pdl_wait();
   if (dev_scale) grad_scale *= *dev_scale;
   const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x, stride = (long long)gridDim.x * blockDim.x;
   long long done = 0;
@@ -88,6 +90,8 @@ __global__ void adamw_kernel(TP* __restrict__ params, float* __restrict__ master
 }
 
 __global__ void norm_sq_partial_kernel(float* __restrict__ partial, const float* __restrict__ x, long long n) {
+  pdl_trigger();
+  pdl_wait();
   __shared__ float red[32];
   float s = 0.f;
   const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x, stride = (long long)gridDim.x * blockDim.x;
@@ -110,6 +114,8 @@ __global__ void norm_sq_partial_kernel(float* __restrict__ partial, const float*
   if (wid == 0) { float t = lane < blockDim.x / 32 ? red[lane] : 0.f; t = warp_sum(t); if (lane == 0) partial[blockIdx.x] = t; }
 }
 __global__ void norm_sq_final_kernel(float* __restrict__ out, const float* __restrict__ partial, int nblocks, int accumulate) {
+  pdl_trigger();
+  pdl_wait();
   __shared__ float red[32];
   float s = 0.f;
   for (int i = threadIdx.x; i < nblocks; i += blockDim.x) s += partial[i];
@@ -132,11 +138,11 @@ LLMB_API int llmb_adamw(void* params, float* master, const float* grads, float* 
                          reinterpret_cast<uintptr_t>(master) | (reinterpret_cast<uintptr_t>(params) << (param_dtype == LLMB_BF16 ? 1 : 0));
   const bool vec = (bits & 15) == 0 && n >= 4;
   if (param_dtype == LLMB_BF16) {
-    if (vec) adamw_kernel<__nv_bfloat16, true><<<grid, 256, 0, st>>>((__nv_bfloat16*)params, master, grads, m, v, n, lr, beta1, beta2, bc1, bc2, eps, wd, grad_scale, dev_scale, seed, use_sr);
-    else adamw_kernel<__nv_bfloat16, false><<<grid, 256, 0, st>>>((__nv_bfloat16*)params, master, grads, m, v, n, lr, beta1, beta2, bc1, bc2, eps, wd, grad_scale, dev_scale, seed, use_sr);
+    if (vec) launch_pdl(adamw_kernel<__nv_bfloat16, true>, grid, 256, 0, st, (__nv_bfloat16*)params, master, grads, m, v, n, lr, beta1, beta2, bc1, bc2, eps, wd, grad_scale, dev_scale, seed, use_sr);
+    else launch_pdl(adamw_kernel<__nv_bfloat16, false>, grid, 256, 0, st, (__nv_bfloat16*)params, master, grads, m, v, n, lr, beta1, beta2, bc1, bc2, eps, wd, grad_scale, dev_scale, seed, use_sr);
   } else {
-    if (vec) adamw_kernel<float, true><<<grid, 256, 0, st>>>((float*)params, master, grads, m, v, n, lr, beta1, beta2, bc1, bc2, eps, wd, grad_scale, dev_scale, seed, 0);
-    else adamw_kernel<float, false><<<grid, 256, 0, st>>>((float*)params, master, grads, m, v, n, lr, beta1, beta2, bc1, bc2, eps, wd, grad_scale, dev_scale, seed, 0);
+    if (vec) launch_pdl(adamw_kernel<float, true>, grid, 256, 0, st, (float*)params, master, grads, m, v, n, lr, beta1, beta2, bc1, bc2, eps, wd, grad_scale, dev_scale, seed, 0);
+    else launch_pdl(adamw_kernel<float, false>, grid, 256, 0, st, (float*)params, master, grads, m, v, n, lr, beta1, beta2, bc1, bc2, eps, wd, grad_scale, dev_scale, seed, 0);
   }
   return (int)cudaGetLastError();
 }
@@ -145,8 +151,8 @@ LLMB_API int llmb_norm_sq_blocks() { return sm_count() * 4; }
 // out[0] (=|+=) sum(x^2); scratch holds llmb_norm_sq_blocks() floats.
 LLMB_API int llmb_global_norm_sq(float* out, const float* x, long long n, float* scratch, int accumulate, cudaStream_t st) {
   int grid = llmb_norm_sq_blocks();
-  norm_sq_partial_kernel<<<grid, 512, 0, st>>>(scratch, x, n);
-  norm_sq_final_kernel<<<1, 256, 0, st>>>(out, scratch, grid, accumulate);
+  launch_pdl(norm_sq_partial_kernel, grid, 512, 0, st, scratch, x, n);
+  launch_pdl(norm_sq_final_kernel, 1, 256, 0, st, out, scratch, grid, accumulate);
   return (int)cudaGetLastError();
 }
 

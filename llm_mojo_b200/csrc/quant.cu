@@ -53,6 +53,8 @@ __device__ __forceinline__ float rng_uniform01(uint64_t seed, uint64_t ctr, uint
 // ------------------------------------------------------------------ amax
 template <typename T>
 __global__ void amax_kernel(unsigned* __restrict__ out_bits, const T* __restrict__ x, long long n) {
+  pdl_trigger();
+  pdl_wait();
   // |x| as raw bits orders like an unsigned integer and NaN patterns sort above +inf, so an
   // integer max is a NaN-infectious float max.
   constexpr int N = Pack<T>::N;
@@ -101,6 +103,8 @@ __global__ void amax_update_kernel(float* state, const float* amax_cur, float fm
 // ------------------------------------------------------------------ FP8 quantise (device scale)
 template <typename T, int FMT>
 __global__ void quantize_fp8_kernel(uint8_t* __restrict__ out, const T* __restrict__ x, const float* __restrict__ scale_ptr, long long n) {
+  pdl_trigger();
+  pdl_wait();
   constexpr int N = Pack<T>::N;
   const float s = *scale_ptr;
   const long long nvec = n / N;
@@ -198,6 +202,8 @@ __global__ void nvfp4_quantize_kernel(uint8_t* __restrict__ q, uint8_t* __restri
                                       const T* __restrict__ x, const float* __restrict__ tensor_scale_ptr, int rows, int cols,
                                       int axis, int rht, int sr, unsigned long long seed, unsigned long long stream,
                                       long long step, long long n_col_tiles) {
+  pdl_trigger();
+  pdl_wait();
   const int outer = axis == 1 ? rows : cols;            // index across blocks' "rows"
   const int K = axis == 1 ? cols : rows;                // length along the block axis
   const int kblocks = K / 16;
@@ -299,6 +305,8 @@ __global__ void __launch_bounds__(256) nvfp4_quantize16_coop_kernel(uint8_t* __r
                                                                    const float* __restrict__ tensor_scale_ptr, int rows, int cols, int axis,
                                                                    int sr, unsigned long long seed, unsigned long long stream, long long step,
                                                                    long long n_col_tiles) {
+  pdl_trigger();
+  pdl_wait();
   const int outer = axis == 1 ? rows : cols, K = axis == 1 ? cols : rows;
   const int kblocks = K / 16, tile_rows = outer / 16;
   const long long gid = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / 16;       // block index (half-warp uniform)
@@ -371,6 +379,8 @@ __global__ void __launch_bounds__(256) nvfp4_quantize16_coop_kernel(uint8_t* __r
 }
 
 __global__ void nvfp4_tensor_scale_kernel(float* ts, const float* amax) {
+  pdl_trigger();
+  pdl_wait();
   const float a = *amax;
   *ts = (a > 0.f && !isnan(a) && !isinf(a)) ? a / (448.0f * 6.0f) : 1.0f;
 }
@@ -425,6 +435,8 @@ __global__ void amax_push_kernel(float* state, const float* amax_cur) {
 template <typename T, int FMT>
 __global__ void __launch_bounds__(512) quantize_fp8_amax_kernel(uint8_t* __restrict__ out, unsigned* __restrict__ amax_bits, const T* __restrict__ x,
                                                                const float* __restrict__ scale_ptr, long long n) {
+  pdl_trigger();
+  pdl_wait();
   constexpr int N = Pack<T>::N;
   const float s = *scale_ptr;
   unsigned m = 0;
@@ -471,6 +483,8 @@ __device__ void derive_scale(float* state, unsigned* amax_bits, float fmt_max, f
 }
 __global__ void fp8_prepare_kernel(float* sa, unsigned* aa, float fa, float ma, float* sb, unsigned* ab, float fb, float mb,
                                    float* alpha1, const float* p1, const float* q1, float* alpha2, const float* p2, const float* q2) {
+  pdl_trigger();
+  pdl_wait();
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
   if (sa) derive_scale(sa, aa, fa, ma);
   if (sb) derive_scale(sb, ab, fb, mb);
@@ -478,6 +492,8 @@ __global__ void fp8_prepare_kernel(float* sa, unsigned* aa, float fa, float ma, 
   if (alpha2) *alpha2 = p2[1] * q2[1];
 }
 __global__ void fp8_push_kernel(float* sa, const float* aa, float* sb, const float* ab) {
+  pdl_trigger();
+  pdl_wait();
   if (threadIdx.x != 0 || blockIdx.x != 0) return;
   if (sa) { const int step = __float_as_int(sa[2]); sa[4 + step % AMAX_HISTORY] = *aa; sa[2] = __int_as_float(step + 1); }
   if (sb) { const int step = __float_as_int(sb[2]); sb[4 + step % AMAX_HISTORY] = *ab; sb[2] = __int_as_float(step + 1); }
@@ -485,11 +501,11 @@ __global__ void fp8_push_kernel(float* sa, const float* aa, float* sb, const flo
 }  // namespace
 LLMB_API int llmb_fp8_prepare(float* sa, float* aa, float fa, float ma, float* sb, float* ab, float fb, float mb, float* alpha1,
                               const float* p1, const float* q1, float* alpha2, const float* p2, const float* q2, cudaStream_t st) {
-  fp8_prepare_kernel<<<1, 32, 0, st>>>(sa, (unsigned*)aa, fa, ma, sb, (unsigned*)ab, fb, mb, alpha1, p1, q1, alpha2, p2, q2);
+  launch_pdl(fp8_prepare_kernel, 1, 32, 0, st, sa, (unsigned*)aa, fa, ma, sb, (unsigned*)ab, fb, mb, alpha1, p1, q1, alpha2, p2, q2);
   return (int)cudaGetLastError();
 }
 LLMB_API int llmb_fp8_push(float* sa, const float* aa, float* sb, const float* ab, cudaStream_t st) {
-  fp8_push_kernel<<<1, 32, 0, st>>>(sa, aa, sb, ab);
+  launch_pdl(fp8_push_kernel, 1, 32, 0, st, sa, aa, sb, ab);
   return (int)cudaGetLastError();
 }
 // out = fp8(x * state[0]) saturated and amax[0] = max(amax[0], max|x|) as raw bits (clear it first); n a multiple of the vector width
@@ -499,11 +515,11 @@ LLMB_API int llmb_quantize_fp8_amax(void* out, const void* x, const float* state
   long long blocks = ceil_div_ll(n, 512 * 8);
   int grid = (int)(blocks < (long long)sm_count() * 4 ? (blocks < 1 ? 1 : blocks) : (long long)sm_count() * 4);
   if (dtype == LLMB_BF16) {
-    if (fmt == 0) quantize_fp8_amax_kernel<__nv_bfloat16, 0><<<grid, 512, 0, st>>>((uint8_t*)out, (unsigned*)amax, (const __nv_bfloat16*)x, state, n);
-    else quantize_fp8_amax_kernel<__nv_bfloat16, 1><<<grid, 512, 0, st>>>((uint8_t*)out, (unsigned*)amax, (const __nv_bfloat16*)x, state, n);
+    if (fmt == 0) launch_pdl(quantize_fp8_amax_kernel<__nv_bfloat16, 0>, grid, 512, 0, st, (uint8_t*)out, (unsigned*)amax, (const __nv_bfloat16*)x, state, n);
+    else launch_pdl(quantize_fp8_amax_kernel<__nv_bfloat16, 1>, grid, 512, 0, st, (uint8_t*)out, (unsigned*)amax, (const __nv_bfloat16*)x, state, n);
   } else {
-    if (fmt == 0) quantize_fp8_amax_kernel<float, 0><<<grid, 512, 0, st>>>((uint8_t*)out, (unsigned*)amax, (const float*)x, state, n);
-    else quantize_fp8_amax_kernel<float, 1><<<grid, 512, 0, st>>>((uint8_t*)out, (unsigned*)amax, (const float*)x, state, n);
+    if (fmt == 0) launch_pdl(quantize_fp8_amax_kernel<float, 0>, grid, 512, 0, st, (uint8_t*)out, (unsigned*)amax, (const float*)x, state, n);
+    else launch_pdl(quantize_fp8_amax_kernel<float, 1>, grid, 512, 0, st, (uint8_t*)out, (unsigned*)amax, (const float*)x, state, n);
   }
   return (int)cudaGetLastError();
 }
@@ -518,11 +534,11 @@ LLMB_API int llmb_quantize_fp8_delayed(void* out, const void* x, float* state, f
   long long blocks = ceil_div_ll(n, 512 * 8);
   int grid = (int)(blocks < (long long)sm_count() * 4 ? (blocks < 1 ? 1 : blocks) : (long long)sm_count() * 4);
   if (dtype == LLMB_BF16) {
-    if (fmt == 0) quantize_fp8_amax_kernel<__nv_bfloat16, 0><<<grid, 512, 0, st>>>((uint8_t*)out, (unsigned*)amax, (const __nv_bfloat16*)x, state, n);
-    else quantize_fp8_amax_kernel<__nv_bfloat16, 1><<<grid, 512, 0, st>>>((uint8_t*)out, (unsigned*)amax, (const __nv_bfloat16*)x, state, n);
+    if (fmt == 0) launch_pdl(quantize_fp8_amax_kernel<__nv_bfloat16, 0>, grid, 512, 0, st, (uint8_t*)out, (unsigned*)amax, (const __nv_bfloat16*)x, state, n);
+    else launch_pdl(quantize_fp8_amax_kernel<__nv_bfloat16, 1>, grid, 512, 0, st, (uint8_t*)out, (unsigned*)amax, (const __nv_bfloat16*)x, state, n);
   } else {
-    if (fmt == 0) quantize_fp8_amax_kernel<float, 0><<<grid, 512, 0, st>>>((uint8_t*)out, (unsigned*)amax, (const float*)x, state, n);
-    else quantize_fp8_amax_kernel<float, 1><<<grid, 512, 0, st>>>((uint8_t*)out, (unsigned*)amax, (const float*)x, state, n);
+    if (fmt == 0) launch_pdl(quantize_fp8_amax_kernel<float, 0>, grid, 512, 0, st, (uint8_t*)out, (unsigned*)amax, (const float*)x, state, n);
+    else launch_pdl(quantize_fp8_amax_kernel<float, 1>, grid, 512, 0, st, (uint8_t*)out, (unsigned*)amax, (const float*)x, state, n);
   }
   amax_push_kernel<<<1, 32, 0, st>>>(state, amax);
   return (int)cudaGetLastError();
@@ -534,8 +550,8 @@ LLMB_API int llmb_amax(float* out, const void* x, long long n, int dtype, cudaSt
   if (e != cudaSuccess) return (int)e;
   long long blocks = ceil_div_ll(n, 512 * 8);
   int grid = (int)(blocks < (long long)sm_count() * 4 ? (blocks < 1 ? 1 : blocks) : (long long)sm_count() * 4);
-  if (dtype == LLMB_BF16) amax_kernel<__nv_bfloat16><<<grid, 512, 0, st>>>((unsigned*)out, (const __nv_bfloat16*)x, n);
-  else amax_kernel<float><<<grid, 512, 0, st>>>((unsigned*)out, (const float*)x, n);
+  if (dtype == LLMB_BF16) launch_pdl(amax_kernel<__nv_bfloat16>, grid, 512, 0, st, (unsigned*)out, (const __nv_bfloat16*)x, n);
+  else launch_pdl(amax_kernel<float>, grid, 512, 0, st, (unsigned*)out, (const float*)x, n);
   return (int)cudaGetLastError();
 }
 // amax of the 16-point randomised Hadamard transform of x taken along `axis` (blocks of 16 consecutive columns
@@ -543,6 +559,8 @@ LLMB_API int llmb_amax(float* out, const void* x, long long n, int dtype, cudaSt
 namespace {
 template <typename T>
 __global__ void amax_rht_kernel(unsigned* __restrict__ out_bits, const T* __restrict__ x, int rows, int cols, int axis) {
+  pdl_trigger();
+  pdl_wait();
   unsigned m = 0;
   const long long nblocks = (long long)rows * cols / 16;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < nblocks; i += (long long)gridDim.x * blockDim.x) {
@@ -583,8 +601,8 @@ LLMB_API int llmb_amax_rht(float* out, const void* x, int rows, int cols, int ax
   const long long nblocks = (long long)rows * cols / 16;
   long long want = (nblocks + 255) / 256;
   const int grid = (int)(want < 8LL * sm_count() ? (want < 1 ? 1 : want) : 8LL * sm_count());
-  if (dtype == LLMB_BF16) amax_rht_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>((unsigned*)out, (const __nv_bfloat16*)x, rows, cols, axis);
-  else amax_rht_kernel<float><<<grid, 256, 0, st>>>((unsigned*)out, (const float*)x, rows, cols, axis);
+  if (dtype == LLMB_BF16) launch_pdl(amax_rht_kernel<__nv_bfloat16>, grid, 256, 0, st, (unsigned*)out, (const __nv_bfloat16*)x, rows, cols, axis);
+  else launch_pdl(amax_rht_kernel<float>, grid, 256, 0, st, (unsigned*)out, (const float*)x, rows, cols, axis);
   return (int)cudaGetLastError();
 }
 LLMB_API int llmb_amax_state_floats() { return 4 + AMAX_HISTORY; }
@@ -598,12 +616,12 @@ LLMB_API int llmb_quantize_fp8(void* out, const void* x, const float* scale, lon
   int grid = sm_count() * 8;
   if (dtype == LLMB_BF16) {
     if (n % 8) return LLMB_ERR_BAD_ARG;
-    if (fmt == 0) quantize_fp8_kernel<__nv_bfloat16, 0><<<grid, 256, 0, st>>>((uint8_t*)out, (const __nv_bfloat16*)x, scale, n);
-    else quantize_fp8_kernel<__nv_bfloat16, 1><<<grid, 256, 0, st>>>((uint8_t*)out, (const __nv_bfloat16*)x, scale, n);
+    if (fmt == 0) launch_pdl(quantize_fp8_kernel<__nv_bfloat16, 0>, grid, 256, 0, st, (uint8_t*)out, (const __nv_bfloat16*)x, scale, n);
+    else launch_pdl(quantize_fp8_kernel<__nv_bfloat16, 1>, grid, 256, 0, st, (uint8_t*)out, (const __nv_bfloat16*)x, scale, n);
   } else {
     if (n % 4) return LLMB_ERR_BAD_ARG;
-    if (fmt == 0) quantize_fp8_kernel<float, 0><<<grid, 256, 0, st>>>((uint8_t*)out, (const float*)x, scale, n);
-    else quantize_fp8_kernel<float, 1><<<grid, 256, 0, st>>>((uint8_t*)out, (const float*)x, scale, n);
+    if (fmt == 0) launch_pdl(quantize_fp8_kernel<float, 0>, grid, 256, 0, st, (uint8_t*)out, (const float*)x, scale, n);
+    else launch_pdl(quantize_fp8_kernel<float, 1>, grid, 256, 0, st, (uint8_t*)out, (const float*)x, scale, n);
   }
   return (int)cudaGetLastError();
 }
@@ -612,7 +630,7 @@ LLMB_API int llmb_dequantize_fp8(float* out, const void* q, const float* scale_i
   return (int)cudaGetLastError();
 }
 LLMB_API int llmb_nvfp4_tensor_scale(float* ts, const float* amax, cudaStream_t st) {
-  nvfp4_tensor_scale_kernel<<<1, 1, 0, st>>>(ts, amax);
+  launch_pdl(nvfp4_tensor_scale_kernel, 1, 1, 0, st, ts, amax);
   return (int)cudaGetLastError();
 }
 // ------------------------------------------------------------------ FP8 with per-128 block scales (fake quantisation)
@@ -715,6 +733,8 @@ __global__ void __launch_bounds__(256) fp8_block_tile_kernel(__nv_bfloat16* __re
 template <int FMT, int GRAN, int TRANS>
 __global__ void __launch_bounds__(256) fp8_block_quant_kernel(uint8_t* __restrict__ q, uint8_t* __restrict__ sf,
                                                               const __nv_bfloat16* __restrict__ x, int rows, int cols) {
+  pdl_trigger();
+  pdl_wait();
   __shared__ float red[16][128];                          // GRAN 1: partial column maxima; GRAN 2: warp maxima in red[0]
   __shared__ float line_scale[128];                       // scale of outer line o of the written tile
   __shared__ __align__(16) uint8_t tile[TRANS ? 128 * 128 : 16];   // transposed bytes, 8-byte chunks XOR-swizzled by line / 8
@@ -813,6 +833,8 @@ __global__ void __launch_bounds__(256) fp8_block_quant_kernel(uint8_t* __restric
 template <int FMT>
 __global__ void __launch_bounds__(256) fp8_block_quant_dual_kernel(uint8_t* __restrict__ q0, uint8_t* __restrict__ sf0, uint8_t* __restrict__ q1,
                                                                    uint8_t* __restrict__ sf1, const __nv_bfloat16* __restrict__ x, int rows, int cols) {
+  pdl_trigger();
+  pdl_wait();
   __shared__ float red[16][128];                          // partial column maxima
   __shared__ float row_scale[128], col_scale[128];
   __shared__ __align__(16) uint8_t tile[128 * 128];       // transposed bytes, 8-byte chunks XOR-swizzled by line / 8
@@ -910,7 +932,7 @@ LLMB_API int llmb_fp8_block_quant(void* q, void* sf, const void* x, int rows, in
   if (rows % 128 || cols % 128 || fmt < 0 || fmt > 1) return LLMB_ERR_BAD_ARG;
   const unsigned grid = (unsigned)((rows / 128) * (cols / 128));
   auto* qo = (uint8_t*)q; auto* so = (uint8_t*)sf; auto* in = (const __nv_bfloat16*)x;
-#define FP8Q(F, G, T) fp8_block_quant_kernel<F, G, T><<<grid, 256, 0, st>>>(qo, so, in, rows, cols)
+#define FP8Q(F, G, T) launch_pdl(fp8_block_quant_kernel<F, G, T>, grid, 256, 0, st, qo, so, in, rows, cols)
   if (gran == 0 && !transpose) { if (fmt == 0) FP8Q(0, 0, 0); else FP8Q(1, 0, 0); }
   else if (gran == 1 && transpose) { if (fmt == 0) FP8Q(0, 1, 1); else FP8Q(1, 1, 1); }
   else if (gran == 2 && !transpose) { if (fmt == 0) FP8Q(0, 2, 0); else FP8Q(1, 2, 0); }
@@ -924,8 +946,8 @@ LLMB_API int llmb_fp8_block_quant(void* q, void* sf, const void* x, int rows, in
 LLMB_API int llmb_fp8_block_quant_dual(void* q0, void* sf0, void* q1, void* sf1, const void* x, int rows, int cols, int fmt, cudaStream_t st) {
   if (rows % 128 || cols % 128 || fmt < 0 || fmt > 1) return LLMB_ERR_BAD_ARG;
   const unsigned grid = (unsigned)((rows / 128) * (cols / 128));
-  if (fmt == 0) fp8_block_quant_dual_kernel<0><<<grid, 256, 0, st>>>((uint8_t*)q0, (uint8_t*)sf0, (uint8_t*)q1, (uint8_t*)sf1, (const __nv_bfloat16*)x, rows, cols);
-  else fp8_block_quant_dual_kernel<1><<<grid, 256, 0, st>>>((uint8_t*)q0, (uint8_t*)sf0, (uint8_t*)q1, (uint8_t*)sf1, (const __nv_bfloat16*)x, rows, cols);
+  if (fmt == 0) launch_pdl(fp8_block_quant_dual_kernel<0>, grid, 256, 0, st, (uint8_t*)q0, (uint8_t*)sf0, (uint8_t*)q1, (uint8_t*)sf1, (const __nv_bfloat16*)x, rows, cols);
+  else launch_pdl(fp8_block_quant_dual_kernel<1>, grid, 256, 0, st, (uint8_t*)q0, (uint8_t*)sf0, (uint8_t*)q1, (uint8_t*)sf1, (const __nv_bfloat16*)x, rows, cols);
   return (int)cudaGetLastError();
 }
 
@@ -946,11 +968,11 @@ LLMB_API int llmb_nvfp4_quantize(void* q, void* scales, void* deq, const void* x
   const unsigned grid = (unsigned)ceil_div_ll(total, threads);
   if (dtype == LLMB_BF16 && block_rows == 16 && !rht && cols % 16 == 0 && outer % 16 == 0 && K % 16 == 0) {
     const long long lanes = total * 16;
-    nvfp4_quantize16_coop_kernel<<<(unsigned)ceil_div_ll(lanes, 256), 256, 0, st>>>((uint8_t*)q, (uint8_t*)scales, (__nv_bfloat16*)deq,
+    launch_pdl(nvfp4_quantize16_coop_kernel, (unsigned)ceil_div_ll(lanes, 256), 256, 0, st, (uint8_t*)q, (uint8_t*)scales, (__nv_bfloat16*)deq,
         (const __nv_bfloat16*)x, tensor_scale, rows, cols, axis, sr, seed, stream, step, n_col_tiles);
     return (int)cudaGetLastError();
   }
-#define NVFP4_LAUNCH(T, BR) nvfp4_quantize_kernel<T, BR><<<grid, threads, 0, st>>>((uint8_t*)q, (uint8_t*)scales, (__nv_bfloat16*)deq, (const T*)x, tensor_scale, rows, cols, axis, rht, sr, seed, stream, step, n_col_tiles)
+#define NVFP4_LAUNCH(T, BR) launch_pdl(nvfp4_quantize_kernel<T, BR>, grid, threads, 0, st, (uint8_t*)q, (uint8_t*)scales, (__nv_bfloat16*)deq, (const T*)x, tensor_scale, rows, cols, axis, rht, sr, seed, stream, step, n_col_tiles)
   if (dtype == LLMB_BF16) { if (block_rows == 1) NVFP4_LAUNCH(__nv_bfloat16, 1); else NVFP4_LAUNCH(__nv_bfloat16, 16); }
   else { if (block_rows == 1) NVFP4_LAUNCH(float, 1); else NVFP4_LAUNCH(float, 16); }
 #undef NVFP4_LAUNCH

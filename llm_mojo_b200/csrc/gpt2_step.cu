@@ -1,0 +1,207 @@
+// One forward or backward micro-step of the bf16 GPT-2 as ONE host call: the launch sequence of models/gpt2.py (reference:
+// train_gpt2.mojo:3050-3848 forward, :3948-5056 backward) issued from native code over the same kernels, buffers and scratch.
+//
+// What it is for: a layer is 7 launches forward and 17 backward, and issuing one from Python (tensor views, pointer reads, a ctypes
+// call) takes 15 - 20 us of host time, more than the kernels of a small batch run: sampling with d12 at 64 positions spent 1.75 ms
+// per token on 0.64 ms of kernels.  From here a launch costs 2 - 3 us: that token takes
+// 0.74 ms (d24 at 776 positions 3.36 -> 2.24), a d6 training step of 2 x 128 tokens 2.75 -> 1.36; steps whose kernels outlast the
+// Python loop (d12 from 4 x 1024 on) keep their time.
+// Nothing is kept between calls: every pointer comes with the call.
+#include "common.cuh"
+using namespace llmb;
+
+// entry points of the other files of this library
+LLMB_API int llmb_encoder_fwd(void* out, const int* tok, const void* wte, const void* wpe, int B, int T, int C, int V, int dtype, cudaStream_t st);
+LLMB_API int llmb_encoder_bwd(float* dwte, float* dwpe, const void* dout, const int* tok, void* scratch, long long scratch_bytes, int B, int T,
+                              int C, int V, int vocab_bits, int dtype, cudaStream_t st);
+LLMB_API int llmb_gelu_fwd(void* out, const void* inp, long long n, int dtype, cudaStream_t st);
+LLMB_API int llmb_dbias(float* dbias, const void* dout, float* scratch, long long scratch_bytes, int rows, int OC, int dtype, cudaStream_t st);
+LLMB_API int llmb_layernorm_fwd(void* out, float* mean, float* rstd, void* resid_out, const void* inp1, const void* inp2, const void* w,
+                                const void* b, int rows, int C, int dtype, cudaStream_t st);
+LLMB_API int llmb_layernorm_bwd(void* dres, float* dw, float* db, float* scratch, long long scratch_bytes, const void* dout, const void* inp,
+                                const void* w, const float* mean, const float* rstd, int rows, int C, int accumulate, int dtype, cudaStream_t st);
+LLMB_API int llmb_gemm(void* D, const void* A, const void* B, const void* bias, void* aux, const float* alpha, int M, int N, int K, long long lda,
+                       long long ldb, long long ldd, long long ldaux, int a_mn, int b_mn, int kind, int a_fmt, int b_fmt, int epi, int splits,
+                       int* status, cudaStream_t st);
+LLMB_API void llmb_gemm_set_colsum(float* colsum);
+LLMB_API int llmb_attention_fwd(void* out, float* lse, const void* qkv, int B, int T, int NH, int* status, cudaStream_t st);
+LLMB_API int llmb_attention_bwd_fused(void* dqkv, float* dbias, float* stats, float* dq_acc, const void* dout, const void* qkv, const void* out,
+                                      const float* lse, int B, int T, int NH, int* status, cudaStream_t st);
+LLMB_API int llmb_fused_classifier(void* logits, float* losses, const int* targets, float dloss, int rows, int V, int Vp, int write_dlogits,
+                                   int dtype, int* status, cudaStream_t st);
+LLMB_API int llmb_ce_pass1(float* stats, const void* tile, const int* targets, int rows, int ld, int col0, int width, int V, int first, int dtype,
+                           cudaStream_t st);
+LLMB_API int llmb_ce_loss(float* losses, const float* stats, int rows, cudaStream_t st);
+LLMB_API int llmb_ce_pass2(void* tile, const float* stats, const int* targets, int rows, int ld, int col0, int width, int V, float dloss, int dtype,
+                           cudaStream_t st);
+
+namespace {
+enum { EPI_NONE = 0, EPI_BIAS = 1, EPI_BIAS_GELU = 2, EPI_DGELU = 3, EPI_ACC_F32 = 4, EPI_BIAS_RESID = 5 };
+
+// acc += scale * sum(x), one CTA: 16-byte loads, eight in flight per thread.  It replaces a sum, a product and an addition (three
+// launches, 9 us of them the sum of 16384 losses on one SM).
+__global__ void __launch_bounds__(1024) loss_accumulate_kernel(float* __restrict__ acc, const float* __restrict__ x, int n, float scale) {
+  pdl_trigger();
+  pdl_wait();
+  __shared__ float red[32];
+  float s[4] = {0.f, 0.f, 0.f, 0.f};
+  const bool vec = (reinterpret_cast<uintptr_t>(x) & 15) == 0;
+  const int nv = vec ? n / 4 : 0;
+  int i = threadIdx.x;
+  for (; i + 7 * 1024 < nv; i += 8 * 1024) {
+    float4 t[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) t[k] = reinterpret_cast<const float4*>(x)[i + k * 1024];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) { s[0] += t[k].x; s[1] += t[k].y; s[2] += t[k].z; s[3] += t[k].w; }
+  }
+  for (; i < nv; i += 1024) { const float4 t = reinterpret_cast<const float4*>(x)[i]; s[0] += t.x; s[1] += t.y; s[2] += t.z; s[3] += t.w; }
+  for (int j = nv * 4 + threadIdx.x; j < n; j += 1024) s[j & 3] += x[j];
+  const float w = warp_sum((s[0] + s[1]) + (s[2] + s[3]));
+  if (threadIdx.x % 32 == 0) red[threadIdx.x / 32] = w;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    const float t = warp_sum(red[threadIdx.x]);
+    if (threadIdx.x == 0) *acc += t * scale;
+  }
+}
+}  // namespace
+
+LLMB_API int llmb_loss_accumulate(float* acc, const float* losses, int n, float scale, cudaStream_t st) {
+  if (n <= 0) return LLMB_ERR_BAD_ARG;
+  return launch_pdl(loss_accumulate_kernel, 1, 1024, 0, st, acc, losses, n, scale);
+}
+
+// Mirrored by ops/step.py.  Pointers are in the order of the enums below; bf16 unless noted.
+enum { P_WTE, P_WPE, P_LN1W, P_LN1B, P_QKVW, P_QKVB, P_ATTW, P_ATTB, P_LN2W, P_LN2B, P_FCW, P_FCB, P_PROJW, P_PROJB, P_LNFW, P_LNFB, P_COUNT };
+enum { A_ENCODED, A_LN1, A_LN1_MEAN, A_LN1_RSTD, A_QKV, A_ATTY, A_LSE, A_RES2, A_LN2, A_LN2_MEAN, A_LN2_RSTD, A_FCH, A_GELU, A_RES3, A_LNF,
+       A_LNF_MEAN, A_LNF_RSTD, A_LOSSES, A_DRES, A_DL, A_DL4, A_LOGITS, A_CE_STATS, A_COUNT };
+struct Gpt2Step {
+  const void* p[P_COUNT];
+  float* g[P_COUNT];             // fp32 gradients (backward only)
+  void* a[A_COUNT];              // means, rstds, lse, losses and ce_stats fp32; A_LOGITS: [rows, Vp], or one vocabulary tile [rows, tile_width]
+  const int* tokens; const int* targets;                      // targets: null = logits only
+  float* loss_acc; int* status;
+  void* s_encoder; float* s_ln; float* s_dbias; float* s_stats; float* s_dq;      // scratch (backward only)
+  long long s_encoder_bytes, s_ln_bytes, s_dbias_bytes;
+  float dloss;
+  int B, T, L, C, NH, V, Vp;
+  int recompute;                 // 1: one GELU buffer for all layers, recomputed in the backward pass
+  int tile_width;                // > 0: LM head in vocabulary tiles of this many columns
+  int fc_colsum;                 // the dGELU GEMM takes the fc bias gradient in its epilogue
+  int splits_qkv, splits_att, splits_fc, splits_proj, splits_head, splits_head_last;   // split-K factors of the weight gradients
+  int vocab_bits;
+  int launches;                  // out: launches issued
+};
+
+namespace {
+struct Step {
+  const Gpt2Step& s; cudaStream_t st; int launches = 0, rc = 0;
+  const int rows, C;
+  Step(const Gpt2Step& s_, cudaStream_t st_) : s(s_), st(st_), rows(s_.B * s_.T), C(s_.C) {}
+
+  const __nv_bfloat16* p(int i, int l, size_t per) const { return reinterpret_cast<const __nv_bfloat16*>(s.p[i]) + l * per; }
+  float* g(int i, int l, size_t per) const { return s.g[i] + l * per; }
+  __nv_bfloat16* a(int i, int l = 0, size_t per = 0) const { return reinterpret_cast<__nv_bfloat16*>(s.a[i]) + l * per; }
+  float* f(int i, int l = 0) const { return reinterpret_cast<float*>(s.a[i]) + l * (size_t)rows; }
+  bool ok(int code, int n = 1) { if (rc == 0) { rc = code; launches += n; } return rc == 0; }
+
+  // D[rows, N] = inp[rows, K] W[N, K]^T with the epilogue
+  bool linear(void* out, const void* inp, const void* w, const void* bias, void* aux, int N, int K, int epi, long long ldd = 0) {
+    return ok(llmb_gemm(out, inp, w, bias, aux, nullptr, rows, N, K, K, K, ldd ? ldd : N, N, 0, 0, 0, 0, 0, epi, 1, s.status, st));
+  }
+  // dinp[rows, K] = dout[rows, N] W[N, K] (times GELU' of aux, or plus aux), then dW[N, K] += dout^T inp
+  bool linear_bwd(void* dinp, float* dw, const void* dout, const void* inp, const void* w, void* aux, int N, int K, int epi, int splits,
+                  float* colsum = nullptr, long long ldo = 0) {
+    const long long lo = ldo ? ldo : N;
+    if (colsum) llmb_gemm_set_colsum(colsum);
+    return ok(llmb_gemm(dinp, dout, w, nullptr, aux, nullptr, rows, K, N, lo, K, K, aux ? K : 0, 0, 1, 0, 0, 0, epi, 1, s.status, st)) &&
+           ok(llmb_gemm(dw, dout, inp, nullptr, nullptr, nullptr, N, K, rows, lo, K, K, 0, 1, 1, 0, 0, 0, EPI_ACC_F32, splits, s.status, st));
+  }
+  bool bias_grad(float* db, const void* dout, int N) { return ok(llmb_dbias(db, dout, s.s_dbias, s.s_dbias_bytes, rows, N, LLMB_BF16, st), 2); }
+  bool ln_bwd(float* dw, float* db, const void* inp, const void* w, const float* mean, const float* rstd, int accumulate) {
+    return ok(llmb_layernorm_bwd(s.a[A_DRES], dw, db, s.s_ln, s.s_ln_bytes, s.a[A_DL], inp, w, mean, rstd, rows, C, accumulate, LLMB_BF16, st), 2);
+  }
+
+  void forward() {
+    const size_t rc1 = (size_t)rows * C, cc = (size_t)C * C, lse = (size_t)s.B * s.NH * s.T;
+    if (!ok(llmb_encoder_fwd(a(A_ENCODED), s.tokens, s.p[P_WTE], s.p[P_WPE], s.B, s.T, C, s.Vp, LLMB_BF16, st))) return;
+    for (int l = 0; l < s.L && !rc; ++l) {
+      void* x = l == 0 ? a(A_ENCODED) : a(A_RES3, l - 1, rc1);
+      void* act = a(A_GELU, s.recompute ? 0 : l, 4 * rc1);
+      ok(llmb_layernorm_fwd(a(A_LN1, l, rc1), f(A_LN1_MEAN, l), f(A_LN1_RSTD, l), nullptr, x, nullptr, p(P_LN1W, l, C), p(P_LN1B, l, C), rows, C, LLMB_BF16, st)) &&
+      linear(a(A_QKV, l, 3 * rc1), a(A_LN1, l, rc1), p(P_QKVW, l, 3 * cc), p(P_QKVB, l, 3 * C), nullptr, 3 * C, C, EPI_BIAS) &&
+      ok(llmb_attention_fwd(a(A_ATTY, l, rc1), reinterpret_cast<float*>(s.a[A_LSE]) + l * lse, a(A_QKV, l, 3 * rc1), s.B, s.T, s.NH, s.status, st)) &&
+      linear(a(A_RES2, l, rc1), a(A_ATTY, l, rc1), p(P_ATTW, l, cc), p(P_ATTB, l, C), x, C, C, EPI_BIAS_RESID) &&
+      ok(llmb_layernorm_fwd(a(A_LN2, l, rc1), f(A_LN2_MEAN, l), f(A_LN2_RSTD, l), nullptr, a(A_RES2, l, rc1), nullptr, p(P_LN2W, l, C), p(P_LN2B, l, C), rows, C, LLMB_BF16, st)) &&
+      linear(act, a(A_LN2, l, rc1), p(P_FCW, l, 4 * cc), p(P_FCB, l, 4 * C), a(A_FCH, l, 4 * rc1), 4 * C, C, EPI_BIAS_GELU) &&
+      linear(a(A_RES3, l, rc1), act, p(P_PROJW, l, 4 * cc), p(P_PROJB, l, C), a(A_RES2, l, rc1), C, 4 * C, EPI_BIAS_RESID);
+    }
+    if (rc || !ok(llmb_layernorm_fwd(a(A_LNF), f(A_LNF_MEAN), f(A_LNF_RSTD), nullptr, a(A_RES3, s.L - 1, rc1), nullptr, s.p[P_LNFW], s.p[P_LNFB], rows, C, LLMB_BF16, st))) return;
+    if (s.tile_width > 0) {
+      for (int c0 = 0; c0 < s.Vp && !rc; c0 += s.tile_width) {
+        const int w = s.Vp - c0 < s.tile_width ? s.Vp - c0 : s.tile_width;
+        linear(a(A_LOGITS), a(A_LNF), p(P_WTE, c0, C), nullptr, nullptr, w, C, EPI_NONE, s.tile_width) &&
+        ok(llmb_ce_pass1(f(A_CE_STATS), a(A_LOGITS), s.targets, rows, s.tile_width, c0, w, s.V, c0 == 0, LLMB_BF16, st));
+      }
+      if (rc || !ok(llmb_ce_loss(f(A_LOSSES), f(A_CE_STATS), rows, st))) return;
+    } else {
+      if (!linear(a(A_LOGITS), a(A_LNF), s.p[P_WTE], nullptr, nullptr, s.Vp, C, EPI_NONE) || !s.targets) return;
+      if (!ok(llmb_fused_classifier(a(A_LOGITS), f(A_LOSSES), s.targets, s.dloss, rows, s.V, s.Vp, 1, LLMB_BF16, s.status, st))) return;
+    }
+    ok(llmb_loss_accumulate(s.loss_acc, f(A_LOSSES), rows, s.dloss, st));
+  }
+
+  void backward() {
+    const size_t rc1 = (size_t)rows * C, cc = (size_t)C * C, lse = (size_t)s.B * s.NH * s.T;
+    void *dres = s.a[A_DRES], *dl = s.a[A_DL], *dl4 = s.a[A_DL4], *dqkv = s.a[A_DL4];
+    if (s.tile_width > 0) {                               // every logits tile again, as dlogits, consumed at once
+      for (int c0 = 0; c0 < s.Vp && !rc; c0 += s.tile_width) {
+        const bool last = s.Vp - c0 <= s.tile_width;
+        const int w = last ? s.Vp - c0 : s.tile_width;
+        linear(a(A_LOGITS), a(A_LNF), p(P_WTE, c0, C), nullptr, nullptr, w, C, EPI_NONE, s.tile_width) &&
+        ok(llmb_ce_pass2(a(A_LOGITS), f(A_CE_STATS), s.targets, rows, s.tile_width, c0, w, s.V, s.dloss, LLMB_BF16, st)) &&
+        linear_bwd(dl, g(P_WTE, c0, C), a(A_LOGITS), a(A_LNF), p(P_WTE, c0, C), c0 ? dl : nullptr, w, C, c0 ? EPI_BIAS_RESID : EPI_NONE,
+                   last ? s.splits_head_last : s.splits_head, nullptr, s.tile_width);
+      }
+    } else {
+      linear_bwd(dl, s.g[P_WTE], a(A_LOGITS), a(A_LNF), s.p[P_WTE], nullptr, s.Vp, C, EPI_NONE, s.splits_head);
+    }
+    if (rc || !ln_bwd(s.g[P_LNFW], s.g[P_LNFB], a(A_RES3, s.L - 1, rc1), s.p[P_LNFW], f(A_LNF_MEAN), f(A_LNF_RSTD), 0)) return;
+    for (int l = s.L - 1; l >= 0 && !rc; --l) {
+      const void* x = l == 0 ? a(A_ENCODED) : a(A_RES3, l - 1, rc1);
+      void* act = a(A_GELU, s.recompute ? 0 : l, 4 * rc1);
+      if (s.recompute && !ok(llmb_gelu_fwd(act, a(A_FCH, l, 4 * rc1), 4 * (long long)rc1, LLMB_BF16, st))) return;
+      float* dfcb = g(P_FCB, l, 4 * C);
+      linear_bwd(dl4, g(P_PROJW, l, 4 * cc), dres, act, p(P_PROJW, l, 4 * cc), a(A_FCH, l, 4 * rc1), C, 4 * C, EPI_DGELU, s.splits_proj,
+                 s.fc_colsum ? dfcb : nullptr) &&
+      (s.fc_colsum || bias_grad(dfcb, dl4, 4 * C)) &&
+      bias_grad(g(P_PROJB, l, C), dres, C) &&
+      linear_bwd(dl, g(P_FCW, l, 4 * cc), dl4, a(A_LN2, l, rc1), p(P_FCW, l, 4 * cc), nullptr, 4 * C, C, EPI_NONE, s.splits_fc) &&
+      ln_bwd(g(P_LN2W, l, C), g(P_LN2B, l, C), a(A_RES2, l, rc1), p(P_LN2W, l, C), f(A_LN2_MEAN, l), f(A_LN2_RSTD, l), 1) &&
+      linear_bwd(dl, g(P_ATTW, l, cc), dres, a(A_ATTY, l, rc1), p(P_ATTW, l, cc), nullptr, C, C, EPI_NONE, s.splits_att) &&
+      bias_grad(g(P_ATTB, l, C), dres, C) &&
+      ok(llmb_attention_bwd_fused(dqkv, g(P_QKVB, l, 3 * C), s.s_stats, s.s_dq, dl, a(A_QKV, l, 3 * rc1), a(A_ATTY, l, rc1),
+                                  reinterpret_cast<float*>(s.a[A_LSE]) + l * lse, s.B, s.T, s.NH, s.status, st), 3) &&
+      linear_bwd(dl, g(P_QKVW, l, 3 * cc), dqkv, a(A_LN1, l, rc1), p(P_QKVW, l, 3 * cc), nullptr, 3 * C, C, EPI_NONE, s.splits_qkv) &&
+      ln_bwd(g(P_LN1W, l, C), g(P_LN1B, l, C), x, p(P_LN1W, l, C), f(A_LN1_MEAN, l), f(A_LN1_RSTD, l), 1);
+    }
+    if (!rc) ok(llmb_encoder_bwd(s.g[P_WTE], s.g[P_WPE], dres, s.tokens, s.s_encoder, s.s_encoder_bytes, s.B, s.T, C, s.Vp, s.vocab_bits, LLMB_BF16, st), 4);
+  }
+};
+}  // namespace
+
+LLMB_API int llmb_gpt2_step_bytes() { return (int)sizeof(Gpt2Step); }
+// Both return 0 or the code of the first entry point that failed; nothing after it is launched.
+LLMB_API int llmb_gpt2_forward(Gpt2Step* s, cudaStream_t st) {
+  Step x(*s, st);
+  x.forward();
+  s->launches = x.launches;
+  return x.rc;
+}
+LLMB_API int llmb_gpt2_backward(Gpt2Step* s, cudaStream_t st) {
+  Step x(*s, st);
+  x.backward();
+  s->launches = x.launches;
+  return x.rc;
+}

@@ -22,6 +22,7 @@ from typing import Dict, List, Optional, Tuple
 import torch
 
 from .. import ops
+from ..ops import step
 from ..config import (GPT2Config, INIT_RNG_SEED, INIT_WEIGHT_STD, PARAM_NAMES, Precision,
                       is_model_descriptor, parse_model_descriptor)
 from ..utils import checkpointing as ckpt
@@ -356,6 +357,11 @@ class GPT2:
             self.targets_dev.copy_(targets.view(B, T), non_blocking=True)
         if on_inputs_copied is not None:      # the host buffers may be reused once these two copies have run
             on_inputs_copied()
+        self._dloss = dloss = 1.0 / (B * T * grad_accum_steps)
+        if "logits" not in a and not (targets is not None and (self.lm_head_chunks > 1 or self.vocab_parallel)):
+            a["logits"] = torch.empty(B, T, cfg.padded_vocab_size, dtype=self.dtype, device=self.device)
+        if step.usable(self):
+            return step.forward(self, targets is not None)
         z = self.zero
         if z is not None:
             z.before_embedding()
@@ -380,8 +386,6 @@ class GPT2:
         if self._fused_gather is not None:
             self._fused_gather.wait_released()          # peers have finished reading the previous lnf rows
         ops.layernorm_fwd(a["lnf"], a["lnf_mean"], a["lnf_rstd"], a["residual3"][L - 1], p["lnfw"], p["lnfb"])
-        dloss = 1.0 / (B * T * grad_accum_steps)
-        self._dloss = dloss
         if self.vocab_parallel and targets is not None:
             self._vocab_parallel_forward(p, dloss)
             return
@@ -392,14 +396,12 @@ class GPT2:
                 ops.matmul_fwd(tile, a["lnf"], p["wte"][c0:c0 + w])
                 ops.chunked_ce_pass1(a["ce_stats"], tile, self.targets_dev, c0, w, V, k == 0)
             ops.chunked_ce_loss(a["losses"], a["ce_stats"])
-            self.loss_acc += a["losses"].sum() * dloss
+            ops.loss_accumulate(self.loss_acc, a["losses"], dloss)
             return
-        if "logits" not in a:
-            a["logits"] = torch.empty(B, T, cfg.padded_vocab_size, dtype=self.dtype, device=self.device)
         ops.matmul_fwd(a["logits"], a["lnf"], p["wte"])
         if targets is not None:
             ops.fused_classifier(a["logits"], a["losses"], self.targets_dev, dloss, V)
-            self.loss_acc += a["losses"].sum() * dloss
+            ops.loss_accumulate(self.loss_acc, a["losses"], dloss)
 
     def read_loss(self) -> float:
         """Synchronising read of the accumulated mean loss; resets the accumulator."""
@@ -422,6 +424,10 @@ class GPT2:
             last_micro_step = micro_step == grad_accum_steps - 1
         if micro_step == 0:
             self.zero_gradients()
+        if step.usable(self):
+            step.backward(self)
+            self.micro_steps_done += 1
+            return
         cfg, a = self.config, self.acts
         L, NH = cfg.num_layer, cfg.num_heads
         z = self.zero

@@ -13,6 +13,7 @@ adamw → ``adamw_update``; global_norm → ``global_norm_squared``.
 """
 from __future__ import annotations
 
+import functools
 import math
 import os
 from typing import Optional
@@ -264,6 +265,7 @@ def _tc_kind(t: torch.Tensor):
     return None
 
 
+@functools.lru_cache(maxsize=None)
 def _splits_for(M: int, N: int, K: int, *, tile: int = 256, tile_n: int = 0, bk: int = 64, units: int = 74) -> int:
     """Split-K factor for the dW GEMMs (by default 256x256 tiles on 74 CTA pairs, 64 values of K per stage; the
     block-scaled kernels have 128x256 tiles on 148 CTAs): the number of splits that minimises waves x (k-blocks per
@@ -534,6 +536,15 @@ def chunked_ce_pass2(tile, stats, targets, col0: int, width: int, vocab_size: in
     cols = torch.arange(width, device=tile.device) + col0
     p[:, cols >= vocab_size] = 0.0
     tile[:, :width] = (p * dloss).to(tile.dtype)
+
+
+def loss_accumulate(acc: torch.Tensor, losses: torch.Tensor, scale: float) -> None:
+    """acc[0] += scale · Σ losses: the micro-step's share of the mean loss, kept on the device."""
+    if losses.is_cuda:
+        check(lib().llmb_loss_accumulate(ptr(acc), ptr(losses), losses.numel(), float(scale), stream()), "loss_accumulate")
+        _count()
+    else:
+        acc += losses.sum() * scale
 
 
 def softmax_rows(logits2d: torch.Tensor, vocab_size: int, temperature: float = 1.0) -> torch.Tensor:

@@ -24,13 +24,13 @@ using namespace llmb;
 
 namespace {
 // ------------------------------------------------------------------ Squares RNG
-__device__ __forceinline__ uint64_t splitmix64(uint64_t x) {
+__host__ __device__ __forceinline__ uint64_t splitmix64(uint64_t x) {
   x += 0x9E3779B97F4A7C15ull;
   x = (x ^ (x >> 30)) * 0xBF58476D1CE4E5B9ull;
   x = (x ^ (x >> 27)) * 0x94D049BB133111EBull;
   return x ^ (x >> 31);
 }
-__device__ __forceinline__ uint64_t rng_key(uint64_t seed, uint64_t stream) { return splitmix64(seed ^ splitmix64(stream)) | 1ull; }
+__host__ __device__ __forceinline__ uint64_t rng_key(uint64_t seed, uint64_t stream) { return splitmix64(seed ^ splitmix64(stream)) | 1ull; }
 __device__ __forceinline__ uint32_t squares32(uint64_t ctr, uint64_t key) {
   uint64_t x = ctr * key, y = x, z = y + key;
   x = x * x + y; x = (x >> 32) | (x << 32);
@@ -638,6 +638,286 @@ LLMB_API int llmb_nvfp4_tensor_scale(float* ts, const float* amax, cudaStream_t 
 // 1 x 128 blocks along `axis` (activations, gradients) or 128 x 128 blocks (weights).  Power-of-two scales make
 // value x scale exactly representable in bf16, so the block-scaled product can run on the bf16 tensor path with
 // the numerics of a block-scaled FP8 GEMM.
+namespace {
+
+// ------------------------------------------------------------------ NVFP4 operands of the linear layers
+// What one operand needs, in two launches: max|x| (of the values, of their 16-point transform along the rows, or both, from one read),
+// then both orientations from one read: q0 / sf0 = blocks along the columns, bytes [rows, cols / 2] (a product contracted over the
+// columns), q1 / sf1 = blocks along the rows, bytes transposed [cols, rows / 2] (contracted over the rows).  Values, scales, random
+// draws and rounding are those of llmb_amax(_rht) + nvfp4_tensor_scale_kernel + llmb_nvfp4_quantize.
+// What bounded those: a thread per block of 16 x 1 wrote the transposed bytes 8 at a time at a stride of rows / 2 and the scales one
+// byte at a time, every orientation read x twice, and the scale factors took a memset and two one-thread kernels per product.  Here a
+// CTA takes a 128 x 128 tile through shared memory (bytes and scale atoms leave as whole 64-byte lines and 16-byte vectors), the
+// maxima go to per-CTA slots that every CTA of the second kernel reduces for itself, and that kernel also writes the product's factor.
+// Measured on a d48 training step (B 4, T 1024, 44 layers with NVFP4 MLPs): 67.0 -> 62.5 ms, 4375 -> 2261 launches.
+constexpr int NVA_GRID = 592;                            // slots of partial maxima (four CTAs per SM)
+constexpr int NVT_PITCH = 272, NVT_OUT_PITCH = 72;       // bytes: 16-byte (8-byte) accesses at a stride of one row are free of bank conflicts
+
+inline int nvfp4_amax_grid(int rows, int cols) {         // 16 rows x 4 columns per thread and step
+  const long long want = ceil_div_ll((long long)ceil_div(rows, 16) * (cols / 4), 256);
+  return (int)(want < NVA_GRID ? want : NVA_GRID);
+}
+// The randomised 16-point transform of two columns at once (packed fp32x2; the additions of fwht16 in the same order)
+__device__ __forceinline__ void rht16x2(float2 (&b)[16]) {
+  const float2 neg = make_float2(-1.f, -1.f);
+#pragma unroll
+  for (int k = 0; k < 16; ++k)
+    if (hadamard_sign(k) < 0.f) b[k] = make_float2(-b[k].x, -b[k].y);
+#pragma unroll
+  for (int s = 0; s < 4; ++s) {
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {                         // the eight pairs of stage s: j and j + 2^s
+      const int j = ((e >> s) << (s + 1)) | (e & ((1 << s) - 1)), h = 1 << s;
+      const float2 x = b[j], y = b[j + h];
+      b[j] = __fadd2_rn(x, y); b[j + h] = __ffma2_rn(y, neg, x);
+    }
+  }
+}
+__device__ __forceinline__ float2 bf16x2_f(uint32_t u) { return make_float2(__uint_as_float(u << 16), __uint_as_float(u & 0xffff0000u)); }
+__device__ __forceinline__ unsigned block_umax(unsigned m, unsigned* red) {      // 256 threads; every thread gets the maximum
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+  if (threadIdx.x % 32 == 0) red[threadIdx.x / 32] = m;
+  __syncthreads();
+  m = red[0];
+#pragma unroll
+  for (int w = 1; w < 8; ++w) m = max(m, red[w]);
+  __syncthreads();
+  return m;
+}
+
+// partial[0 .. gridDim): raw bits of max|x| (NaN sorts above infinity); partial[NVA_GRID .. +gridDim): of the transform along the rows
+template <bool PLAIN, bool RHT>
+__global__ void __launch_bounds__(256) nvfp4_amax_kernel(unsigned* __restrict__ partial, const __nv_bfloat16* __restrict__ x, int rows, int cols) {
+  pdl_trigger();
+  pdl_wait();
+  __shared__ unsigned red[8];
+  unsigned m0 = 0, m1 = 0;
+  const int c4 = cols / 4;
+  const long long n = (long long)ceil_div(rows, 16) * c4;
+  for (long long i = (long long)blockIdx.x * 256 + threadIdx.x; i < n; i += (long long)gridDim.x * 256) {
+    const int rb = (int)(i / c4), c = (int)(i % c4) * 4;
+    const __nv_bfloat16* p = x + (long long)rb * 16 * cols + c;
+    uint2 u[16];
+#pragma unroll
+    for (int k = 0; k < 16; ++k) u[k] = rb * 16 + k < rows ? *reinterpret_cast<const uint2*>(p + (long long)k * cols) : make_uint2(0u, 0u);
+    if (PLAIN) {
+#pragma unroll
+      for (int k = 0; k < 16; ++k) {                      // 16-bit magnitudes order like the values
+        const uint32_t a = u[k].x & 0x7fff7fffu, b = u[k].y & 0x7fff7fffu;
+        const uint32_t t = __vmaxu2(a, b);
+        m0 = __vmaxu2(m0, t);
+      }
+    }
+    if (RHT) {
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        float2 b[16];
+#pragma unroll
+        for (int k = 0; k < 16; ++k) b[k] = bf16x2_f(half ? u[k].y : u[k].x);
+        rht16x2(b);
+#pragma unroll
+        for (int k = 0; k < 16; ++k) m1 = max(m1, max(__float_as_uint(b[k].x) & 0x7fffffffu, __float_as_uint(b[k].y) & 0x7fffffffu));
+      }
+    }
+  }
+  if (PLAIN) { const unsigned m = block_umax(max(m0 & 0xffffu, m0 >> 16) << 16, red); if (threadIdx.x == 0) partial[blockIdx.x] = m; }
+  if (RHT) { const unsigned m = block_umax(m1, red); if (threadIdx.x == 0) partial[NVA_GRID + blockIdx.x] = m; }
+}
+
+struct NvAlpha { float* out; const float* other; float factor; };       // *out = factor * this operand's tensor scale * *other
+struct NvTile {
+  uint8_t *q0, *sf0, *q1, *sf1;
+  const __nv_bfloat16* x;
+  float* ts;                                              // [2]: tensor scales of the two orientations
+  const unsigned* partial; int nparts;
+  int rows, cols;
+  unsigned long long key0, key1; long long step;          // stochastic rounding (0: nearest); the keys are odd
+  NvAlpha alpha0, alpha1;
+};
+__device__ __forceinline__ float nvfp4_ts(unsigned bits) {
+  const float a = __uint_as_float(bits);
+  return (a > 0.f && !isnan(a) && !isinf(a)) ? a / (448.0f * 6.0f) : 1.0f;
+}
+__device__ __forceinline__ uint8_t nvfp4_block_scale(float amax, float ts, float& inv) {
+  const float raw = (amax <= 0.f || ts <= 0.f) ? 1.0f : (amax / 6.0f) / ts;
+  const uint8_t code = encode_e4m3(raw);
+  float val = decode_e4m3(code) * ts;
+  if (val <= 0.f) val = 1.0f;
+  inv = 1.0f / val;
+  return code;
+}
+// sixteen values to e2m1, the first in the lowest nibble; ctr counts the first value (one 64-bit draw per eight)
+__device__ __forceinline__ uint2 nvfp4_pack16(const float (&v)[16], float inv, unsigned long long ctr, unsigned long long key) {
+  uint2 o;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const float* s = v + 8 * h;
+    uint32_t lo, hi;
+    if (key) {
+      const uint64_t r = squares64(ctr + 8 * h, key);
+      lo = e2m1x4_rs(s[0] * inv, s[1] * inv, s[2] * inv, s[3] * inv, (uint32_t)r);
+      hi = e2m1x4_rs(s[4] * inv, s[5] * inv, s[6] * inv, s[7] * inv, (uint32_t)(r >> 32));
+    } else {
+      lo = e2m1x2_rn(s[0] * inv, s[1] * inv) | (e2m1x2_rn(s[2] * inv, s[3] * inv) << 8);
+      hi = e2m1x2_rn(s[4] * inv, s[5] * inv) | (e2m1x2_rn(s[6] * inv, s[7] * inv) << 8);
+    }
+    (h ? o.y : o.x) = (lo & 0xffffu) | (hi << 16);
+  }
+  return o;
+}
+
+// ROW / COL: which orientations; B16: 16 x 16 blocks (weights) instead of 16 x 1; RHT: transform the row blocks (COL).
+template <bool ROW, bool COL, bool B16, bool RHT>
+__global__ void __launch_bounds__(256) nvfp4_tile_kernel(const NvTile p) {
+  __shared__ __align__(16) unsigned char xs[128 * NVT_PITCH];
+  __shared__ __align__(16) unsigned char qs[128 * NVT_OUT_PITCH];
+  __shared__ __align__(16) unsigned char ss[1024];        // two scale atoms of 128 lines x 4 blocks
+  __shared__ unsigned red[8];
+  pdl_trigger();
+  pdl_wait();
+  const int tiles_c = ceil_div(p.cols, 128);
+  const int tr = blockIdx.x / tiles_c, tc = blockIdx.x % tiles_c, r0 = tr * 128, c0 = tc * 128;
+  const int t = threadIdx.x, lane = t % 32, w = t / 32;
+  {
+    uint4 u[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int id = t + i * 256, r = r0 + id / 16, c = c0 + (id % 16) * 8;
+      u[i] = r < p.rows && c < p.cols ? *reinterpret_cast<const uint4*>(p.x + (long long)r * p.cols + c) : make_uint4(0u, 0u, 0u, 0u);
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) { const int id = t + i * 256; *reinterpret_cast<uint4*>(xs + (id / 16) * NVT_PITCH + (id % 16) * 16) = u[i]; }
+  }
+  float ts0 = 1.f, ts1 = 1.f;
+  {
+    const bool plain = ROW || !RHT;
+    unsigned m0 = 0, m1 = 0;
+    for (int i = t; i < p.nparts; i += 256) {
+      if (plain) m0 = max(m0, p.partial[i]);
+      if (COL && RHT) m1 = max(m1, p.partial[NVA_GRID + i]);
+    }
+    if (plain) ts0 = ts1 = nvfp4_ts(block_umax(m0, red));            // (the barriers in here also order the tile's stores)
+    if (COL && RHT) ts1 = nvfp4_ts(block_umax(m1, red));
+  }
+  if (blockIdx.x == 0 && t == 0) {
+    if (ROW) p.ts[0] = ts0;
+    if (COL) p.ts[1] = ts1;
+    if (ROW && p.alpha0.out) *p.alpha0.out = ts0 * *p.alpha0.other * p.alpha0.factor;
+    if (COL && p.alpha1.out) *p.alpha1.out = ts1 * *p.alpha1.other * p.alpha1.factor;
+  }
+
+  // lines of 64 bytes in `qs` (one per line of the orientation: `n` of them, `len` bytes each) and the atoms in `ss` to memory
+  auto flush = [&](uint8_t* q, uint8_t* sf, int line0, int n, long long pitch, long long off, int len, long long atom0, int atoms) {
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int id = t + i * 256, l = id / 8, b = (id % 8) * 8;
+      if (l < n && b < len) *reinterpret_cast<uint2*>(q + (long long)(line0 + l) * pitch + off + b) = *reinterpret_cast<const uint2*>(qs + l * NVT_OUT_PITCH + b);
+    }
+    if (t < 32 * atoms) *reinterpret_cast<uint4*>(sf + atom0 * 512 + t * 16) = *reinterpret_cast<const uint4*>(ss + t * 16);
+  };
+
+  if (ROW) {
+    const int kb = w, kblocks = p.cols / 16;              // warp w: block w of the 128 columns; lane: row
+    const bool kv = c0 + kb * 16 < p.cols;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int r = i * 32 + lane;
+      const unsigned char* src = xs + r * NVT_PITCH + kb * 32;
+      const uint4 a = *reinterpret_cast<const uint4*>(src), b = *reinterpret_cast<const uint4*>(src + 16);
+      const uint32_t uu[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+      float v[16], amax = 0.f;
+#pragma unroll
+      for (int k = 0; k < 8; ++k) { const float2 f = bf16x2_f(uu[k]); v[2 * k] = f.x; v[2 * k + 1] = f.y; }
+#pragma unroll
+      for (int k = 0; k < 16; ++k) amax = fmaxf(amax, fabsf(v[k]));
+      if (B16) {
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o, 16));
+      }
+      float inv;
+      const uint8_t code = nvfp4_block_scale(amax, ts0, inv);
+      const unsigned long long ctr = ((unsigned long long)p.step << 32) | ((unsigned long long)(r0 + r) * p.cols + c0 + kb * 16);
+      *reinterpret_cast<uint2*>(qs + r * NVT_OUT_PITCH + kb * 8) = nvfp4_pack16(v, inv, ctr, p.key0);
+      ss[(kb / 4) * 512 + lane * 16 + i * 4 + (kb & 3)] = kv && r0 + r < p.rows ? code : 0;
+    }
+    const int atoms_k = ceil_div(kblocks, 4);
+    flush(p.q0, p.sf0, r0, min(128, p.rows - r0), p.cols / 2, c0 / 2, min(64, (p.cols - c0) / 2), (long long)tr * atoms_k + tc * 2, min(2, atoms_k - tc * 2));
+  }
+  if (COL) {
+    if (ROW) __syncthreads();
+    const int rb = w, kblocks = p.rows / 16;              // warp w: block w of the 128 rows; lane: two adjacent columns
+    const bool kv = r0 + rb * 16 < p.rows;
+#pragma unroll 1
+    for (int i = 0; i < 2; ++i) {
+      const int c = (i * 32 + lane) * 2;
+      float2 b[16];
+#pragma unroll
+      for (int k = 0; k < 16; ++k) b[k] = bf16x2_f(*reinterpret_cast<const uint32_t*>(xs + (rb * 16 + k) * NVT_PITCH + c * 2));
+      if (RHT) rht16x2(b);
+      float ax = 0.f, ay = 0.f;
+#pragma unroll
+      for (int k = 0; k < 16; ++k) { ax = fmaxf(ax, fabsf(b[k].x)); ay = fmaxf(ay, fabsf(b[k].y)); }
+      if (B16) {
+        ax = fmaxf(ax, ay);
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) ax = fmaxf(ax, __shfl_xor_sync(0xffffffffu, ax, o, 8));
+        ay = ax;
+      }
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        float v[16], inv;
+#pragma unroll
+        for (int k = 0; k < 16; ++k) v[k] = h ? b[k].y : b[k].x;
+        const uint8_t code = nvfp4_block_scale(h ? ay : ax, ts1, inv);
+        const int cc = c + h;
+        const unsigned long long ctr = ((unsigned long long)p.step << 32) | ((unsigned long long)(c0 + cc) * p.rows + r0 + rb * 16);
+        *reinterpret_cast<uint2*>(qs + cc * NVT_OUT_PITCH + rb * 8) = nvfp4_pack16(v, inv, ctr, p.key1);
+        ss[(rb / 4) * 512 + (cc % 32) * 16 + (cc / 32) * 4 + (rb & 3)] = kv && c0 + cc < p.cols ? code : 0;
+      }
+    }
+    const int atoms_k = ceil_div(kblocks, 4);
+    flush(p.q1, p.sf1, c0, min(128, p.cols - c0), p.rows / 2, r0 / 2, min(64, (p.rows - r0) / 2), (long long)tc * atoms_k + tr * 2, min(2, atoms_k - tr * 2));
+  }
+}
+}  // namespace
+
+// One NVFP4 operand of a linear layer (see above).  x: contiguous bf16 [rows, cols], 16-byte aligned, cols % 16 == 0, and rows % 16 == 0
+// where q1 is wanted or block16 is set.  q0 / sf0 and q1 / sf1: 16-byte aligned, either pair may be null.  block16: 16 x 16 blocks (no
+// transform, nearest rounding).  rht: transform the row blocks of q1.  ws: llmb_nvfp4_operand_ws_floats() floats; on return ws[0] and
+// ws[1] are the tensor scales of q0 and q1 and, with alpha_other0 / 1 (another operand's tensor scale), ws[2] and ws[3] =
+// factor * tensor scale * *alpha_other: the factor of the product of the two operands.
+LLMB_API int llmb_nvfp4_operand_ws_floats() { return 4 + 2 * NVA_GRID; }
+LLMB_API int llmb_nvfp4_operand(void* q0, void* sf0, void* q1, void* sf1, float* ws, const void* x, int rows, int cols, int block16, int rht,
+                                int sr, unsigned long long seed, unsigned long long stream0, unsigned long long stream1, long long step,
+                                const float* alpha_other0, float factor0, const float* alpha_other1, float factor1, cudaStream_t st) {
+  const bool row = q0 && sf0, col = q1 && sf1;
+  if (rows <= 0 || cols <= 0 || !(row || col) || cols % 16 || ((col || block16) && rows % 16) || (block16 && (sr || rht))) return LLMB_ERR_BAD_ARG;
+  if ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(q0) | reinterpret_cast<uintptr_t>(sf0) | reinterpret_cast<uintptr_t>(q1) |
+       reinterpret_cast<uintptr_t>(sf1)) & 15) return LLMB_ERR_BAD_ARG;
+  const bool tr = col && rht, plain = row || !tr;
+  NvTile p{};
+  p.q0 = (uint8_t*)q0; p.sf0 = (uint8_t*)sf0; p.q1 = (uint8_t*)q1; p.sf1 = (uint8_t*)sf1;
+  p.x = (const __nv_bfloat16*)x; p.ts = ws; p.partial = reinterpret_cast<unsigned*>(ws + 4); p.nparts = nvfp4_amax_grid(rows, cols);
+  p.rows = rows; p.cols = cols; p.step = step;
+  p.key0 = sr ? rng_key(seed, stream0) : 0ull;
+  p.key1 = sr ? rng_key(seed, stream1) : 0ull;
+  p.alpha0 = {alpha_other0 ? ws + 2 : nullptr, alpha_other0, factor0};
+  p.alpha1 = {alpha_other1 ? ws + 3 : nullptr, alpha_other1, factor1};
+  unsigned* part = reinterpret_cast<unsigned*>(ws + 4);
+  int rc = plain && tr ? launch_pdl(nvfp4_amax_kernel<true, true>, p.nparts, 256, 0, st, part, p.x, rows, cols)
+           : plain     ? launch_pdl(nvfp4_amax_kernel<true, false>, p.nparts, 256, 0, st, part, p.x, rows, cols)
+                       : launch_pdl(nvfp4_amax_kernel<false, true>, p.nparts, 256, 0, st, part, p.x, rows, cols);
+  if (rc) return rc;
+  const long long tiles = (long long)ceil_div(rows, 128) * ceil_div(cols, 128);
+  if (tiles > 0x7fffffffLL) return LLMB_ERR_BAD_ARG;
+#define NVT(R, C, B, H) launch_pdl(nvfp4_tile_kernel<R, C, B, H>, (unsigned)tiles, 256, 0, st, p)
+  if (block16) return row && col ? NVT(true, true, true, false) : row ? NVT(true, false, true, false) : NVT(false, true, true, false);
+  if (tr) return row ? NVT(true, true, false, true) : NVT(false, true, false, true);
+  return row && col ? NVT(true, true, false, false) : row ? NVT(true, false, false, false) : NVT(false, true, false, false);
+#undef NVT
+}
 namespace {
 __device__ __forceinline__ float pow2_scale(float amax, float fmt_max) {
   if (!(amax > 0.f) || isinf(amax)) return 1.0f;

@@ -73,6 +73,8 @@ _SIGS = {
     "llmb_nvfp4_scale_bytes": [c_ll, c_ll, c_int],
     "llmb_nvfp4_quantize": [c_p, c_p, c_p, c_p, c_p, c_int, c_int, c_int, c_int, c_int, c_int, c_ull, c_ull, c_ll, c_int,
                             c_int, c_p],
+    "llmb_nvfp4_operand_ws_floats": [],
+    "llmb_nvfp4_operand": [c_p, c_p, c_p, c_p, c_p, c_p, c_int, c_int, c_int, c_int, c_int, c_ull, c_ull, c_ull, c_ll, c_p, c_f, c_p, c_f, c_p],
     "llmb_nvfp4_dequantize": [c_p, c_p, c_p, c_p, c_int, c_int, c_int, c_p],
     "llmb_hadamard16": [c_p, c_p, c_ll, c_int, c_int, c_p],
     "llmb_rng_uniform": [c_p, c_ll, c_ull, c_ull, c_ull, c_p],

@@ -16,6 +16,7 @@ throughput is that of the bf16 tensor path.  CPU tensors run an emulation of the
 """
 from __future__ import annotations
 
+import functools
 import math
 import os
 from typing import Dict, Optional, Tuple
@@ -24,7 +25,7 @@ import torch
 
 from . import (EPI_ACC_F32, EPI_BIAS, EPI_BIAS_GELU, EPI_BIAS_RESID, EPI_DGELU, EPI_NONE, _count, _gelu_grad_t, _gelu_t,
                _splits_for, dbias_reduce, gemm, gemm_mxfp8, gemm_nvfp4, scratch)
-from ._lib import check, dtype_code, lib, ptr, stream
+from ._lib import check, dtype_code, lib, ptr, status_word, stream
 from . import matmul_fwd as ops_matmul_fwd, matmul_bwd as ops_matmul_bwd
 
 E4M3, E5M2 = 0, 1
@@ -463,12 +464,63 @@ def _qp(x, axis, block_rows, **kw):
     return q, sc, ts
 
 
+class Fp4Operand:
+    """A bf16 matrix [rows, cols] as the NVFP4 operand of one or two products, in one buffer: packed bytes and scale atoms of the
+    blocks along the columns (``q0``, ``sf0``) and / or of the blocks along the rows, transposed (``q1``, ``sf1``); their tensor scales
+    ``ts0``, ``ts1``; and the factors ``alpha0`` / ``alpha1`` of the products with ``other`` (addresses; GPU only, two launches)."""
+
+    def __init__(self, x, row: bool, col: bool, *, block16=False, rht=False, sr=False, seed=0, streams=(0, 0), step=0, other0=None,
+                 other1=None, factor1: float = 1.0):
+        rows, cols = x.shape
+        up = lambda n: -(-n // 16) * 16
+        nq, n0, n1 = up(rows * cols // 2), -(-rows // 128) * -(-cols // 64) * 512, -(-cols // 128) * -(-rows // 64) * 512
+        ws = 4 * _ws_floats()
+        self.buf = torch.empty(ws + row * (nq + n0) + col * (nq + n1), dtype=torch.uint8, device=x.device)
+        base = self.buf.data_ptr()
+        self.ts0, self.ts1, self.alpha0, self.alpha1 = base, base + 4, base + 8, base + 12
+        at = base + ws
+        self.q0 = self.sf0 = self.q1 = self.sf1 = None
+        if row:
+            self.q0, self.sf0, at = at, at + nq, at + nq + n0
+        if col:
+            self.q1, self.sf1 = at, at + nq
+        check(lib().llmb_nvfp4_operand(self.q0, self.sf0, self.q1, self.sf1, base, ptr(x), rows, cols, int(block16), int(rht), int(sr), seed,
+                                       streams[0], streams[1], step, other0, 1.0, other1, factor1, stream()), "nvfp4_operand")
+        _count(2)
+
+
+@functools.lru_cache(maxsize=None)
+def _ws_floats() -> int:
+    return -(-lib().llmb_nvfp4_operand_ws_floats() // 4) * 4
+
+
+def _fp4_tiled(*tensors) -> bool:
+    """Matrices that ``Fp4Operand`` takes: contiguous bf16, 16-byte aligned, whole 16 x 16 blocks; others are quantised by
+    ``nvfp4_fake_quant`` (any strides and types)."""
+    return all(t.is_cuda and t.dtype == torch.bfloat16 and t.is_contiguous() and t.shape[0] % 16 == 0 and t.shape[1] % 16 == 0
+               and t.data_ptr() % 16 == 0 for t in tensors)
+
+
+def _gemm_fp4(D, qa, sfa, qb, sfb, K, alpha, *, epi, bias=None, aux=None, splits=1) -> None:
+    M, N = D.shape
+    check(lib().llmb_gemm_nvfp4(ptr(D), qa, qb, sfa, sfb, ptr(bias), ptr(aux), alpha, M, N, K, D.stride(0),
+                                aux.stride(0) if aux is not None else 0, epi, splits, ptr(status_word(D.device)), stream()), "gemm_nvfp4")
+    _count()
+
+
 def matmul_fwd_fp4(out, inp, weight, bias, *, pre_gelu=None, residual=None) -> None:
     """NVFP4 forward: activations 1x16 blocks, weights 16x16 blocks, RNE (``llmm/matmul.mojo:2038-2138``)."""
     OC, C = weight.shape
     rows = inp.numel() // C
     x = inp.reshape(rows, C)
     o = out.view(rows, OC)
+    if out.is_cuda and nvfp4_native(C) and _fp4_tiled(x, weight):
+        qx = Fp4Operand(x, True, False)
+        qw = Fp4Operand(weight, True, False, block16=True, other0=qx.ts0)
+        epi, aux = (EPI_BIAS_GELU, pre_gelu) if pre_gelu is not None else (EPI_BIAS_RESID, residual) if residual is not None else \
+            (EPI_BIAS if bias is not None else EPI_NONE, None)
+        _gemm_fp4(o, qx.q0, qx.sf0, qw.q0, qw.sf0, C, qw.alpha0, epi=epi, bias=bias, aux=aux.view(rows, OC) if aux is not None else None)
+        return
     if out.is_cuda and nvfp4_native(C):
         qx, sx, tsx = _qp(x, 1, 1)
         qw, sw, tsw = _qp(weight, 1, 16)
@@ -502,6 +554,19 @@ def matmul_bwd_fp4(dinp, dweight, dbias, dout, inp, weight, *, gelu_pre=None, rh
     OC, C = weight.shape
     rows = inp.numel() // C
     d, x = dout.reshape(rows, OC), inp.reshape(rows, C)
+    if dout.is_cuda and nvfp4_native(OC, rows) and _fp4_tiled(d, x, weight):
+        # both orientations of the output gradient from one read; the operands contracted over the rows are written transposed
+        qd = Fp4Operand(d, dinp is not None, True, rht=rht, sr=sr, seed=seed, streams=(NVFP4_SR_STREAM + 2, NVFP4_SR_STREAM + 3), step=step)
+        if dinp is not None:
+            qw = Fp4Operand(weight, False, True, block16=True, other1=qd.ts0)
+            _gemm_fp4(dinp.view(rows, C), qd.q0, qd.sf0, qw.q1, qw.sf1, OC, qw.alpha1, epi=EPI_DGELU if gelu_pre is not None else EPI_NONE,
+                      aux=gelu_pre.view(rows, C) if gelu_pre is not None else None)
+        qx = Fp4Operand(x, False, True, rht=rht, other1=qd.ts1, factor1=(1.0 / 16.0) if rht else 1.0)
+        _gemm_fp4(dweight.view(OC, C), qd.q1, qd.sf1, qx.q1, qx.sf1, rows, qx.alpha1, epi=EPI_ACC_F32,
+                  splits=_splits_for(OC, C, rows, tile=128, tile_n=256, bk=256, units=148))
+        if dbias is not None:
+            dbias_reduce(dbias, d)
+        return
     if dout.is_cuda and nvfp4_native(OC, rows):
         # the packed operand of a product contracted over axis 0 is written transposed ([cols, rows/2]), so all three
         # products are K-major x K-major on the block-scaled tensor path

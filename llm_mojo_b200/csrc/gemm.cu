@@ -69,7 +69,6 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
   if (p.g.W <= 1 && p.pull.nseg == 0 && p.pull.nwait == 0) pdl_trigger();   // else this kernel waits for other GPUs or streams
-  pdl_wait();
 
   const int m_tiles = ceil_div(p.M, 2 * BM);            // cluster tiles of 256 rows
   const int tiles_per_split = m_tiles * p.n_tiles;
@@ -88,6 +87,20 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     kb0 = split * p.kb_per_split;
     kb1 = min(p.kb_total, kb0 + p.kb_per_split);
   };
+
+  // While the kernel before this one drains: the first ring of B (a forward or input-gradient GEMM's weights) into L2, once per column
+  // of tiles.  A hint only, so it may run before the wait; if that kernel writes B, the loads below still read what it wrote.
+  if (warp == 0 && cluster_id < total_units && p.pull.nwait == 0) {
+    int m_blk, n_blk, kb0, kb1; unit_coords(cluster_id, m_blk, n_blk, kb0, kb1);
+    const int n0 = n_blk * BN + (int)cta * 128;
+    if (m_blk % BAND2 == 0 && elect_one())
+      for (int kb = kb0; kb < kb1 && kb < kb0 + NST; ++kb) {
+        if (!p.b_mn) tma_prefetch_l2_2d(&tmB, kb * p.bke, n0);
+        else if (p.b_3d) tma_prefetch_l2_3d(&tmB, 0, kb * p.bke, n0 / p.bke);
+      }
+    __syncwarp();
+  }
+  pdl_wait();
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer (both CTAs)
@@ -441,7 +454,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       // nothing of this CTA's shared memory may still be a source or a destination of a copy at exit
       for (int ls = 0; ls < 2; ++ls)
         if (aux_pending & (1u << ls)) (void)mbar_wait(&abar[ls], (aux_phase >> ls) & 1);
-      if (lane == 0) bulk_wait<0>();
+      if (lane == 0) bulk_wait_read<0>();
       __syncwarp();
     }
   }
@@ -907,7 +920,7 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       if (lane == 0) mbar_arrive(&tempty_bar[acc]);
     }
     if (tma_epi) {                                        // no copy may still read this CTA's shared memory at exit
-      if (lane == 0) bulk_wait<0>();
+      if (lane == 0) bulk_wait_read<0>();
       __syncwarp();
     }
   }

@@ -71,6 +71,16 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
   pdl_trigger();
+  // While the kernel before this one drains: B (weights, as a rule) into L2.  A hint only, so it may run before the wait; if that kernel
+  // writes B, the loads below still read what it wrote.
+  if (warp == 0 && m_blk == 0 && elect_one()) {
+    for (int kb = kb0; kb < kb1 && kb < kb0 + 16; ++kb) {
+      const int k0 = kb * p.bke;
+      if (!p.b_mn) tma_prefetch_l2_2d(&tmB, k0, n0);
+      else if (p.b_3d) tma_prefetch_l2_3d(&tmB, 0, k0, n0 / p.bke);
+    }
+  }
+  __syncwarp();
   pdl_wait();
 
   // the 32-row band this warp runs the epilogue of: its own quarter, or one of the 4 / CL bands that this CTA collects
@@ -218,7 +228,7 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
         bulk_commit();
       }
     }
-    if (lane == 0) bulk_wait<0>();                         // shared memory must outlive the stores
+    if (lane == 0) bulk_wait_read<0>();                    // shared memory must outlive the stores' reads of it
     __syncwarp();
   }
   fence_before_sync();

@@ -104,6 +104,10 @@ __device__ __forceinline__ void tma_prefetch_l2_3d(const CUtensorMap* t, int c0,
   asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global.tile [%0, {%1, %2, %3}];"
                ::"l"(reinterpret_cast<uint64_t>(t)), "r"(c0), "r"(c1), "r"(c2) : "memory");
 }
+__device__ __forceinline__ void tma_prefetch_l2_2d(const CUtensorMap* t, int c0, int c1) {
+  asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];"
+               ::"l"(reinterpret_cast<uint64_t>(t)), "r"(c0), "r"(c1) : "memory");
+}
 // TMA store of a shared-memory box to global memory (bulk async-group completion, tracked per issuing thread)
 __device__ __forceinline__ void tma_store_2d(const CUtensorMap* t, const void* src, int c0, int c1) {
   asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];"

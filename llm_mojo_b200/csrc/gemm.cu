@@ -25,19 +25,30 @@ namespace {
 // the tiles it owns; the peer's TMA completions are reported to the leader's mbarrier.
 constexpr int B2_STAGE = 128 * ROW_BYTES;             // 16 KB: this CTA's half of the B tile
 constexpr int STAGE2_BYTES = A_STAGE + B2_STAGE;      // 32 KB
-constexpr int PAIR_THREADS = 384;                      // TMA producer, MMA issuer, 8 epilogue warps, 2 gather copier warps
+// TMA producer, MMA issuer, 8 or 16 epilogue warps, 2 gather copier warps.  Sixteen where an auxiliary input has to be read and worked
+// in (bf16 outputs): a slab of 64 columns is a chain of TMEM loads, MUFU and FMA latencies, staging and column sums, and with two warps
+// per scheduler a tile of such slabs took twice the time of its MMAs at K = 768.  K = 768, 8 -> 16 warps, us: dGELU + column sums N 3072, M
+// 4096 32.2 -> 30.8, M 5439 40.0 -> 36.2, M 12288 72.4 -> 65.0; bias + residual N 768, M 5439 14.1 -> 13.2, M 12288 22.4 -> 20.2 (K 3072, M
+// 5439 26.1 -> 25.2).  Without an auxiliary input the operands' L2 traffic bounds a tile (12 TB/s at M 12288) and eight warps keep up.
+template <int KIND, int EPI> struct PairCfg {
+  static constexpr bool WIDE = EpiCfg<EPI>::AUX_IN && KIND != KIND_TF32;
+  static constexpr int EPI_WARPS = WIDE ? 16 : 8;
+  static constexpr int THREADS = 32 * (4 + EPI_WARPS);
+};
 constexpr int FLAG_ROWS_READY = 6;                     // flag kind (layout of comm.cu: flags[kind][8 ranks])
 constexpr int FLAG_PARAM = 3;                          // owners announce the optimizer step their parameter shard holds
 constexpr int SMEM2_TAIL = 512;                        // barriers, TMEM slot, abort flag
 template <int EPI> constexpr int smem2_bytes() { return EpiCfg<EPI>::STAGES * STAGE2_BYTES + 4 * EpiCfg<EPI>::WARP_STAGE + 1024 + SMEM2_TAIL; }
 
 template <int KIND, int EPI>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PairCfg<KIND, EPI>::THREADS, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                  const __grid_constant__ CUtensorMap tmD, const __grid_constant__ CUtensorMap tmAux, const GemmParams p) {
   using Cfg = EpiCfg<EPI>;
   constexpr int NST = Cfg::STAGES;
   constexpr int WSB = Cfg::WARP_STAGE;
+  constexpr int EPI_WARPS = PairCfg<KIND, EPI>::EPI_WARPS;
+  constexpr bool WIDE = PairCfg<KIND, EPI>::WIDE;
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   unsigned char* epi_stage = smem + NST * STAGE2_BYTES;
@@ -45,7 +56,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   uint64_t* empty_bar = full_bar + NST;
   uint64_t* tfull_bar = empty_bar + NST;
   uint64_t* tempty_bar = tfull_bar + 2;
-  uint64_t* aux_bar = tempty_bar + 2;                   // [8 warps][2 slabs] auxiliary-input tiles landed
+  uint64_t* aux_bar = tempty_bar + 2;                   // [8 warps][2 slabs] or [16 warps]: auxiliary-input tiles landed
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(aux_bar + 16);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
@@ -55,7 +66,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < NST; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
-    for (int a = 0; a < 2; ++a) { mbar_init(&tfull_bar[a], 1); mbar_init(&tempty_bar[a], 16); }   // 8 warps x 2 CTAs
+    for (int a = 0; a < 2; ++a) { mbar_init(&tfull_bar[a], 1); mbar_init(&tempty_bar[a], 2 * EPI_WARPS); }
     for (int a = 0; a < 16; ++a) mbar_init(&aux_bar[a], 1);
     *abort_flag = 0;
     fence_barrier_init();
@@ -211,8 +222,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       }
       if (!ok && lane == 0) { *abort_flag = 1; atomicExch(p.status, LLMB_ERR_TIMEOUT); }
     }
-  } else if (warp >= 10) {
-    // ------------------------------------------------------------ gather copiers (warps 10, 11, both CTAs)
+  } else if (warp >= 2 + EPI_WARPS) {
+    // ------------------------------------------------------------ gather copiers (the last two warps, both CTAs)
     if (p.g.W > 1) {
       // Slices of 32 KB are handed out by ticket, so the copy completes with whatever CTAs are resident.
       constexpr long long SLICE = 2048;                  // 16-byte vectors
@@ -296,6 +307,63 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       }
       if (!ok && lane == 0) { *abort_flag = 1; atomicExch(p.status, LLMB_ERR_TIMEOUT); }
     }
+  } else if (WIDE && p.tma_epi) {
+    // ------------------------------------------------------------ epilogue with an auxiliary input (warps 2..17, both CTAs)
+    // warp % 4 selects the 32-row band (the TMEM lane quarter a warp may read), (warp - 2) / 4 the 64-column slab: one slab per warp
+    // and tile, worked in halves of 32 columns (few enough registers for 16 warps), in place in the warp's one box.  The next tile's
+    // auxiliary box is on its way to L2 while this tile's MMAs run and is loaded once this tile's store has read the box.
+    const int q = warp & 3, e = warp - 2, coff = (e >> 2) * 64;
+    unsigned char* box = epi_stage + e * SLAB_BYTES;
+    uint64_t* abar = aux_bar + e;
+    const int band_off = (int)cta * BM + q * 32;
+    uint32_t aux_phase = 0;
+    auto unit_box = [&](int unit, int& row0, int& col0) {  // false: outside the matrix (warp-uniform)
+      int m_blk, n_blk, kb0, kb1; unit_coords(unit, m_blk, n_blk, kb0, kb1);
+      row0 = m_blk * 2 * BM + band_off; col0 = n_blk * BN + coff;
+      return row0 < p.M && col0 < p.N;
+    };
+    int row0 = 0, col0 = 0;
+    bool valid = cluster_id < total_units && unit_box(cluster_id, row0, col0), loading = valid;
+    if (valid && lane == 0) { mbar_expect_tx(abar, SLAB_BYTES); tma_load_2d(box, &tmAux, abar, col0, row0); }
+    int it = 0;
+    for (int unit = cluster_id; unit < total_units && !*abort_flag; unit += num_clusters, ++it) {
+      const int acc = it & 1;
+      int nrow0 = 0, ncol0 = 0;
+      const bool nvalid = unit + num_clusters < total_units && unit_box(unit + num_clusters, nrow0, ncol0);
+      if (nvalid && lane == 0) tma_prefetch_l2_2d(&tmAux, ncol0, nrow0);
+      if (!mbar_wait(&tfull_bar[acc], (it >> 1) & 1)) { *abort_flag = 1; atomicExch(p.status, LLMB_ERR_TIMEOUT); break; }
+      fence_after_sync();
+      const float alpha = p.alpha ? *p.alpha : 1.0f;
+      const uint32_t tacc = tmem_base + ((uint32_t)(q * 32) << 16) + acc * BN + coff;
+      uint32_t r[32];
+      if (valid) {
+        if (!mbar_wait(abar, aux_phase)) { *abort_flag = 1; atomicExch(p.status, LLMB_ERR_TIMEOUT); break; }
+        aux_phase ^= 1; loading = false;
+        tmem_ld32(tacc, r);
+        tmem_wait_ld();
+        epi_half_bf16<EPI, 0>(p, r, box, col0, alpha, lane);
+        tmem_ld32(tacc + 32, r);
+        tmem_wait_ld();
+      }
+      fence_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive_cluster(mapa_u32(smem_u32(&tempty_bar[acc]), 0));   // the slab has left TMEM; the leader owns the hand-back
+      if (valid) {
+        epi_half_bf16<EPI, 1>(p, r, box, col0, alpha, lane);
+        fence_proxy_async();
+        __syncwarp();
+        if (EPI == EPI_DGELU && p.colsum) { epi_slab_colsum(p, box, row0, col0, lane); __syncwarp(); }
+        if (lane == 0) { tma_store_2d(&tmD, box, col0, row0); bulk_commit(); }
+      }
+      if (nvalid) {
+        if (lane == 0) { bulk_wait_read<0>(); mbar_expect_tx(abar, SLAB_BYTES); tma_load_2d(box, &tmAux, abar, ncol0, nrow0); }
+        loading = true;
+      }
+      valid = nvalid; row0 = nrow0; col0 = ncol0;
+    }
+    if (loading) (void)mbar_wait(abar, aux_phase);
+    if (lane == 0) bulk_wait_read<0>();
+    __syncwarp();
   } else {
     // ------------------------------------------------------------ epilogue (warps 2..9, both CTAs)
     // Eight warps: warp % 4 selects the 32-row band (the TMEM lane quarter a warp may read), (warp - 2) / 4 the
@@ -390,7 +458,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             aux_phase ^= 1u << b; aux_pending &= ~(1u << b);
           } else {
             buf = wstage;
-            if (lane == 0) bulk_wait_read<0>();           // the previous slab's stores have read the buffer
+            // the previous slab's stores have read the buffer (two outputs: its pre-activations have; the newest store is of the other box)
+            if (lane == 0) { if (Cfg::TWO_OUT && !F32_IO) bulk_wait_read<1>(); else bulk_wait_read<0>(); }
             __syncwarp();
           }
           if (F32_IO) {
@@ -414,7 +483,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             epi_slab_pre(p, r0, r1, buf, col0, alpha, lane, pre);
             fence_proxy_async();
             __syncwarp();
-            if (lane == 0) { tma_store_2d(&tmAux, buf, col0, row0); bulk_commit(); }
+            if (lane == 0) { tma_store_2d(&tmAux, buf, col0, row0); bulk_commit(); bulk_wait_read<1>(); }   // the previous slab's activations have left
+            __syncwarp();
             epi_slab_gelu(p, pre, buf + SLAB_BYTES, lane);
             fence_proxy_async();
             __syncwarp();
@@ -486,7 +556,7 @@ int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap&
     if (e != cudaSuccess) return (int)e;
     attr_done = true;
   }
-  return launch_pdl(gemm_pair_kernel<KIND, EPI>, grid, PAIR_THREADS, SMEM, st, ta, tb, td, taux, p);
+  return launch_pdl(gemm_pair_kernel<KIND, EPI>, grid, PairCfg<KIND, EPI>::THREADS, SMEM, st, ta, tb, td, taux, p);
 }
 
 // Tile configuration of one problem: bn = 256 is the CTA-pair kernel, 64 / 128 the kernel of gemm_small.cu with cl CTAs per tile.

@@ -232,16 +232,16 @@ __device__ __forceinline__ void unpack8(const uint4& u, float (&x)[8]) {
   for (int i = 0; i < 4; ++i) { const float2 f = __bfloat1622float2(h[i]); x[2 * i] = f.x; x[2 * i + 1] = f.y; }
 }
 
-// One slab (this lane's row, 64 columns) from registers to the swizzled staging buffer.  With an
-// auxiliary input the buffer holds it on entry and the result replaces it; BIAS_GELU writes the
-// pre-activation to `buf` and the activation to `buf + SLAB_BYTES`.
-template <int EPI>
-__device__ __forceinline__ void epi_slab_bf16(const GemmParams& p, const uint32_t (&r0)[32], const uint32_t (&r1)[32],
-                                              unsigned char* buf, int col0, float alpha, int lane) {
+// Half a slab (this lane's row, 32 columns: chunks 4 * H .. 4 * H + 3) from registers to the swizzled staging buffer.  With an
+// auxiliary input the buffer holds it on entry and the result replaces it; BIAS_GELU writes the pre-activation to `buf` and the
+// activation to `buf + SLAB_BYTES`.
+template <int EPI, int H>
+__device__ __forceinline__ void epi_half_bf16(const GemmParams& p, const uint32_t (&r)[32], unsigned char* buf, int col0, float alpha, int lane) {
   unsigned char* myrow = buf + lane * 128;
   const __nv_bfloat16* bias = reinterpret_cast<const __nv_bfloat16*>(p.bias);
 #pragma unroll
-  for (int c = 0; c < 8; ++c) {
+  for (int c4 = 0; c4 < 4; ++c4) {
+    const int c = H * 4 + c4;
     float v[8], b[8];
     const int col = col0 + c * 8;
 #pragma unroll
@@ -257,8 +257,7 @@ __device__ __forceinline__ void epi_slab_bf16(const GemmParams& p, const uint32_
     }
 #pragma unroll
     for (int j = 0; j < 8; j += 2) {
-      const uint32_t (&r)[32] = c < 4 ? r0 : r1;
-      const float2 y = __ffma2_rn(make_float2(__uint_as_float(r[(c & 3) * 8 + j]), __uint_as_float(r[(c & 3) * 8 + j + 1])),
+      const float2 y = __ffma2_rn(make_float2(__uint_as_float(r[c4 * 8 + j]), __uint_as_float(r[c4 * 8 + j + 1])),
                                   make_float2(alpha, alpha), make_float2(b[j], b[j + 1]));
       v[j] = y.x; v[j + 1] = y.y;
     }
@@ -286,6 +285,12 @@ __device__ __forceinline__ void epi_slab_bf16(const GemmParams& p, const uint32_
       *reinterpret_cast<uint4*>(slot) = pack8(v);
     }
   }
+}
+template <int EPI>
+__device__ __forceinline__ void epi_slab_bf16(const GemmParams& p, const uint32_t (&r0)[32], const uint32_t (&r1)[32],
+                                              unsigned char* buf, int col0, float alpha, int lane) {
+  epi_half_bf16<EPI, 0>(p, r0, buf, col0, alpha, lane);
+  epi_half_bf16<EPI, 1>(p, r1, buf, col0, alpha, lane);
 }
 
 // Column sums of a 32 x 64 slab as stored (bf16): lane l adds up columns 2l and 2l + 1 of the warp's rows out of the swizzled box

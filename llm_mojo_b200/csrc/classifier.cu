@@ -199,6 +199,7 @@ __global__ void __launch_bounds__(1024, 1) classifier_stream_kernel(__nv_bfloat1
 // only compute; warp 31 moves rows: it stores a buffer once the compute warps hand it over (`done`), waits for that
 // store to have read the buffer and refills it with the row after next (`full`).  Per row the steady state is
 // max(arithmetic, (arithmetic + store + load) / 2) instead of store + arithmetic.
+template <int MAXV>
 __global__ void __launch_bounds__(1024, 1) classifier_stream2_kernel(__nv_bfloat16* __restrict__ logits, float* __restrict__ losses,
                                                                      const int* __restrict__ targets, float dloss, int rows, int V,
                                                                      int Vp, int write_dlogits, int buf_bytes, int* status) {
@@ -209,8 +210,7 @@ __global__ void __launch_bounds__(1024, 1) classifier_stream2_kernel(__nv_bfloat
   constexpr int NC = 992, NCW = 31;                       // compute threads / warps
   extern __shared__ __align__(128) unsigned char smraw[];
   __shared__ uint64_t full[2], done[2];
-  __shared__ float red[32];
-  __shared__ float bcast[2];
+  __shared__ float red[32], reds[32];
   __shared__ int fail_s;
   const int tid = threadIdx.x, lane = tid % 32, wid = tid / 32;
   const uint32_t row_bytes = (uint32_t)Vp * 2;
@@ -242,12 +242,17 @@ __global__ void __launch_bounds__(1024, 1) classifier_stream2_kernel(__nv_bfloat
           bulk_load_1d(buf, logits + (size_t)rn * Vp, row_bytes, &full[b]);
         }
       }
-      bulk_wait<0>();                                     // shared memory must outlive the last store
+      bulk_wait_read<0>();                                // shared memory must outlive the last store's reads of it
     }
     return;
   }
 
   // -------------------------------------------------------------- compute warps
+  // A thread holds its part of the row (MAXV 16-byte vectors) in registers from the one read of the buffer to the one write:
+  // packed bf16 maximum, exponentials packed back into the same registers, scaled by 1 / sum on the way out.  Re-reading the buffer
+  // for each pass, with two barriers around every reduction, took 6.5 us a row against the 4.5 us in which an SM's share of the
+  // memory bandwidth moves it.  4096 x 50304: 175 -> 162 us, 16384 x 50304: 623 -> 608 us (5.4 TB/s; what is left is the buffers' cycle of
+  // load, arithmetic and store: a third buffer does not fit).
   const float L2E = 1.4426950408889634f;
   const int nfull = V / N;                                // vectors entirely below V
   int it = 0;
@@ -255,61 +260,67 @@ __global__ void __launch_bounds__(1024, 1) classifier_stream2_kernel(__nv_bfloat
     const int b = it & 1;
     T* row_s = reinterpret_cast<T*>(smraw + (size_t)b * buf_bytes);
     if (!mbar_wait(&full[b], (it >> 1) & 1)) { atomicExch(status, LLMB_ERR_TIMEOUT); fail_s = 1; }
-    csync();
-    if (fail_s) break;
-    // pass 1: row maximum over the real vocabulary
-    float mx = -INFINITY;
-    for (int v = tid; v < nfull; v += NC) {
-      Pack<T> p; p.load(row_s + v * N);
+    uint4 u[MAXV];
 #pragma unroll
-      for (int k = 0; k < N; ++k) mx = fmaxf(mx, p.v[k]);
-    }
-    for (int v = nfull + tid; v < nvec; v += NC) {
-      Pack<T> p; p.load(row_s + v * N);
+    for (int j = 0; j < MAXV; ++j) {
+      const int v = tid + j * NC;
+      u[j] = v < nvec ? *reinterpret_cast<const uint4*>(row_s + v * N) : make_uint4(0xff80ff80u, 0xff80ff80u, 0xff80ff80u, 0xff80ff80u);
+      if (v >= nfull && v < nvec) {                       // padded columns count as -infinity
+        unsigned short* h = reinterpret_cast<unsigned short*>(&u[j]);
 #pragma unroll
-      for (int k = 0; k < N; ++k) if (v * N + k < V) mx = fmaxf(mx, p.v[k]);
+        for (int k = 0; k < N; ++k) if (v * N + k >= V) h[k] = 0xff80u;
+      }
     }
-    mx = warp_max(mx);
+    float x_tgt = 0.f;
+    int tgt = 0;
+    if (tid == 0) {
+      tgt = targets[r];
+      if (!llmb_in_range(tgt, V, LLMB_SITE_CLASSIFIER_TARGET)) tgt = 0;               // checked build: a bad target is recorded and clamped
+      x_tgt = __bfloat162float(row_s[tgt]);
+    }
+    __nv_bfloat162 m2 = __floats2bfloat162_rn(-INFINITY, -INFINITY);
+#pragma unroll
+    for (int j = 0; j < MAXV; ++j) {
+      const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&u[j]);
+      m2 = __hmax2(m2, __hmax2(__hmax2(h[0], h[1]), __hmax2(h[2], h[3])));
+    }
+    float mx = warp_max(fmaxf(__low2float(m2), __high2float(m2)));
     if (lane == 0) red[wid] = mx;
     csync();
-    if (wid == 0) { float m = lane < NCW ? red[lane] : -INFINITY; m = warp_max(m); if (lane == 0) bcast[0] = m; }
-    csync();
-    mx = bcast[0];
-    const int tgt_raw = targets[r];
-  const int tgt = llmb_in_range(tgt_raw, V, LLMB_SITE_CLASSIFIER_TARGET) ? tgt_raw : 0;   // checked build: a bad target is recorded and clamped
-    const float x_tgt = __bfloat162float(row_s[tgt]);     // read before the buffer is overwritten
-    csync();
-    // pass 2: e = 2^((x - max) log2 e), once per element, written back over the row
-    float sum = 0.f;
+    if (fail_s) break;
+    mx = warp_max(lane < NCW ? red[lane] : -INFINITY);
     const float mb = mx * L2E;
-    for (int v = tid; v < nfull; v += NC) {
-      Pack<T> p; p.load(row_s + v * N);
+    float s0 = 0.f, s1 = 0.f;
 #pragma unroll
-      for (int k = 0; k < N; ++k) { p.v[k] = ex2_fast(fmaf(p.v[k], L2E, -mb)); sum += p.v[k]; }
-      if (write_dlogits) p.store(row_s + v * N);
-    }
-    for (int v = nfull + tid; v < nvec; v += NC) {
-      Pack<T> p; p.load(row_s + v * N);
+    for (int j = 0; j < MAXV; ++j) {
+      uint32_t* h = reinterpret_cast<uint32_t*>(&u[j]);
 #pragma unroll
-      for (int k = 0; k < N; ++k) { p.v[k] = (v * N + k < V) ? ex2_fast(fmaf(p.v[k], L2E, -mb)) : 0.f; sum += p.v[k]; }
-      if (write_dlogits) p.store(row_s + v * N);
+      for (int k = 0; k < 4; ++k) {
+        const float e0 = ex2_fast(fmaf(__uint_as_float(h[k] << 16), L2E, -mb)), e1 = ex2_fast(fmaf(__uint_as_float(h[k] & 0xffff0000u), L2E, -mb));
+        s0 += e0; s1 += e1;
+        const __nv_bfloat162 e = __floats2bfloat162_rn(e0, e1);
+        h[k] = *reinterpret_cast<const uint32_t*>(&e);
+      }
     }
-    sum = warp_sum(sum);
-    if (lane == 0) red[wid] = sum;
+    float sum = warp_sum(s0 + s1);
+    if (lane == 0) reds[wid] = sum;
     csync();
-    if (wid == 0) { float s = lane < NCW ? red[lane] : 0.f; s = warp_sum(s); if (lane == 0) bcast[1] = s; }
-    csync();
-    sum = bcast[1];
+    sum = warp_sum(lane < NCW ? reds[lane] : 0.f);
     if (tid == 0 && losses) losses[r] = -(x_tgt - mx - logf(sum));
     if (write_dlogits) {
-      // pass 3: dlogits = (e / sum - 1[target]) dloss in place (padded columns hold e = 0); the target column is
-      // corrected afterwards by one thread; then the row is handed to the mover
+      // dlogits = (e / sum - 1[target]) dloss (padded columns hold e = 0); the target column is corrected afterwards by one thread;
+      // then the row is handed to the mover
       const float inv = dloss / sum;
-      for (int v = tid; v < nvec; v += NC) {
-        Pack<T> p; p.load(row_s + v * N);
 #pragma unroll
-        for (int k = 0; k < N; ++k) p.v[k] *= inv;
-        p.store(row_s + v * N);
+      for (int j = 0; j < MAXV; ++j) {
+        const int v = tid + j * NC;
+        uint32_t* h = reinterpret_cast<uint32_t*>(&u[j]);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const __nv_bfloat162 o = __floats2bfloat162_rn(__uint_as_float(h[k] << 16) * inv, __uint_as_float(h[k] & 0xffff0000u) * inv);
+          h[k] = *reinterpret_cast<const uint32_t*>(&o);
+        }
+        if (v < nvec) *reinterpret_cast<uint4*>(row_s + v * N) = u[j];
       }
       fence_proxy_async();                                // these writes, before the mover's bulk store reads them
       csync();
@@ -473,8 +484,9 @@ LLMB_API int llmb_fused_classifier(void* logits, float* losses, const int* targe
         launch_pdl(classifier_stream_kernel, grid, 1024, 2 * buf_bytes, st, (__nv_bfloat16*)logits, losses, targets, dloss, rows, V, Vp,
                                                                    write_dlogits, buf_bytes, status);
       } else {
-        cudaFuncSetAttribute(classifier_stream2_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * buf_bytes);
-        launch_pdl(classifier_stream2_kernel, grid, 1024, 2 * buf_bytes, st, (__nv_bfloat16*)logits, losses, targets, dloss, rows, V, Vp,
+        auto kern = Vp <= 7 * 992 * 8 ? classifier_stream2_kernel<7> : classifier_stream2_kernel<8>;      // two buffers fit up to Vp = 57344
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * buf_bytes);
+        launch_pdl(kern, grid, 1024, 2 * buf_bytes, st, (__nv_bfloat16*)logits, losses, targets, dloss, rows, V, Vp,
                                                                     write_dlogits, buf_bytes, status);
       }
       return (int)cudaGetLastError();

@@ -171,3 +171,25 @@ def test_gemm_residual_right_edge_many_tiles():
         out = torch.empty(M, N, dtype=torch.bfloat16, device=DEV)
         ops.matmul_fwd(out, X, W, torch.zeros(N, dtype=torch.bfloat16, device=DEV), residual=Rs)
         assert_close(out, ref, 2.0 ** -6, 2.0 ** -8, "residual at the right edge")
+
+
+# a thread of the classifier holds 7 or 8 vectors of a row: widths around whole and partial last vectors, the switch and the largest
+@pytest.mark.parametrize("V,Vp", [(3, 8), (7930, 7936), (7944, 7944), (50257, 50304), (55546, 55552), (55553, 55560), (57344, 57344)])
+@pytest.mark.parametrize("rows", [1, 3, 400])
+def test_fused_classifier_row_widths(V, Vp, rows):
+    x = rnd(rows, Vp, scale=3.0)
+    tgt = torch.randint(0, V, (rows,), generator=torch.Generator().manual_seed(rows), dtype=torch.int32)
+    tgt[0], tgt[-1] = 0, V - 1
+    got, losses = x.to(DEV), torch.empty(rows, device=DEV)
+    ops.fused_classifier(got, losses, tgt.to(DEV), 0.5, V)
+    p = torch.softmax(x[:, :V].float(), dim=1)
+    at = (torch.arange(rows), tgt.long())
+    # the target column is a difference: absolute error of the bf16 exponential (p <= 1) and of the result
+    assert_close(got.cpu()[at], 0.5 * (p[at] - 1), 0.5 * 2.0 ** -8, 0.0, "dlogits of the targets")
+    got = got.cpu()
+    got[at], p[at] = 0, 0
+    assert_close(got[:, :V], 0.5 * p, 1e-7, 2.0 ** -7, "dlogits")        # two bf16 roundings: of the exponential and of the result
+    assert bool((got[:, V:] == 0).all())
+    want = torch.nn.functional.cross_entropy(x[:, :V].float(), tgt.long(), reduction="none")
+    assert_close(losses, want, 1e-4, 1e-4, "losses")
+    assert _lib.read_status() == 0

@@ -24,6 +24,7 @@ struct AttnParams {
   float scale;          // 1/sqrt(HS)
   float* dbias;         // bwd, optional: fp32 [3C], += column sums of dqkv (the gradient of the qkv bias)
   int* status;
+  int tpi;              // fwd: query tiles per work item (2, or 1 where the grid has an SM for every tile)
 };
 
 // byte offset of 16-byte chunk `chunk` (0..7) of row `row` inside a 128B-swizzled tile

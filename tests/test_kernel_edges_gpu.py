@@ -193,3 +193,17 @@ def test_fused_classifier_row_widths(V, Vp, rows):
     want = torch.nn.functional.cross_entropy(x[:, :V].float(), tgt.long(), reduction="none")
     assert_close(losses, want, 1e-4, 1e-4, "losses")
     assert _lib.read_status() == 0
+
+
+# the forward takes one query tile per CTA up to as many tiles as the chip has SMs and pairs beyond: both sides of the switch, one tile,
+# even and odd tile counts, ragged ends
+@pytest.mark.parametrize("B,T,NH", [(1, 64, 12), (1, 128, 1), (1, 776, 16), (1, 1024, 18), (1, 1100, 16), (2, 1024, 9), (1, 1024, 19), (3, 300, 49), (3, 300, 50)])
+def test_attention_fwd_tiles_per_item(B, T, NH):
+    qkv = rnd(B, T, 3 * 64 * NH)
+    ref, lse_ref = torch.empty(B, T, 64 * NH), torch.empty(B, NH, T)
+    ops.attention_fwd(ref, lse_ref, qkv.float(), NH)
+    out, lse = torch.empty(B, T, 64 * NH, dtype=torch.bfloat16, device=DEV), torch.empty(B, NH, T, device=DEV)
+    ops.attention_fwd(out, lse, qkv.to(DEV), NH)
+    assert_close(out, ref, 2.0 ** -7, 2.0 ** -7, "out")          # bf16 probabilities and output, values of order one
+    assert_close(lse, lse_ref, 1e-3, 1e-4, "lse")
+    assert _lib.read_status() == 0

@@ -163,15 +163,15 @@ __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.lau
 // Launch with the attribute, in clusters of `cl` CTAs (1: none, or as the kernel declares); every thread of `kern` that touches global
 // memory must call pdl_wait() first.
 template <typename... KArgs, typename... Args>
-inline int launch_pdl_cluster(int cl, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args&&... args) {
+inline int launch_pdl_cluster(dim3 cl, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args&&... args) {
   cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = st;
   at[1].id = cudaLaunchAttributeClusterDimension;
-  at[1].val.clusterDim.x = (unsigned)cl; at[1].val.clusterDim.y = 1; at[1].val.clusterDim.z = 1;
-  cfg.attrs = at; cfg.numAttrs = cl > 1 ? 2 : 1;
+  at[1].val.clusterDim.x = cl.x; at[1].val.clusterDim.y = cl.y; at[1].val.clusterDim.z = cl.z;
+  cfg.attrs = at; cfg.numAttrs = cl.x * cl.y * cl.z > 1 ? 2 : 1;
   return (int)cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...);
 }
 template <typename... KArgs, typename... Args>

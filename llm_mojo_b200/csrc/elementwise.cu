@@ -6,7 +6,7 @@
 // B200 design: all accesses are 16-byte vectors; dwte is made deterministic by a device-side
 // radix sort of (token, position) keys followed by one block per token run, instead of the
 // reference's host-side counting sort.
-#include "common.cuh"
+#include "tc05.cuh"
 #include <cub/device/device_radix_sort.cuh>
 
 using namespace llmb;
@@ -68,9 +68,13 @@ __global__ void make_keys_kernel(unsigned long long* keys, const int* tok, int B
 // that lies inside one segment is added to dwte at once (nothing else touches that row); the piece of a run that crosses a
 // segment border goes to a per-segment partial row (slot 0: the run began in an earlier segment, slot 1: it goes on in the
 // next one), and wte_bwd_combine_kernel adds up the pieces of each such run in segment order.
+// Latency bounds it: the sixteen rows of a segment are loaded together, the additions to dwte (one per element, so their result does
+// not depend on timing) are left to L2, and the channels of a segment are shared by the warps of blockIdx.y.  One row at a time, with
+// a read-modify-write of dwte per run and all channels in one warp, 4096 x 768 took 51 us, 5439 x 768 49 us; with the
+// shorter sort and the single-launch bias gradients below, a d6 training step of 2 x 128 went from 1.335 to 1.304 ms.
 constexpr int WTE_SEG = 16;
 template <typename T>
-__global__ void __launch_bounds__(256) wte_bwd_kernel(float* __restrict__ dwte, float* __restrict__ partial, const T* __restrict__ dout,
+__global__ void __launch_bounds__(128) wte_bwd_kernel(float* __restrict__ dwte, float* __restrict__ partial, const T* __restrict__ dout,
                                                       const unsigned long long* __restrict__ keys, int BT, int C, int V) {
   pdl_trigger();
   pdl_wait();
@@ -79,44 +83,54 @@ __global__ void __launch_bounds__(256) wte_bwd_kernel(float* __restrict__ dwte, 
   const int j0 = seg * WTE_SEG;
   if (j0 >= BT) return;
   const int cnt = min(WTE_SEG, BT - j0);
-  unsigned long long mykey = lane < cnt ? keys[j0 + lane] : 0ull;
+  const unsigned long long mykey = lane < cnt ? keys[j0 + lane] : 0ull;
   const unsigned prev_tok = j0 > 0 ? (unsigned)(keys[j0 - 1] >> 32) : 0xffffffffu;
   const unsigned next_tok = j0 + cnt < BT ? (unsigned)(keys[j0 + cnt] >> 32) : 0xffffffffu;
-  const int vec_per_row = C / N;
-  for (int vc0 = 0; vc0 < vec_per_row; vc0 += 32) {       // this lane's channel vectors, one after the other; every lane walks the
-    const int vc = vc0 + lane;                             // loop (the shuffles below need the whole warp), idle ones past the row end
-    const bool live = vc < vec_per_row;
-    float acc[N];
+  const int vc = blockIdx.y * 32 + lane;                  // this lane's channel vector; lanes past the row end take part in the shuffles only
+  const bool live = vc * N < C;
+  uint4 raw[WTE_SEG];
 #pragma unroll
-    for (int k = 0; k < N; ++k) acc[k] = 0.f;
-    int a = 0;                                              // first position of the current run inside the segment
-    for (int j = 0; j < cnt; ++j) {
-      const unsigned long long key = __shfl_sync(0xffffffffu, mykey, j);
-      const unsigned tokv = (unsigned)(key >> 32);
-      const bool ok = llmb_in_range((long long)tokv, V, LLMB_SITE_ENCODER_BWD_TOKEN);
+  for (int j = 0; j < WTE_SEG; ++j) {
+    const unsigned pos = (unsigned)(__shfl_sync(0xffffffffu, mykey, j) & 0xffffffffu);
+    if (live && j < cnt) raw[j] = *reinterpret_cast<const uint4*>(dout + (size_t)pos * C + vc * N);
+  }
+  float acc[N];
+#pragma unroll
+  for (int k = 0; k < N; ++k) acc[k] = 0.f;
+  int a = 0;                                                // first position of the current run inside the segment
+#pragma unroll
+  for (int j = 0; j < WTE_SEG; ++j) {
+    if (j >= cnt) break;
+    const unsigned tokv = (unsigned)(__shfl_sync(0xffffffffu, mykey, j) >> 32);
+    const bool ok = llmb_in_range((long long)tokv, V, LLMB_SITE_ENCODER_BWD_TOKEN);
+    if (ok && live) {
+      Pack<T> p; p.load(reinterpret_cast<const T*>(&raw[j]));
+#pragma unroll
+      for (int k = 0; k < N; ++k) acc[k] += p.v[k];
+    }
+    const unsigned nxt = j + 1 < cnt ? (unsigned)(__shfl_sync(0xffffffffu, mykey, (j + 1) % WTE_SEG) >> 32) : next_tok;
+    if (j + 1 == cnt || nxt != tokv) {                      // the run (or its piece in this segment) ends here
+      const bool from_before = a == 0 && prev_tok == tokv, goes_on = j + 1 == cnt && next_tok == tokv;
       if (ok && live) {
-        Pack<T> p; p.load(dout + (size_t)(unsigned)(key & 0xffffffffu) * C + vc * N);
+        if (from_before || goes_on) {
+          float* dst = partial + ((size_t)seg * 2 + (from_before ? 0 : 1)) * C + vc * N;
 #pragma unroll
-        for (int k = 0; k < N; ++k) acc[k] += p.v[k];
-      }
-      const unsigned nxt = j + 1 < cnt ? (unsigned)(__shfl_sync(0xffffffffu, mykey, j + 1) >> 32) : next_tok;
-      if (j + 1 == cnt || nxt != tokv) {                    // the run (or its piece in this segment) ends here
-        const bool from_before = a == 0 && prev_tok == tokv, goes_on = j + 1 == cnt && next_tok == tokv;
-        if (ok && live) {
-          float* dst = (from_before || goes_on) ? partial + ((size_t)seg * 2 + (from_before ? 0 : 1)) * C + vc * N
-                                                : dwte + (size_t)tokv * C + vc * N;
-          if (from_before || goes_on) {
+          for (int k = 0; k < N; ++k) dst[k] = acc[k];
+        } else {
+          float* dst = dwte + (size_t)tokv * C + vc * N;
+          if ((reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
 #pragma unroll
-            for (int k = 0; k < N; ++k) dst[k] = acc[k];
+            for (int k = 0; k < N; k += 4)
+              asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(dst + k), "f"(acc[k]), "f"(acc[k + 1]), "f"(acc[k + 2]), "f"(acc[k + 3]) : "memory");
           } else {
 #pragma unroll
-            for (int k = 0; k < N; ++k) dst[k] += acc[k];
+            for (int k = 0; k < N; ++k) asm volatile("red.global.add.f32 [%0], %1;" ::"l"(dst + k), "f"(acc[k]) : "memory");
           }
         }
-#pragma unroll
-        for (int k = 0; k < N; ++k) acc[k] = 0.f;
-        a = j + 1;
       }
+#pragma unroll
+      for (int k = 0; k < N; ++k) acc[k] = 0.f;
+      a = j + 1;
     }
   }
 }
@@ -195,18 +209,19 @@ LLMB_API int llmb_encoder_bwd(float* dwte, float* dwpe, const void* dout, const 
   size_t temp_bytes = sort_bytes - 2 * (size_t)BT * sizeof(unsigned long long);
   float* partial = reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(scratch) + sort_bytes);
   launch_pdl(make_keys_kernel, ceil_div(BT, 256), 256, 0, st, kin, tok, BT);
-  // position bits live in [0, 32); token bits in [32, 32 + vocab_bits). Sort only the used bits.
-  cudaError_t e = cub::DeviceRadixSort::SortKeys(temp, temp_bytes, kin, kout, BT, 0, 32 + vocab_bits, st);
+  // Position bits live in [0, 32), token bits in [32, 32 + vocab_bits).  The keys come in order of position and the radix sort is
+  // stable, so sorting by the token bits alone (two passes instead of six) leaves the positions of a token in order.
+  cudaError_t e = cub::DeviceRadixSort::SortKeys(temp, temp_bytes, kin, kout, BT, 32, 32 + vocab_bits, st);
   if (e != cudaSuccess) return (int)e;
   const int nseg = ceil_div(BT, WTE_SEG);
   if (dtype == LLMB_BF16) {
     if (C % 8) return LLMB_ERR_BAD_ARG;
-    launch_pdl(wte_bwd_kernel<__nv_bfloat16>, ceil_div(nseg, 8), 256, 0, st, dwte, partial, (const __nv_bfloat16*)dout, kout, BT, C, V);
+    launch_pdl(wte_bwd_kernel<__nv_bfloat16>, dim3(ceil_div(nseg, 4), ceil_div(C / 8, 32)), 128, 0, st, dwte, partial, (const __nv_bfloat16*)dout, kout, BT, C, V);
     launch_pdl(wte_bwd_combine_kernel, nseg, 256, 0, st, dwte, partial, kout, BT, C, V);
     launch_pdl(wpe_bwd_kernel<__nv_bfloat16>, ceil_div(T * (C / 8), 256), 256, 0, st, dwpe, (const __nv_bfloat16*)dout, B, T, C);
   } else {
     if (C % 4) return LLMB_ERR_BAD_ARG;
-    launch_pdl(wte_bwd_kernel<float>, ceil_div(nseg, 8), 256, 0, st, dwte, partial, (const float*)dout, kout, BT, C, V);
+    launch_pdl(wte_bwd_kernel<float>, dim3(ceil_div(nseg, 4), ceil_div(C / 4, 32)), 128, 0, st, dwte, partial, (const float*)dout, kout, BT, C, V);
     launch_pdl(wte_bwd_combine_kernel, nseg, 256, 0, st, dwte, partial, kout, BT, C, V);
     launch_pdl(wpe_bwd_kernel<float>, ceil_div(T * (C / 4), 256), 256, 0, st, dwpe, (const float*)dout, B, T, C);
   }
@@ -254,13 +269,17 @@ LLMB_API int llmb_gelu_bwd(void* dinp, const void* inp, const void* dout, long l
 // ---------------------------------------------------------------- dbias: dbias[c] += sum_rows dout[row, c]
 // Stage 1: grid (col blocks, row slabs); each block owns 32*N columns... threads (8 row lanes x 32 col vecs).
 // partial[slab][c] written to scratch; stage 2 sums slabs in order (deterministic) and accumulates.
-template <typename T, int RL>
+// DIRECT (up to 8192 rows): the slabs of a column block are the CTAs of one cluster; they hand their sums to the first through
+// distributed shared memory, which adds them up in slab order and into dbias: one launch instead of two (24 a d12 micro-step, 2 - 3 us each).
+template <typename T, int RL, bool DIRECT>
 __global__ void __launch_bounds__(256) dbias_partial_kernel(float* __restrict__ partial, const T* __restrict__ dout, int rows, int OC, int rows_per_slab) {
+  if (DIRECT) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");     // waited for before anything is sent
   pdl_trigger();
   pdl_wait();
   constexpr int N = Pack<T>::N;
   constexpr int CV = 256 / RL;                           // column vectors per block; RL row lanes
   __shared__ float sm[RL][CV * N + 1];
+  __shared__ float mine[DIRECT ? CV * N : 1], all[DIRECT ? 8 : 1][DIRECT ? CV * N : 1];
   int cv = threadIdx.x % CV, rl = threadIdx.x / CV;
   int c0 = (blockIdx.x * CV + cv) * N;
   int r0 = blockIdx.y * rows_per_slab, r1 = min(rows, r0 + rows_per_slab);
@@ -291,21 +310,43 @@ __global__ void __launch_bounds__(256) dbias_partial_kernel(float* __restrict__ 
       float s = 0.f;
 #pragma unroll
       for (int l = 0; l < RL; ++l) s += sm[l][c];
-      partial[(size_t)blockIdx.y * OC + col] = s;
+      if (DIRECT) mine[c] = s; else partial[(size_t)blockIdx.y * OC + col] = s;
     }
   }
+  if (DIRECT) {
+    __syncthreads();
+    asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+    for (int c = threadIdx.x; c < CV * N; c += blockDim.x)
+      asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(tc05::mapa_u32(tc05::smem_u32(&all[blockIdx.y][c]), 0)), "f"(mine[c]) : "memory");
+    tc05::cluster_sync_all();
+    if (blockIdx.y == 0)
+      for (int c = threadIdx.x; c < CV * N; c += blockDim.x) {
+        const int col = blockIdx.x * CV * N + c;
+        float s = 0.f;
+        for (int y = 0; y < (int)gridDim.y; ++y) s += all[y][c];
+        if (col < OC) partial[col] += s;                  // dbias itself
+      }
+  }
 }
+constexpr int DBIAS_DIRECT_ROWS = 8192, DBIAS_MAX_CLUSTER = 8;
 // narrow matrices get more row lanes per block (fewer columns per block) so that the grid still fills the machine
 template <typename T>
 void dbias_partial_launch(float* partial, const T* dout, int rows, int OC, int rows_per_slab, int slabs, cudaStream_t st) {
   constexpr int N = Pack<T>::N;
   const int want = 6 * sm_count();
   if (ceil_div(OC, 32 * N) * slabs >= want)
-    launch_pdl(dbias_partial_kernel<T, 8>, dim3(ceil_div(OC, 32 * N), slabs), 256, 0, st, partial, dout, rows, OC, rows_per_slab);
+    launch_pdl(dbias_partial_kernel<T, 8, false>, dim3(ceil_div(OC, 32 * N), slabs), 256, 0, st, partial, dout, rows, OC, rows_per_slab);
   else if (ceil_div(OC, 16 * N) * slabs >= want)
-    launch_pdl(dbias_partial_kernel<T, 16>, dim3(ceil_div(OC, 16 * N), slabs), 256, 0, st, partial, dout, rows, OC, rows_per_slab);
+    launch_pdl(dbias_partial_kernel<T, 16, false>, dim3(ceil_div(OC, 16 * N), slabs), 256, 0, st, partial, dout, rows, OC, rows_per_slab);
   else
-    launch_pdl(dbias_partial_kernel<T, 32>, dim3(ceil_div(OC, 8 * N), slabs), 256, 0, st, partial, dout, rows, OC, rows_per_slab);
+    launch_pdl(dbias_partial_kernel<T, 32, false>, dim3(ceil_div(OC, 8 * N), slabs), 256, 0, st, partial, dout, rows, OC, rows_per_slab);
+}
+template <typename T>
+int dbias_direct_launch(float* dbias, const T* dout, int rows, int OC, cudaStream_t st) {
+  int slabs = 1;                                          // at most 512 rows per CTA until the cluster is full
+  while (slabs < DBIAS_MAX_CLUSTER && slabs * 512 < rows) slabs *= 2;
+  return launch_pdl_cluster(dim3(1, slabs), dbias_partial_kernel<T, 32, true>, dim3(ceil_div(OC, 8 * Pack<T>::N), slabs), 256, 0, st, dbias, dout,
+                            rows, OC, ceil_div(rows, slabs));
 }
 // Stage 2: 32 columns per block, eight threads per column each summing every eighth slab (independent loads in flight
 // instead of one thread walking all slabs), then a fixed-order sum of the eight: deterministic.
@@ -331,16 +372,19 @@ __global__ void __launch_bounds__(256) dbias_final_kernel(float* __restrict__ db
 }
 LLMB_API int llmb_dbias_slabs(int rows) { int s = ceil_div(rows, 128); return s > 128 ? 128 : (s < 1 ? 1 : s); }
 LLMB_API long long llmb_dbias_scratch_bytes(int rows, int OC) { return (long long)llmb_dbias_slabs(rows) * OC * sizeof(float); }
+LLMB_API int llmb_dbias_launches(int rows) { return rows <= DBIAS_DIRECT_ROWS ? 1 : 2; }
 LLMB_API int llmb_dbias(float* dbias, const void* dout, float* scratch, long long scratch_bytes, int rows, int OC,
                         int dtype, cudaStream_t st) {
   int slabs = llmb_dbias_slabs(rows);
   if (scratch_bytes < (long long)slabs * OC * (long long)sizeof(float)) return LLMB_ERR_BAD_ARG;  // regression guard: never overrun
   int rows_per_slab = ceil_div(rows, slabs);
+  if (OC % (dtype == LLMB_BF16 ? 8 : 4)) return LLMB_ERR_BAD_ARG;
+  if (rows <= DBIAS_DIRECT_ROWS)
+    return dtype == LLMB_BF16 ? dbias_direct_launch<__nv_bfloat16>(dbias, (const __nv_bfloat16*)dout, rows, OC, st)
+                              : dbias_direct_launch<float>(dbias, (const float*)dout, rows, OC, st);
   if (dtype == LLMB_BF16) {
-    if (OC % 8) return LLMB_ERR_BAD_ARG;
     dbias_partial_launch<__nv_bfloat16>(scratch, (const __nv_bfloat16*)dout, rows, OC, rows_per_slab, slabs, st);
   } else {
-    if (OC % 4) return LLMB_ERR_BAD_ARG;
     dbias_partial_launch<float>(scratch, (const float*)dout, rows, OC, rows_per_slab, slabs, st);
   }
   launch_pdl(dbias_final_kernel, ceil_div(OC, 32), 256, 0, st, dbias, scratch, OC, slabs);

@@ -15,6 +15,7 @@ LLMB_API int llmb_encoder_fwd(void* out, const int* tok, const void* wte, const 
 LLMB_API int llmb_encoder_bwd(float* dwte, float* dwpe, const void* dout, const int* tok, void* scratch, long long scratch_bytes, int B, int T,
                               int C, int V, int vocab_bits, int dtype, cudaStream_t st);
 LLMB_API int llmb_gelu_fwd(void* out, const void* inp, long long n, int dtype, cudaStream_t st);
+LLMB_API int llmb_dbias_launches(int rows);
 LLMB_API int llmb_dbias(float* dbias, const void* dout, float* scratch, long long scratch_bytes, int rows, int OC, int dtype, cudaStream_t st);
 LLMB_API int llmb_layernorm_fwd(void* out, float* mean, float* rstd, void* resid_out, const void* inp1, const void* inp2, const void* w,
                                 const void* b, int rows, int C, int dtype, cudaStream_t st);
@@ -118,7 +119,7 @@ struct Step {
     return ok(llmb_gemm(dinp, dout, w, nullptr, aux, nullptr, rows, K, N, lo, K, K, aux ? K : 0, 0, 1, 0, 0, 0, epi, 1, s.status, st)) &&
            ok(llmb_gemm(dw, dout, inp, nullptr, nullptr, nullptr, N, K, rows, lo, K, K, 0, 1, 1, 0, 0, 0, EPI_ACC_F32, splits, s.status, st));
   }
-  bool bias_grad(float* db, const void* dout, int N) { return ok(llmb_dbias(db, dout, s.s_dbias, s.s_dbias_bytes, rows, N, LLMB_BF16, st), 2); }
+  bool bias_grad(float* db, const void* dout, int N) { return ok(llmb_dbias(db, dout, s.s_dbias, s.s_dbias_bytes, rows, N, LLMB_BF16, st), llmb_dbias_launches(rows)); }
   bool ln_bwd(float* dw, float* db, const void* inp, const void* w, const float* mean, const float* rstd, int accumulate) {
     return ok(llmb_layernorm_bwd(s.a[A_DRES], dw, db, s.s_ln, s.s_ln_bytes, s.a[A_DL], inp, w, mean, rstd, rows, C, accumulate, LLMB_BF16, st), 2);
   }

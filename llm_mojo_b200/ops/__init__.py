@@ -380,7 +380,7 @@ def dbias_reduce(dbias, dout2d) -> None:
         nb = L.llmb_dbias_scratch_bytes(rows, OC)
         s = scratch("dbias", nb, dout2d.device)
         check(L.llmb_dbias(ptr(dbias), ptr(dout2d), ptr(s), s.numel(), rows, OC, dtype_code(dout2d), stream()), "dbias")
-        _count(2)
+        _count(L.llmb_dbias_launches(rows))
     else:
         dbias += dout2d.float().sum(0)
 

@@ -29,6 +29,7 @@ _SIGS = {
     "llmb_gelu_fwd": [c_p, c_p, c_ll, c_int, c_p],
     "llmb_gelu_bwd": [c_p, c_p, c_p, c_ll, c_int, c_p],
     "llmb_dbias_scratch_bytes": [c_int, c_int],
+    "llmb_dbias_launches": [c_int],
     "llmb_dbias": [c_p, c_p, c_p, c_ll, c_int, c_int, c_int, c_p],
     "llmb_cast_f32_to_bf16": [c_p, c_p, c_ll, c_p],
     "llmb_nan_census": [c_p, c_p, c_ll, c_int, c_p],

@@ -195,6 +195,36 @@ def test_fused_classifier_row_widths(V, Vp, rows):
     assert _lib.read_status() == 0
 
 
+# one CTA, clusters of 2, 4 and 8 with even and uneven slabs, the last row count of the single launch and the first of the pair
+@pytest.mark.parametrize("rows", [1, 511, 513, 1025, 3001, 8192, 8193])
+@pytest.mark.parametrize("OC", [8, 72, 776])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_dbias_edges(rows, OC, dtype):
+    x = rnd(rows, OC, dtype=dtype)
+    got = torch.full((OC,), 3.0, device=DEV)
+    ops.dbias_reduce(got, x.to(DEV))
+    want = 3.0 + x.double().sum(0)
+    assert_close(got, want, 2.0 ** -24 * 4 * rows ** 0.5 * 16, 1e-5, "dbias")      # fp32 sums of unit normals in short chains
+    again = torch.full((OC,), 3.0, device=DEV)
+    ops.dbias_reduce(again, x.to(DEV))
+    assert torch.equal(got, again)
+
+
+# segments of 16 positions, 4 segments and 32 channel vectors per CTA; a token that fills several segments, every token once
+@pytest.mark.parametrize("BT,C,V", [(1, 8, 8), (15, 256, 40), (65, 264, 40), (300, 768, 7), (513, 384, 5000), (64, 1600, 1)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("off", [0, 1])
+def test_encoder_bwd_edges(BT, C, V, dtype, off):
+    tok = torch.randint(0, V, (1, BT), generator=torch.Generator().manual_seed(BT), dtype=torch.int32)
+    d = rnd(1, BT, C, dtype=dtype)
+    store = torch.full((V * C + 1,), 0.5, device=DEV)
+    dwte, dwpe = store[off:off + V * C].view(V, C), torch.full((BT, C), 0.25, device=DEV)      # off = 1: not 16-byte aligned
+    ops.encoder_bwd(dwte, dwpe, d.to(DEV), tok.to(DEV))
+    want = torch.full((V, C), 0.5, dtype=torch.float64).index_add_(0, tok[0].long(), d[0].double())
+    assert_close(dwte, want, 1e-5, 1e-5, "dwte")
+    assert_close(dwpe, 0.25 + d[0].double(), 1e-6, 1e-6, "dwpe")
+
+
 # the forward takes one query tile per CTA up to as many tiles as the chip has SMs and pairs beyond: both sides of the switch, one tile,
 # even and odd tile counts, ragged ends
 @pytest.mark.parametrize("B,T,NH", [(1, 64, 12), (1, 128, 1), (1, 776, 16), (1, 1024, 18), (1, 1100, 16), (2, 1024, 9), (1, 1024, 19), (3, 300, 49), (3, 300, 50)])

@@ -386,6 +386,12 @@ def dbias_reduce(dbias, dout2d) -> None:
 
 
 # ----------------------------------------------------------------------------- attention
+def _attn_f32(num_heads: int, *tensors) -> bool:
+    """fp32 storage on the FMA-pipe kernels: 64-wide heads, contiguous 16-byte aligned tensors."""
+    return (ATTN_IMPL == "tcgen05" and tensors[0].shape[-1] == 3 * 64 * num_heads
+            and all(t.is_cuda and t.dtype == torch.float32 and t.is_contiguous() and t.data_ptr() % 16 == 0 for t in tensors))
+
+
 def attention_fwd(out, lse, qkv, num_heads: int) -> None:
     """Causal multi-head attention on packed qkv [B,T,3C] → out [B,T,C], lse [B,NH,T].
 
@@ -396,6 +402,10 @@ def attention_fwd(out, lse, qkv, num_heads: int) -> None:
     if qkv.is_cuda and ATTN_IMPL == "tcgen05" and hs == 64 and qkv.dtype == torch.bfloat16:
         check(lib().llmb_attention_fwd(ptr(out), ptr(lse), ptr(qkv), B, T, num_heads, ptr(status_word(qkv.device)),
                                        stream()), "attention_fwd")
+        _count()
+        return
+    if qkv.is_cuda and _attn_f32(num_heads, qkv, out, lse):
+        check(lib().llmb_attention_f32_fwd(ptr(out), ptr(lse), ptr(qkv), B, T, num_heads, stream()), "attention_f32_fwd")
         _count()
         return
     if qkv.is_cuda:      # library comparator (LLMB_ATTN=sdpa) and head sizes other than 64
@@ -436,6 +446,12 @@ def attention_bwd(dqkv, dout, qkv, out, lse, num_heads: int, dbias=None) -> None
     if dbias is not None:
         attention_bwd(dqkv, dout, qkv, out, lse, num_heads)
         dbias_reduce(dbias, dqkv.view(B * T, C3))
+        return
+    if qkv.is_cuda and _attn_f32(num_heads, qkv, out, lse, dqkv, dout):
+        dots = scratch("attn_f32_dots", B * num_heads * T * 4, qkv.device)
+        check(lib().llmb_attention_f32_bwd(ptr(dqkv), ptr(dots), ptr(dout), ptr(qkv), ptr(out), ptr(lse), B, T, num_heads, stream()),
+              "attention_f32_bwd")
+        _count(2)
         return
     if qkv.is_cuda:      # library comparator: recompute through SDPA under autograd
         with torch.enable_grad():

@@ -1,0 +1,70 @@
+"""fp32 attention on the GPU (forward, log-sum-exp, backward) against the same formulas in 64 bits."""
+import math
+
+import pytest
+import torch
+
+from llm_mojo_b200 import ops
+
+pytestmark = pytest.mark.gpu
+
+
+def reference(qkv, dout, NH):
+    """out, lse (log2 domain) and dqkv in float64."""
+    B, T, C3 = qkv.shape
+    q, k, v = (t.view(B, T, NH, 64).transpose(1, 2) for t in qkv.double().split(C3 // 3, dim=2))
+    do = dout.double().view(B, T, NH, 64).transpose(1, 2)
+    s = (q @ k.transpose(-1, -2) / 8).masked_fill(~torch.ones(T, T, dtype=torch.bool, device=qkv.device).tril(), float("-inf"))
+    lse = torch.logsumexp(s, dim=-1)
+    p = torch.exp(s - lse.unsqueeze(-1))
+    o = p @ v
+    ds = p * (do @ v.transpose(-1, -2) - (do * o).sum(-1, keepdim=True)) / 8
+    back = lambda t: t.transpose(1, 2).reshape(B, T, C3 // 3)
+    return back(o), lse * math.log2(math.e), torch.cat([back(ds @ k), back(ds.transpose(-1, -2) @ q), back(p.transpose(-1, -2) @ do)], dim=2)
+
+
+def rel(a, b):
+    return ((a.double() - b).norm() / b.norm().clamp_min(1e-300)).item()
+
+
+# one row, part of a tile, tiles of 64 rows exactly and one more, several tiles with a ragged last one; one and several heads
+@pytest.mark.parametrize("B,T,NH", [(1, 1, 1), (2, 16, 3), (1, 63, 2), (1, 64, 1), (2, 65, 2), (1, 128, 5), (3, 200, 2), (1, 1000, 2)])
+@pytest.mark.parametrize("scale", [1.0, 6.0])
+def test_attention_f32(B, T, NH, scale):
+    g = torch.Generator().manual_seed(T)
+    C = 64 * NH
+    qkv = (torch.randn(B, T, 3 * C, generator=g) * scale).cuda()
+    dout = torch.randn(B, T, C, generator=g).cuda()
+    out, lse = torch.empty(B, T, C, device="cuda"), torch.empty(B, NH, T, device="cuda")
+    dqkv = torch.full((B, T, 3 * C), 7.0, device="cuda")
+    dbias = torch.ones(3 * C, device="cuda")
+    assert ops._attn_f32(NH, qkv, out, lse, dqkv, dout)
+    ops.attention_fwd(out, lse, qkv, NH)
+    ops.attention_bwd(dqkv, dout, qkv, out, lse, NH, dbias=dbias)
+    o, l, d = reference(qkv, dout, NH)
+    # a score is a sum of 64 products of size scale^2 (error of order 2^-24 * 8 * scale^2), which the exponential passes on; the sums that
+    # follow add a few 2^-24 each
+    tol = 2.0 ** -24 * (16 + 16 * scale * scale)
+    assert rel(out, o) < tol and rel(dqkv, d) < 2 * tol if T > 1 else rel(out, o) < tol
+    # largest single error of a score: 64 serial additions, each off by at most 2^-24 of a partial sum of the |q k| (mean below scale^2),
+    # in the units of lse
+    assert (lse.double() - l).abs().max() < 64 * 2.0 ** -24 * 64 * scale * scale * math.log2(math.e) / 8 + 2.0 ** -22
+    if T == 1:
+        # one key: dq and dk vanish and dv is dout times a probability of 1, recomputed as 2^(score - lse) from two roundings of the same
+        # score, so off by up to 2^-23 of the score, which is of order 8 * scale^2
+        assert rel(dqkv[..., 2 * C:], dout.double()) < tol and dqkv[..., :2 * C].abs().max() < 1e-4 * scale
+    assert (dbias.double() - 1 - d.sum((0, 1))).abs().max() < 1e-3 * scale
+
+
+def test_layouts_outside_the_kernel_keep_the_library_path():
+    qkv = torch.randn(1, 32, 3 * 64, device="cuda")
+    out, lse = torch.empty(1, 32, 64, device="cuda"), torch.empty(1, 1, 32, device="cuda")
+    assert ops._attn_f32(1, qkv, out, lse)
+    assert not ops._attn_f32(2, qkv, out, lse)                       # 32-wide heads
+    assert not ops._attn_f32(1, qkv.double(), out, lse)
+    assert not ops._attn_f32(1, torch.randn(1, 32, 6 * 64, device="cuda")[..., ::2], out, lse)
+    wide = torch.empty(1, 32, 128, device="cuda")
+    assert not ops._attn_f32(1, qkv, wide[..., :64], lse)
+    ops.attention_fwd(wide[..., :64], lse, qkv, 1)
+    ops.attention_fwd(out, lse, qkv, 1)
+    assert (wide[..., :64] - out).abs().max() < 1e-4                 # fp32 rounding of either path

@@ -138,6 +138,7 @@ class GPT2:
         self.use_stochastic_rounding = False
         self.micro_steps_done = 0
         self.lowp = None
+        self.step_kept: Optional[torch.Tensor] = None     # ops/step.py: operands that a forward pass leaves for its backward pass
         if self.precision.name == "fp8":
             from ..ops.lowp import LowpState
             self.lowp = LowpState(cfg.num_layer, self.device)
@@ -360,8 +361,8 @@ class GPT2:
         self._dloss = dloss = 1.0 / (B * T * grad_accum_steps)
         if "logits" not in a and not (targets is not None and (self.lm_head_chunks > 1 or self.vocab_parallel)):
             a["logits"] = torch.empty(B, T, cfg.padded_vocab_size, dtype=self.dtype, device=self.device)
-        if step.usable(self):
-            return step.forward(self, targets is not None)
+        if step.usable(self) and step.forward(self, targets is not None):
+            return
         z = self.zero
         if z is not None:
             z.before_embedding()
@@ -424,8 +425,7 @@ class GPT2:
             last_micro_step = micro_step == grad_accum_steps - 1
         if micro_step == 0:
             self.zero_gradients()
-        if step.usable(self):
-            step.backward(self)
+        if step.usable(self) and step.backward(self):
             self.micro_steps_done += 1
             return
         cfg, a = self.config, self.acts

@@ -89,11 +89,13 @@ _SIGS = {
     "llmb_attention_bwd_fused_acc_floats": [c_int, c_int, c_int],
     "llmb_loss_accumulate": [c_p, c_p, c_int, c_f, c_p],
     "llmb_gpt2_step_bytes": [],
+    "llmb_gpt2_lowp_scratch_bytes": [c_p],
+    "llmb_gpt2_lowp_kept_bytes": [c_p],
     "llmb_gpt2_forward": [c_p, c_p],
     "llmb_gpt2_backward": [c_p, c_p],
 }
 _RET_LL = {"llmb_encoder_bwd_scratch_bytes", "llmb_dbias_scratch_bytes", "llmb_layernorm_bwd_scratch_bytes",
-           "llmb_nvfp4_scale_bytes", "llmb_attention_bwd_fused_stats_floats", "llmb_attention_bwd_fused_acc_floats"}
+           "llmb_nvfp4_scale_bytes", "llmb_gpt2_lowp_scratch_bytes", "llmb_gpt2_lowp_kept_bytes", "llmb_attention_bwd_fused_stats_floats", "llmb_attention_bwd_fused_acc_floats"}
 
 
 def lib_path() -> str:

@@ -10,9 +10,9 @@ from llm_mojo_b200.ops import _lib, step
 pytestmark = pytest.mark.gpu
 
 
-def run(native, monkeypatch, cfg, B, T, accum, recompute, chunks, targets=True):
+def run(native, monkeypatch, cfg, B, T, accum, recompute, chunks, targets=True, precision="bf16"):
     g = torch.Generator().manual_seed(3)
-    m = GPT2(cfg, "bf16", "cuda", recompute=recompute, lm_head_chunks=chunks)
+    m = GPT2(cfg, precision, "cuda", recompute=recompute, lm_head_chunks=chunks)
     used = []
     if native:
         monkeypatch.setattr(step, "usable", lambda mm, f=step.usable: used.append(f(mm)) or used[-1])
@@ -50,6 +50,31 @@ def test_native_step_matches_op_by_op(L, NH, B, T, accum, recompute, chunks, mon
             assert ((got[k] == 0) == (want[k] == 0)).float().mean() > 0.999, k
         else:
             assert torch.equal(got[k], want[k]), k
+
+
+# TF32 on fp32 storage at lengths no tile divides; FP8 with block scales at whole 128-row tiles; NVFP4 in the middle layers only
+@pytest.mark.parametrize("precision,L,NH,B,T,accum,recompute,chunks", [
+    ("tf32", 2, 2, 2, 77, 2, False, 1), ("tf32", 1, 3, 1, 128, 1, True, 3), ("fp8b", 2, 2, 2, 128, 2, False, 1), ("fp8b", 2, 4, 1, 256, 1, True, 4),
+    ("fp4", 6, 2, 2, 48, 2, False, 1), ("fp4", 5, 4, 1, 224, 1, True, 3)])
+def test_native_step_in_other_precisions(precision, L, NH, B, T, accum, recompute, chunks, monkeypatch):
+    cfg = GPT2Config(max_seq_len=256, vocab_size=1000, num_layer=L, num_heads=NH, channels=64 * NH, padded_vocab_size=1024)
+    want, n_want = run(False, monkeypatch, cfg, B, T, accum, recompute, chunks, precision=precision)
+    got, n_got = run(True, monkeypatch, cfg, B, T, accum, recompute, chunks, precision=precision)
+    assert n_got == n_want
+    for k in want:
+        # gradients: fp32 atomics in another order from run to run; where they are quantised again on the way (NVFP4: to a grid of 1/4 to
+        # 1/2 of a value, the draws being the same) a last bit can move a value to its neighbour
+        if k == "grads":
+            assert (got[k] - want[k]).norm() <= (2.0 ** -5 if precision == "fp4" else 2.0 ** -8) * want[k].norm(), k
+        else:
+            assert torch.equal(got[k], want[k]), k
+
+
+@pytest.mark.parametrize("precision,NH,T", [("fp8b", 2, 96), ("fp8b", 3, 128), ("fp8", 2, 128), ("fp4", 2, 40)])
+def test_other_shapes_and_precisions_stay_op_by_op(precision, NH, T):
+    m = GPT2(GPT2Config(max_seq_len=256, vocab_size=1000, num_layer=1, num_heads=NH, channels=64 * NH, padded_vocab_size=1024), precision, "cuda")
+    m.allocate_activations(1, T)
+    assert not step.usable(m)
 
 
 def test_native_forward_without_targets(monkeypatch):

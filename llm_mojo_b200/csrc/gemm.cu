@@ -1028,6 +1028,14 @@ LLMB_API int llmb_gemm(void* D, const void* A, const void* B, const void* bias, 
   return LLMB_ERR_BAD_ARG;
 }
 
+// How many parts of the contraction an accumulating llmb_gemm (epilogue 4, both operands stored [K, *]) of this size is cut into: with
+// one part the result may as well be stored (epilogue 6) where nothing has to be added to.
+LLMB_API int llmb_gemm_dw_splits(int kind, int M, int N, int K, int splits) {
+  const int kb = ceil_div(K, kind == 0 ? 64 : 32);
+  splits = splits < 1 ? 1 : splits > kb ? kb : splits;
+  return pick_tile(kind == 0 ? KIND_F16 : KIND_TF32, EPI_ACC_F32, M, N, kb, splits, 1, 1).splits;
+}
+
 // Arms the calling thread's NEXT llmb_gemm call to gather its A matrix from W ranks (see GatherArgs): A must be the
 // local [W*n, K] buffer, n a multiple of 256; peer_src[r] = address of chunk r in rank r's buffer; flags = this
 // rank's flag words; counts = 16 local counters that the caller zeroes (stream-ordered) before the GEMM.

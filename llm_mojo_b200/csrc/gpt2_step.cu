@@ -25,6 +25,7 @@ LLMB_API int llmb_gemm(void* D, const void* A, const void* B, const void* bias, 
                        long long ldb, long long ldd, long long ldaux, int a_mn, int b_mn, int kind, int a_fmt, int b_fmt, int epi, int splits,
                        int* status, cudaStream_t st);
 LLMB_API void llmb_gemm_set_colsum(float* colsum);
+LLMB_API int llmb_gemm_dw_splits(int kind, int M, int N, int K, int splits);
 LLMB_API int llmb_attention_fwd(void* out, float* lse, const void* qkv, int B, int T, int NH, int* status, cudaStream_t st);
 LLMB_API int llmb_attention_bwd_fused(void* dqkv, float* dbias, float* stats, float* dq_acc, const void* dout, const void* qkv, const void* out,
                                       const float* lse, int B, int T, int NH, int* status, cudaStream_t st);
@@ -52,7 +53,7 @@ LLMB_API int llmb_ce_pass2(void* tile, const float* stats, const int* targets, i
                            cudaStream_t st);
 
 namespace {
-enum { EPI_NONE = 0, EPI_BIAS = 1, EPI_BIAS_GELU = 2, EPI_DGELU = 3, EPI_ACC_F32 = 4, EPI_BIAS_RESID = 5 };
+enum { EPI_NONE = 0, EPI_BIAS = 1, EPI_BIAS_GELU = 2, EPI_DGELU = 3, EPI_ACC_F32 = 4, EPI_BIAS_RESID = 5, EPI_STORE_F32 = 6 };
 
 // acc += scale * sum(x), one CTA: 16-byte loads, eight in flight per thread.  It replaces a sum, a product and an addition (three
 // launches, 9 us of them the sum of 16384 losses on one SM).
@@ -116,6 +117,8 @@ struct Gpt2Step {
   unsigned char* s_lowp;         // scratch, llmb_gpt2_lowp_scratch_bytes()
   unsigned char* kept;           // FP8B: the layer inputs as operands of the weight gradients, from forward to backward (null in the backward
                                  // pass: quantised again); llmb_gpt2_lowp_kept_bytes()
+  int first;                     // backward: the gradients start from zero (see Step::begin_gradients)
+  int T_max;                     // rows of wpe
 };
 enum { LP_FP8B = 2, LP_FP4 = 3 };
 enum { S_QKV, S_ATT, S_FC, S_PROJ };
@@ -179,14 +182,47 @@ struct Step {
   }
   // dinp[rows, K] = dout[rows, N] W[N, K] (times GELU' of aux, or plus aux), then dW[N, K] += dout^T inp
   bool linear_bwd(void* dinp, float* dw, const void* dout, const void* inp, const void* w, void* aux, int N, int K, int epi, int splits,
-                  float* colsum = nullptr, long long ldo = 0) {
+                  bool store, float* colsum = nullptr, long long ldo = 0) {
     const long long lo = ldo ? ldo : N;
     if (colsum) llmb_gemm_set_colsum(colsum);
     return ok(llmb_gemm(dinp, dout, w, nullptr, aux, nullptr, rows, K, N, lo, K, K, aux ? K : 0, 0, 1, kind, 0, 0, epi, 1, s.status, st)) &&
-           ok(llmb_gemm(dw, dout, inp, nullptr, nullptr, nullptr, N, K, rows, lo, K, K, 0, 1, 1, kind, 0, 0, EPI_ACC_F32, splits, s.status, st));
+           ok(llmb_gemm(dw, dout, inp, nullptr, nullptr, nullptr, N, K, rows, lo, K, K, 0, 1, 1, kind, 0, 0, store ? EPI_STORE_F32 : EPI_ACC_F32, splits,
+                        s.status, st));
+  }
+  // A micro-step that starts the accumulation leaves out the zero fill and the read of every gradient that ONE kernel writes as a whole
+  // (weights whose contraction is not split: the widest ones, where these bytes count); what is added to in parts - split weights,
+  // biases, LayerNorms, positions - is filled here.
+  // d36 fp8b, B 4, T 1024: 36.07 -> 35.63 ms a step, d48 NVFP4 61.63 -> 60.73; d12, where the layers' weights are split, unchanged.
+  bool store_qkv = false, store_att = false, store_fc = false, store_proj = false, store_head = false;
+  bool begin_gradients() {
+    if (!s.first) return true;
+    const size_t cc = (size_t)C * C, LC = (size_t)s.L * C;
+    // one rule for a tensor of all layers: every layer's product must be in one part
+    auto one = [&](int st_, int N, int K, int splits, int lp_splits) {
+      bool plain = false, lp = false;
+      for (int l = 0; l < s.L; ++l) (mode(st_, l) ? lp : plain) = true;
+      return (!plain || llmb_gemm_dw_splits(kind, N, K, rows, splits) == 1) && (!lp || lp_splits == 1);
+    };
+    store_qkv = one(S_QKV, 3 * C, C, s.splits_qkv, s.lp_splits_qkv);
+    store_att = one(S_ATT, C, C, s.splits_att, s.lp_splits_att);
+    store_fc = one(S_FC, 4 * C, C, s.splits_fc, s.lp_splits_fc);
+    store_proj = one(S_PROJ, C, 4 * C, s.splits_proj, s.lp_splits_proj);
+    const int tile = s.tile_width > 0 ? s.tile_width : s.Vp, rest = s.Vp - (s.Vp - 1) / tile * tile;
+    store_head = llmb_gemm_dw_splits(kind, tile, C, rows, s.splits_head) == 1 && llmb_gemm_dw_splits(kind, rest, C, rows, s.splits_head_last) == 1;
+    const size_t n[P_COUNT] = {store_head ? 0 : (size_t)s.Vp * C, (size_t)s.T_max * C, LC, LC, store_qkv ? 0 : 3 * cc * s.L, 3 * LC, store_att ? 0 : cc * s.L, LC,
+                               LC, LC, store_fc ? 0 : 4 * cc * s.L, 4 * LC, store_proj ? 0 : 4 * cc * s.L, LC, (size_t)C, (size_t)C};
+    float *from = nullptr, *to = nullptr;                 // neighbours in memory are filled together
+    for (int i = 0; i <= P_COUNT; ++i) {
+      if (i < P_COUNT && n[i] && s.g[i] == to) { to += n[i]; continue; }
+      if (i < P_COUNT && !n[i]) continue;
+      if (from != to && !ok((int)cudaMemsetAsync(from, 0, (to - from) * sizeof(float), st), 0)) return false;
+      if (i < P_COUNT) { from = s.g[i]; to = from + n[i]; }
+    }
+    return true;
   }
   bool site_bwd(int st_, int l, void* dinp, float* dw, const void* dout, const void* inp, const void* w, void* aux, int N, int K, int epi,
-                int splits, int lp_splits, float* colsum = nullptr) {
+                int splits, int lp_splits, bool store, float* colsum = nullptr) {
+    const int acc = store ? EPI_STORE_F32 : EPI_ACC_F32;
     if (mode(st_, l) == LP_FP8B) {
       const size_t nd = (size_t)rows * N, sd_n = sf8_bytes(rows, N);
       unsigned char *qd = s.s_lowp, *sd = qd + nd, *qdt = sd + sd_n, *sdt = qdt + nd, *wq = sdt + sd_n, *wsf = wq + (size_t)N * K;
@@ -197,7 +233,7 @@ struct Step {
         qx = wsf + sf8_bytes(N, K);
         if (!ok(llmb_fp8_block_quant(qx, qx + (size_t)rows * K, inp, rows, K, 1, 0, 1, st))) return false;
       }
-      return ok(llmb_gemm_mxfp8(dw, qdt, qx, sdt, qx + (size_t)rows * K, nullptr, nullptr, nullptr, N, K, rows, 1, 0, K, 0, EPI_ACC_F32, lp_splits, s.status, st));
+      return ok(llmb_gemm_mxfp8(dw, qdt, qx, sdt, qx + (size_t)rows * K, nullptr, nullptr, nullptr, N, K, rows, 1, 0, K, 0, acc, lp_splits, s.status, st));
     }
     if (mode(st_, l) == LP_FP4) {
       const Op4 d(s.s_lowp, rows, N, true, true), ww(d.end, N, K, false, true), x(ww.end, rows, K, false, true);
@@ -207,9 +243,9 @@ struct Step {
              ok(llmb_gemm_nvfp4(dinp, d.q0, ww.q1, d.sf0, ww.sf1, nullptr, aux, ww.ws + 3, rows, K, N, K, aux ? K : 0, epi, 1, s.status, st)) &&
              ok(llmb_nvfp4_operand(nullptr, nullptr, x.q1, x.sf1, x.ws, inp, rows, K, 0, s.fp4_rht, 0, 0, 0, 0, 0, nullptr, 1.f, d.ws + 1,
                                    s.fp4_rht ? 1.f / 16.f : 1.f, st), 2) &&
-             ok(llmb_gemm_nvfp4(dw, d.q1, x.q1, d.sf1, x.sf1, nullptr, nullptr, x.ws + 3, N, K, rows, K, 0, EPI_ACC_F32, lp_splits, s.status, st));
+             ok(llmb_gemm_nvfp4(dw, d.q1, x.q1, d.sf1, x.sf1, nullptr, nullptr, x.ws + 3, N, K, rows, K, 0, acc, lp_splits, s.status, st));
     }
-    return linear_bwd(dinp, dw, dout, inp, w, aux, N, K, epi, splits, colsum);
+    return linear_bwd(dinp, dw, dout, inp, w, aux, N, K, epi, splits, store, colsum);
   }
   static constexpr unsigned long long FP4_STREAM = 16;    // NVFP4_SR_STREAM of ops/lowp.py
   bool attention(int l, size_t rc1, size_t lse) {
@@ -263,6 +299,7 @@ struct Step {
 
   void backward() {
     const size_t rc1 = (size_t)rows * C, cc = (size_t)C * C, lse = (size_t)s.B * s.NH * s.T;
+    if (!begin_gradients()) return;
     void *dres = s.a[A_DRES], *dl = s.a[A_DL], *dl4 = s.a[A_DL4], *dqkv = s.a[A_DL4];
     if (s.tile_width > 0) {                               // every logits tile again, as dlogits, consumed at once
       for (int c0 = 0; c0 < s.Vp && !rc; c0 += s.tile_width) {
@@ -271,10 +308,10 @@ struct Step {
         linear(a(A_LOGITS), a(A_LNF), p(P_WTE, c0, C), nullptr, nullptr, w, C, EPI_NONE, s.tile_width) &&
         ok(llmb_ce_pass2(a(A_LOGITS), f(A_CE_STATS), s.targets, rows, s.tile_width, c0, w, s.V, s.dloss, dt, st)) &&
         linear_bwd(dl, g(P_WTE, c0, C), a(A_LOGITS), a(A_LNF), p(P_WTE, c0, C), c0 ? dl : nullptr, w, C, c0 ? EPI_BIAS_RESID : EPI_NONE,
-                   last ? s.splits_head_last : s.splits_head, nullptr, s.tile_width);
+                   last ? s.splits_head_last : s.splits_head, store_head, nullptr, s.tile_width);
       }
     } else {
-      linear_bwd(dl, s.g[P_WTE], a(A_LOGITS), a(A_LNF), s.p[P_WTE], nullptr, s.Vp, C, EPI_NONE, s.splits_head);
+      linear_bwd(dl, s.g[P_WTE], a(A_LOGITS), a(A_LNF), s.p[P_WTE], nullptr, s.Vp, C, EPI_NONE, s.splits_head, store_head);
     }
     if (rc || !ln_bwd(s.g[P_LNFW], s.g[P_LNFB], a(A_RES3, s.L - 1, rc1), s.p[P_LNFW], f(A_LNF_MEAN), f(A_LNF_RSTD), 0)) return;
     for (int l = s.L - 1; l >= 0 && !rc; --l) {
@@ -284,15 +321,15 @@ struct Step {
       float* dfcb = g(P_FCB, l, 4 * C);
       const bool fused = s.fc_colsum && mode(S_PROJ, l) == 0;               // the dGELU GEMM takes the fc bias gradient
       site_bwd(S_PROJ, l, dl4, g(P_PROJW, l, 4 * cc), dres, act, p(P_PROJW, l, 4 * cc), a(A_FCH, l, 4 * rc1), C, 4 * C, EPI_DGELU, s.splits_proj,
-               s.lp_splits_proj, fused ? dfcb : nullptr) &&
+               s.lp_splits_proj, store_proj, fused ? dfcb : nullptr) &&
       (fused || bias_grad(dfcb, dl4, 4 * C)) &&
       bias_grad(g(P_PROJB, l, C), dres, C) &&
-      site_bwd(S_FC, l, dl, g(P_FCW, l, 4 * cc), dl4, a(A_LN2, l, rc1), p(P_FCW, l, 4 * cc), nullptr, 4 * C, C, EPI_NONE, s.splits_fc, s.lp_splits_fc) &&
+      site_bwd(S_FC, l, dl, g(P_FCW, l, 4 * cc), dl4, a(A_LN2, l, rc1), p(P_FCW, l, 4 * cc), nullptr, 4 * C, C, EPI_NONE, s.splits_fc, s.lp_splits_fc, store_fc) &&
       ln_bwd(g(P_LN2W, l, C), g(P_LN2B, l, C), a(A_RES2, l, rc1), p(P_LN2W, l, C), f(A_LN2_MEAN, l), f(A_LN2_RSTD, l), 1) &&
-      site_bwd(S_ATT, l, dl, g(P_ATTW, l, cc), dres, a(A_ATTY, l, rc1), p(P_ATTW, l, cc), nullptr, C, C, EPI_NONE, s.splits_att, s.lp_splits_att) &&
+      site_bwd(S_ATT, l, dl, g(P_ATTW, l, cc), dres, a(A_ATTY, l, rc1), p(P_ATTW, l, cc), nullptr, C, C, EPI_NONE, s.splits_att, s.lp_splits_att, store_att) &&
       bias_grad(g(P_ATTB, l, C), dres, C) &&
       attention_bwd(dqkv, l, rc1, lse) &&
-      site_bwd(S_QKV, l, dl, g(P_QKVW, l, 3 * cc), dqkv, a(A_LN1, l, rc1), p(P_QKVW, l, 3 * cc), nullptr, 3 * C, C, EPI_NONE, s.splits_qkv, s.lp_splits_qkv) &&
+      site_bwd(S_QKV, l, dl, g(P_QKVW, l, 3 * cc), dqkv, a(A_LN1, l, rc1), p(P_QKVW, l, 3 * cc), nullptr, 3 * C, C, EPI_NONE, s.splits_qkv, s.lp_splits_qkv, store_qkv) &&
       ln_bwd(g(P_LN1W, l, C), g(P_LN1B, l, C), x, p(P_LN1W, l, C), f(A_LN1_MEAN, l), f(A_LN1_RSTD, l), 1);
     }
     if (!rc) ok(llmb_encoder_bwd(s.g[P_WTE], s.g[P_WPE], dres, s.tokens, s.s_encoder, s.s_encoder_bytes, s.B, s.T, C, s.Vp, s.vocab_bits, dt, st), 4);

@@ -423,11 +423,11 @@ class GPT2:
         soon as it is complete."""
         if last_micro_step is None:
             last_micro_step = micro_step == grad_accum_steps - 1
-        if micro_step == 0:
-            self.zero_gradients()
-        if step.usable(self) and step.backward(self):
+        if step.usable(self) and step.backward(self, micro_step == 0):
             self.micro_steps_done += 1
             return
+        if micro_step == 0:
+            self.zero_gradients()
         cfg, a = self.config, self.acts
         L, NH = cfg.num_layer, cfg.num_heads
         z = self.zero

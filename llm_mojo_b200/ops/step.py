@@ -29,7 +29,7 @@ class Gpt2Step(ctypes.Structure):
                 ("splits_qkv", I), ("splits_att", I), ("splits_fc", I), ("splits_proj", I), ("splits_head", I), ("splits_head_last", I),
                 ("vocab_bits", I), ("launches", I), ("dtype", I), ("lowp", I), ("fp4_first", I), ("fp4_end", I), ("fp4_rht", I), ("fp4_sr", I),
                 ("lp_splits_qkv", I), ("lp_splits_att", I), ("lp_splits_fc", I), ("lp_splits_proj", I), ("seed", ctypes.c_ulonglong),
-                ("micro", LL), ("s_lowp", P), ("kept", P)]
+                ("micro", LL), ("s_lowp", P), ("kept", P), ("first", I), ("T_max", I)]
 
 
 PLAIN, FP8B, FP4 = 0, 2, 3      # what the linear sites run in (LP_* of the C side)
@@ -108,14 +108,18 @@ def forward(m, targets: bool) -> bool:
     return True
 
 
-def backward(m) -> bool:
-    """As ``forward``."""
+def backward(m, first: bool) -> bool:
+    """As ``forward``.  ``first``: whatever the gradients hold is discarded."""
     cfg, a, dev = m.config, m.acts, m.device
     tiled = m.lm_head_chunks > 1
     s = _fill(m, tiled, True)
     if s is None:
         return False
-    s.g[:] = [m.g[n].data_ptr() for n in PARAM_NAMES]
+    grads = _addresses(m.g, PARAM_NAMES, torch.float32)
+    if grads is None:
+        return False
+    s.g[:] = grads
+    s.first, s.T_max = int(first), m.config.max_seq_len
     B, T, C, NH, Vp = m.B, m.T, cfg.channels, cfg.num_heads, cfg.padded_vocab_size
     rows, L = B * T, lib()
     s.fc_colsum = int(colsum_usable(a["dl_bt4c"].view(rows, 4 * C), a["fch"][0].view(rows, 4 * C)))

@@ -19,6 +19,7 @@ def run(native, monkeypatch, cfg, B, T, accum, recompute, chunks, targets=True, 
     else:
         monkeypatch.setattr(step, "usable", lambda mm: False)
     n0 = ops.LAUNCHES
+    m.grads.fill_(float("nan"))      # the first micro-step discards whatever is there
     for micro in range(accum):
         toks = torch.randint(0, cfg.vocab_size, (B * T + 1,), generator=g, dtype=torch.int32)
         m.forward(toks[:-1].view(B, T), toks[1:].view(B, T) if targets else None, accum)
@@ -27,6 +28,8 @@ def run(native, monkeypatch, cfg, B, T, accum, recompute, chunks, targets=True, 
     launches = ops.LAUNCHES - n0
     monkeypatch.undo()
     assert all(used) and (used or not native)
+    if not targets:
+        m.grads.zero_()
     out = {"grads": m.grads.clone(), "loss": torch.tensor(m.read_loss()), "lnf": m.acts["lnf"].clone()}
     if targets:
         out["losses"] = m.acts["losses"].clone()
@@ -38,7 +41,8 @@ def run(native, monkeypatch, cfg, B, T, accum, recompute, chunks, targets=True, 
 
 # sequence lengths around the 128-row tiles and the smallest; vocabulary tiles of equal and unequal width; one and several layers
 @pytest.mark.parametrize("L,NH,B,T,accum,recompute,chunks", [
-    (1, 1, 1, 16, 1, False, 1), (2, 3, 2, 127, 2, False, 1), (3, 2, 1, 129, 1, True, 1), (2, 2, 3, 200, 2, True, 3), (2, 4, 2, 256, 1, False, 4)])
+    (1, 1, 1, 16, 1, False, 1), (2, 3, 2, 127, 2, False, 1), (3, 2, 1, 129, 1, True, 1), (2, 2, 3, 200, 2, True, 3), (2, 4, 2, 256, 1, False, 4),
+    (1, 12, 16, 256, 2, False, 1)])      # the last: head stored, layer weights split
 def test_native_step_matches_op_by_op(L, NH, B, T, accum, recompute, chunks, monkeypatch):
     cfg = GPT2Config(max_seq_len=256, vocab_size=1000, num_layer=L, num_heads=NH, channels=64 * NH, padded_vocab_size=1024)
     want, n_want = run(False, monkeypatch, cfg, B, T, accum, recompute, chunks)

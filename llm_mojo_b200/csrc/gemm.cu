@@ -591,9 +591,14 @@ Tile pick_tile(int kind, int epi, int M, int N, int kb_total, int splits, int a_
       if (acc)                                            // one round of CTAs, at least four k-blocks each
         while (sp < 16 && tiles * (sp + 1) <= sms && kb_total / (sp + 1) >= 4) ++sp;
       const float per_sm = (float)(tiles * cl * sp) / sms;
-      const float w = per_sm <= 1.f ? 1.f : 0.5f * (per_sm + ceilf(per_sm));
+      // one to two CTAs per SM and operands stored along K: the second CTA of an SM overlaps the first one's epilogue, and the kernels
+      // before and after overlap the short tail (in a chain of layers: M 776, K 1024, N 3072, 168 CTAs 2.8 us less than the pair kernel,
+      // N 4096 with GELU, 224 CTAs, 3.1 us less; as isolated launches the two are level).  Not with an auxiliary input: bias + residual at
+      // M 4096, N 768 (192 CTAs) on these tiles made a d12 step of 4 x 1024 2 % slower.
+      const bool beside = per_sm > 1.f && per_sm <= 2.f && !a_mn && !b_mn && epi != EPI_BIAS_RESID && epi != EPI_DGELU;
+      const float w = per_sm <= 1.f ? 1.f : beside ? per_sm : 0.5f * (per_sm + ceilf(per_sm));
       const float fixed = (cl == 1 ? (bn == 64 ? 4.2f : 5.0f) : cl == 2 ? 5.6f : 6.2f) + (aux ? (bn == 64 ? 0.3f : 1.2f) : 0.f) + f32;
-      const float est = fixed + w * ceil_div(kb_total, cl * sp) * 0.24f * mn + (w - 1.f) * (aux ? 3.0f : 0.7f) * (bn / 64);
+      const float est = fixed + w * ceil_div(kb_total, cl * sp) * 0.24f * mn + (w - 1.f) * (!aux ? 0.7f : beside ? 1.0f : 3.0f) * (bn / 64);
       if (est < best) { best = est; t = {bn, cl, sp}; }
     }
   }

@@ -386,10 +386,36 @@ def dbias_reduce(dbias, dout2d) -> None:
 
 
 # ----------------------------------------------------------------------------- attention
-def _attn_f32(num_heads: int, *tensors) -> bool:
-    """fp32 storage on the FMA-pipe kernels: 64-wide heads, contiguous 16-byte aligned tensors."""
-    return (ATTN_IMPL == "tcgen05" and tensors[0].shape[-1] == 3 * 64 * num_heads
-            and all(t.is_cuda and t.dtype == torch.float32 and t.is_contiguous() and t.data_ptr() % 16 == 0 for t in tensors))
+def _attn_f32(num_heads: int, qkv, out, lse, *more) -> bool:
+    """fp32 storage on the FMA-pipe kernels: 64-wide heads; contiguous 16-byte aligned tensors of the sizes that the kernels read and
+    write (``more``: dqkv and dout of the backward pass).  They write while they read, so no output may lie over an input."""
+    B, T, C3 = qkv.shape
+    tensors = [qkv, out, lse, *more]
+    if ATTN_IMPL != "tcgen05" or C3 != 3 * 64 * num_heads or qkv.numel() == 0 or any(t is None for t in tensors):
+        return False
+    sizes = (B * T * C3, B * T * C3 // 3, B * num_heads * T, B * T * C3, B * T * C3 // 3)
+    if not all(t.is_cuda and t.dtype == torch.float32 and t.is_contiguous() and t.data_ptr() % 16 == 0 and t.numel() == n
+               for t, n in zip(tensors, sizes)):
+        return False
+    if not more and torch.is_grad_enabled() and qkv.requires_grad:       # a forward that autograd records
+        return False
+    spans = [(t.data_ptr(), t.data_ptr() + 4 * n) for t, n in zip(tensors, sizes)]
+    apart = lambda i, j: spans[i][1] <= spans[j][0] or spans[j][1] <= spans[i][0]
+    return all(apart(i, j) for i in ((3,) if more else (1, 2)) for j in range(len(tensors)) if i != j)
+
+
+def _attn_f32_fwd_any(out, lse, qkv, num_heads: int) -> None:
+    """The fp32 forward kernel through temporaries, for tensors that it does not take as they are.  Whatever form the forward's tensors
+    had, the backward kernel then finds the log-sum-exp that it reads."""
+    B, T, C3 = qkv.shape
+    x = qkv.detach().clone(memory_format=torch.contiguous_format)
+    o = torch.empty(B, T, C3 // 3, dtype=torch.float32, device=qkv.device)
+    l = torch.empty(B, num_heads, T, dtype=torch.float32, device=qkv.device)
+    check(lib().llmb_attention_f32_fwd(ptr(o), ptr(l), ptr(x), B, T, num_heads, stream()), "attention_f32_fwd")
+    _count()
+    if out is not None:
+        out.copy_(o)
+    lse.detach().copy_(l.view(lse.shape))
 
 
 def attention_fwd(out, lse, qkv, num_heads: int) -> None:
@@ -409,6 +435,14 @@ def attention_fwd(out, lse, qkv, num_heads: int) -> None:
         _count()
         return
     if qkv.is_cuda:      # library comparator (LLMB_ATTN=sdpa) and head sizes other than 64
+        # an lse of the right size may be read by the backward kernel, which chooses its path by its own tensors
+        wants_lse = (ATTN_IMPL == "tcgen05" and hs == 64 and qkv.dtype == torch.float32 and qkv.numel() > 0 and lse is not None
+                     and lse.numel() == B * num_heads * T)
+        recorded = torch.is_grad_enabled() and qkv.requires_grad
+        if wants_lse:
+            _attn_f32_fwd_any(None if recorded else out, lse, qkv, num_heads)
+            if not recorded:
+                return
         q, k, v = (t.view(B, T, num_heads, hs).transpose(1, 2) for t in qkv.split(C, dim=2))
         out.copy_(F.scaled_dot_product_attention(q, k, v, is_causal=True).transpose(1, 2).reshape(B, T, C))
         return

@@ -68,3 +68,72 @@ def test_layouts_outside_the_kernel_keep_the_library_path():
     ops.attention_fwd(wide[..., :64], lse, qkv, 1)
     ops.attention_fwd(out, lse, qkv, 1)
     assert (wide[..., :64] - out).abs().max() < 1e-4                 # fp32 rounding of either path
+
+
+def _inputs(B=2, T=80, NH=2):
+    g = torch.Generator().manual_seed(4)
+    qkv, dout = torch.randn(B, T, 192 * NH, generator=g).cuda(), torch.randn(B, T, 64 * NH, generator=g).cuda()
+    return qkv, dout, torch.empty(B, T, 64 * NH, device="cuda"), torch.full((B, NH, T), float("nan"), device="cuda")
+
+
+TOL = 2.0 ** -24 * 64          # as in test_attention_f32 at scale 1, either path
+
+
+# the forward and the backward choose their path by their own tensors: each form of the forward, followed by the backward kernel
+@pytest.mark.parametrize("form", ["plain", "strided out", "strided qkv", "unaligned qkv", "strided lse", "unaligned lse", "bf16 out", "recorded"])
+def test_backward_after_every_form_of_the_forward(form):
+    qkv, dout, out, lse = _inputs()
+    B, T, C = out.shape
+    o, l, x = out, lse, qkv
+    if form == "strided out":
+        o = torch.empty(B, T, 2 * C, device="cuda")[..., :C]
+    elif form == "bf16 out":
+        o = torch.empty(B, T, C, device="cuda", dtype=torch.bfloat16)
+    elif form == "strided qkv":
+        x = torch.empty(B, T, 6 * C, device="cuda")[..., ::2].copy_(qkv)
+    elif form == "unaligned qkv":
+        x = torch.empty(qkv.numel() + 1, device="cuda")[1:].view(qkv.shape).copy_(qkv)
+    elif form == "strided lse":
+        l = torch.empty(*lse.shape, 2, device="cuda")[..., 0]
+    elif form == "unaligned lse":
+        l = torch.empty(lse.numel() + 1, device="cuda")[1:].view(lse.shape)
+    elif form == "recorded":
+        x = qkv.clone().requires_grad_(True)
+    assert ops._attn_f32(2, x, o, l) == (form == "plain")
+    ops.attention_fwd(o, l, x, 2)
+    want_o, want_l, want_d = reference(qkv, dout, 2)
+    assert rel(o.detach(), want_o) < (2.0 ** -8 if form == "bf16 out" else TOL)
+    assert (l.double() - want_l).abs().max() < 1e-5
+    if form == "recorded":        # autograd saw the forward
+        o.backward(dout)
+        assert rel(x.grad, want_d) < 2 * TOL
+    saved, lse = o.detach().float().contiguous(), l.clone(memory_format=torch.contiguous_format)
+    dqkv = torch.empty_like(qkv)
+    assert ops._attn_f32(2, qkv, saved, lse, dqkv, dout)
+    ops.attention_bwd(dqkv, dout, qkv, saved, lse, 2)
+    # a rounded output enters through sum(dO * O) only
+    assert rel(dqkv, want_d) < (2.0 ** -8 if form == "bf16 out" else 2 * TOL)
+
+
+# what the library path took without looking at lse or out: no lse, one of another size, gradients over their inputs, nothing at all
+@pytest.mark.parametrize("form", ["no lse", "short lse", "no out", "in place", "empty"])
+def test_calls_that_need_no_saved_statistics(form):
+    qkv, dout, out, lse = _inputs()
+    want_o, _, want_d = reference(qkv, dout, 2)
+    dqkv = torch.empty_like(qkv)
+    if form == "no lse":
+        lse = None
+    elif form == "short lse":
+        lse = torch.full((4,), 9.0, device="cuda")
+    elif form == "in place":
+        dqkv = qkv
+    elif form == "empty":
+        qkv, dout, out, lse, dqkv = qkv[:0], dout[:0], out[:0], lse[:0], dqkv[:0]
+    ops.attention_fwd(out, lse, qkv, 2)
+    saved = None if form == "no out" else out
+    ops.attention_bwd(dqkv, dout, qkv, saved, lse, 2)
+    if form == "empty":
+        return
+    assert rel(out, want_o) < TOL and rel(dqkv, want_d) < 2 * TOL
+    if form == "short lse":
+        assert bool((lse == 9.0).all())

@@ -343,12 +343,17 @@ template <typename T> __device__ __forceinline__ float exp_row(float d);
 template <> __device__ __forceinline__ float exp_row<float>(float d) { return expf(d); }
 template <> __device__ __forceinline__ float exp_row<__nv_bfloat16>(float d) { return ex2_fast(d * 1.4426950408889634f); }
 
-// (max, sum of exp(x - max)) of two disjoint sets of values
+// (max, sum of exp(x - max)) of two disjoint sets of values.  fmaxf passes over NaN: a set of nothing but NaN and -infinity has the
+// maximum -infinity, and its sum says which (NaN, or 0 where all are -infinity).
 __device__ __forceinline__ float2 merge_ms(float2 a, float2 b) {
   const float m = fmaxf(a.x, b.x);
-  if (m == -INFINITY) return make_float2(m, 0.f);
+  if (m == -INFINITY) return make_float2(m, a.x + b.x != m ? NAN : a.y + b.y);
   return make_float2(m, a.y * expf(a.x - m) + b.y * expf(b.x - m));
 }
+// the set of one value
+__device__ __forceinline__ float2 single_ms(float x) { return make_float2(x, x == -INFINITY ? 0.f : 1.f); }
+// what the exponents of a set are taken relative to: its maximum, if that is finite
+__device__ __forceinline__ float base_ms(float m) { return m == -INFINITY ? 0.f : m; }
 __device__ __forceinline__ float2 warp_merge_ms(float2 v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v = merge_ms(v, make_float2(__shfl_xor_sync(0xffffffffu, v.x, o), __shfl_xor_sync(0xffffffffu, v.y, o)));
@@ -385,9 +390,9 @@ __global__ void __launch_bounds__(512) softmax_rows_kernel(float* __restrict__ o
     }
 #pragma unroll
     for (int k = 0; k < N; ++k) m = fmaxf(m, x[k]);
-    if (m == -INFINITY) continue;
+    const float m0 = base_ms(m);
 #pragma unroll
-    for (int k = 0; k < N; ++k) sum += expf(x[k] - m);
+    for (int k = 0; k < N; ++k) sum += expf(x[k] - m0);
     ms = merge_ms(ms, make_float2(m, sum));
   }
   ms = warp_merge_ms(ms);
@@ -542,18 +547,18 @@ __global__ void __launch_bounds__(256) ce_pass1_kernel(float4* __restrict__ stat
 #pragma unroll
         for (int k = 0; k < N; ++k) m = fmaxf(m, p.v[k]);
       }
-    if (m == -INFINITY) continue;
     float s = ms.x == m ? ms.y : ms.y * exp_row<T>(ms.x - m);
+    const float m0 = base_ms(m);
 #pragma unroll
     for (int u = 0; u < U; ++u)
       if (v0 + u * 256 < nvec) {
         Pack<T> p; p.load(reinterpret_cast<const T*>(&raw[u]));
 #pragma unroll
-        for (int k = 0; k < N; ++k) s += exp_row<T>(p.v[k] - m);
+        for (int k = 0; k < N; ++k) s += exp_row<T>(p.v[k] - m0);
       }
     ms = make_float2(m, s);
   }
-  for (int i = nvec * N + tid; i < valid; i += 256) ms = merge_ms(ms, make_float2(to_f<T>(g[i]), 1.f));
+  for (int i = nvec * N + tid; i < valid; i += 256) ms = merge_ms(ms, single_ms(to_f<T>(g[i])));
   ms = warp_merge_ms(ms);
   if (lane == 0) red[wid] = ms;
   __syncthreads();

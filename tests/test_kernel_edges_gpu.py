@@ -237,3 +237,44 @@ def test_attention_fwd_tiles_per_item(B, T, NH):
     assert_close(out, ref, 2.0 ** -7, 2.0 ** -7, "out")          # bf16 probabilities and output, values of order one
     assert_close(lse, lse_ref, 1e-3, 1e-4, "lse")
     assert _lib.read_status() == 0
+
+
+# NaN and -infinity where a whole vector, a thread's whole share, a scalar tail or a row holds nothing else; masks of -infinity
+@pytest.mark.parametrize("rows", [3, 64])              # softmax: a cluster of CTAs per row / one CTA per row
+@pytest.mark.parametrize("V", [9, 4099])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_nan_reaches_every_denominator(rows, V, dtype):
+    ld = (V + 15) // 8 * 8
+    for where in (slice(0, 8), slice(V - 1, V), slice(0, V), slice(V // 2, V // 2 + 1)):
+        for around in (0.5, float("-inf")):
+            x = rnd(rows, ld, dtype=dtype)
+            x[1] = around
+            x[1, where] = float("nan")
+            got = ops.softmax_rows(x.to(DEV), V).cpu()
+            assert bool(torch.isnan(got[1]).all()), (where, around)
+            assert_close(got[[0, 2]], torch.softmax(x[[0, 2], :V].float(), dim=-1), 1e-7, 2e-5, "rows beside it")
+            stats, losses = torch.empty(rows, 4, device=DEV), torch.empty(rows, device=DEV)
+            tgt = torch.zeros(rows, dtype=torch.int32, device=DEV)
+            for c0 in range(0, ld, 2048):                  # several tiles: the NaN has to last
+                w = min(2048, ld - c0)
+                ops.chunked_ce_pass1(stats, x.to(DEV)[:, c0:c0 + w], tgt, c0, w, V, c0 == 0)
+            ops.chunked_ce_loss(losses, stats)
+            assert bool(torch.isnan(losses[1])), (where, around)
+            assert_close(losses[[0, 2]], torch.nn.functional.cross_entropy(x[[0, 2], :V].float(), torch.zeros(2, dtype=torch.long), reduction="none"),
+                         1e-5, 1e-5, "losses beside it")
+
+
+@pytest.mark.parametrize("mask", [float("-inf"), "lowest"])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_masked_logits_count_as_nothing(mask, dtype):
+    rows, V = 5, 3001
+    x = rnd(rows, 3008, dtype=dtype, scale=3.0)
+    x[:, 100:2900] = torch.finfo(dtype).min if mask == "lowest" else mask
+    assert_close(ops.softmax_rows(x.to(DEV), V), torch.softmax(x[:, :V].double(), dim=-1), 1e-7, 2e-5, "softmax")
+    stats, losses = torch.empty(rows, 4, device=DEV), torch.empty(rows, device=DEV)
+    tgt = torch.tensor([0, 99, 2900, 3000, 5], dtype=torch.int32)
+    for c0 in (0, 1000, 2000):                             # the middle tile is masked as a whole
+        ops.chunked_ce_pass1(stats, x.to(DEV)[:, c0:c0 + 1008 if c0 == 2000 else c0 + 1000], tgt.to(DEV), c0, 1008 if c0 == 2000 else 1000, V, c0 == 0)
+    ops.chunked_ce_loss(losses, stats)
+    want = torch.nn.functional.cross_entropy(x[:, :V].double(), tgt.long(), reduction="none")
+    assert_close(losses, want, 1e-5, 1e-5, "losses")

@@ -588,8 +588,8 @@ Tile pick_tile(int kind, int epi, int M, int N, int kb_total, int splits, int a_
     for (int cl = 1; cl <= (bn == 64 ? 4 : 2); cl *= 2) {
       if (cl > 1 && (acc || kind == KIND_TF32 || tiles * cl > sms || cl > kb_total)) break;
       int sp = 1;
-      if (acc)                                            // one round of CTAs, at least four k-blocks each
-        while (sp < 16 && tiles * (sp + 1) <= sms && kb_total / (sp + 1) >= 4) ++sp;
+      if (acc)                                            // one round of CTAs, at least four k-blocks each, no more parts than asked for
+        while (sp < splits && tiles * (sp + 1) <= sms && kb_total / (sp + 1) >= 4) ++sp;
       const float per_sm = (float)(tiles * cl * sp) / sms;
       // one to two CTAs per SM and operands stored along K: the second CTA of an SM overlaps the first one's epilogue, and the kernels
       // before and after overlap the short tail (in a chain of layers: M 776, K 1024, N 3072, 168 CTAs 2.8 us less than the pair kernel,
@@ -1020,7 +1020,8 @@ int launch_nvfp4(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap
 
 // D[M,N] = epi(alpha * A·B^T).  a_mn/b_mn = 1 when the operand is stored [K, M] / [K, N].
 // kind: 0 bf16, 1 tf32 (fp32 storage), 2 fp8 (a_fmt/b_fmt: 0 e4m3, 1 e5m2).  D is bf16 except for the
-// fp32 epilogues (4 = accumulate with red.add, split-K allowed; 6 = plain fp32 store).
+// fp32 epilogues (4 = accumulate with red.add; 6 = plain fp32 store).  splits: the most parts that K may be cut into by an accumulating
+// product.  Parts are added in the order in which they finish, so with one part the result is the same on every run.
 // `status` is a device int the kernel sets to LLMB_ERR_TIMEOUT if a bounded wait expires.
 LLMB_API int llmb_gemm(void* D, const void* A, const void* B, const void* bias, void* aux, const float* alpha, int M,
                        int N, int K, long long lda, long long ldb, long long ldd, long long ldaux, int a_mn, int b_mn,

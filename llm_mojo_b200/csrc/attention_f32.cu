@@ -13,7 +13,9 @@
 //   tn: sum_k A[k][i] B[k][j]   dV += P^T dO, dK += dS^T Q        columns tx * 4 + j
 // Forward: a CTA per 64 query rows walks the key tiles up to its own (longest rows first).  Backward: a CTA per 64 keys walks the
 // query tiles from its own on, recomputes P once, keeps dK and dV in registers and adds its part of dQ to the zeroed output by
-// vector reductions; the row dots D = sum(dO * O) come from a small kernel before it.
+// vector reductions; the row dots D = sum(dO * O) come from a small kernel before it.  The parts of dQ arrive in any order, so its last
+// bits differ from run to run; the split form leaves dQ to a kernel of its own, a CTA per 64 query rows that walks the key tiles in
+// order and recomputes P and dP (seven products instead of five), and is the same on every run.
 // Measured, B 4, T 512, 12 heads: forward 92 us, backward 164 us (library: 76 and 314, which for this path included a second forward);
 // B 2, T 2048, 16 heads 457 and 1158 us (499 and 1972).  Relative error against 64 bits, unit normal inputs: 1.7e-7 and 2.8e-7 (library 4.3e-7
 // and 6.6e-7): scores in four partial sums, tile sums before running sums.  The wavefronts of the 16-byte shared-memory reads bound it.
@@ -204,7 +206,8 @@ __global__ void __launch_bounds__(256) attn_f32_dot_kernel(float* __restrict__ D
   }
 }
 
-// The dQ part of dqkv must be zero on entry.
+// DQ: parts of dQ are added to dqkv, where it must be zero on entry; otherwise dQ is left alone.
+template <bool DQ>
 __global__ void __launch_bounds__(F32_THREADS, 2) attn_f32_bwd_kernel(float* __restrict__ dqkv, const float* __restrict__ dout, const float* __restrict__ qkv,
                                                                    const float* __restrict__ lse, const float* __restrict__ D, int T, int NH, int n_t) {
   extern __shared__ __align__(16) float smf[];
@@ -255,6 +258,7 @@ __global__ void __launch_bounds__(F32_THREADS, 2) attn_f32_bwd_kernel(float* __r
     add(dv, acc);
     mm_tn(acc, sS, sQ, ty, tx);
     add(dk, acc);
+    if (!DQ) continue;
     mm_nn(acc, sS, sK, ty, tx);
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
@@ -274,7 +278,57 @@ __global__ void __launch_bounds__(F32_THREADS, 2) attn_f32_bwd_kernel(float* __r
   }
 }
 
-constexpr int FWD_SMEM = 4 * TILE_WORDS * 4, BWD_SMEM = 6 * TILE_WORDS * 4;
+// dQ of 64 query rows, the key tiles in order.
+__global__ void __launch_bounds__(F32_THREADS, 2) attn_f32_dq_kernel(float* __restrict__ dqkv, const float* __restrict__ dout, const float* __restrict__ qkv,
+                                                                  const float* __restrict__ lse, const float* __restrict__ D, int T, int NH, int n_t) {
+  extern __shared__ __align__(16) float smf[];
+  float *sQ = smf, *sO = sQ + TILE_WORDS, *sK = sO + TILE_WORDS, *sV = sK + TILE_WORDS, *sS = sV + TILE_WORDS;
+  pdl_trigger();
+  pdl_wait();
+  const int BH = gridDim.x / n_t, qt = n_t - 1 - (int)(blockIdx.x / BH), bh = blockIdx.x % BH;      // the longest walks first
+  const int b = bh / NH, h = bh % NH, C = NH * FT;
+  const long long pitch = 3LL * C;
+  const float* base = qkv + (long long)b * T * pitch + h * FT;
+  const int ty = threadIdx.x / 16, tx = threadIdx.x % 16, q0 = qt * FT;
+  load_tile(sQ, base, pitch, q0, T);
+  load_tile(sO, dout + (long long)b * T * C + h * FT, C, q0, T);
+  float dq[8][4], ls[8], d[8];
+  zero(dq);
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int q = q0 + ty * 8 + i;
+    ls[i] = q < T ? lse[(long long)bh * T + q] : INFINITY;                   // rows beyond T: p = 0
+    d[i] = q < T ? D[(long long)bh * T + q] : 0.f;
+  }
+  for (int kt = 0; kt <= qt; ++kt) {
+    __syncthreads();                                      // the previous tile's products have read sK, sV and sS
+    load_tile(sK, base + C, pitch, kt * FT, T);
+    load_tile(sV, base + 2 * C, pitch, kt * FT, T);
+    __syncthreads();
+    float p[8][4], acc[8][4];
+    mm_nt(p, sQ, sK, ty, tx);
+    mm_nt(acc, sO, sV, ty, tx);
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const bool seen = kt < qt || j * 16 + tx <= ty * 8 + i;
+        sS[(ty * 8 + i) * FP + j * 16 + tx] = seen ? exp2f(p[i][j] * SCALE_LOG2 - ls[i]) * (acc[i][j] - d[i]) : 0.f;
+      }
+    __syncwarp();                                         // (a warp's rows of dS are written and read by that warp only)
+    mm_nn(acc, sS, sK, ty, tx);
+    add(dq, acc);
+  }
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int q = q0 + ty * 8 + i;
+    if (q < T)
+      *reinterpret_cast<float4*>(dqkv + ((long long)b * T + q) * pitch + h * FT + tx * 4) =
+          make_float4(dq[i][0] * SCALE, dq[i][1] * SCALE, dq[i][2] * SCALE, dq[i][3] * SCALE);
+  }
+}
+
+constexpr int FWD_SMEM = 4 * TILE_WORDS * 4, BWD_SMEM = 6 * TILE_WORDS * 4, DQ_SMEM = 5 * TILE_WORDS * 4;
 bool bad(const void* a, const void* b, const void* c) { return (reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(b) | reinterpret_cast<uintptr_t>(c)) & 15; }
 }  // namespace
 
@@ -286,17 +340,21 @@ LLMB_API int llmb_attention_f32_fwd(float* out, float* lse, const float* qkv, in
   if (e != cudaSuccess) return (int)e;
   return launch_pdl(attn_f32_fwd_kernel, (unsigned)grid, F32_THREADS, FWD_SMEM, st, out, lse, qkv, T, NH, (int)n_t);
 }
-// dqkv [B,T,3C] (overwritten) from dout and out [B,T,C], qkv and the forward's lse; D: scratch of B * NH * T floats.
+// dqkv [B,T,3C] (overwritten) from dout and out [B,T,C], qkv and the forward's lse; D: scratch of B * NH * T floats.  split: dQ by a
+// kernel of its own, the same on every run (one launch more: three kernels).
 LLMB_API int llmb_attention_f32_bwd(float* dqkv, float* D, const float* dout, const float* qkv, const float* out, const float* lse, int B, int T,
-                                    int NH, cudaStream_t st) {
+                                    int NH, int split, cudaStream_t st) {
   const long long n_t = ceil_div(T, FT), grid = n_t * B * NH, rows = (long long)B * T * NH, dots = ceil_div_ll(rows * 16, 256);
   if (B <= 0 || T <= 0 || NH <= 0 || grid > 0x7fffffffLL || dots > 0x7fffffffLL || bad(dqkv, dout, qkv) || bad(out, nullptr, nullptr)) return LLMB_ERR_BAD_ARG;
-  cudaError_t e = cudaFuncSetAttribute(attn_f32_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, BWD_SMEM);
-  if (e != cudaSuccess) return (int)e;
+  auto kern = split ? attn_f32_bwd_kernel<false> : attn_f32_bwd_kernel<true>;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, BWD_SMEM);
+  if (e == cudaSuccess && split) e = cudaFuncSetAttribute(attn_f32_dq_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, DQ_SMEM);
   const size_t row = (size_t)NH * FT * sizeof(float);
-  e = cudaMemset2DAsync(dqkv, 3 * row, 0, row, (size_t)B * T, st);
+  if (e == cudaSuccess && !split) e = cudaMemset2DAsync(dqkv, 3 * row, 0, row, (size_t)B * T, st);
   if (e != cudaSuccess) return (int)e;
-  const int rc = launch_pdl(attn_f32_dot_kernel, (unsigned)dots, 256, 0, st, D, dout, out, T, NH, rows);
+  int rc = launch_pdl(attn_f32_dot_kernel, (unsigned)dots, 256, 0, st, D, dout, out, T, NH, rows);
   if (rc) return rc;
-  return launch_pdl(attn_f32_bwd_kernel, (unsigned)grid, F32_THREADS, BWD_SMEM, st, dqkv, dout, qkv, lse, D, T, NH, (int)n_t);
+  rc = launch_pdl(kern, (unsigned)grid, F32_THREADS, BWD_SMEM, st, dqkv, dout, qkv, lse, D, T, NH, (int)n_t);
+  if (rc || !split) return rc;
+  return launch_pdl(attn_f32_dq_kernel, (unsigned)grid, F32_THREADS, DQ_SMEM, st, dqkv, dout, qkv, lse, D, T, NH, (int)n_t);
 }

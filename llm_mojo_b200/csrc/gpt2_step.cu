@@ -31,7 +31,7 @@ LLMB_API int llmb_attention_bwd_fused(void* dqkv, float* dbias, float* stats, fl
                                       const float* lse, int B, int T, int NH, int* status, cudaStream_t st);
 LLMB_API int llmb_attention_f32_fwd(float* out, float* lse, const float* qkv, int B, int T, int NH, cudaStream_t st);
 LLMB_API int llmb_attention_f32_bwd(float* dqkv, float* D, const float* dout, const float* qkv, const float* out, const float* lse, int B, int T,
-                                    int NH, cudaStream_t st);
+                                    int NH, int split, cudaStream_t st);
 LLMB_API int llmb_fp8_block_quant(void* q, void* sf, const void* x, int rows, int cols, int gran, int fmt, int transpose, cudaStream_t st);
 LLMB_API int llmb_fp8_block_quant_dual(void* q0, void* sf0, void* q1, void* sf1, const void* x, int rows, int cols, int fmt, cudaStream_t st);
 LLMB_API int llmb_gemm_mxfp8(void* D, const void* A, const void* B, const void* sfa, const void* sfb, const void* bias, void* aux,
@@ -261,7 +261,7 @@ struct Step {
     float* db = g(P_QKVB, l, 3 * C);
     if (dt == LLMB_BF16) return ok(llmb_attention_bwd_fused(dqkv, db, s.s_stats, s.s_dq, s.a[A_DL], qkv, o, ls, s.B, s.T, s.NH, s.status, st), 3);
     return ok(llmb_attention_f32_bwd(reinterpret_cast<float*>(dqkv), s.s_stats, reinterpret_cast<float*>(s.a[A_DL]), reinterpret_cast<const float*>(qkv),
-                                     reinterpret_cast<const float*>(o), ls, s.B, s.T, s.NH, st), 2) && bias_grad(db, dqkv, 3 * C);
+                                     reinterpret_cast<const float*>(o), ls, s.B, s.T, s.NH, 0, st), 2) && bias_grad(db, dqkv, 3 * C);
   }
   bool bias_grad(float* db, const void* dout, int N) { return ok(llmb_dbias(db, dout, s.s_dbias, s.s_dbias_bytes, rows, N, dt, st), llmb_dbias_launches(rows)); }
   bool ln_bwd(float* dw, float* db, const void* inp, const void* w, const float* mean, const float* rstd, int accumulate) {

@@ -483,9 +483,10 @@ def attention_bwd(dqkv, dout, qkv, out, lse, num_heads: int, dbias=None) -> None
         return
     if qkv.is_cuda and _attn_f32(num_heads, qkv, out, lse, dqkv, dout):
         dots = scratch("attn_f32_dots", B * num_heads * T * 4, qkv.device)
-        check(lib().llmb_attention_f32_bwd(ptr(dqkv), ptr(dots), ptr(dout), ptr(qkv), ptr(out), ptr(lse), B, T, num_heads, stream()),
+        split = ATTN_BWD != "fused"
+        check(lib().llmb_attention_f32_bwd(ptr(dqkv), ptr(dots), ptr(dout), ptr(qkv), ptr(out), ptr(lse), B, T, num_heads, int(split), stream()),
               "attention_f32_bwd")
-        _count(2)
+        _count(3 if split else 2)
         return
     if qkv.is_cuda:      # library comparator: recompute through SDPA under autograd
         with torch.enable_grad():

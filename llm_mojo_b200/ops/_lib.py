@@ -81,7 +81,7 @@ _SIGS = {
     "llmb_rng_uniform": [c_p, c_ll, c_ull, c_ull, c_ull, c_p],
     "llmb_attention_fwd": [c_p, c_p, c_p, c_int, c_int, c_int, c_p, c_p],
     "llmb_attention_f32_fwd": [c_p, c_p, c_p, c_int, c_int, c_int, c_p],
-    "llmb_attention_f32_bwd": [c_p, c_p, c_p, c_p, c_p, c_p, c_int, c_int, c_int, c_p],
+    "llmb_attention_f32_bwd": [c_p, c_p, c_p, c_p, c_p, c_p, c_int, c_int, c_int, c_int, c_p],
     "llmb_attention_bwd": [c_p, c_p, c_p, c_p, c_p, c_p, c_int, c_int, c_int, c_p, c_p],
     "llmb_attention_bwd_dbias": [c_p, c_p, c_p, c_p, c_p, c_p, c_p, c_int, c_int, c_int, c_p, c_p],
     "llmb_attention_bwd_fused": [c_p, c_p, c_p, c_p, c_p, c_p, c_p, c_p, c_int, c_int, c_int, c_p, c_p],

@@ -137,3 +137,22 @@ def test_calls_that_need_no_saved_statistics(form):
     assert rel(out, want_o) < TOL and rel(dqkv, want_d) < 2 * TOL
     if form == "short lse":
         assert bool((lse == 9.0).all())
+
+
+@pytest.mark.parametrize("B,T,NH", [(1, 1, 1), (1, 64, 1), (2, 65, 2), (3, 200, 2), (1, 1000, 2), (4, 512, 12)])
+def test_split_backward_repeats_itself(B, T, NH, monkeypatch):
+    """LLMB_ATTN_BWD=split: the fp32 backward without additions in arrival order."""
+    monkeypatch.setattr(ops, "ATTN_BWD", "split")
+    qkv, dout, out, lse = _inputs(B, T, NH)
+    ops.attention_fwd(out, lse, qkv, NH)
+    got = []
+    for _ in range(3):
+        dqkv = torch.full_like(qkv, float("nan"))
+        ops.attention_bwd(dqkv, dout, qkv, out, lse, NH)
+        got.append(dqkv)
+    assert torch.equal(got[0], got[1]) and torch.equal(got[0], got[2])
+    want = reference(qkv, dout, NH)[2]
+    if T == 1:                     # dq and dk vanish
+        assert rel(got[0][..., 128 * NH:], dout.double()) < TOL and got[0][..., :128 * NH].abs().max() < 1e-4
+    else:
+        assert rel(got[0], want) < 2 * TOL

@@ -337,12 +337,6 @@ __global__ void __launch_bounds__(1024, 1) classifier_stream2_kernel(__nv_bfloat
   }
 }
 
-// Natural exponential of a difference to a row maximum: ex2.approx for values that came from bf16 (as in the fused classifier),
-// the library function for fp32 rows.
-template <typename T> __device__ __forceinline__ float exp_row(float d);
-template <> __device__ __forceinline__ float exp_row<float>(float d) { return expf(d); }
-template <> __device__ __forceinline__ float exp_row<__nv_bfloat16>(float d) { return ex2_fast(d * 1.4426950408889634f); }
-
 // (max, sum of exp(x - max)) of two disjoint sets of values.  fmaxf passes over NaN: a set of nothing but NaN and -infinity has the
 // maximum -infinity, and its sum says which (NaN, or 0 where all are -infinity).
 __device__ __forceinline__ float2 merge_ms(float2 a, float2 b) {
@@ -547,14 +541,14 @@ __global__ void __launch_bounds__(256) ce_pass1_kernel(float4* __restrict__ stat
 #pragma unroll
         for (int k = 0; k < N; ++k) m = fmaxf(m, p.v[k]);
       }
-    float s = ms.x == m ? ms.y : ms.y * exp_row<T>(ms.x - m);
+    float s = ms.x == m ? ms.y : ms.y * expf(ms.x - m);
     const float m0 = base_ms(m);
 #pragma unroll
     for (int u = 0; u < U; ++u)
       if (v0 + u * 256 < nvec) {
         Pack<T> p; p.load(reinterpret_cast<const T*>(&raw[u]));
 #pragma unroll
-        for (int k = 0; k < N; ++k) s += exp_row<T>(p.v[k] - m0);
+        for (int k = 0; k < N; ++k) s += expf(p.v[k] - m0);
       }
     ms = make_float2(m, s);
   }
@@ -591,7 +585,7 @@ __global__ void __launch_bounds__(256) ce_pass2_kernel(T* __restrict__ tile, con
   const float lse = st.x + logf(st.y);
   const int tgt = targets[row] - col0;
   const int nvec = (reinterpret_cast<uintptr_t>(g) & 15) == 0 ? width / N : 0;
-  auto value = [&](float x, int i) { return col0 + i < V ? (exp_row<T>(x - lse) - (i == tgt ? 1.f : 0.f)) * dloss : 0.f; };
+  auto value = [&](float x, int i) { return col0 + i < V ? (expf(x - lse) - (i == tgt ? 1.f : 0.f)) * dloss : 0.f; };
   for (int v0 = tid; v0 < nvec; v0 += 256 * U) {
     uint4 raw[U];
 #pragma unroll

@@ -278,3 +278,19 @@ def test_masked_logits_count_as_nothing(mask, dtype):
     ops.chunked_ce_loss(losses, stats)
     want = torch.nn.functional.cross_entropy(x[:, :V].double(), tgt.long(), reduction="none")
     assert_close(losses, want, 1e-5, 1e-5, "losses")
+
+
+def test_chunked_ce_exponentials_do_not_depend_on_the_storage_type():
+    """The same logits as a bf16 and as an fp32 tile: the fp32 dlogits, rounded, are the bf16 dlogits."""
+    rows, V = 200, 4096
+    x = rnd(rows, V, scale=6.0).to(DEV)
+    tgt = torch.randint(0, V, (rows,), dtype=torch.int32, generator=torch.Generator().manual_seed(2)).to(DEV)
+    both = [x.clone(), x.float()]
+    stats = [torch.empty(rows, 4, device=DEV) for _ in both]
+    for t, s in zip(both, stats):
+        ops.chunked_ce_pass1(s, t, tgt, 0, V, V, True)
+    # two orders of 4096 additions of terms up to 1, the longest chain 32 of them; each exponential within 2^-23
+    assert_close(stats[0], stats[1].cpu(), 0.0, 2.0 ** -21, "statistics")
+    for t in both:
+        ops.chunked_ce_pass2(t, stats[1], tgt, 0, V, V, 0.125)
+    assert torch.equal(both[0], both[1].bfloat16())

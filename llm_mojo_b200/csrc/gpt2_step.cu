@@ -337,6 +337,7 @@ struct Step {
 };
 }  // namespace
 
+LLMB_API int llmb_abi() { return LLMB_ABI; }
 LLMB_API int llmb_gpt2_step_bytes() { return (int)sizeof(Gpt2Step); }
 // the largest site, backward: both orientations of the output gradient, the weight and the input
 LLMB_API long long llmb_gpt2_lowp_scratch_bytes(const Gpt2Step* s) {

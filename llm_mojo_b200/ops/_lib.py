@@ -106,6 +106,26 @@ def available() -> bool:
     return os.path.exists(_LIB_PATH)
 
 
+# Counts the changes of the C entry points' arguments; LLMB_ABI in csrc/common.cuh is the library's side of it.
+ABI = 1
+
+
+def _declare(L) -> None:
+    """Argument and result types of the entry points.  A library that was built from other sources than this file takes other arguments
+    and another ``Gpt2Step``: it is refused here, before a kernel is handed an address that is none."""
+    stale = f"{_LIB_PATH} was built from other sources: build it again with `python -m llm_mojo_b200.build`"
+    for name, sig in {"llmb_abi": [], **_SIGS}.items():
+        fn = getattr(L, name, None)
+        if fn is None:
+            raise RuntimeError(f"{stale} ({name} is missing)")
+        fn.argtypes = sig
+        fn.restype = c_ll if name in _RET_LL else c_int
+    from .step import Gpt2Step
+    for what, have, want in (("argument lists", L.llmb_abi(), ABI), ("Gpt2Step", L.llmb_gpt2_step_bytes(), ctypes.sizeof(Gpt2Step))):
+        if have != want:
+            raise RuntimeError(f"{stale} ({what}: {have}, not {want})")
+
+
 def lib() -> ctypes.CDLL:
     global _LIB
     if _LIB is None:
@@ -114,12 +134,7 @@ def lib() -> ctypes.CDLL:
                 f"{_LIB_PATH} is missing: build it with `python -m llm_mojo_b200.build` "
                 "(CUDA tensors never fall back to PyTorch ops)")
         L = ctypes.CDLL(_LIB_PATH)
-        for name, sig in _SIGS.items():
-            if not hasattr(L, name):
-                continue
-            fn = getattr(L, name)
-            fn.argtypes = sig
-            fn.restype = c_ll if name in _RET_LL else c_int
+        _declare(L)
         _LIB = L
     return _LIB
 

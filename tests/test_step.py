@@ -1,5 +1,8 @@
-"""The ctypes mirror of the native step's argument block has the layout of the C struct."""
+"""The ctypes side of the kernel library: argument block, argument lists, refusal of a library built from other sources."""
 import ctypes
+import glob
+import os
+import re
 
 import pytest
 
@@ -24,3 +27,40 @@ def test_weight_gradients_are_cut_into_no_more_parts_than_asked_for(kind):
                     assert 1 <= got <= splits, (M, N, K, splits, got)
                     seen.add(got)
     assert len(seen) > 2
+
+
+class _Fn:
+    def __init__(self, value):
+        self.value = value
+
+    def __call__(self):
+        return self.value
+
+
+class _Library:
+    """A stand-in for a loaded library: every entry point is there, ``without`` one of them, with the given answers."""
+
+    def __init__(self, abi=_lib.ABI, step_bytes=ctypes.sizeof(step.Gpt2Step), without=None):
+        for name in _lib._SIGS:
+            if name != without:
+                setattr(self, name, _Fn(0))
+        self.llmb_abi, self.llmb_gpt2_step_bytes = _Fn(abi), _Fn(step_bytes)
+
+
+def test_a_library_of_other_sources_is_refused_at_load():
+    _lib._declare(_Library())
+    for other in (_Library(abi=_lib.ABI - 1), _Library(step_bytes=ctypes.sizeof(step.Gpt2Step) - 8), _Library(without="llmb_gpt2_forward")):
+        with pytest.raises(RuntimeError, match="build it again"):
+            _lib._declare(other)
+
+
+def test_argument_lists_match_the_sources():
+    csrc = os.path.join(os.path.dirname(_lib.__file__), os.pardir, "csrc")
+    text = "\n".join(open(f).read() for f in sorted(glob.glob(os.path.join(csrc, "*.cu"))))
+    declared = {}
+    for name, args in re.findall(r"LLMB_API\s+(?:int|long long|void)\s+(\w+)\(([^)]*)\)", text):
+        declared.setdefault(name, set()).add(len(args.split(",")) if args.strip() else 0)
+    for name, sig in _lib._SIGS.items():
+        if name.startswith("llmb_bounds_report"):          # defined by a macro
+            continue
+        assert declared.get(name) == {len(sig)}, name

@@ -309,8 +309,9 @@ LLMB_API int llmb_layernorm_bwd_colsum(void* dres, float* dw, float* db, float* 
                                        const void* dout, const void* inp, const void* w, const float* mean,
                                        const float* rstd, int rows, int C, int accumulate, int dtype, cudaStream_t st) {
   const bool sumout = dsum != nullptr;
+  if (rows <= 0 || C <= 0) return LLMB_ERR_BAD_ARG;       // (before the plan divides by them)
   const int grid = ln_bwd_plan(rows, C, 8).grid;
-  if (rows <= 0 || scratch_bytes < (long long)grid * (sumout ? 3 : 2) * C * (long long)sizeof(float)) return LLMB_ERR_BAD_ARG;
+  if (scratch_bytes < (long long)grid * (sumout ? 3 : 2) * C * (long long)sizeof(float)) return LLMB_ERR_BAD_ARG;
   const int rc = dtype == LLMB_BF16 ? ln_bwd_launch<__nv_bfloat16>(dres, scratch, dout, inp, w, mean, rstd, rows, C, accumulate, sumout, st)
                                     : ln_bwd_launch<float>(dres, scratch, dout, inp, w, mean, rstd, rows, C, accumulate, sumout, st);
   if (rc) return rc;

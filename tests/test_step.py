@@ -3,6 +3,8 @@ import ctypes
 import glob
 import os
 import re
+import subprocess
+import sys
 
 import pytest
 
@@ -64,3 +66,14 @@ def test_argument_lists_match_the_sources():
         if name.startswith("llmb_bounds_report"):          # defined by a macro
             continue
         assert declared.get(name) == {len(sig)}, name
+
+
+@pytest.mark.skipif(not _lib.available(), reason="kernel library not built")
+def test_layernorm_backward_of_nothing_is_an_error():
+    """In a process of its own: an integer division by zero would end it."""
+    code = ("from llm_mojo_b200.ops import _lib\n"
+            "for rows, C in ((0, 768), (4, 0), (-1, 768)):\n"
+            "    for dtype in (0, 1):\n"
+            "        assert _lib.lib().llmb_layernorm_bwd_colsum(*[None] * 5, 1 << 20, *[None] * 5, rows, C, 1, dtype, None) == 2   # BAD_ARG\n")
+    root = os.path.dirname(os.path.dirname(os.path.dirname(os.path.abspath(_lib.__file__))))
+    assert subprocess.run([sys.executable, "-c", code], cwd=root).returncode == 0

@@ -163,8 +163,9 @@ __device__ __forceinline__ float2 gelu_grad_fast2(float2 x) {
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
-// Launch with the attribute, in clusters of `cl` CTAs (1: none, or as the kernel declares); every thread of `kern` that touches global
-// memory must call pdl_wait() first.
+// Launch with the attribute, in clusters of `cl` CTAs (1: none, or as the kernel declares).  Every thread of `kern` must call pdl_wait()
+// before it touches global memory and on every path to its exit: a grid that exits without it completes while the kernel before it may
+// still be running, and the next kernel's wait covers this grid only.
 template <typename... KArgs, typename... Args>
 inline int launch_pdl_cluster(dim3 cl, void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args&&... args) {
   cudaLaunchAttribute at[2];

@@ -775,6 +775,7 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   if (smem - smem_raw > 768) {                          // the alignment slack this launch was given does not cover the base it got
+    pdl_wait();                                         // (the kernel after this one counts on it, on this path too)
     if (threadIdx.x == 0) atomicExch(p.status, LLMB_ERR_BAD_ARG);
     return;
   }

@@ -561,7 +561,7 @@ int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap&
 
 // Tile configuration of one problem: bn = 256 is the CTA-pair kernel, 64 / 128 the kernel of gemm_small.cu with cl CTAs per tile.
 struct Tile { int bn, cl, splits; };
-int g_force_bn = 0, g_force_cl = 1;                       // test hook (llmb_gemm_force_tile): 0 = the rule decides
+thread_local int g_force_bn = 0, g_force_cl = 1;          // test hook (llmb_gemm_force_tile): 0 = the rule decides
 
 // The configuration with the smallest estimated time, in microseconds on a B200 from linear fits over M = 64 ... 5439, K and N =
 // 384 ... 5120 (the fits are within 15 %; the small kernel must win by 5 %): a fixed part (launch, set-up, epilogue) plus a cost per
@@ -1079,7 +1079,7 @@ LLMB_API void llmb_gemm_set_colsum(float* colsum) { g_pending_colsum = colsum; }
 LLMB_API void llmb_gemm_debug_mn_strides(int lbo_bytes, int sbo_bytes) { g_dbg_mn_lbo = lbo_bytes; g_dbg_mn_sbo = sbo_bytes; }
 // 0: single-CTA 128x128 tiles, 1: the rule of pick_tile() (default; env LLMB_GEMM_PAIR=0 selects the former)
 LLMB_API void llmb_gemm_set_pair_mode(int on) { g_pair_mode = on ? 1 : 0; }
-// Test hook: every following llmb_gemm call uses tiles of bn columns (256: CTA pair; 64 / 128: gemm_small.cu with cl = 1, 2 or 4 CTAs
+// Test hook: every following llmb_gemm call of the calling thread uses tiles of bn columns (256: CTA pair; 64 / 128: gemm_small.cu with cl = 1, 2 or 4 CTAs
 // per tile); bn = 0 gives the choice back to pick_tile().
 LLMB_API void llmb_gemm_force_tile(int bn, int cl) { g_force_bn = bn; g_force_cl = cl; }
 

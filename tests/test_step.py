@@ -5,6 +5,7 @@ import os
 import re
 import subprocess
 import sys
+import threading
 
 import pytest
 
@@ -77,3 +78,19 @@ def test_layernorm_backward_of_nothing_is_an_error():
             "        assert _lib.lib().llmb_layernorm_bwd_colsum(*[None] * 5, 1 << 20, *[None] * 5, rows, C, 1, dtype, None) == 2   # BAD_ARG\n")
     root = os.path.dirname(os.path.dirname(os.path.dirname(os.path.abspath(_lib.__file__))))
     assert subprocess.run([sys.executable, "-c", code], cwd=root).returncode == 0
+
+
+@pytest.mark.skipif(not _lib.available(), reason="kernel library not built")
+def test_forced_tiles_are_the_calling_threads_own():
+    L = _lib.lib()
+    parts = lambda: L.llmb_gemm_dw_splits(0, 768, 768, 2048, 15)
+    rule, other = parts(), []
+    try:
+        L.llmb_gemm_force_tile(64, 1)
+        assert parts() == 15 != rule                       # a forced tile takes the parts as given
+        t = threading.Thread(target=lambda: other.append(parts()))
+        t.start()
+        t.join()
+    finally:
+        L.llmb_gemm_force_tile(0, 1)
+    assert other == [rule] and parts() == rule

@@ -538,6 +538,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 int g_dbg_mn_lbo = -1, g_dbg_mn_sbo = -1;   // test hooks: override the MN-major descriptor strides
 thread_local float* g_pending_colsum = nullptr;   // armed by llmb_gemm_set_colsum, consumed by the calling thread's next llmb_gemm
 thread_local GatherArgs g_pending_gather{};   // armed by llmb_gemm_set_gather, consumed (and cleared) by the calling thread's next llmb_gemm
+thread_local bool g_pending_pair = false;     // armed by llmb_gemm_set_pair, consumed the same way
 thread_local PullArgs g_pending_pull{};       // armed by llmb_gemm_set_pull, consumed (and cleared) the same way
 // LLMB_GEMM_PAIR=0 / llmb_gemm_set_pair_mode(0): 128 x 128 tiles on single CTAs wherever the layout allows (a comparator)
 int g_pair_mode = -1;
@@ -624,6 +625,8 @@ int gemm_dispatch(void* D, const void* A, const void* B, const void* bias, void*
   g_pending_pull.nseg = 0; g_pending_pull.nwait = 0;
   p.colsum = g_pending_colsum;
   g_pending_colsum = nullptr;
+  const bool keep_pair = g_pending_pair;
+  g_pending_pair = false;
   if ((p.pull.nseg > 0 || p.pull.nwait > 0) && p.g.W > 1) return LLMB_ERR_BAD_ARG;
   if (p.colsum && !(epi == EPI_DGELU && (KIND == KIND_F16 || KIND == KIND_F8F6F4))) return LLMB_ERR_BAD_ARG;   // bf16 output, TMA epilogue
   if (p.g.W > 1) {
@@ -651,7 +654,7 @@ int gemm_dispatch(void* D, const void* A, const void* B, const void* bias, void*
   if (splits < 1 || epi != EPI_ACC_F32) splits = 1;
   if (splits > kb_total) splits = kb_total;
   Tile tile{256, 1, splits};
-  if (p.tma_epi && p.g.W <= 1 && p.pull.nseg == 0 && p.pull.nwait == 0) tile = pick_tile(KIND, epi, M, N, kb_total, splits, a_mn, b_mn);
+  if (p.tma_epi && !keep_pair && p.g.W <= 1 && p.pull.nseg == 0 && p.pull.nwait == 0) tile = pick_tile(KIND, epi, M, N, kb_total, splits, a_mn, b_mn);
   while (tile.cl > 1 && tile.cl > kb_total) tile.cl >>= 1;
   splits = tile.splits;
   const bool pair = tile.bn == 256;
@@ -1076,6 +1079,9 @@ LLMB_API int llmb_gemm_set_pull(const void* const* src, void* const* dst, const 
 // Arms the calling thread's NEXT llmb_gemm call (bf16, epilogue 3 = dGELU, CTA-pair kernel with the TMA epilogue) to add the column
 // sums of its result to colsum[N] (fp32, red.add): the bias gradient of the layer that produced the pre-activations.
 LLMB_API void llmb_gemm_set_colsum(float* colsum) { g_pending_colsum = colsum; }
+// Arms the calling thread's NEXT llmb_gemm call to run as the CTA-pair kernel, whose sums run through K in one chain, as they do where a
+// pull is armed: for a product whose result has to be that of an armed one, bit by bit (the tile rule may cut K among four CTAs).
+LLMB_API void llmb_gemm_set_pair() { g_pending_pair = true; }
 LLMB_API void llmb_gemm_debug_mn_strides(int lbo_bytes, int sbo_bytes) { g_dbg_mn_lbo = lbo_bytes; g_dbg_mn_sbo = sbo_bytes; }
 // 0: single-CTA 128x128 tiles, 1: the rule of pick_tile() (default; env LLMB_GEMM_PAIR=0 selects the former)
 LLMB_API void llmb_gemm_set_pair_mode(int on) { g_pair_mode = on ? 1 : 0; }

@@ -538,9 +538,11 @@ class ZeroEngine:
         waits for it.  Only the small tensors of a layer (LayerNorm parameters, biases) still come by the gather kernel.
         ``LLMM_FUSED_Z3=0`` selects the whole-layer gather, prefetched one layer ahead."""
         m = self.model
-        self.fused_z3 = bool(p2p and self.world_size > 1 and m.dtype == torch.bfloat16 and m.precision.name == "bf16"
-                             and ops.GEMM_IMPL == "tcgen05" and os.environ.get("LLMB_GEMM_PAIR", "1") != "0"
-                             and os.environ.get("LLMM_FUSED_Z3", "1") != "0")
+        able = bool(p2p and self.world_size > 1 and m.dtype == torch.bfloat16 and m.precision.name == "bf16"
+                    and ops.GEMM_IMPL == "tcgen05" and os.environ.get("LLMB_GEMM_PAIR", "1") != "0")
+        self.fused_z3 = able and os.environ.get("LLMM_FUSED_Z3", "1") != "0"
+        # the two paths give the same bits: a GEMM that pulls runs as the CTA-pair kernel, so its counterpart does too
+        self.pair_z3 = able and not self.fused_z3
         if not self.fused_z3:
             return
         L = m.config.num_layer
@@ -586,6 +588,8 @@ class ZeroEngine:
     def arm_linear(self, site: str, l: int, backward: bool) -> None:
         """Called right before the GEMM that reads the weight of ``site`` in layer ``l`` (forward GEMM, or the input-
         gradient GEMM in backward): arms that GEMM with the pull of the next weight and the wait for its own."""
+        if getattr(self, "pair_z3", False):
+            self.backend.L.llmb_gemm_set_pair()
         if not getattr(self, "fused_z3", False):
             return
         name = self.SITE_WEIGHT[site]

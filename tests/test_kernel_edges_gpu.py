@@ -294,3 +294,25 @@ def test_chunked_ce_exponentials_do_not_depend_on_the_storage_type():
     for t in both:
         ops.chunked_ce_pass2(t, stats[1], tgt, 0, V, V, 0.125)
     assert torch.equal(both[0], both[1].bfloat16())
+
+
+# sizes at which the rule takes one CTA per tile, two and four CTAs per tile, and CTA pairs
+@pytest.mark.parametrize("M,N,K", [(776, 1024, 1024), (64, 768, 768), (64, 768, 3072), (4096, 2304, 768)])
+def test_gemm_armed_for_the_pair_kernel(M, N, K, force_tile):
+    """The armed call, and only that one, gives the bits of the CTA-pair kernel."""
+    x, w, b, r = rnd(M, K).to(DEV), rnd(N, K, scale=0.05, seed=1).to(DEV), rnd(N, seed=2).to(DEV), rnd(M, N, seed=3).to(DEV)
+
+    def product():
+        out = torch.empty(M, N, dtype=torch.bfloat16, device=DEV)
+        ops.matmul_fwd(out, x, w, b, residual=r)
+        return out
+
+    rule = product()
+    force_tile(256, 1)
+    pair = product()
+    force_tile(0, 1)
+    _lib.lib().llmb_gemm_set_pair()
+    assert torch.equal(product(), pair)
+    assert torch.equal(product(), rule)
+    if (M, K) == (64, 3072):
+        assert not torch.equal(rule, pair)           # four CTAs add their parts of K: another order

@@ -216,3 +216,27 @@ def test_coordinator_scalar_and_or_and_agreement():
     for r in range(W):
         assert out[r][0] == 10.0 and out[r][1] == [15, 0]
     assert out[2][2] or out[0][2]          # divergent ranges are rejected
+
+
+@pytest.mark.parametrize("switch,precision,world,armed", [("0", "bf16", 2, True), ("1", "bf16", 2, None), ("0", "fp8", 2, False), ("0", "bf16", 1, False)])
+def test_zero3_gather_path_keeps_the_kernel_of_the_pulling_gemm(switch, precision, world, armed, monkeypatch):
+    """A GEMM that pulls weights always runs as the CTA-pair kernel.  Where the pulls are switched off its counterpart is armed to do so as
+    well: both paths then sum in the same order (the tile rule may cut K among several CTAs)."""
+    from types import SimpleNamespace
+    from llm_mojo_b200.config import Precision
+    from llm_mojo_b200.parallel.zero import ZeroEngine
+    monkeypatch.setenv("LLMM_FUSED_Z3", switch)
+    calls = []
+    eng = ZeroEngine.__new__(ZeroEngine)
+    eng.world_size = world
+    eng.model = SimpleNamespace(dtype=torch.bfloat16, precision=Precision(precision))
+    eng.backend = SimpleNamespace(L=SimpleNamespace(llmb_gemm_set_pair=lambda: calls.append("pair")))
+    if switch == "1":              # the pulling path: it needs the peers' arena, which is not there
+        with pytest.raises(AttributeError):
+            eng._setup_fused_pull(True)
+        assert eng.fused_z3 and not eng.pair_z3
+        return
+    eng._setup_fused_pull(True)
+    for site in ("qkv", "attproj", "fc", "fcproj"):
+        eng.arm_linear(site, 0, False)
+    assert calls == ["pair"] * 4 * armed and not eng.fused_z3

@@ -6,6 +6,7 @@ tensors on every call."""
 from __future__ import annotations
 
 import ctypes
+import functools
 import os
 
 import torch
@@ -56,27 +57,46 @@ def usable(m) -> bool:
             and env.get("LLMM_FUSED_LN_DBIAS", "0") == "0" and env.get("LLMM_FUSED_QKV_DBIAS", "1") != "0" and _mode(m) is not None)
 
 
-def _addresses(tensors, names, dtype):
-    """Addresses of the named tensors, or None if one of them is not what the kernels take (they see no strides)."""
+@functools.lru_cache(maxsize=64)
+def _act_specs(L, C, NH, B, T, Vp, recompute, tile_width, dtype):
+    """(name, type, bytes) of the buffers in ``ACTS`` and of the logits or the vocabulary tile, as the sequence indexes them."""
+    rows = B * T
+    once = {"encoded", "lnf", "lnf_mean", "lnf_rstd", "losses", "dres", "dl_btc", "dl_bt4c"} | ({"fch_gelu"} if recompute else set())
+    width = {"qkv": 3 * C, "fch": 4 * C, "fch_gelu": 4 * C, "dl_bt4c": 4 * C, "lse": NH, "losses": 1}
+    specs = [(n, torch.float32 if n in F32_ACTS else dtype, (1 if n in once else L) * rows * (1 if n.endswith(("_mean", "_rstd")) else width.get(n, C)))
+             for n in ACTS]
+    specs += [("logits_tile", dtype, rows * tile_width), ("ce_stats", torch.float32, 4 * rows)] if tile_width else [("logits", dtype, rows * Vp)]
+    return tuple((n, t, e * t.itemsize) for n, t, e in specs)
+
+
+@functools.lru_cache(maxsize=64)
+def _param_specs(sizes, dtype):
+    return tuple((n, dtype, e * dtype.itemsize) for n, e in zip(PARAM_NAMES, sizes))
+
+
+def _addresses(tensors, specs):
+    """Addresses of the named tensors, or None if one of them is not what the kernels take: they see no strides, read 16 bytes at a time
+    and find a layer by its place (a model whose options were changed after its buffers were allocated keeps to the op-by-op path)."""
     out = []
-    for n in names:
-        t = tensors[n]
-        if t.dtype is not (torch.float32 if n in F32_ACTS else dtype) or not (t.is_cuda and t.is_contiguous()):
+    for name, dtype, nbytes in specs:
+        t = tensors[name]
+        at = t.data_ptr()
+        if t.dtype is not dtype or t.nbytes != nbytes or at & 15 or not (t.is_cuda and t.is_contiguous()):
             return None
-        out.append(t.data_ptr())
+        out.append(at)
     return out
 
 
 def _fill(m, tiled: bool, targets: bool):
     cfg, a = m.config, m.acts
     s = Gpt2Step()
-    params, acts = _addresses(m.p, PARAM_NAMES, m.dtype), _addresses(a, ACTS, m.dtype)
+    params = _addresses(m.p, _param_specs(tuple(m.param_sizes), m.dtype))
+    acts = _addresses(a, _act_specs(cfg.num_layer, cfg.channels, cfg.num_heads, m.B, m.T, cfg.padded_vocab_size, m.recompute,
+                                    m.tile_width if tiled else 0, m.dtype))
     if params is None or acts is None:
         return None
-    s.p[:], s.a[:len(ACTS)] = params, acts
-    s.a[len(ACTS)] = a["logits_tile" if tiled else "logits"].data_ptr()
+    s.p[:], s.a[:len(acts)] = params, acts
     if tiled:
-        s.a[len(ACTS) + 1] = a["ce_stats"].data_ptr()
         s.tile_width = m.tile_width
     s.tokens, s.targets = m.inputs_dev.data_ptr(), m.targets_dev.data_ptr() if targets else None
     s.loss_acc, s.status, s.dloss = m.loss_acc.data_ptr(), status_word(m.device).data_ptr(), m._dloss
@@ -115,7 +135,7 @@ def backward(m, first: bool) -> bool:
     s = _fill(m, tiled, True)
     if s is None:
         return False
-    grads = _addresses(m.g, PARAM_NAMES, torch.float32)
+    grads = _addresses(m.g, _param_specs(tuple(m.param_sizes), torch.float32))
     if grads is None:
         return False
     s.g[:] = grads

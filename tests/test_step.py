@@ -8,7 +8,10 @@ import sys
 import threading
 
 import pytest
+import torch
 
+from llm_mojo_b200.config import GPT2Config
+from llm_mojo_b200.models import GPT2
 from llm_mojo_b200.ops import _lib, step
 
 
@@ -94,3 +97,33 @@ def test_forced_tiles_are_the_calling_threads_own():
     finally:
         L.llmb_gemm_force_tile(0, 1)
     assert other == [rule] and parts() == rule
+
+
+class _Tensor:
+    def __init__(self, n, dtype=torch.bfloat16, at=1 << 20, cuda=True, contiguous=True):
+        self.nbytes, self.dtype, self.at, self.is_cuda, self.contiguous = n * dtype.itemsize, dtype, at, cuda, contiguous
+
+    data_ptr = lambda self: self.at
+    is_contiguous = lambda self: self.contiguous
+
+
+def test_addresses_of_plain_buffers_only():
+    good = {"qkv": _Tensor(12), "lse": _Tensor(4, torch.float32, at=1 << 21)}
+    specs = (("qkv", torch.bfloat16, 24), ("lse", torch.float32, 16))
+    assert step._addresses(good, specs) == [1 << 20, 1 << 21]
+    for bad in (_Tensor(11), _Tensor(6, torch.float32), _Tensor(12, torch.float16), _Tensor(12, at=(1 << 20) + 8), _Tensor(12, cuda=False),
+                _Tensor(12, contiguous=False)):
+        assert step._addresses({**good, "qkv": bad}, specs) is None
+
+
+@pytest.mark.parametrize("recompute,chunks", [(False, 1), (True, 1), (False, 3)])
+def test_buffer_sizes_are_those_that_the_model_allocates(recompute, chunks):
+    cfg = GPT2Config(max_seq_len=16, vocab_size=300, num_layer=3, num_heads=2, channels=128, padded_vocab_size=384)
+    m = GPT2(cfg, "fp32", "cpu", recompute=recompute, lm_head_chunks=chunks)
+    m.allocate_activations(2, 5)
+    specs = lambda r: step._act_specs(3, 128, 2, 2, 5, 384, r, m.tile_width if chunks > 1 else 0, torch.float32)
+    sizes = {n: (t.dtype, t.nbytes) for n, t in m.acts.items()}
+    assert {n: (t, b) for n, t, b in specs(recompute)} == sizes != {n: (t, b) for n, t, b in specs(not recompute)}
+    assert [n for n, _, _ in specs(recompute)][:len(step.ACTS)] == list(step.ACTS)
+    assert [(m.p[n].dtype, m.p[n].nbytes) for n, _, _ in step._param_specs(tuple(m.param_sizes), torch.float32)] == \
+        [(t, b) for _, t, b in step._param_specs(tuple(m.param_sizes), torch.float32)]

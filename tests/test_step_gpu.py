@@ -98,3 +98,18 @@ def test_loss_accumulate(n):
         ops.loss_accumulate(acc, v, 0.25)
         want = 2.0 + 0.25 * v.double().sum().item()
         assert abs(acc.item() - want) <= 2e-6 * want, (n, off)      # at most 64 serial fp32 additions of positive terms, then a tree
+
+
+def test_options_changed_after_the_buffers_take_the_op_by_op_path():
+    """One GELU buffer, and a backward pass that would index one per layer."""
+    m = GPT2(GPT2Config(max_seq_len=64, vocab_size=1000, num_layer=2, num_heads=1, channels=64, padded_vocab_size=1024), "bf16", "cuda", recompute=True)
+    toks = torch.zeros(1, 32, dtype=torch.int32)
+    m.forward(toks, toks)
+    m.recompute = False
+    with pytest.raises(IndexError):
+        m.forward(toks, toks)
+    m.recompute = True
+    m.forward(toks, toks)
+    m.backward()
+    torch.cuda.synchronize()
+    assert _lib.read_status() == 0

@@ -139,6 +139,7 @@ class GPT2:
         self.micro_steps_done = 0
         self.lowp = None
         self.step_kept: Optional[torch.Tensor] = None     # ops/step.py: operands that a forward pass leaves for its backward pass
+        self.step_kept_stream = 0
         if self.precision.name == "fp8":
             from ..ops.lowp import LowpState
             self.lowp = LowpState(cfg.num_layer, self.device)
@@ -361,6 +362,7 @@ class GPT2:
         self._dloss = dloss = 1.0 / (B * T * grad_accum_steps)
         if "logits" not in a and not (targets is not None and (self.lm_head_chunks > 1 or self.vocab_parallel)):
             a["logits"] = torch.empty(B, T, cfg.padded_vocab_size, dtype=self.dtype, device=self.device)
+        self.step_kept = None                 # of the forward pass before, whichever way this one goes
         if step.usable(self) and step.forward(self, targets is not None):
             return
         z = self.zero

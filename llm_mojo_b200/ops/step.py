@@ -116,12 +116,11 @@ def _fill(m, tiled: bool, targets: bool):
 def forward(m, targets: bool) -> bool:
     """Issues the forward pass; False (nothing issued) if a buffer is not a plain contiguous tensor."""
     s = _fill(m, targets and m.lm_head_chunks > 1, targets)
-    m.step_kept = None
     if s is None:
         return False
     if s.lowp == FP8B and targets:                       # a backward pass may follow
         m.step_kept = torch.empty(lib().llmb_gpt2_lowp_kept_bytes(ctypes.byref(s)), dtype=torch.uint8, device=m.device)
-        s.kept = m.step_kept.data_ptr()
+        s.kept, m.step_kept_stream = m.step_kept.data_ptr(), stream()
     rc = lib().llmb_gpt2_forward(ctypes.byref(s), stream())
     _count(s.launches)
     check(rc, "gpt2_forward")
@@ -152,6 +151,8 @@ def backward(m, first: bool) -> bool:
     if s.lowp:
         if m.step_kept is not None and m.step_kept.numel() == L.llmb_gpt2_lowp_kept_bytes(ctypes.byref(s)):
             s.kept = m.step_kept.data_ptr()              # of this micro-step's forward pass
+            if m.step_kept_stream != stream():           # it is let go below, while this stream may still have to read it
+                m.step_kept.record_stream(torch.cuda.current_stream())
         lp = lambda n, k: _splits_for(n, k, rows, tile=128, tile_n=256, bk=128 if s.lowp == FP8B else 256, units=148)
         s.lp_splits_qkv, s.lp_splits_att, s.lp_splits_fc, s.lp_splits_proj = lp(3 * C, C), lp(C, C), lp(4 * C, C), lp(C, 4 * C)
     s.vocab_bits = max(1, (Vp - 1).bit_length())

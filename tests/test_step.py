@@ -127,3 +127,11 @@ def test_buffer_sizes_are_those_that_the_model_allocates(recompute, chunks):
     assert [n for n, _, _ in specs(recompute)][:len(step.ACTS)] == list(step.ACTS)
     assert [(m.p[n].dtype, m.p[n].nbytes) for n, _, _ in step._param_specs(tuple(m.param_sizes), torch.float32)] == \
         [(t, b) for _, t, b in step._param_specs(tuple(m.param_sizes), torch.float32)]
+
+
+def test_a_forward_pass_lets_go_of_what_the_one_before_left():
+    m = GPT2(GPT2Config(max_seq_len=16, vocab_size=60, num_layer=1, num_heads=1, channels=64, padded_vocab_size=64), "fp32", "cpu")
+    m.step_kept = torch.zeros(3)              # as a native forward would
+    toks = torch.zeros(1, 4, dtype=torch.int32)
+    m.forward(toks, toks)                     # op by op
+    assert m.step_kept is None

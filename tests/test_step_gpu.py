@@ -113,3 +113,29 @@ def test_options_changed_after_the_buffers_take_the_op_by_op_path():
     m.backward()
     torch.cuda.synchronize()
     assert _lib.read_status() == 0
+
+
+def test_operands_kept_for_a_backward_pass_on_another_stream():
+    """The forward's stream may not have their memory back while the backward's stream still reads them."""
+    cfg = GPT2Config(max_seq_len=128, vocab_size=1000, num_layer=2, num_heads=2, channels=128, padded_vocab_size=1024)
+    toks = torch.randint(0, 1000, (2 * 128 + 1,), generator=torch.Generator().manual_seed(5), dtype=torch.int32).cuda()
+    x, y = toks[:-1].view(2, 128), toks[1:].view(2, 128)
+    grads = []
+    for apart in (False, True):
+        m = GPT2(cfg, "fp8b", "cuda")
+        first, second = torch.cuda.Stream(), torch.cuda.Stream()
+        first.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(first):
+            m.forward(x, y)
+        n = m.step_kept.numel()
+        second.wait_stream(first)
+        with torch.cuda.stream(second if apart else first):
+            torch.cuda._sleep(100_000_000)
+            m.backward()
+        assert m.step_kept is None
+        with torch.cuda.stream(first):            # what a program may do next on its own stream
+            reused = torch.full((n,), 0x7f, dtype=torch.uint8, device="cuda") if apart else None
+        torch.cuda.synchronize()
+        grads.append(m.grads.clone())
+        del reused
+    assert torch.isfinite(grads[1]).all() and (grads[1] - grads[0]).norm() <= 2.0 ** -8 * grads[0].norm()

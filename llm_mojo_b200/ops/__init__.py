@@ -265,7 +265,7 @@ def _tc_kind(t: torch.Tensor):
     return None
 
 
-@functools.lru_cache(maxsize=None)
+@functools.lru_cache(maxsize=4096)
 def _splits_for(M: int, N: int, K: int, *, tile: int = 256, tile_n: int = 0, bk: int = 64, units: int = 74) -> int:
     """Split-K factor for the dW GEMMs (by default 256x256 tiles on 74 CTA pairs, 64 values of K per stage; the
     block-scaled kernels have 128x256 tiles on 148 CTAs): the number of splits that minimises waves x (k-blocks per

@@ -130,7 +130,7 @@ __device__ __forceinline__ float gelu_grad_fast_f(float x) {
 }
 
 // The same two functions on pairs, with packed fp32x2 arithmetic (half the FMA-pipe instructions per element; the two
-// tanh stay scalar MUFU operations).  Used by the GEMM epilogues, whose eight warps, not the tensor core, bound the GELU layers.
+// tanh stay scalar MUFU operations).  Used by the GEMM epilogues, whose warps, not the tensor core, bound the GELU layers at short K.
 __device__ __forceinline__ float2 gelu_fast2(float2 x) {
   const float k = 0.7978845608028654f, kc = 0.7978845608028654f * 0.044715f;
   const float2 x2 = __fmul2_rn(x, x);

@@ -10,7 +10,7 @@
 // MN-major (the UMMA descriptor and the TMA box change, not the data), which is how dinp (B = W as stored) and dW (A = dout^T,
 // B = inp^T as stored) run without any transposes.  Split-K work units add into the (fp32) gradient buffer.
 //
-// gemm_pair_kernel (two CTAs per 256 x 256 tile with cta_group::2 MMAs, persistent, eight epilogue warps, optional all-gather of A
+// gemm_pair_kernel (two CTAs per 256 x 256 tile with cta_group::2 MMAs, persistent, 8 or 16 epilogue warps, optional all-gather of A
 // from peer GPUs and optional column sums of the result) runs what fills the chip with such tiles; gemm_small.cu runs the rest on
 // 128-row tiles; gemm_nvfp4_kernel has block-scaled NVFP4 / MXFP8 operands with their scales in tensor memory.  pick_tile() chooses.
 #include <math.h>
@@ -370,7 +370,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     // 128-column half of the tile, i.e. two 64-column slabs per warp and tile.  The register epilogue (fp32
     // outputs, layouts without a tensor map) keeps four working warps with all four slabs of a band each.
     // An fp32-storage problem (tf32) moves its 128 columns as four 32-column boxes through the same buffers.
-    constexpr bool F32_IO = KIND == KIND_TF32 && !Cfg::F32_OUT;
+    // Auxiliary inputs come this way for fp32 storage only.
+    constexpr bool F32_IO = KIND == KIND_TF32 && !Cfg::F32_OUT, AUX = Cfg::AUX_IN && F32_IO;
     constexpr int NBOX = F32_IO ? 4 : 2, BOXC = F32_IO ? 32 : 64;
     const int q = warp & 3, e = warp - 2, hcol = e >> 2;
     const bool tma_epi = p.tma_epi;                       // warp-uniform
@@ -389,7 +390,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         tma_load_2d(wstage + b * SLAB_BYTES, &tmAux, &abar[b], n0 + hcol * 128 + ls * BOXC, row0);
       }
     };
-    if (Cfg::AUX_IN && tma_epi && cluster_id < total_units) {
+    if (AUX && tma_epi && cluster_id < total_units) {
       int m_blk, n_blk, kb0, kb1; unit_coords(cluster_id, m_blk, n_blk, kb0, kb1);
       for (int ls = 0; ls < 2; ++ls) aux_issue(m_blk * 2 * BM + band_off, n_blk * BN, ls);
     }
@@ -408,7 +409,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         if (e < 4) epilogue_warp<EPI>(p, tacc, wstage, row0, n0, alpha, lane);
       } else {
         const int nunit = unit + num_clusters;
-        const bool has_next = Cfg::AUX_IN && nunit < total_units;
+        const bool has_next = AUX && nunit < total_units;
         int nrow0 = 0, nn0 = 0;
         if (has_next) { int mb, nb, k0, k1; unit_coords(nunit, mb, nb, k0, k1); nrow0 = mb * 2 * BM + band_off; nn0 = nb * BN; }
         bool ok = true;
@@ -451,7 +452,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
             }
             continue;
           }
-          if (Cfg::AUX_IN) {
+          if (AUX) {
             const int b = ls & 1;
             buf = wstage + b * SLAB_BYTES;
             if (!mbar_wait(&abar[b], (aux_phase >> b) & 1)) { ok = false; break; }
@@ -471,7 +472,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
               else tma_store_2d(&tmD, buf, col0, row0);
               bulk_commit();
             }
-            if (Cfg::AUX_IN && ls + 2 < NBOX && slab_valid(row0, n0, ls + 2)) {   // this buffer's next box, once the store has read it
+            if (AUX && ls + 2 < NBOX && slab_valid(row0, n0, ls + 2)) {   // this buffer's next box, once the store has read it
               if (lane == 0) bulk_wait_read<0>();
               __syncwarp();
               aux_issue(row0, n0, ls + 2);
@@ -494,19 +495,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           epi_slab_bf16<EPI>(p, r0, r1, buf, col0, alpha, lane);
           fence_proxy_async();
           __syncwarp();
-          if (EPI == EPI_DGELU && p.colsum) epi_slab_colsum(p, buf, row0, col0, lane);
-          if (lane == 0) {
-            if (Cfg::TWO_OUT) {
-              tma_store_2d(&tmAux, buf, col0, row0);
-              tma_store_2d(&tmD, buf + SLAB_BYTES, col0, row0);
-            } else {
-              tma_store_2d(&tmD, buf, col0, row0);
-            }
-            bulk_commit();
-          }
+          if (lane == 0) { tma_store_2d(&tmD, buf, col0, row0); bulk_commit(); }
         }
         if (!ok) { *abort_flag = 1; atomicExch(p.status, LLMB_ERR_TIMEOUT); break; }
-        if (Cfg::AUX_IN && has_next) {                    // refill each buffer once its store has been read
+        if (AUX && has_next) {                            // refill each buffer once its store has been read
           // (a unit at the right edge may have stored its last slab from buffer 0: then both stores must have been read)
           if (lane == 0) { if (slab_valid(row0, n0, NBOX - 1)) bulk_wait_read<1>(); else bulk_wait_read<0>(); }
           __syncwarp();
@@ -1076,7 +1068,7 @@ LLMB_API int llmb_gemm_set_pull(const void* const* src, void* const* dst, const 
   g_pending_pull = a;
   return 0;
 }
-// Arms the calling thread's NEXT llmb_gemm call (bf16, epilogue 3 = dGELU, CTA-pair kernel with the TMA epilogue) to add the column
+// Arms the calling thread's NEXT llmb_gemm call (bf16 result, epilogue 3 = dGELU, any tile, TMA epilogue) to add the column
 // sums of its result to colsum[N] (fp32, red.add): the bias gradient of the layer that produced the pre-activations.
 LLMB_API void llmb_gemm_set_colsum(float* colsum) { g_pending_colsum = colsum; }
 // Arms the calling thread's NEXT llmb_gemm call to run as the CTA-pair kernel, whose sums run through K in one chain, as they do where a

@@ -197,26 +197,23 @@ __device__ __forceinline__ void epilogue_warp(const GemmParams& p, uint32_t tacc
 }
 
 // ------------------------------------------------------------------------------------------------
-// Epilogue through TMA (bf16 outputs of the CTA-pair kernel).  Each of the eight epilogue warps owns
-// 32 rows x 128 columns of the accumulator and moves them as two slabs of 64 columns = one
-// 128-byte-swizzled box of 32 rows x 128 B (4 KB) each:
-//   * tcgen05.ld gives each lane one row of the slab; bias, GELU, dGELU and the residual add happen in
-//     registers in that layout;
-//   * the auxiliary INPUT (residual stream, pre-GELU activations) arrives by TMA loads that are issued a
-//     whole tile ahead - while the tensor core is still busy with that tile - into the buffer the
-//     result is then written to in place;
-//   * results leave by TMA stores (bulk groups), so no lane ever waits on global memory and every
-//     global access of the epilogue is a full 128-byte row segment; out-of-range rows and columns are
-//     clipped by the tensor maps.
-// Epilogues with an auxiliary input or a second output (BIAS_GELU stores the pre-activation too) get
-// two 4 KB buffers per warp and a 5-deep operand ring, and so do the fp32 outputs (two 32-column boxes of a 64-column slab,
-// added into or stored to global memory by TMA); the others one buffer and a 6-deep ring.
+// Epilogue through TMA.  A warp moves its part of the accumulator in boxes of 32 rows x 128 bytes (4 KB, 128-byte swizzle):
+// 64 columns of bf16 or 32 of fp32.
+//   * tcgen05.ld gives each lane one row of a box; bias, GELU, dGELU and the residual add happen in registers in that layout;
+//   * the auxiliary INPUT (residual stream, pre-GELU activations) arrives by TMA in the buffer that the result is then written to in
+//     place.  In the CTA-pair kernel a tile's boxes are on their way to L2 (bf16, fp8 operands: sixteen warps, one box each) or into
+//     their buffers (fp32 storage: eight warps, four boxes in two buffers) while the tile before it is worked; a buffer is filled
+//     again once the store of its last result has read it;
+//   * results leave by TMA stores (fp32 accumulate: by TMA additions), so no lane ever waits on global memory and every global access
+//     of the epilogue is a full 128-byte row segment; out-of-range rows and columns are clipped by the tensor maps.
+// Epilogues with an auxiliary input or a second output (BIAS_GELU stores the pre-activation too) and the fp32 outputs get 64 KB of
+// boxes and a 5-deep operand ring in the CTA-pair kernel; the others 32 KB and a 6-deep ring.
 template <int EPI> struct EpiCfg {
   static constexpr bool AUX_IN = EPI == EPI_DGELU || EPI == EPI_BIAS_RESID;
   static constexpr bool TWO_OUT = EPI == EPI_BIAS_GELU;
   static constexpr bool F32_OUT = EPI == EPI_ACC_F32 || EPI == EPI_STORE_F32;
   static constexpr int STAGES = (F32_OUT || AUX_IN || TWO_OUT) ? 5 : 6;
-  static constexpr int WARP_STAGE = STAGES == 5 ? 16384 : 8192;     // staging bytes per warp of the 4-warp register epilogue (half that per warp of the 8-warp TMA epilogue)
+  static constexpr int WARP_STAGE = STAGES == 5 ? 16384 : 8192;     // staging bytes per warp of the 4-warp register epilogue (half that per warp of 8, a quarter per warp of 16 in the TMA epilogues)
 };
 constexpr int SLAB_BYTES = 32 * 128;
 

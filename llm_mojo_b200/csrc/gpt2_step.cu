@@ -1,5 +1,6 @@
-// One forward or backward micro-step of GPT-2 (bf16, fp32 storage, block-scaled FP8 or NVFP4 sites) as ONE host call: the launch sequence of models/gpt2.py (reference:
-// train_gpt2.mojo:3050-3848 forward, :3948-5056 backward) issued from native code over the same kernels, buffers and scratch.
+// One forward or backward micro-step of GPT-2 (bf16, fp32 storage with TF32 products, block-scaled FP8 or NVFP4 sites) as ONE host call:
+// the launch sequence of models/gpt2.py (reference: train_gpt2.mojo:3050-3848 forward, :3948-5056 backward) issued from native code
+// over the same kernels, buffers and scratch.
 //
 // What it is for: a layer is 7 launches forward and 17 backward, and issuing one from Python (tensor views, pointer reads, a ctypes
 // call) takes 15 - 20 us of host time, more than the kernels of a small batch run: sampling with d12 at 64 positions spent 1.75 ms

@@ -209,8 +209,8 @@ EPI_NONE, EPI_BIAS, EPI_BIAS_GELU, EPI_DGELU, EPI_ACC_F32, EPI_BIAS_RESID, EPI_S
 def gemm(D, A, B, *, a_mn=False, b_mn=False, epi=EPI_NONE, bias=None, aux=None, alpha=None, splits=1,
          kind: int = 0, a_fmt: int = 0, b_fmt: int = 0, colsum=None) -> None:
     """Raw tcgen05 GEMM: D[M,N] = epi(A·Bᵀ).  A is [M,K] (or [K,M] when ``a_mn``), B is [N,K]
-    (or [K,N] when ``b_mn``); all row-major with arbitrary row pitch.  ``colsum`` (fp32 [N], dGELU epilogue of
-    the bf16 kernel only, see ``colsum_usable``) accumulates the column sums of D inside the epilogue."""
+    (or [K,N] when ``b_mn``); all row-major with arbitrary row pitch.  ``colsum`` (fp32 [N], dGELU epilogue with
+    a bf16 result only, see ``colsum_usable``) accumulates the column sums of D inside the epilogue."""
     M, N = D.shape
     K = A.shape[0] if a_mn else A.shape[1]
     if colsum is not None:
@@ -245,8 +245,8 @@ def gemm_mxfp8(D, qa, sfa, qb, sfb, *, a_fmt=0, b_fmt=0, epi=EPI_NONE, bias=None
 
 
 def colsum_usable(D: torch.Tensor, aux: torch.Tensor) -> bool:
-    """The dGELU GEMM can add the column sums of its result (the bias gradient of the layer below) in its epilogue when
-    it runs as the bf16 CTA-pair kernel with the TMA epilogue: 16-byte aligned bf16 rows of D and aux."""
+    """The dGELU GEMM can add the column sums of its bf16 result (the bias gradient of the layer below) in its TMA epilogue, whatever its
+    tiles: 16-byte aligned bf16 rows of D and aux.  (With ``LLMB_GEMM_PAIR=0`` the comparator takes them in a pass of their own.)"""
     if not (D.is_cuda and D.dtype == torch.bfloat16 and aux.dtype == torch.bfloat16 and GEMM_IMPL == "tcgen05"):
         return False
     if os.environ.get("LLMB_GEMM_PAIR", "1") == "0" or os.environ.get("LLMB_GEMM_TMA_EPI", "1") == "0":

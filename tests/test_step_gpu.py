@@ -1,4 +1,5 @@
-"""The native launch sequence of a bf16 micro-step against the op-by-op sequence of the model: same kernels, same buffers."""
+"""The native launch sequence of a micro-step (bf16, TF32, block-scaled FP8, NVFP4) against the op-by-op sequence of the model: same
+kernels, same buffers."""
 import pytest
 import torch
 

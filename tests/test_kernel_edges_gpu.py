@@ -160,17 +160,35 @@ def test_gemm_fp8_tile_configurations(bn, cl, force_tile):
     assert _lib.read_status() == 0
 
 
-def test_gemm_residual_right_edge_many_tiles():
-    """Several tiles per CTA pair with a right edge that leaves one 64-column slab in a warp's half of the tile: the slab's buffer is
-    refilled with the next tile's residual, which must wait for the store that still reads it."""
-    M, N, K = 256 * 74 * 3 + 40, 320, 64
-    x, w, r = rnd(M, K), rnd(N, K, scale=0.1, seed=1), rnd(M, N, seed=2)
-    ref = x.float() @ w.float().t() + r.float()
+# columns in the last 256-wide tile: its first warps' halves hold 1, 2, 3 (and 4, then 1) boxes of 32 columns; 1 and 2 slabs of 64
+@pytest.mark.parametrize("N", [288, 320, 352, 416])
+@pytest.mark.parametrize("epi", ["residual", "dgelu"])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])      # 16 warps with one box each / 8 warps with two buffers for four boxes
+def test_gemm_residual_right_edge_many_tiles(dtype, epi, N, force_tile):
+    """Several tiles per CTA pair, the right edge leaving part of a warp's boxes: a buffer is refilled with the next tile's auxiliary
+    input, which must wait for the store that still reads it."""
+    force_tile(256, 1)
+    M, K = 256 * 74 * 3 + 40, 64
+    x, w, r = rnd(M, K, dtype=dtype), rnd(N, K, dtype=dtype, scale=0.1, seed=1), rnd(M, N, dtype=dtype, seed=2)
+    ref = x.float() @ w.float().t()
+    if epi == "residual":
+        ref += r.float()
+    else:
+        xg = r.float().requires_grad_(True)
+        torch.nn.functional.gelu(xg, approximate="tanh").backward(ref)
+        ref = xg.grad
     X, W, Rs = x.to(DEV), w.to(DEV), r.to(DEV)
-    for _ in range(5):
-        out = torch.empty(M, N, dtype=torch.bfloat16, device=DEV)
-        ops.matmul_fwd(out, X, W, torch.zeros(N, dtype=torch.bfloat16, device=DEV), residual=Rs)
-        assert_close(out, ref, 2.0 ** -6, 2.0 ** -8, "residual at the right edge")
+    zero = torch.zeros(N, dtype=dtype, device=DEV)
+    # bf16: one rounding of the result, GELU' by a tanh within 2^-11; fp32: operands rounded to tf32 (2^-11 each, 64 terms of size ~0.1)
+    tol = (2.0 ** -6, 2.0 ** -7 if epi == "dgelu" else 2.0 ** -8) if dtype == torch.bfloat16 else (2.0 ** -8, 2.0 ** -9)
+    for _ in range(3):
+        out = torch.empty(M, N, dtype=dtype, device=DEV)
+        if epi == "residual":
+            ops.matmul_fwd(out, X, W, zero, residual=Rs)
+        else:
+            ops.gemm(out, X, W, epi=ops.EPI_DGELU, aux=Rs, kind=0 if dtype == torch.bfloat16 else 1)
+        assert_close(out, ref, *tol, f"{epi} at the right edge")
+    assert _lib.read_status() == 0
 
 
 # a thread of the classifier holds 7 or 8 vectors of a row: widths around whole and partial last vectors, the switch and the largest

@@ -3,6 +3,9 @@
 
     python profile_kernels.py attn        # flash attention forward + backward, B=32 T=1024 NH=12
     python profile_kernels.py gemm        # fc GEMM with the fused bias+GELU epilogue, its dinp (dGELU) and dW GEMMs
+    python profile_kernels.py small       # layer GEMMs of 776 rows (d24 sampling): 128-row tiles, one CTA each or a cluster per contraction
+    python profile_kernels.py f32attn     # fp32 attention forward + backward, B=8 T=1024 NH=12
+    python profile_kernels.py nvfp4       # NVFP4 operands (maxima, both orientations) and block-scaled GEMMs, 8192 x 1600 x 6400
     python profile_kernels.py lmhead      # LM-head GEMM on 8192 rows + fused softmax/cross-entropy
     python profile_kernels.py layernorm   # LayerNorm forward + backward on 65536 x 768
     python profile_kernels.py fusedpull   # a layer GEMM that pulls its own weight (four emulated owners) with its copier warps
@@ -51,6 +54,31 @@ def case_gemm(reps):
         ops.matmul_fwd(act, x, w, b, pre_gelu=pre)                       # bias + GELU epilogue, two outputs
         ops.matmul_bwd(dact, dw2, None, dy, act, w2, gelu_pre=pre)       # fcproj backward: dGELU epilogue on dinp
         ops.matmul_bwd(dx, dw, db, dact, x, w)                           # fc backward: dinp (B MN-major), split-K dW
+
+
+def case_small(reps):
+    rows, C, L = 776, 1024, 16            # 16 layers of weights (403 MB): every product reads its own from memory, as a token's pass does
+    rand = lambda *s: torch.randn(*s, device="cuda").bfloat16()
+    x, o3, o4, o1 = rand(rows, C), rand(rows, 3 * C), rand(rows, 4 * C), rand(rows, C)
+    pre = torch.empty_like(o4)
+    layers = [[rand(n, k) * 0.02 for n, k in ((3 * C, C), (C, C), (4 * C, C), (C, 4 * C))] for _ in range(L)]
+    b = torch.zeros(4 * C, device="cuda", dtype=torch.bfloat16)
+    for _ in range(reps):
+        for wq, wa, wf, wp in layers:
+            ops.matmul_fwd(o3, x, wq, b[:3 * C])
+            ops.matmul_fwd(o1, x, wa, b[:C], residual=x)
+            ops.matmul_fwd(o4, x, wf, b, pre_gelu=pre)
+            ops.matmul_fwd(o1, o4, wp, b[:C], residual=x)
+
+
+def case_f32attn(reps):
+    B, T, NH, C = 8, 1024, 12, 768
+    qkv = torch.randn(B, T, 3 * C, device="cuda")
+    out, lse = torch.empty(B, T, C, device="cuda"), torch.empty(B, NH, T, device="cuda")
+    dqkv, dout = torch.empty_like(qkv), torch.randn(B, T, C, device="cuda")
+    for _ in range(reps):
+        ops.attention_fwd(out, lse, qkv, NH)
+        ops.attention_bwd(dqkv, dout, qkv, out, lse, NH)
 
 
 def case_lmhead(reps):
@@ -159,7 +187,7 @@ def case_nvfp4(reps):
         lowp.matmul_bwd_fp4(dinp, dw, None, d, x, w, seed=1, step=i)
 
 
-CASES = {"nvfp4": case_nvfp4, "fusedgather": case_fusedgather, "fusedpull": case_fusedpull, "attn": case_attn, "gemm": case_gemm, "lmhead": case_lmhead, "layernorm": case_layernorm}
+CASES = {"small": case_small, "f32attn": case_f32attn, "nvfp4": case_nvfp4, "fusedgather": case_fusedgather, "fusedpull": case_fusedpull, "attn": case_attn, "gemm": case_gemm, "lmhead": case_lmhead, "layernorm": case_layernorm}
 
 if __name__ == "__main__":
     ap = argparse.ArgumentParser(description=__doc__, formatter_class=argparse.RawDescriptionHelpFormatter)

@@ -16,9 +16,12 @@
 // vector reductions; the row dots D = sum(dO * O) come from a small kernel before it.  The parts of dQ arrive in any order, so its last
 // bits differ from run to run; the split form leaves dQ to a kernel of its own, a CTA per 64 query rows that walks the key tiles in
 // order and recomputes P and dP (seven products instead of five), and is the same on every run.
-// Measured, B 4, T 512, 12 heads: forward 92 us, backward 164 us (library: 76 and 314, which for this path included a second forward);
-// B 2, T 2048, 16 heads 457 and 1158 us (499 and 1972).  Relative error against 64 bits, unit normal inputs: 1.7e-7 and 2.8e-7 (library 4.3e-7
-// and 6.6e-7): scores in four partial sums, tile sums before running sums.  The wavefronts of the 16-byte shared-memory reads bound it.
+// Measured (us, with the library in brackets; its backward included a second forward): forward B 8, T 64, 6 heads 9.2 (25.6), B 2, T 512, 12
+// heads 82 (64), B 4, T 512 97 (76), B 8, T 1024 351 (359), B 2, T 2048, 16 heads 455 (500); backward 27 (189), 162 (237), 164 (314), 891
+// (1487), 1158 (1982).  The library's forward is ahead at two to six tiles per SM: there the longest CTA, eight tiles one after the other
+// with one warp per scheduler, is the whole time.  Split backward: 208 at B 4, T 512, 1607 at B 2, T 2048.
+// Relative error against 64 bits, unit normal inputs: 1.7e-7 and 2.8e-7 (library 4.3e-7 and 6.6e-7): scores in four partial sums, tile sums
+// before running sums.  At B 8, T 1024 the SMs are 75 % (forward) and 67 % (backward) busy, L1 62 %, with 19 % and 12 % of the warp slots taken.
 #include "common.cuh"
 using namespace llmb;
 

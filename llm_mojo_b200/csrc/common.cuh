@@ -159,7 +159,7 @@ __device__ __forceinline__ float2 gelu_grad_fast2(float2 x) {
 // first and then wait for this one), and a kernel that waits for another stream or another GPU does not call it at all (the waiting
 // CTAs of the next kernel could keep out what it waits for).  Without the attribute, as after any other kernel, copy or event, both
 // do nothing.  Measured: the 1.3 - 2.5 us between two kernels of a step disappear; d12 B 7 T 777 8.87 -> 8.27 ms (356 launches), d36 fp8
-// B 8 T 1024 51.2 -> 47.8 ms (1989), d12 B 64 T 1024 68.6 -> 66.7 ms (356, longer kernels: their ragged last waves overlap too).
+// B 8 T 1024 51.2 -> 47.8 ms (1989); d12 B 64 T 1024 (356 long kernels, 67 ms) no change beyond the 1 % by which its runs differ.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

@@ -563,6 +563,9 @@ thread_local int g_force_bn = 0, g_force_cl = 1;          // test hook (llmb_gem
 // further round of pair tiles costs its epilogue if that is longer than its k-loop.  Clusters only while they fit in one round:
 // beyond it they were 1.5 - 4 times slower than one CTA per tile.  Measured, bias + residual: M 64, K 3072, N 768: pair 22.4 us,
 // 128 x 128 17.8, 64 x 4 CTAs 8.7; M 776, K 1024, N 1024: 14.3 / 10.7 / (64 x 1) 8.8; M 4096, K 768, N 3072: 27.1 / 50.6 / 44.8.
+// Beyond the fits, every configuration forced on the seven products of a layer at M up to 16384 and C 768, 1024, 1600: from M 4096 on the
+// pair kernel is the fastest but for two products (M 5439, C 1600, input gradients: 128 x 128 11 - 13 % less) and the rule takes it;
+// elsewhere it is off by 10 - 19 % at three of the 42 products below that (M 776: C x C at C 1600 17.0 against 14.3 us).
 Tile pick_tile(int kind, int epi, int M, int N, int kb_total, int splits, int a_mn, int b_mn) {
   if (g_force_bn) return {kind == KIND_F8F6F4 && g_force_bn == 64 ? 128 : g_force_bn, g_force_cl, splits};
   if (!pair_mode()) return {128, 1, splits};
@@ -585,9 +588,10 @@ Tile pick_tile(int kind, int epi, int M, int N, int kb_total, int splits, int a_
         while (sp < splits && tiles * (sp + 1) <= sms && kb_total / (sp + 1) >= 4) ++sp;
       const float per_sm = (float)(tiles * cl * sp) / sms;
       // one to two CTAs per SM and operands stored along K: the second CTA of an SM overlaps the first one's epilogue, and the kernels
-      // before and after overlap the short tail (in a chain of layers: M 776, K 1024, N 3072, 168 CTAs 2.8 us less than the pair kernel,
-      // N 4096 with GELU, 224 CTAs, 3.1 us less; as isolated launches the two are level).  Not with an auxiliary input: bias + residual at
-      // M 4096, N 768 (192 CTAs) on these tiles made a d12 step of 4 x 1024 2 % slower.
+      // before and after overlap the short tail.  M 776, us, pair / 128 x 128: K 1024, N 3072 (168 CTAs) 14.6 / 12.8, N 4096 with GELU
+      // (224) 17.1 / 15.6; K 1600, N 4800 (266) 28.9 / 20.9.  Not with an auxiliary input, which the pair kernel works in with 16
+      // warps: bias + residual, M 4096, N 768 (192), K 768 13.0 / 18.4, K 3072 25.4 / 37.5; dGELU, M 776, N 3072 (168) 13.0 / 18.7, N 4096
+      // (224) 15.2 / 23.2 (a backward product, whose weights lie along N, is out by that already).
       const bool beside = per_sm > 1.f && per_sm <= 2.f && !a_mn && !b_mn && epi != EPI_BIAS_RESID && epi != EPI_DGELU;
       const float w = per_sm <= 1.f ? 1.f : beside ? per_sm : 0.5f * (per_sm + ceilf(per_sm));
       const float fixed = (cl == 1 ? (bn == 64 ? 4.2f : 5.0f) : cl == 2 ? 5.6f : 6.2f) + (aux ? (bn == 64 ? 0.3f : 1.2f) : 0.f) + f32;

@@ -591,8 +591,9 @@ def chunked_ce_pass2(tile, stats, targets, col0: int, width: int, vocab_size: in
 
 def loss_accumulate(acc: torch.Tensor, losses: torch.Tensor, scale: float) -> None:
     """acc[0] += scale · Σ losses: the micro-step's share of the mean loss, kept on the device."""
-    if losses.is_cuda:
-        check(lib().llmb_loss_accumulate(ptr(acc), ptr(losses), losses.numel(), float(scale), stream()), "loss_accumulate")
+    if losses.is_cuda and acc.dtype == losses.dtype == torch.float32 and losses.numel() > 0:
+        flat = losses.contiguous()
+        check(lib().llmb_loss_accumulate(ptr(acc), ptr(flat), flat.numel(), float(scale), stream()), "loss_accumulate")
         _count()
     else:
         acc += losses.sum() * scale

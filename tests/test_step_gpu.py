@@ -118,6 +118,16 @@ def test_loss_accumulate(n):
         assert abs(acc.item() - want) <= 2e-6 * want, (n, off)      # at most 64 serial fp32 additions of positive terms, then a tree
 
 
+@pytest.mark.parametrize("form", ["strided", "transposed", "double", "empty"])
+def test_loss_accumulate_takes_what_a_sum_takes(form):
+    x = torch.rand(64, 96, generator=torch.Generator().manual_seed(1)).cuda()
+    x = {"strided": x[:, ::2], "transposed": x.t(), "double": x.double(), "empty": x[:0]}[form]
+    acc = torch.full((1,), 2.0, dtype=x.dtype, device="cuda")
+    ops.loss_accumulate(acc, x, 0.25)
+    want = 2.0 + 0.25 * x.double().sum().item()
+    assert abs(acc.item() - want) <= 2e-6 * want
+
+
 def test_options_changed_after_the_buffers_take_the_op_by_op_path():
     """One GELU buffer, and a backward pass that would index one per layer."""
     m = GPT2(GPT2Config(max_seq_len=64, vocab_size=1000, num_layer=2, num_heads=1, channels=64, padded_vocab_size=1024), "bf16", "cuda", recompute=True)

@@ -566,7 +566,8 @@ thread_local int g_force_bn = 0, g_force_cl = 1;          // test hook (llmb_gem
 // Beyond the fits, every configuration forced on the seven products of a layer at M up to 16384 and C 768, 1024, 1600: from M 4096 on the
 // pair kernel is the fastest but for two products (M 5439, C 1600, input gradients: 128 x 128 11 - 13 % less) and the rule takes it;
 // elsewhere it is off by 10 - 19 % at three of the 42 products below that (M 776: C x C at C 1600 17.0 against 14.3 us).
-Tile pick_tile(int kind, int epi, int M, int N, int kb_total, int splits, int a_mn, int b_mn) {
+// splits: parts of K in the pair kernel; most: the most that this kernel's CTAs may cut it into.
+Tile pick_tile(int kind, int epi, int M, int N, int kb_total, int splits, int most, int a_mn, int b_mn) {
   if (g_force_bn) return {kind == KIND_F8F6F4 && g_force_bn == 64 ? 128 : g_force_bn, g_force_cl, splits};
   if (!pair_mode()) return {128, 1, splits};
   const bool aux = epi == EPI_BIAS_GELU || epi == EPI_DGELU || epi == EPI_BIAS_RESID, acc = epi == EPI_ACC_F32;
@@ -584,8 +585,8 @@ Tile pick_tile(int kind, int epi, int M, int N, int kb_total, int splits, int a_
     for (int cl = 1; cl <= (bn == 64 ? 4 : 2); cl *= 2) {
       if (cl > 1 && (acc || kind == KIND_TF32 || tiles * cl > sms || cl > kb_total)) break;
       int sp = 1;
-      if (acc)                                            // one round of CTAs, at least four k-blocks each, no more parts than asked for
-        while (sp < splits && tiles * (sp + 1) <= sms && kb_total / (sp + 1) >= 4) ++sp;
+      if (acc)                                            // one round of CTAs, at least four k-blocks each, no more parts than allowed
+        while (sp < most && tiles * (sp + 1) <= sms && kb_total / (sp + 1) >= 4) ++sp;
       const float per_sm = (float)(tiles * cl * sp) / sms;
       // one to two CTAs per SM and operands stored along K: the second CTA of an SM overlaps the first one's epilogue, and the kernels
       // before and after overlap the short tail.  M 776, us, pair / 128 x 128: K 1024, N 3072 (168 CTAs) 14.6 / 12.8, N 4096 with GELU
@@ -600,6 +601,14 @@ Tile pick_tile(int kind, int epi, int M, int N, int kb_total, int splits, int a_
     }
   }
   return t;
+}
+
+// The caller's `splits` (see llmb_gemm): makes it the parts of the pair kernel, 1 ... kb_total, and returns the most parts for other tiles.
+int parts(int& splits, int kb_total) {
+  const bool rule = splits < 0;
+  if (rule) splits = splits < -kb_total ? kb_total : -splits;
+  splits = splits < 1 ? 1 : splits > kb_total ? kb_total : splits;
+  return rule ? 16 : splits;
 }
 
 template <int KIND>
@@ -647,10 +656,10 @@ int gemm_dispatch(void* D, const void* A, const void* B, const void* bias, void*
   }
   if (p.colsum && !p.tma_epi) return LLMB_ERR_BAD_ARG;    // the column sums are taken in the TMA epilogue only
   const int kb_total = ceil_div(K, BKE);
-  if (splits < 1 || epi != EPI_ACC_F32) splits = 1;
-  if (splits > kb_total) splits = kb_total;
+  const int most = parts(splits, kb_total);
+  if (epi != EPI_ACC_F32) splits = 1;
   Tile tile{256, 1, splits};
-  if (p.tma_epi && !keep_pair && p.g.W <= 1 && p.pull.nseg == 0 && p.pull.nwait == 0) tile = pick_tile(KIND, epi, M, N, kb_total, splits, a_mn, b_mn);
+  if (p.tma_epi && !keep_pair && p.g.W <= 1 && p.pull.nseg == 0 && p.pull.nwait == 0) tile = pick_tile(KIND, epi, M, N, kb_total, splits, most, a_mn, b_mn);
   while (tile.cl > 1 && tile.cl > kb_total) tile.cl >>= 1;
   splits = tile.splits;
   const bool pair = tile.bn == 256;
@@ -1021,7 +1030,8 @@ int launch_nvfp4(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap
 // D[M,N] = epi(alpha * A·B^T).  a_mn/b_mn = 1 when the operand is stored [K, M] / [K, N].
 // kind: 0 bf16, 1 tf32 (fp32 storage), 2 fp8 (a_fmt/b_fmt: 0 e4m3, 1 e5m2).  D is bf16 except for the
 // fp32 epilogues (4 = accumulate with red.add; 6 = plain fp32 store).  splits: the most parts that K may be cut into by an accumulating
-// product.  Parts are added in the order in which they finish, so with one part the result is the same on every run.
+// product.  Parts are added in the order in which they finish, so with one part the result is the same on every run.  splits < 0: -splits
+// parts on CTA pairs, and as many as fill the chip (up to 16) where the tile rule takes other tiles.
 // `status` is a device int the kernel sets to LLMB_ERR_TIMEOUT if a bounded wait expires.
 LLMB_API int llmb_gemm(void* D, const void* A, const void* B, const void* bias, void* aux, const float* alpha, int M,
                        int N, int K, long long lda, long long ldb, long long ldd, long long ldaux, int a_mn, int b_mn,
@@ -1038,8 +1048,8 @@ LLMB_API int llmb_gemm(void* D, const void* A, const void* B, const void* bias, 
 // one part the result may as well be stored (epilogue 6) where nothing has to be added to.
 LLMB_API int llmb_gemm_dw_splits(int kind, int M, int N, int K, int splits) {
   const int kb = ceil_div(K, kind == 0 ? 64 : 32);
-  splits = splits < 1 ? 1 : splits > kb ? kb : splits;
-  return pick_tile(kind == 0 ? KIND_F16 : KIND_TF32, EPI_ACC_F32, M, N, kb, splits, 1, 1).splits;
+  const int most = parts(splits, kb);
+  return pick_tile(kind == 0 ? KIND_F16 : KIND_TF32, EPI_ACC_F32, M, N, kb, splits, most, 1, 1).splits;
 }
 
 // Arms the calling thread's NEXT llmb_gemm call to gather its A matrix from W ranks (see GatherArgs): A must be the

@@ -276,7 +276,7 @@ class GPT2:
             ops.chunked_ce_pass2(tile, a["ce_stats"], self._tgt_all, v0, w, V, self._dloss)
             ops.gemm(p32, tile, p["wte"][v0:v0 + w], b_mn=True, epi=ops.EPI_STORE_F32)
             ops.gemm(g["wte"][v0:v0 + w], tile, self._lnf_all, a_mn=True, b_mn=True, epi=ops.EPI_ACC_F32,
-                     splits=ops._splits_for(w, C, n_all))
+                     splits=ops._dw_splits(w, C, n_all))
             z.reduce_scatter_rows_f32(p32.view(-1), own32)
             dl.view(-1).copy_(own32)
             return

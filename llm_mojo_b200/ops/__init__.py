@@ -209,7 +209,8 @@ EPI_NONE, EPI_BIAS, EPI_BIAS_GELU, EPI_DGELU, EPI_ACC_F32, EPI_BIAS_RESID, EPI_S
 def gemm(D, A, B, *, a_mn=False, b_mn=False, epi=EPI_NONE, bias=None, aux=None, alpha=None, splits=1,
          kind: int = 0, a_fmt: int = 0, b_fmt: int = 0, colsum=None) -> None:
     """Raw tcgen05 GEMM: D[M,N] = epi(A·Bᵀ).  A is [M,K] (or [K,M] when ``a_mn``), B is [N,K]
-    (or [K,N] when ``b_mn``); all row-major with arbitrary row pitch.  ``colsum`` (fp32 [N], dGELU epilogue with
+    (or [K,N] when ``b_mn``); all row-major with arbitrary row pitch.  ``splits``: the most parts of K in an accumulating
+    product, added in the order in which they finish (one part: the same bits on every run).  ``colsum`` (fp32 [N], dGELU epilogue with
     a bf16 result only, see ``colsum_usable``) accumulates the column sums of D inside the epilogue."""
     M, N = D.shape
     K = A.shape[0] if a_mn else A.shape[1]
@@ -282,6 +283,14 @@ def _splits_for(M: int, N: int, K: int, *, tile: int = 256, tile_n: int = 0, bk:
     return best
 
 
+def _dw_splits(M: int, N: int, K: int) -> int:
+    """The parts of a weight gradient's contraction, as ``llmb_gemm`` takes them: those that fill the CTA pairs, and what fills the chip where
+    other tiles are taken.  ``LLMB_ATTN_BWD=split``, the repeatable choice, holds these to the former, so that a product of one part
+    stays one."""
+    s = _splits_for(M, N, K)
+    return -s if ATTN_BWD == "fused" else s
+
+
 def matmul_fwd(out, inp, weight, bias=None, *, pre_gelu=None, residual=None) -> None:
     """out = inp·weightᵀ (+bias) — optionally out = GELU(pre), pre_gelu = inp·Wᵀ+b, or
     out = inp·Wᵀ + b + residual (llmm/matmul.mojo:1526-1722: BIAS / GELU_AUX_BIAS epilogues)."""
@@ -334,7 +343,7 @@ def matmul_bwd(dinp, dweight, dbias, dout, inp, weight, *, gelu_pre=None, dinp_c
                 if dinp_colsum is not None:
                     dbias_reduce(dinp_colsum, di)
         if dweight is not None:
-            gemm(dweight.view(OC, C), d, x, a_mn=True, b_mn=True, epi=EPI_ACC_F32, splits=_splits_for(OC, C, rows), kind=kind)
+            gemm(dweight.view(OC, C), d, x, a_mn=True, b_mn=True, epi=EPI_ACC_F32, splits=_dw_splits(OC, C, rows), kind=kind)
         if dbias is not None:
             dbias_reduce(dbias, d)
         return
@@ -363,7 +372,7 @@ def lm_head_bwd_tile(dinp, dweight_tile, dlogits_tile, inp, weight_tile, accumul
             gemm(di, d, weight_tile, b_mn=True, epi=EPI_BIAS_RESID, aux=di, kind=kind)
         else:
             gemm(di, d, weight_tile, b_mn=True, kind=kind)
-        gemm(dweight_tile, d, x, a_mn=True, b_mn=True, epi=EPI_ACC_F32, splits=_splits_for(w, C, rows), kind=kind)
+        gemm(dweight_tile, d, x, a_mn=True, b_mn=True, epi=EPI_ACC_F32, splits=_dw_splits(w, C, rows), kind=kind)
         return
     g = d.float() @ weight_tile.float()
     if accumulate:

@@ -24,7 +24,7 @@ from typing import Dict, Optional, Tuple
 import torch
 
 from . import (EPI_ACC_F32, EPI_BIAS, EPI_BIAS_GELU, EPI_BIAS_RESID, EPI_DGELU, EPI_NONE, _count, _gelu_grad_t, _gelu_t,
-               _splits_for, dbias_reduce, gemm, gemm_mxfp8, gemm_nvfp4, scratch)
+               _dw_splits, _splits_for, dbias_reduce, gemm, gemm_mxfp8, gemm_nvfp4, scratch)
 from ._lib import check, dtype_code, lib, ptr, status_word, stream
 from . import matmul_fwd as ops_matmul_fwd, matmul_bwd as ops_matmul_bwd
 
@@ -337,7 +337,7 @@ def matmul_bwd_fp8(dinp, dweight, dbias, dout, inp, weight, site: LinearSite, *,
     else:
         alpha2 = site.dout.scale_inv * site.inp.scale_inv
     if dout.is_cuda:
-        gemm(dweight.view(OC, C), qd, qx, a_mn=True, b_mn=True, epi=EPI_ACC_F32, splits=_splits_for(OC, C, rows), alpha=alpha2,
+        gemm(dweight.view(OC, C), qd, qx, a_mn=True, b_mn=True, epi=EPI_ACC_F32, splits=_dw_splits(OC, C, rows), alpha=alpha2,
              kind=2, a_fmt=E5M2, b_fmt=E4M3)
         if dbias is not None:
             dbias_reduce(dbias, d)
@@ -602,7 +602,7 @@ def matmul_bwd_fp4(dinp, dweight, dbias, dout, inp, weight, *, gelu_pre=None, rh
     dx, tsx = nvfp4_fake_quant(x, axis=0, block_rows=1, rht=usable_rht)
     alpha = tsd * tsx * ((1.0 / 16.0) if usable_rht else 1.0)
     if dout.is_cuda:
-        gemm(dweight.view(OC, C), dd, dx, a_mn=True, b_mn=True, epi=EPI_ACC_F32, splits=_splits_for(OC, C, rows), alpha=alpha)
+        gemm(dweight.view(OC, C), dd, dx, a_mn=True, b_mn=True, epi=EPI_ACC_F32, splits=_dw_splits(OC, C, rows), alpha=alpha)
         if dbias is not None:
             dbias_reduce(dbias, d)
     else:

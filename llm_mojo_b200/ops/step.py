@@ -11,7 +11,7 @@ import os
 
 import torch
 
-from . import colsum_usable, lowp, scratch, _count, _splits_for
+from . import colsum_usable, lowp, scratch, _count, _dw_splits, _splits_for
 from ._lib import check, dtype_code, lib, status_word, stream
 from ..config import PARAM_NAMES
 from .. import ops
@@ -142,12 +142,12 @@ def backward(m, first: bool) -> bool:
     B, T, C, NH, Vp = m.B, m.T, cfg.channels, cfg.num_heads, cfg.padded_vocab_size
     rows, L = B * T, lib()
     s.fc_colsum = int(colsum_usable(a["dl_bt4c"].view(rows, 4 * C), a["fch"][0].view(rows, 4 * C)))
-    s.splits_qkv, s.splits_att = _splits_for(3 * C, C, rows), _splits_for(C, C, rows)
-    s.splits_fc, s.splits_proj = _splits_for(4 * C, C, rows), _splits_for(C, 4 * C, rows)
+    s.splits_qkv, s.splits_att = _dw_splits(3 * C, C, rows), _dw_splits(C, C, rows)
+    s.splits_fc, s.splits_proj = _dw_splits(4 * C, C, rows), _dw_splits(C, 4 * C, rows)
     if tiled:
-        s.splits_head, s.splits_head_last = (_splits_for(w, C, rows) for w in (m.tile_width, Vp - (Vp - 1) // m.tile_width * m.tile_width))
+        s.splits_head, s.splits_head_last = (_dw_splits(w, C, rows) for w in (m.tile_width, Vp - (Vp - 1) // m.tile_width * m.tile_width))
     else:
-        s.splits_head = s.splits_head_last = _splits_for(Vp, C, rows)
+        s.splits_head = s.splits_head_last = _dw_splits(Vp, C, rows)
     if s.lowp:
         if m.step_kept is not None and m.step_kept.numel() == L.llmb_gpt2_lowp_kept_bytes(ctypes.byref(s)):
             s.kept = m.step_kept.data_ptr()              # of this micro-step's forward pass

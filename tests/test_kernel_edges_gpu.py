@@ -334,3 +334,18 @@ def test_gemm_armed_for_the_pair_kernel(M, N, K, force_tile):
     assert torch.equal(product(), rule)
     if (M, K) == (64, 3072):
         assert not torch.equal(rule, pair)           # four CTAs add their parts of K: another order
+
+
+@pytest.mark.parametrize("M,N,K", [(384, 384, 777), (768, 768, 2048), (1536, 384, 1024)])      # the rule alone would cut K into 3, 4 and 4 parts
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_weight_gradient_in_one_part_repeats_itself(M, N, K, dtype):
+    a, b = rnd(K, M, dtype=dtype).to(DEV), rnd(K, N, dtype=dtype, seed=1).to(DEV)
+    start = rnd(M, N, dtype=torch.float32, seed=2).to(DEV)
+    got = []
+    for _ in range(4):
+        d = start.clone()
+        ops.gemm(d, a, b, a_mn=True, b_mn=True, epi=ops.EPI_ACC_F32, splits=1, kind=0 if dtype == torch.bfloat16 else 1)
+        got.append(d)
+    assert all(torch.equal(got[0], d) for d in got[1:])
+    want = start.double() + a.double().t() @ b.double()
+    assert_close(got[0], want, (1e-4 if dtype == torch.bfloat16 else 2.0 ** -8) * math.sqrt(K), 1e-4 if dtype == torch.bfloat16 else 2.0 ** -10, "dW")

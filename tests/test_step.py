@@ -10,6 +10,7 @@ import threading
 import pytest
 import torch
 
+from llm_mojo_b200 import ops
 from llm_mojo_b200.config import GPT2Config
 from llm_mojo_b200.models import GPT2
 from llm_mojo_b200.ops import _lib, step
@@ -33,6 +34,17 @@ def test_weight_gradients_are_cut_into_no_more_parts_than_asked_for(kind):
                     assert 1 <= got <= splits, (M, N, K, splits, got)
                     seen.add(got)
     assert len(seen) > 2
+    # a negative number leaves the parts of other tiles than CTA pairs to the rule, and means the same on CTA pairs
+    assert L.llmb_gemm_dw_splits(kind, 384, 384, 777, -1) > L.llmb_gemm_dw_splits(kind, 384, 384, 777, 1) == 1
+    assert L.llmb_gemm_dw_splits(kind, 3072, 3072, 8192, -2) == L.llmb_gemm_dw_splits(kind, 3072, 3072, 8192, 2) == 2
+    assert 1 <= L.llmb_gemm_dw_splits(kind, 384, 384, 64, -(1 << 31)) <= 2
+
+
+@pytest.mark.parametrize("bwd,sign", [("fused", -1), ("split", 1)])
+def test_the_repeatable_choice_holds_weight_gradients_to_their_parts(bwd, sign, monkeypatch):
+    monkeypatch.setattr(ops, "ATTN_BWD", bwd)
+    for size in ((384, 384, 777), (768, 768, 65536)):
+        assert ops._dw_splits(*size) == sign * ops._splits_for(*size)
 
 
 class _Fn:

@@ -49,6 +49,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   constexpr int WSB = Cfg::WARP_STAGE;
   constexpr int EPI_WARPS = PairCfg<KIND, EPI>::EPI_WARPS;
   constexpr bool WIDE = PairCfg<KIND, EPI>::WIDE;
+  constexpr int BKE = KindTraits<KIND>::BKE;            // elements of a swizzled row: K of a stage, and the columns of an MN-major chunk
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   unsigned char* epi_stage = smem + NST * STAGE2_BYTES;
@@ -106,8 +107,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     const int n0 = n_blk * BN + (int)cta * 128;
     if (m_blk % BAND2 == 0 && elect_one())
       for (int kb = kb0; kb < kb1 && kb < kb0 + NST; ++kb) {
-        if (!p.b_mn) tma_prefetch_l2_2d(&tmB, kb * p.bke, n0);
-        else if (p.b_3d) tma_prefetch_l2_3d(&tmB, 0, kb * p.bke, n0 / p.bke);
+        if (!p.b_mn) tma_prefetch_l2_2d(&tmB, kb * BKE, n0);
+        else if (p.b_3d) tma_prefetch_l2_3d(&tmB, 0, kb * BKE, n0 / BKE);
       }
     __syncwarp();
   }
@@ -115,7 +116,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer (both CTAs)
-    // warp-uniform loop, one elected lane issues (same reasoning as for the MMA issuer below)
+    // warp-uniform loop, one elected lane issues (same reasoning as for the MMA issuer below).
+    // The loop, not TMA, can be what paces an MN-major operand: the four MMAs of a k-block take 512 cycles, the barrier round trips of a
+    // turn about 300, and a chunk index m0 / (k-block size) with a divisor known at run time only cost 155 more per operand and turn
+    // (690 cycles in all for a weight gradient; 380 as it is now).  Hence BKE.  M 65536, C 768: weight gradients of a layer 891 -> 636
+    // us, input gradients 917 -> 730; M 4096, C 768: 82.8 -> 69.0, 82.0 -> 77.4.
     {
       int stage = 0; uint32_t phase = 0;
       const uint32_t lead_full0 = mapa_u32(smem_u32(&full_bar[0]), 0);
@@ -152,20 +157,20 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           unsigned char* sa = smem + stage * STAGE2_BYTES;
           unsigned char* sb = sa + A_STAGE;
           const uint32_t lead_full = lead_full0 + stage * 8;
-          const int k0 = kb * p.bke;
+          const int k0 = kb * BKE;
           if (elect_one()) {
             if (leader) mbar_expect_tx(&full_bar[stage], 2 * STAGE2_BYTES);     // bytes of both CTAs
             if (!p.a_mn) tma_load_2d_pair(sa, &tmA, lead_full, k0, m0);
-            else if (p.a_3d) tma_load_3d_pair(sa, &tmA, lead_full, 0, k0, m0 / p.bke);
+            else if (p.a_3d) tma_load_3d_pair(sa, &tmA, lead_full, 0, k0, m0 / BKE);
             else {
-              const int chunk_elems = p.bke, nchunk = BM / chunk_elems;
-              for (int c = 0; c < nchunk; ++c) tma_load_2d_pair(sa + c * p.bke * ROW_BYTES, &tmA, lead_full, m0 + c * chunk_elems, k0);
+#pragma unroll
+              for (int c = 0; c < BM / BKE; ++c) tma_load_2d_pair(sa + c * BKE * ROW_BYTES, &tmA, lead_full, m0 + c * BKE, k0);
             }
             if (!p.b_mn) tma_load_2d_pair(sb, &tmB, lead_full, k0, n0);
-            else if (p.b_3d) tma_load_3d_pair(sb, &tmB, lead_full, 0, k0, n0 / p.bke);
+            else if (p.b_3d) tma_load_3d_pair(sb, &tmB, lead_full, 0, k0, n0 / BKE);
             else {
-              const int chunk_elems = p.bke, nchunk = 128 / chunk_elems;
-              for (int c = 0; c < nchunk; ++c) tma_load_2d_pair(sb + c * p.bke * ROW_BYTES, &tmB, lead_full, n0 + c * chunk_elems, k0);
+#pragma unroll
+              for (int c = 0; c < 128 / BKE; ++c) tma_load_2d_pair(sb + c * BKE * ROW_BYTES, &tmB, lead_full, n0 + c * BKE, k0);
             }
           }
           __syncwarp();
@@ -709,7 +714,6 @@ int gemm_dispatch(void* D, const void* A, const void* B, const void* bias, void*
   p.a_lbo = a_mn ? mn_lbo : 16; p.a_sbo = a_mn ? mn_sbo : 1024; p.a_kstep = a_mn ? MMA_K * ROW_BYTES : 32;
   p.b_lbo = b_mn ? mn_lbo : 16; p.b_sbo = b_mn ? mn_sbo : 1024; p.b_kstep = b_mn ? MMA_K * ROW_BYTES : 32;
   p.idesc = make_idesc((uint32_t)a_fmt, (uint32_t)b_fmt, (uint32_t)a_mn, (uint32_t)b_mn, pair ? 2 * BM : BM, (uint32_t)tile.bn);
-  p.bke = BKE;                                          // a 128-byte stage row holds BKE / MMA_K = 4 MMA k-steps for every kind
   p.m_tiles = ceil_div(M, BM); p.n_tiles = ceil_div(N, tile.bn);
   p.kb_total = kb_total;
   p.kb_per_split = ceil_div(kb_total, splits);
@@ -1121,7 +1125,6 @@ int gemm_block_scaled(void* D, const void* A, const void* B, const void* sfa, co
   GemmParams& p = q.g;
   p.D = D; p.bias = bias; p.aux = aux; p.alpha = alpha;
   p.M = M; p.N = N; p.K = K; p.ldd = ldd; p.ldaux = ldaux;
-  p.bke = BKE;
   p.m_tiles = ceil_div(M, BM); p.n_tiles = ceil_div(N, NV_BN);
   p.kb_total = ceil_div(K, BKE);
   if (splits < 1) splits = 1;

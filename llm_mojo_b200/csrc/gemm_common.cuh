@@ -69,7 +69,6 @@ struct GemmParams {
   uint32_t a_lbo, a_sbo, a_kstep, b_lbo, b_sbo, b_kstep;   // bytes
   uint32_t a_layout, b_layout; // UMMA layout type: 2 = SWIZZLE_128B, 1 = SWIZZLE_128B with 32-byte base (fp32 MN-major)
   uint32_t idesc;
-  int bke;                     // K elements per stage
   int m_tiles, n_tiles, splits, kb_per_split, kb_total;
   int io_f32;                  // 1: D, bias and aux are fp32 (tf32 kind); 0: bf16
   int tma_epi;                 // 1: bf16 outputs leave (and auxiliary inputs arrive) by TMA; 0: register/shared-memory epilogue
@@ -387,9 +386,9 @@ __device__ __forceinline__ void epi_box_f32(const GemmParams& p, const uint32_t 
 }
 
 template <int KIND> struct KindTraits;
-template <> struct KindTraits<KIND_F16> { static constexpr int ESZ = 2; static constexpr CUtensorMapDataType DT = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16; };
-template <> struct KindTraits<KIND_TF32> { static constexpr int ESZ = 4; static constexpr CUtensorMapDataType DT = CU_TENSOR_MAP_DATA_TYPE_FLOAT32; };
-template <> struct KindTraits<KIND_F8F6F4> { static constexpr int ESZ = 1; static constexpr CUtensorMapDataType DT = CU_TENSOR_MAP_DATA_TYPE_UINT8; };
+template <> struct KindTraits<KIND_F16> { static constexpr int ESZ = 2, BKE = ROW_BYTES / ESZ; static constexpr CUtensorMapDataType DT = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16; };
+template <> struct KindTraits<KIND_TF32> { static constexpr int ESZ = 4, BKE = ROW_BYTES / ESZ; static constexpr CUtensorMapDataType DT = CU_TENSOR_MAP_DATA_TYPE_FLOAT32; };
+template <> struct KindTraits<KIND_F8F6F4> { static constexpr int ESZ = 1, BKE = ROW_BYTES / ESZ; static constexpr CUtensorMapDataType DT = CU_TENSOR_MAP_DATA_TYPE_UINT8; };
 }  // namespace lgemm
 using namespace lgemm;
 

@@ -36,6 +36,7 @@ __global__ void __launch_bounds__(SM_THREADS)
 gemm_small_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                   const __grid_constant__ CUtensorMap tmD, const __grid_constant__ CUtensorMap tmAux, const GemmParams p, int stages) {
   using Cfg = SmallCfg<KIND, EPI, BN_, CL>;
+  constexpr int BKE = KindTraits<KIND>::BKE;
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   unsigned char* aux_s = smem + stages * Cfg::STAGE;
@@ -75,9 +76,9 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   // writes B, the loads below still read what it wrote.
   if (warp == 0 && m_blk == 0 && elect_one()) {
     for (int kb = kb0; kb < kb1 && kb < kb0 + 16; ++kb) {
-      const int k0 = kb * p.bke;
+      const int k0 = kb * BKE;
       if (!p.b_mn) tma_prefetch_l2_2d(&tmB, k0, n0);
-      else if (p.b_3d) tma_prefetch_l2_3d(&tmB, 0, k0, n0 / p.bke);
+      else if (p.b_3d) tma_prefetch_l2_3d(&tmB, 0, k0, n0 / BKE);
     }
   }
   __syncwarp();
@@ -105,15 +106,15 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
       if (kb - kb0 >= stages && !mbar_wait(&empty_bar[stage], phase ^ 1)) { ok = false; break; }
       unsigned char* sa = smem + stage * Cfg::STAGE;
       unsigned char* sb = sa + A_STAGE;
-      const int k0 = kb * p.bke;
+      const int k0 = kb * BKE;
       if (elect_one()) {
         mbar_expect_tx(&full_bar[stage], Cfg::STAGE);
         if (!p.a_mn) tma_load_2d(sa, &tmA, &full_bar[stage], k0, m0);
-        else if (p.a_3d) tma_load_3d(sa, &tmA, &full_bar[stage], 0, k0, m0 / p.bke);
-        else for (int c = 0; c < BM / p.bke; ++c) tma_load_2d(sa + c * p.bke * ROW_BYTES, &tmA, &full_bar[stage], m0 + c * p.bke, k0);
+        else if (p.a_3d) tma_load_3d(sa, &tmA, &full_bar[stage], 0, k0, m0 / BKE);
+        else for (int c = 0; c < BM / BKE; ++c) tma_load_2d(sa + c * BKE * ROW_BYTES, &tmA, &full_bar[stage], m0 + c * BKE, k0);
         if (!p.b_mn) tma_load_2d(sb, &tmB, &full_bar[stage], k0, n0);
-        else if (p.b_3d) tma_load_3d(sb, &tmB, &full_bar[stage], 0, k0, n0 / p.bke);
-        else for (int c = 0; c < BN_ / p.bke; ++c) tma_load_2d(sb + c * p.bke * ROW_BYTES, &tmB, &full_bar[stage], n0 + c * p.bke, k0);
+        else if (p.b_3d) tma_load_3d(sb, &tmB, &full_bar[stage], 0, k0, n0 / BKE);
+        else for (int c = 0; c < BN_ / BKE; ++c) tma_load_2d(sb + c * BKE * ROW_BYTES, &tmB, &full_bar[stage], n0 + c * BKE, k0);
       }
       __syncwarp();
       if (++stage == stages) { stage = 0; phase ^= 1; }

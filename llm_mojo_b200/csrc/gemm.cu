@@ -10,528 +10,14 @@
 // MN-major (the UMMA descriptor and the TMA box change, not the data), which is how dinp (B = W as stored) and dW (A = dout^T,
 // B = inp^T as stored) run without any transposes.  Split-K work units add into the (fp32) gradient buffer.
 //
-// gemm_pair_kernel (two CTAs per 256 x 256 tile with cta_group::2 MMAs, persistent, 8 or 16 epilogue warps, optional all-gather of A
-// from peer GPUs and optional column sums of the result) runs what fills the chip with such tiles; gemm_small.cu runs the rest on
-// 128-row tiles; gemm_nvfp4_kernel has block-scaled NVFP4 / MXFP8 operands with their scales in tensor memory.  pick_tile() chooses.
+// gemm_pair_kernel (gemm_pair.cuh: two CTAs per 256 x 256 tile with cta_group::2 MMAs, persistent, 8 epilogue warps, optional
+// all-gather of A from peer GPUs and optional column sums of the result) runs what fills the chip with such tiles; gemm_small.cu runs the
+// rest on 128-row tiles; pick_tile() chooses.
+// gemm_nvfp4_kernel has block-scaled NVFP4 / MXFP8 operands with their scales in tensor memory.
 #include <math.h>
-#include "gemm_common.cuh"
+#include "gemm_pair.cuh"
 
 namespace {
-// ------------------------------------------------------------------------------------------------
-// CTA-pair variant: a cluster of two CTAs computes a 256 x 256 tile with cta_group::2 MMAs.  Each
-// CTA stages its own 128 rows of A and its own 128-row half of B (half the B traffic per SM, and
-// a ring of 32 KB stages instead of 48 KB ones), the leader issues the MMAs, and both
-// CTAs drain their 128 x 256 accumulator halves.  No load is multicast: every CTA fetches only
-// the tiles it owns; the peer's TMA completions are reported to the leader's mbarrier.
-constexpr int B2_STAGE = 128 * ROW_BYTES;             // 16 KB: this CTA's half of the B tile
-constexpr int STAGE2_BYTES = A_STAGE + B2_STAGE;      // 32 KB
-// TMA producer, MMA issuer, 8 or 16 epilogue warps, 2 gather copier warps.  Sixteen where an auxiliary input has to be read and worked
-// in (bf16 outputs): a slab of 64 columns is a chain of TMEM loads, MUFU and FMA latencies, staging and column sums, and with two warps
-// per scheduler a tile of such slabs took twice the time of its MMAs at K = 768.  K = 768, 8 -> 16 warps, us: dGELU + column sums N 3072, M
-// 4096 32.2 -> 30.8, M 5439 40.0 -> 36.2, M 12288 72.4 -> 65.0; bias + residual N 768, M 5439 14.1 -> 13.2, M 12288 22.4 -> 20.2 (K 3072, M
-// 5439 26.1 -> 25.2).  Without an auxiliary input the operands' L2 traffic bounds a tile (12 TB/s at M 12288) and eight warps keep up.
-template <int KIND, int EPI> struct PairCfg {
-  static constexpr bool WIDE = EpiCfg<EPI>::AUX_IN && KIND != KIND_TF32;
-  static constexpr int EPI_WARPS = WIDE ? 16 : 8;
-  static constexpr int THREADS = 32 * (4 + EPI_WARPS);
-};
-constexpr int FLAG_ROWS_READY = 6;                     // flag kind (layout of comm.cu: flags[kind][8 ranks])
-constexpr int FLAG_PARAM = 3;                          // owners announce the optimizer step their parameter shard holds
-constexpr int SMEM2_TAIL = 512;                        // barriers, TMEM slot, abort flag
-template <int EPI> constexpr int smem2_bytes() { return EpiCfg<EPI>::STAGES * STAGE2_BYTES + 4 * EpiCfg<EPI>::WARP_STAGE + 1024 + SMEM2_TAIL; }
-
-template <int KIND, int EPI>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PairCfg<KIND, EPI>::THREADS, 1)
-gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                 const __grid_constant__ CUtensorMap tmD, const __grid_constant__ CUtensorMap tmAux, const GemmParams p) {
-  using Cfg = EpiCfg<EPI>;
-  constexpr int NST = Cfg::STAGES;
-  constexpr int WSB = Cfg::WARP_STAGE;
-  constexpr int EPI_WARPS = PairCfg<KIND, EPI>::EPI_WARPS;
-  constexpr bool WIDE = PairCfg<KIND, EPI>::WIDE;
-  constexpr int BKE = KindTraits<KIND>::BKE;            // elements of a swizzled row: K of a stage, and the columns of an MN-major chunk
-  extern __shared__ unsigned char smem_raw[];
-  unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  unsigned char* epi_stage = smem + NST * STAGE2_BYTES;
-  uint64_t* full_bar = reinterpret_cast<uint64_t*>(epi_stage + 4 * WSB);
-  uint64_t* empty_bar = full_bar + NST;
-  uint64_t* tfull_bar = empty_bar + NST;
-  uint64_t* tempty_bar = tfull_bar + 2;
-  uint64_t* aux_bar = tempty_bar + 2;                   // [8 warps][2 slabs] or [16 warps]: auxiliary-input tiles landed
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(aux_bar + 16);
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-
-  const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-  const uint32_t cta = cluster_ctarank();              // 0 = leader
-  const bool leader = cta == 0;
-
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < NST; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
-    for (int a = 0; a < 2; ++a) { mbar_init(&tfull_bar[a], 1); mbar_init(&tempty_bar[a], 2 * EPI_WARPS); }
-    for (int a = 0; a < 16; ++a) mbar_init(&aux_bar[a], 1);
-    *abort_flag = 0;
-    fence_barrier_init();
-    prefetch_tmap(&tmA); prefetch_tmap(&tmB);
-    if (p.tma_epi) { prefetch_tmap(&tmD); prefetch_tmap(&tmAux); }
-  }
-  if (warp == 1) tmem_alloc_pair<512>(tmem_slot);
-  fence_before_sync();
-  __syncthreads();
-  cluster_sync_all();                                   // both CTAs' barriers exist before any remote signal
-  fence_after_sync();
-  const uint32_t tmem_base = *tmem_slot;
-  if (p.g.W <= 1 && p.pull.nseg == 0 && p.pull.nwait == 0) pdl_trigger();   // else this kernel waits for other GPUs or streams
-
-  const int m_tiles = ceil_div(p.M, 2 * BM);            // cluster tiles of 256 rows
-  const int tiles_per_split = m_tiles * p.n_tiles;
-  const int total_units = tiles_per_split * p.splits;
-  const int cluster_id = blockIdx.x >> 1, num_clusters = gridDim.x >> 1;
-  constexpr int BAND2 = 8;
-
-  auto unit_coords = [&](int unit, int& m_blk, int& n_blk, int& kb0, int& kb1) {
-    int split = unit / tiles_per_split, t = unit % tiles_per_split;
-    int band_sz = BAND2 * p.n_tiles;
-    int b = t / band_sz, r = t % band_sz;
-    int m_in_band = min(BAND2, m_tiles - b * BAND2);
-    m_blk = b * BAND2 + r % m_in_band;
-    n_blk = r / m_in_band;
-    if (p.g.W > 1) m_blk = (m_blk + p.g.me * p.g.tiles_per_chunk) % m_tiles;   // the local chunk's tiles come first
-    kb0 = split * p.kb_per_split;
-    kb1 = min(p.kb_total, kb0 + p.kb_per_split);
-  };
-
-  // While the kernel before this one drains: the first ring of B (a forward or input-gradient GEMM's weights) into L2, once per column
-  // of tiles.  A hint only, so it may run before the wait; if that kernel writes B, the loads below still read what it wrote.
-  if (warp == 0 && cluster_id < total_units && p.pull.nwait == 0) {
-    int m_blk, n_blk, kb0, kb1; unit_coords(cluster_id, m_blk, n_blk, kb0, kb1);
-    const int n0 = n_blk * BN + (int)cta * 128;
-    if (m_blk % BAND2 == 0 && elect_one())
-      for (int kb = kb0; kb < kb1 && kb < kb0 + NST; ++kb) {
-        if (!p.b_mn) tma_prefetch_l2_2d(&tmB, kb * BKE, n0);
-        else if (p.b_3d) tma_prefetch_l2_3d(&tmB, 0, kb * BKE, n0 / BKE);
-      }
-    __syncwarp();
-  }
-  pdl_wait();
-
-  if (warp == 0) {
-    // ------------------------------------------------------------ TMA producer (both CTAs)
-    // warp-uniform loop, one elected lane issues (same reasoning as for the MMA issuer below).
-    // The loop, not TMA, can be what paces an MN-major operand: the four MMAs of a k-block take 512 cycles, the barrier round trips of a
-    // turn about 300, and a chunk index m0 / (k-block size) with a divisor known at run time only cost 155 more per operand and turn
-    // (690 cycles in all for a weight gradient; 380 as it is now).  Hence BKE.  M 65536, C 768: weight gradients of a layer 891 -> 636
-    // us, input gradients 917 -> 730; M 4096, C 768: 82.8 -> 69.0, 82.0 -> 77.4.
-    {
-      int stage = 0; uint32_t phase = 0;
-      const uint32_t lead_full0 = mapa_u32(smem_u32(&full_bar[0]), 0);
-      bool ok = true;
-      int landed = -1;
-      // B operand pulled from peers (by this kernel's copier warps or by an earlier kernel's): all of it must have landed
-      for (int w = 0; w < p.pull.nwait && ok; ++w) {
-        unsigned spins = 0;
-        while ((int)(ld_acquire_gpu(p.pull.wait_counts[w]) - p.pull.wait_target[w]) < 0) {
-          if (++spins > (1u << 24)) { ok = false; break; }
-          __nanosleep(100);
-        }
-      }
-      if (p.pull.nwait) fence_proxy_async_all();          // the copiers' generic-proxy stores before this warp's TMA reads
-      if (!ok && lane == 0) { *abort_flag = 1; atomicExch(p.status, LLMB_ERR_TIMEOUT); }
-      for (int unit = cluster_id; unit < total_units && ok && !*abort_flag; unit += num_clusters) {
-        int m_blk, n_blk, kb0, kb1; unit_coords(unit, m_blk, n_blk, kb0, kb1);
-        const int m0 = m_blk * 2 * BM + (int)cta * BM, n0 = n_blk * BN + (int)cta * 128;
-        if (p.g.W > 1) {                                 // gathered A: this tile's chunk must have landed in local memory
-          const int chunk = m_blk / p.g.tiles_per_chunk;
-          if (chunk != p.g.me && chunk != landed) {
-            unsigned spins = 0;
-            while ((int)(ld_acquire_gpu(&p.g.counts[chunk]) - p.g.target) < 0) {
-              if (++spins > (1u << 24)) { ok = false; break; }
-              __nanosleep(100);
-            }
-            if (!ok) break;
-            fence_proxy_async_all();                      // the copiers' generic-proxy stores before this warp's TMA reads
-            landed = chunk;
-          }
-        }
-        for (int kb = kb0; kb < kb1; ++kb) {
-          if (!mbar_wait(&empty_bar[stage], phase ^ 1)) { ok = false; break; }
-          unsigned char* sa = smem + stage * STAGE2_BYTES;
-          unsigned char* sb = sa + A_STAGE;
-          const uint32_t lead_full = lead_full0 + stage * 8;
-          const int k0 = kb * BKE;
-          if (elect_one()) {
-            if (leader) mbar_expect_tx(&full_bar[stage], 2 * STAGE2_BYTES);     // bytes of both CTAs
-            if (!p.a_mn) tma_load_2d_pair(sa, &tmA, lead_full, k0, m0);
-            else if (p.a_3d) tma_load_3d_pair(sa, &tmA, lead_full, 0, k0, m0 / BKE);
-            else {
-#pragma unroll
-              for (int c = 0; c < BM / BKE; ++c) tma_load_2d_pair(sa + c * BKE * ROW_BYTES, &tmA, lead_full, m0 + c * BKE, k0);
-            }
-            if (!p.b_mn) tma_load_2d_pair(sb, &tmB, lead_full, k0, n0);
-            else if (p.b_3d) tma_load_3d_pair(sb, &tmB, lead_full, 0, k0, n0 / BKE);
-            else {
-#pragma unroll
-              for (int c = 0; c < 128 / BKE; ++c) tma_load_2d_pair(sb + c * BKE * ROW_BYTES, &tmB, lead_full, n0 + c * BKE, k0);
-            }
-          }
-          __syncwarp();
-          if (++stage == NST) { stage = 0; phase ^= 1; }
-        }
-        if (!ok) break;
-      }
-      if (!ok && lane == 0) { *abort_flag = 1; atomicExch(p.status, LLMB_ERR_TIMEOUT); }
-    }
-  } else if (warp == 1) {
-    // ------------------------------------------------------------ MMA issuer (leader CTA only)
-    // The whole warp walks the loop (uniform control flow, so descriptors and barrier addresses stay in
-    // uniform registers) and one elected lane issues.  Everything that does not change per k-block is
-    // computed once: the descriptors of stage 0 (a later stage only adds its byte offset >> 4 to the
-    // address field), the per-MMA descriptor increments and the cluster addresses of the barriers.
-    if (leader) {
-      int stage = 0; uint32_t phase = 0;
-      int it = 0;
-      const uint64_t adesc0 = make_smem_desc(smem_u32(smem), p.a_lbo, p.a_sbo, p.a_layout);
-      const uint64_t bdesc0 = make_smem_desc(smem_u32(smem) + A_STAGE, p.b_lbo, p.b_sbo, p.b_layout);
-      const uint64_t a_inc = (uint64_t)(p.a_kstep >> 4), b_inc = (uint64_t)(p.b_kstep >> 4);
-      const uint32_t idesc = p.idesc;
-      const uint32_t eb0 = mapa_u32(smem_u32(&empty_bar[0]), 0), eb1 = mapa_u32(smem_u32(&empty_bar[0]), 1);
-      const uint32_t tb0 = mapa_u32(smem_u32(&tfull_bar[0]), 0), tb1 = mapa_u32(smem_u32(&tfull_bar[0]), 1);
-      bool ok = true;
-      for (int unit = cluster_id; unit < total_units && !*abort_flag; unit += num_clusters, ++it) {
-        int m_blk, n_blk, kb0, kb1; unit_coords(unit, m_blk, n_blk, kb0, kb1);
-        const int acc = it & 1;
-        const uint32_t acc_phase = (it >> 1) & 1;
-        if (!mbar_wait(&tempty_bar[acc], acc_phase ^ 1)) { ok = false; break; }
-        fence_after_sync();
-        const uint32_t d_tmem = tmem_base + acc * BN;
-        for (int kb = kb0; kb < kb1; ++kb) {
-          if (!mbar_wait(&full_bar[stage], phase)) { ok = false; break; }
-          fence_after_sync();
-          const uint64_t adesc = adesc0 + (uint64_t)(stage * (STAGE2_BYTES >> 4));
-          const uint64_t bdesc = bdesc0 + (uint64_t)(stage * (STAGE2_BYTES >> 4));
-          if (elect_one()) {
-            umma_ss_pair<KIND>(d_tmem, adesc, bdesc, idesc, kb > kb0 ? 1u : 0u);
-#pragma unroll
-            for (int k = 1; k < 4; ++k) umma_ss_pair<KIND>(d_tmem, adesc + k * a_inc, bdesc + k * b_inc, idesc, 1u);
-            umma_commit_pair(eb0 + stage * 8);            // stage free in both CTAs once these MMAs have read it
-            umma_commit_pair(eb1 + stage * 8);
-          }
-          __syncwarp();
-          if (++stage == NST) { stage = 0; phase ^= 1; }
-        }
-        if (!ok) break;
-        if (elect_one()) {
-          umma_commit_pair(tb0 + acc * 8);
-          umma_commit_pair(tb1 + acc * 8);
-        }
-        __syncwarp();
-      }
-      if (!ok && lane == 0) { *abort_flag = 1; atomicExch(p.status, LLMB_ERR_TIMEOUT); }
-    }
-  } else if (warp >= 2 + EPI_WARPS) {
-    // ------------------------------------------------------------ gather copiers (the last two warps, both CTAs)
-    if (p.g.W > 1) {
-      // Slices of 32 KB are handed out by ticket, so the copy completes with whatever CTAs are resident.
-      constexpr long long SLICE = 2048;                  // 16-byte vectors
-      bool ok = true;
-      for (int step = 1; step < p.g.W && ok; ++step) {
-        const int r = (p.g.me + step) % p.g.W;
-        // rank r has announced that its chunk is complete (bounded wait, one lane polls)
-        if (lane == 0) {
-          const unsigned* f = reinterpret_cast<const unsigned*>(p.g.flags) + FLAG_ROWS_READY * 8 + r;
-          unsigned spins = 0;
-          while ((int)(ld_acquire_sys(f) - p.g.seq) < 0) {
-            if (++spins > (1u << 24)) { ok = false; break; }
-            __nanosleep(200);
-          }
-        }
-        ok = __shfl_sync(0xffffffffu, ok, 0);
-        if (!ok) break;
-        const uint4* src = reinterpret_cast<const uint4*>(p.g.peer_src[r]);
-        uint4* dst = reinterpret_cast<uint4*>(p.g.local) + (long long)r * p.g.chunk_vecs;
-        for (;;) {
-          unsigned ticket = 0;
-          if (lane == 0) ticket = atomicAdd(&p.g.counts[8 + r], 1u);
-          ticket = __shfl_sync(0xffffffffu, ticket, 0);
-          if (ticket >= p.g.target) break;
-          const long long v0 = (long long)ticket * SLICE;
-          const long long v1 = v0 + SLICE < p.g.chunk_vecs ? v0 + SLICE : p.g.chunk_vecs;
-          long long v = v0 + lane;
-          for (; v + 7 * 32 < v1; v += 8 * 32) {         // eight peer loads in flight per thread
-            uint4 t[8];
-#pragma unroll
-            for (int k = 0; k < 8; ++k) t[k] = ld_nc_v4(src + v + k * 32);
-#pragma unroll
-            for (int k = 0; k < 8; ++k) dst[v + k * 32] = t[k];
-          }
-          for (; v < v1; v += 32) dst[v] = ld_nc_v4(src + v);
-          __threadfence();
-          __syncwarp();
-          if (lane == 0) atomicAdd(&p.g.counts[r], 1u);
-        }
-      }
-      if (!ok && lane == 0) { *abort_flag = 1; atomicExch(p.status, LLMB_ERR_TIMEOUT); }
-    } else if (p.pull.nseg > 0) {
-      // ZeRO-3 parameter pull: same ticketed 32 KB slices, one list of segments instead of one chunk per rank
-      constexpr long long SLICE = 2048;                  // 16-byte vectors
-      bool ok = true;
-      for (int sgm = 0; sgm < p.pull.nseg && ok; ++sgm) {
-        if (p.pull.seq && lane == 0) {                    // the owner's shard holds this step's parameters
-          const unsigned* f = reinterpret_cast<const unsigned*>(p.pull.flags) + FLAG_PARAM * 8 + p.pull.owner[sgm];
-          unsigned spins = 0;
-          while ((int)(ld_acquire_sys(f) - p.pull.seq) < 0) {
-            if (++spins > (1u << 24)) { ok = false; break; }
-            __nanosleep(200);
-          }
-        }
-        ok = __shfl_sync(0xffffffffu, ok, 0);
-        if (!ok) break;
-        const uint4* src = reinterpret_cast<const uint4*>(p.pull.src[sgm]);
-        uint4* dst = reinterpret_cast<uint4*>(p.pull.dst[sgm]);
-        const long long nvec = p.pull.vecs[sgm];
-        const unsigned target = (unsigned)((nvec + SLICE - 1) / SLICE);
-        for (;;) {
-          unsigned ticket = 0;
-          if (lane == 0) ticket = atomicAdd(&p.pull.counts[8 + sgm], 1u);
-          ticket = __shfl_sync(0xffffffffu, ticket, 0);
-          if (ticket >= target) break;
-          const long long v0 = (long long)ticket * SLICE;
-          const long long v1 = v0 + SLICE < nvec ? v0 + SLICE : nvec;
-          long long v = v0 + lane;
-          for (; v + 7 * 32 < v1; v += 8 * 32) {         // eight loads in flight per thread
-            uint4 t[8];
-#pragma unroll
-            for (int k = 0; k < 8; ++k) t[k] = ld_nc_v4(src + v + k * 32);
-#pragma unroll
-            for (int k = 0; k < 8; ++k) dst[v + k * 32] = t[k];
-          }
-          for (; v < v1; v += 32) dst[v] = ld_nc_v4(src + v);
-          __threadfence();
-          __syncwarp();
-          if (lane == 0) atomicAdd(&p.pull.counts[sgm], 1u);
-        }
-      }
-      if (!ok && lane == 0) { *abort_flag = 1; atomicExch(p.status, LLMB_ERR_TIMEOUT); }
-    }
-  } else if (WIDE && p.tma_epi) {
-    // ------------------------------------------------------------ epilogue with an auxiliary input (warps 2..17, both CTAs)
-    // warp % 4 selects the 32-row band (the TMEM lane quarter a warp may read), (warp - 2) / 4 the 64-column slab: one slab per warp
-    // and tile, worked in halves of 32 columns (few enough registers for 16 warps), in place in the warp's one box.  The next tile's
-    // auxiliary box is on its way to L2 while this tile's MMAs run and is loaded once this tile's store has read the box.
-    const int q = warp & 3, e = warp - 2, coff = (e >> 2) * 64;
-    unsigned char* box = epi_stage + e * SLAB_BYTES;
-    uint64_t* abar = aux_bar + e;
-    const int band_off = (int)cta * BM + q * 32;
-    uint32_t aux_phase = 0;
-    auto unit_box = [&](int unit, int& row0, int& col0) {  // false: outside the matrix (warp-uniform)
-      int m_blk, n_blk, kb0, kb1; unit_coords(unit, m_blk, n_blk, kb0, kb1);
-      row0 = m_blk * 2 * BM + band_off; col0 = n_blk * BN + coff;
-      return row0 < p.M && col0 < p.N;
-    };
-    int row0 = 0, col0 = 0;
-    bool valid = cluster_id < total_units && unit_box(cluster_id, row0, col0), loading = valid;
-    if (valid && lane == 0) { mbar_expect_tx(abar, SLAB_BYTES); tma_load_2d(box, &tmAux, abar, col0, row0); }
-    int it = 0;
-    for (int unit = cluster_id; unit < total_units && !*abort_flag; unit += num_clusters, ++it) {
-      const int acc = it & 1;
-      int nrow0 = 0, ncol0 = 0;
-      const bool nvalid = unit + num_clusters < total_units && unit_box(unit + num_clusters, nrow0, ncol0);
-      if (nvalid && lane == 0) tma_prefetch_l2_2d(&tmAux, ncol0, nrow0);
-      if (!mbar_wait(&tfull_bar[acc], (it >> 1) & 1)) { *abort_flag = 1; atomicExch(p.status, LLMB_ERR_TIMEOUT); break; }
-      fence_after_sync();
-      const float alpha = p.alpha ? *p.alpha : 1.0f;
-      const uint32_t tacc = tmem_base + ((uint32_t)(q * 32) << 16) + acc * BN + coff;
-      uint32_t r[32];
-      if (valid) {
-        if (!mbar_wait(abar, aux_phase)) { *abort_flag = 1; atomicExch(p.status, LLMB_ERR_TIMEOUT); break; }
-        aux_phase ^= 1; loading = false;
-        tmem_ld32(tacc, r);
-        tmem_wait_ld();
-        epi_half_bf16<EPI, 0>(p, r, box, col0, alpha, lane);
-        tmem_ld32(tacc + 32, r);
-        tmem_wait_ld();
-      }
-      fence_before_sync();
-      __syncwarp();
-      if (lane == 0) mbar_arrive_cluster(mapa_u32(smem_u32(&tempty_bar[acc]), 0));   // the slab has left TMEM; the leader owns the hand-back
-      if (valid) {
-        epi_half_bf16<EPI, 1>(p, r, box, col0, alpha, lane);
-        fence_proxy_async();
-        __syncwarp();
-        if (EPI == EPI_DGELU && p.colsum) { epi_slab_colsum(p, box, row0, col0, lane); __syncwarp(); }
-        if (lane == 0) { tma_store_2d(&tmD, box, col0, row0); bulk_commit(); }
-      }
-      if (nvalid) {
-        if (lane == 0) { bulk_wait_read<0>(); mbar_expect_tx(abar, SLAB_BYTES); tma_load_2d(box, &tmAux, abar, ncol0, nrow0); }
-        loading = true;
-      }
-      valid = nvalid; row0 = nrow0; col0 = ncol0;
-    }
-    if (loading) (void)mbar_wait(abar, aux_phase);
-    if (lane == 0) bulk_wait_read<0>();
-    __syncwarp();
-  } else {
-    // ------------------------------------------------------------ epilogue (warps 2..9, both CTAs)
-    // Eight warps: warp % 4 selects the 32-row band (the TMEM lane quarter a warp may read), (warp - 2) / 4 the
-    // 128-column half of the tile, i.e. two 64-column slabs per warp and tile.  The register epilogue (fp32
-    // outputs, layouts without a tensor map) keeps four working warps with all four slabs of a band each.
-    // An fp32-storage problem (tf32) moves its 128 columns as four 32-column boxes through the same buffers.
-    // Auxiliary inputs come this way for fp32 storage only.
-    constexpr bool F32_IO = KIND == KIND_TF32 && !Cfg::F32_OUT, AUX = Cfg::AUX_IN && F32_IO;
-    constexpr int NBOX = F32_IO ? 4 : 2, BOXC = F32_IO ? 32 : 64;
-    const int q = warp & 3, e = warp - 2, hcol = e >> 2;
-    const bool tma_epi = p.tma_epi;                       // warp-uniform
-    unsigned char* wstage = epi_stage + e * (tma_epi ? WSB / 2 : WSB);
-    uint64_t* abar = aux_bar + e * 2;
-    const int band_off = (int)cta * BM + q * 32;
-    uint32_t aux_phase = 0, aux_pending = 0;              // per-slab-buffer phase bits / loads in flight (warp-uniform)
-    // auxiliary-input tiles of a work unit: one box per slab that lies inside the matrix (ls < NBOX), in buffer ls & 1
-    auto slab_valid = [&](int row0, int n0, int ls) { return row0 < p.M && n0 + hcol * 128 + ls * BOXC < p.N; };
-    auto aux_issue = [&](int row0, int n0, int ls) {      // all lanes keep the books, lane 0 issues
-      if (!slab_valid(row0, n0, ls)) return;
-      const int b = ls & 1;
-      aux_pending |= 1u << b;
-      if (lane == 0) {
-        mbar_expect_tx(&abar[b], SLAB_BYTES);
-        tma_load_2d(wstage + b * SLAB_BYTES, &tmAux, &abar[b], n0 + hcol * 128 + ls * BOXC, row0);
-      }
-    };
-    if (AUX && tma_epi && cluster_id < total_units) {
-      int m_blk, n_blk, kb0, kb1; unit_coords(cluster_id, m_blk, n_blk, kb0, kb1);
-      for (int ls = 0; ls < 2; ++ls) aux_issue(m_blk * 2 * BM + band_off, n_blk * BN, ls);
-    }
-    int it = 0;
-    for (int unit = cluster_id; unit < total_units && !*abort_flag; unit += num_clusters, ++it) {
-      int m_blk, n_blk, kb0, kb1; unit_coords(unit, m_blk, n_blk, kb0, kb1);
-      const int acc = it & 1;
-      const uint32_t acc_phase = (it >> 1) & 1;
-      if (!mbar_wait(&tfull_bar[acc], acc_phase)) { *abort_flag = 1; atomicExch(p.status, LLMB_ERR_TIMEOUT); break; }
-      fence_after_sync();
-      const int n0 = n_blk * BN;
-      const int row0 = m_blk * 2 * BM + band_off;
-      const float alpha = p.alpha ? *p.alpha : 1.0f;
-      const uint32_t tacc = tmem_base + ((uint32_t)(q * 32) << 16) + acc * BN;
-      if (!tma_epi) {
-        if (e < 4) epilogue_warp<EPI>(p, tacc, wstage, row0, n0, alpha, lane);
-      } else {
-        const int nunit = unit + num_clusters;
-        const bool has_next = AUX && nunit < total_units;
-        int nrow0 = 0, nn0 = 0;
-        if (has_next) { int mb, nb, k0, k1; unit_coords(nunit, mb, nb, k0, k1); nrow0 = mb * 2 * BM + band_off; nn0 = nb * BN; }
-        bool ok = true;
-#pragma unroll 1
-        for (int ls = 0; ls < NBOX; ++ls) {
-          if (!slab_valid(row0, n0, ls)) break;            // warp-uniform
-          const int col0 = n0 + hcol * 128 + ls * BOXC;
-          uint32_t r0[32], r1[32];
-          tmem_ld32(tacc + hcol * 128 + ls * BOXC, r0);
-          if (!F32_IO) tmem_ld32(tacc + hcol * 128 + ls * BOXC + 32, r1);
-          tmem_wait_ld();
-          unsigned char* buf;
-          if (Cfg::F32_OUT) {
-            // fp32 accumulate / store: the slab leaves as two boxes of 32 rows x 32 fp32 columns (128-byte rows, swizzled), which
-            // the TMA engine adds into (split-K partial sums, gradient accumulation) or writes to the output; the warp goes on
-            // to its next slab at once instead of waiting on 64 vector reductions per lane.
-            buf = wstage;
-            if (lane == 0) bulk_wait_read<0>();           // the previous slab's boxes have been read
-            __syncwarp();
-            unsigned char* myrow = buf + lane * 128;
-#pragma unroll
-            for (int c = 0; c < 8; ++c) {
-              const int sw = (c ^ (lane & 7)) << 4;
-              *reinterpret_cast<float4*>(myrow + sw) = make_float4(__uint_as_float(r0[4 * c]) * alpha, __uint_as_float(r0[4 * c + 1]) * alpha,
-                                                                   __uint_as_float(r0[4 * c + 2]) * alpha, __uint_as_float(r0[4 * c + 3]) * alpha);
-              *reinterpret_cast<float4*>(myrow + SLAB_BYTES + sw) = make_float4(__uint_as_float(r1[4 * c]) * alpha, __uint_as_float(r1[4 * c + 1]) * alpha,
-                                                                                __uint_as_float(r1[4 * c + 2]) * alpha, __uint_as_float(r1[4 * c + 3]) * alpha);
-            }
-            fence_proxy_async();
-            __syncwarp();
-            if (lane == 0) {
-              if (EPI == EPI_ACC_F32) {
-                tma_reduce_add_2d(&tmD, buf, col0, row0);
-                if (col0 + 32 < p.N) tma_reduce_add_2d(&tmD, buf + SLAB_BYTES, col0 + 32, row0);
-              } else {
-                tma_store_2d(&tmD, buf, col0, row0);
-                if (col0 + 32 < p.N) tma_store_2d(&tmD, buf + SLAB_BYTES, col0 + 32, row0);
-              }
-              bulk_commit();
-            }
-            continue;
-          }
-          if (AUX) {
-            const int b = ls & 1;
-            buf = wstage + b * SLAB_BYTES;
-            if (!mbar_wait(&abar[b], (aux_phase >> b) & 1)) { ok = false; break; }
-            aux_phase ^= 1u << b; aux_pending &= ~(1u << b);
-          } else {
-            buf = wstage;
-            // the previous slab's stores have read the buffer (two outputs: its pre-activations have; the newest store is of the other box)
-            if (lane == 0) { if (Cfg::TWO_OUT && !F32_IO) bulk_wait_read<1>(); else bulk_wait_read<0>(); }
-            __syncwarp();
-          }
-          if (F32_IO) {
-            epi_box_f32<EPI>(p, r0, buf, buf + SLAB_BYTES, col0, alpha, lane);
-            fence_proxy_async();
-            __syncwarp();
-            if (lane == 0) {
-              if (Cfg::TWO_OUT) { tma_store_2d(&tmAux, buf, col0, row0); tma_store_2d(&tmD, buf + SLAB_BYTES, col0, row0); }
-              else tma_store_2d(&tmD, buf, col0, row0);
-              bulk_commit();
-            }
-            if (AUX && ls + 2 < NBOX && slab_valid(row0, n0, ls + 2)) {   // this buffer's next box, once the store has read it
-              if (lane == 0) bulk_wait_read<0>();
-              __syncwarp();
-              aux_issue(row0, n0, ls + 2);
-            }
-            continue;
-          }
-          if (Cfg::TWO_OUT) {
-            uint4 pre[8];
-            epi_slab_pre(p, r0, r1, buf, col0, alpha, lane, pre);
-            fence_proxy_async();
-            __syncwarp();
-            if (lane == 0) { tma_store_2d(&tmAux, buf, col0, row0); bulk_commit(); bulk_wait_read<1>(); }   // the previous slab's activations have left
-            __syncwarp();
-            epi_slab_gelu(p, pre, buf + SLAB_BYTES, lane);
-            fence_proxy_async();
-            __syncwarp();
-            if (lane == 0) { tma_store_2d(&tmD, buf + SLAB_BYTES, col0, row0); bulk_commit(); }
-            continue;
-          }
-          epi_slab_bf16<EPI>(p, r0, r1, buf, col0, alpha, lane);
-          fence_proxy_async();
-          __syncwarp();
-          if (lane == 0) { tma_store_2d(&tmD, buf, col0, row0); bulk_commit(); }
-        }
-        if (!ok) { *abort_flag = 1; atomicExch(p.status, LLMB_ERR_TIMEOUT); break; }
-        if (AUX && has_next) {                            // refill each buffer once its store has been read
-          // (a unit at the right edge may have stored its last slab from buffer 0: then both stores must have been read)
-          if (lane == 0) { if (slab_valid(row0, n0, NBOX - 1)) bulk_wait_read<1>(); else bulk_wait_read<0>(); }
-          __syncwarp();
-          aux_issue(nrow0, nn0, 0);
-          if (lane == 0) bulk_wait_read<0>();
-          __syncwarp();
-          aux_issue(nrow0, nn0, 1);
-        }
-      }
-      fence_before_sync();
-      __syncwarp();
-      if (lane == 0) mbar_arrive_cluster(mapa_u32(smem_u32(&tempty_bar[acc]), 0));   // the leader owns the accumulator hand-back
-    }
-    if (tma_epi) {
-      // nothing of this CTA's shared memory may still be a source or a destination of a copy at exit
-      for (int ls = 0; ls < 2; ++ls)
-        if (aux_pending & (1u << ls)) (void)mbar_wait(&abar[ls], (aux_phase >> ls) & 1);
-      if (lane == 0) bulk_wait_read<0>();
-      __syncwarp();
-    }
-  }
-
-  fence_before_sync();
-  __syncthreads();
-  cluster_sync_all();                                   // the peer may still be signalling / reading this CTA's smem
-  if (warp == 1) { fence_after_sync(); tmem_dealloc_pair<512>(tmem_base); }
-}
-
 int g_dbg_mn_lbo = -1, g_dbg_mn_sbo = -1;   // test hooks: override the MN-major descriptor strides
 thread_local float* g_pending_colsum = nullptr;   // armed by llmb_gemm_set_colsum, consumed by the calling thread's next llmb_gemm
 thread_local GatherArgs g_pending_gather{};   // armed by llmb_gemm_set_gather, consumed (and cleared) by the calling thread's next llmb_gemm
@@ -542,19 +28,6 @@ int g_pair_mode = -1;
 bool pair_mode() {
   if (g_pair_mode < 0) { const char* e = getenv("LLMB_GEMM_PAIR"); g_pair_mode = (e && e[0] == '0') ? 0 : 1; }
   return g_pair_mode == 1;
-}
-
-template <int KIND, int EPI>
-int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td, const CUtensorMap& taux,
-                const GemmParams& p, int grid, cudaStream_t st) {
-  static bool attr_done = false;
-  constexpr int SMEM = smem2_bytes<EPI>();
-  if (!attr_done) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_pair_kernel<KIND, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
-    if (e != cudaSuccess) return (int)e;
-    attr_done = true;
-  }
-  return launch_pdl(gemm_pair_kernel<KIND, EPI>, grid, PairCfg<KIND, EPI>::THREADS, SMEM, st, ta, tb, td, taux, p);
 }
 
 // Tile configuration of one problem: bn = 256 is the CTA-pair kernel, 64 / 128 the kernel of gemm_small.cu with cl CTAs per tile.
@@ -723,19 +196,7 @@ int gemm_dispatch(void* D, const void* A, const void* B, const void* bias, void*
   p.bias_vec = (reinterpret_cast<uintptr_t>(bias) & 15) == 0;
   if (!pair) return llmb_gemm_small_launch(KIND, epi, tile.bn, tile.cl, ta, tb, td, taux, p, st);
 
-  const long long units2 = (long long)ceil_div(M, 2 * BM) * p.n_tiles * p.splits;
-  const int max_clusters = sm_count() / 2;
-  const int grid2 = 2 * (int)(units2 < max_clusters ? units2 : max_clusters);
-  switch (epi) {
-    case EPI_NONE: return launch_pair<KIND, EPI_NONE>(ta, tb, td, taux, p, grid2, st);
-    case EPI_BIAS: return launch_pair<KIND, EPI_BIAS>(ta, tb, td, taux, p, grid2, st);
-    case EPI_BIAS_GELU: return launch_pair<KIND, EPI_BIAS_GELU>(ta, tb, td, taux, p, grid2, st);
-    case EPI_DGELU: return launch_pair<KIND, EPI_DGELU>(ta, tb, td, taux, p, grid2, st);
-    case EPI_ACC_F32: return launch_pair<KIND, EPI_ACC_F32>(ta, tb, td, taux, p, grid2, st);
-    case EPI_BIAS_RESID: return launch_pair<KIND, EPI_BIAS_RESID>(ta, tb, td, taux, p, grid2, st);
-    case EPI_STORE_F32: return launch_pair<KIND, EPI_STORE_F32>(ta, tb, td, taux, p, grid2, st);
-  }
-  return LLMB_ERR_BAD_ARG;
+  return launch_pair_epi<KIND>(epi, ta, tb, td, taux, p, st);
 }
 // ------------------------------------------------------------------------------------------------
 // Native block-scaled GEMMs:  D[M,N] = epi(alpha * sum_k (A[m,k] sfa[m,k/B]) (B[n,k] sfb[n,k/B])).

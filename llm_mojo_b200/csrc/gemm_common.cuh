@@ -200,9 +200,8 @@ __device__ __forceinline__ void epilogue_warp(const GemmParams& p, uint32_t tacc
 // 64 columns of bf16 or 32 of fp32.
 //   * tcgen05.ld gives each lane one row of a box; bias, GELU, dGELU and the residual add happen in registers in that layout;
 //   * the auxiliary INPUT (residual stream, pre-GELU activations) arrives by TMA in the buffer that the result is then written to in
-//     place.  In the CTA-pair kernel a tile's boxes are on their way to L2 (bf16, fp8 operands: sixteen warps, one box each) or into
-//     their buffers (fp32 storage: eight warps, four boxes in two buffers) while the tile before it is worked; a buffer is filled
-//     again once the store of its last result has read it;
+//     place.  In the CTA-pair kernel a warp has two boxes (bf16: its two 64-column slabs of a tile; fp32 storage: four 32-column ones in
+//     turn); a box is filled again, with the next tile's input, once the store of its last result has read it;
 //   * results leave by TMA stores (fp32 accumulate: by TMA additions), so no lane ever waits on global memory and every global access
 //     of the epilogue is a full 128-byte row segment; out-of-range rows and columns are clipped by the tensor maps.
 // Epilogues with an auxiliary input or a second output (BIAS_GELU stores the pre-activation too) and the fp32 outputs get 64 KB of
@@ -212,7 +211,7 @@ template <int EPI> struct EpiCfg {
   static constexpr bool TWO_OUT = EPI == EPI_BIAS_GELU;
   static constexpr bool F32_OUT = EPI == EPI_ACC_F32 || EPI == EPI_STORE_F32;
   static constexpr int STAGES = (F32_OUT || AUX_IN || TWO_OUT) ? 5 : 6;
-  static constexpr int WARP_STAGE = STAGES == 5 ? 16384 : 8192;     // staging bytes per warp of the 4-warp register epilogue (half that per warp of 8, a quarter per warp of 16 in the TMA epilogues)
+  static constexpr int WARP_STAGE = STAGES == 5 ? 16384 : 8192;     // staging bytes per warp of the 4-warp register epilogue (half that per warp of 8 in the TMA epilogues)
 };
 constexpr int SLAB_BYTES = 32 * 128;
 
@@ -228,117 +227,125 @@ __device__ __forceinline__ void unpack8(const uint4& u, float (&x)[8]) {
   for (int i = 0; i < 4; ++i) { const float2 f = __bfloat1622float2(h[i]); x[2 * i] = f.x; x[2 * i + 1] = f.y; }
 }
 
+// Eight bias values from column `col` on (N is a multiple of 8; columns beyond it, which no store writes, read the last ones).
+__device__ __forceinline__ uint4 bias8(const GemmParams& p, const __nv_bfloat16* bias, int col) {
+  bias += min(col, p.N - 8);
+  if (p.bias_vec) return __ldg(reinterpret_cast<const uint4*>(bias));
+  const unsigned short* h = reinterpret_cast<const unsigned short*>(bias);
+  uint4 u;
+  u.x = __ldg(h) | (uint32_t)__ldg(h + 1) << 16; u.y = __ldg(h + 2) | (uint32_t)__ldg(h + 3) << 16;
+  u.z = __ldg(h + 4) | (uint32_t)__ldg(h + 5) << 16; u.w = __ldg(h + 6) | (uint32_t)__ldg(h + 7) << 16;
+  return u;
+}
+// The bias of a 64-column slab into L1 while the warp has nothing else to do (a lane reads two values; the L2 latency of the first use was
+// 700 cycles of every tile).
+__device__ __forceinline__ void bias_prefetch(const GemmParams& p, int col0, int lane) {
+  const __nv_bfloat16* bias = reinterpret_cast<const __nv_bfloat16*>(p.bias);
+  const int col = col0 + 2 * lane;
+  unsigned short v;
+  if (bias && col < p.N) asm volatile("ld.global.nc.u16 %0, [%1];" : "=h"(v) : "l"(bias + col));
+}
+// alpha * accumulator + bias of 32 columns (this lane's row)
+template <bool BIAS>
+__device__ __forceinline__ void epi_affine32(const GemmParams& p, const uint32_t (&r)[32], int col0, float alpha, float (&v)[32]) {
+  const __nv_bfloat16* bias = reinterpret_cast<const __nv_bfloat16*>(p.bias);
+  if (BIAS && bias) {
+    uint4 bq[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) bq[c] = bias8(p, bias, col0 + c * 8);
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      float b[8]; unpack8(bq[c], b);
+#pragma unroll
+      for (int j = 0; j < 8; j += 2) {
+        const float2 y = __ffma2_rn(make_float2(__uint_as_float(r[c * 8 + j]), __uint_as_float(r[c * 8 + j + 1])), make_float2(alpha, alpha), make_float2(b[j], b[j + 1]));
+        v[c * 8 + j] = y.x; v[c * 8 + j + 1] = y.y;
+      }
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < 32; j += 2) {
+      const float2 y = __fmul2_rn(make_float2(__uint_as_float(r[j]), __uint_as_float(r[j + 1])), make_float2(alpha, alpha));
+      v[j] = y.x; v[j + 1] = y.y;
+    }
+  }
+}
+
 // Half a slab (this lane's row, 32 columns: chunks 4 * H .. 4 * H + 3) from registers to the swizzled staging buffer.  With an
-// auxiliary input the buffer holds it on entry and the result replaces it; BIAS_GELU writes the pre-activation to `buf` and the
-// activation to `buf + SLAB_BYTES`.
+// auxiliary input the buffer holds it on entry and the result replaces it.
 template <int EPI, int H>
 __device__ __forceinline__ void epi_half_bf16(const GemmParams& p, const uint32_t (&r)[32], unsigned char* buf, int col0, float alpha, int lane) {
   unsigned char* myrow = buf + lane * 128;
-  const __nv_bfloat16* bias = reinterpret_cast<const __nv_bfloat16*>(p.bias);
+  float v[32];
+  epi_affine32<EPI == EPI_BIAS || EPI == EPI_BIAS_RESID>(p, r, col0 + H * 32, alpha, v);
 #pragma unroll
   for (int c4 = 0; c4 < 4; ++c4) {
     const int c = H * 4 + c4;
-    float v[8], b[8];
-    const int col = col0 + c * 8;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) b[j] = 0.f;
-    if (EPI == EPI_BIAS || EPI == EPI_BIAS_GELU || EPI == EPI_BIAS_RESID) {
-      if (bias && col < p.N) {
-        if (p.bias_vec) unpack8(__ldg(reinterpret_cast<const uint4*>(bias + col)), b);
-        else {
-#pragma unroll
-          for (int j = 0; j < 8; ++j) b[j] = __bfloat162float(bias[col + j]);
-        }
-      }
-    }
-#pragma unroll
-    for (int j = 0; j < 8; j += 2) {
-      const float2 y = __ffma2_rn(make_float2(__uint_as_float(r[c4 * 8 + j]), __uint_as_float(r[c4 * 8 + j + 1])),
-                                  make_float2(alpha, alpha), make_float2(b[j], b[j + 1]));
-      v[j] = y.x; v[j + 1] = y.y;
-    }
     unsigned char* slot = myrow + ((c ^ (lane & 7)) << 4);
-    if (EPI == EPI_BIAS_GELU) {
-      const uint4 pre = pack8(v);
-      *reinterpret_cast<uint4*>(slot) = pre;
-      float x[8]; unpack8(pre, x);
+    float o[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) o[j] = v[c4 * 8 + j];
+    if (EPI == EPI_DGELU || EPI == EPI_BIAS_RESID) {
+      float x[8]; unpack8(*reinterpret_cast<const uint4*>(slot), x);
 #pragma unroll
       for (int j = 0; j < 8; j += 2) {
-        const float2 y = gelu_fast2(make_float2(x[j], x[j + 1]));
-        v[j] = y.x; v[j + 1] = y.y;
+        const float2 xx = make_float2(x[j], x[j + 1]), vv = make_float2(o[j], o[j + 1]);
+        const float2 y = (EPI == EPI_DGELU) ? __fmul2_rn(vv, gelu_grad_fast2(xx)) : __fadd2_rn(vv, xx);
+        o[j] = y.x; o[j + 1] = y.y;
       }
-      *reinterpret_cast<uint4*>(slot + SLAB_BYTES) = pack8(v);
-    } else {
-      if (EPI == EPI_DGELU || EPI == EPI_BIAS_RESID) {
-        float x[8]; unpack8(*reinterpret_cast<const uint4*>(slot), x);
-#pragma unroll
-        for (int j = 0; j < 8; j += 2) {
-          const float2 xx = make_float2(x[j], x[j + 1]), vv = make_float2(v[j], v[j + 1]);
-          const float2 y = (EPI == EPI_DGELU) ? __fmul2_rn(vv, gelu_grad_fast2(xx)) : __fadd2_rn(vv, xx);
-          v[j] = y.x; v[j + 1] = y.y;
-        }
-      }
-      *reinterpret_cast<uint4*>(slot) = pack8(v);
     }
+    *reinterpret_cast<uint4*>(slot) = pack8(o);
   }
 }
-template <int EPI>
-__device__ __forceinline__ void epi_slab_bf16(const GemmParams& p, const uint32_t (&r0)[32], const uint32_t (&r1)[32],
-                                              unsigned char* buf, int col0, float alpha, int lane) {
-  epi_half_bf16<EPI, 0>(p, r0, buf, col0, alpha, lane);
-  epi_half_bf16<EPI, 1>(p, r1, buf, col0, alpha, lane);
-}
-
-// Column sums of a 32 x 64 slab as stored (bf16): lane l adds up columns 2l and 2l + 1 of the warp's rows out of the swizzled box
-// (conflict-free: the 32 lanes read the 128 bytes of one row) and adds them to colsum.
+// Column sums of a 32 x 64 slab as stored (bf16), added to colsum.  Lane l reads 16-byte chunk l % 8 (eight columns) of the rows l / 8 + 4 i out of
+// the swizzled box (the 8 lanes of a row read its 128 bytes); the four partial sums of a column meet in two exchanges that leave every
+// lane two columns.
 __device__ __forceinline__ void epi_slab_colsum(const GemmParams& p, const unsigned char* buf, int row0, int col0, int lane) {
-  float s0 = 0.f, s1 = 0.f;
-  const int nrows = min(32, p.M - row0);
-#pragma unroll 8
-  for (int r = 0; r < nrows; ++r) {
-    const uint32_t w = *reinterpret_cast<const uint32_t*>(buf + r * 128 + ((((lane >> 2) ^ (r & 7))) << 4) + (lane & 3) * 4);
-    s0 += __uint_as_float(w << 16); s1 += __uint_as_float(w & 0xffff0000u);
+  const int nrows = min(32, p.M - row0), c = lane & 7, g = lane >> 3;
+  float2 s[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) s[k] = make_float2(0.f, 0.f);
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int r = g + 4 * i;
+    uint4 u = *reinterpret_cast<const uint4*>(buf + r * 128 + ((c ^ (r & 7)) << 4));
+    if (r >= nrows) u = make_uint4(0u, 0u, 0u, 0u);
+    const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+    for (int k = 0; k < 4; ++k) s[k] = __fadd2_rn(s[k], make_float2(__uint_as_float(w[k] << 16), __uint_as_float(w[k] & 0xffff0000u)));
   }
-  const int col = col0 + 2 * lane;
+  auto swap = [&](float2 give, float2 keep, int mask) {
+    return __fadd2_rn(keep, make_float2(__shfl_xor_sync(0xffffffffu, give.x, mask), __shfl_xor_sync(0xffffffffu, give.y, mask)));
+  };
+  const bool hi = g & 2, odd = g & 1;
+  const float2 t0 = swap(hi ? s[0] : s[2], hi ? s[2] : s[0], 16), t1 = swap(hi ? s[1] : s[3], hi ? s[3] : s[1], 16);
+  const float2 t = swap(odd ? t0 : t1, odd ? t1 : t0, 8);
+  const int col = col0 + c * 8 + (hi ? 4 : 0) + (odd ? 2 : 0);
   if (col < p.N) {
-    asm volatile("red.global.add.f32 [%0], %1;" ::"l"(p.colsum + col), "f"(s0) : "memory");
-    asm volatile("red.global.add.f32 [%0], %1;" ::"l"(p.colsum + col + 1), "f"(s1) : "memory");
+    asm volatile("red.global.add.f32 [%0], %1;" ::"l"(p.colsum + col), "f"(t.x) : "memory");
+    asm volatile("red.global.add.f32 [%0], %1;" ::"l"(p.colsum + col + 1), "f"(t.y) : "memory");
   }
 }
 
-// The two halves of the bias + GELU epilogue, so that the pre-activation box can start leaving by TMA while the GELU of the
-// same slab is still being computed: first alpha, bias and the bf16 pre-activations (kept in registers as well) ...
-__device__ __forceinline__ void epi_slab_pre(const GemmParams& p, const uint32_t (&r0)[32], const uint32_t (&r1)[32],
-                                             unsigned char* buf, int col0, float alpha, int lane, uint4 (&pre)[8]) {
+// The bias + GELU epilogue in two steps, so that the pre-activation box can leave by TMA while the GELU of the same slab is computed: first
+// alpha, bias and the bf16 pre-activations of half a slab, kept in registers as well ...
+template <int H>
+__device__ __forceinline__ void epi_half_pre(const GemmParams& p, const uint32_t (&r)[32], unsigned char* buf, int col0, float alpha, int lane, uint4 (&pre)[8]) {
   unsigned char* myrow = buf + lane * 128;
-  const __nv_bfloat16* bias = reinterpret_cast<const __nv_bfloat16*>(p.bias);
+  float v[32];
+  epi_affine32<true>(p, r, col0 + H * 32, alpha, v);
 #pragma unroll
-  for (int c = 0; c < 8; ++c) {
-    float v[8], b[8];
-    const int col = col0 + c * 8;
+  for (int c4 = 0; c4 < 4; ++c4) {
+    const int c = H * 4 + c4;
+    float o[8];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) b[j] = 0.f;
-    if (bias && col < p.N) {
-      if (p.bias_vec) unpack8(__ldg(reinterpret_cast<const uint4*>(bias + col)), b);
-      else {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) b[j] = __bfloat162float(bias[col + j]);
-      }
-    }
-#pragma unroll
-    for (int j = 0; j < 8; j += 2) {
-      const uint32_t (&r)[32] = c < 4 ? r0 : r1;
-      const float2 y = __ffma2_rn(make_float2(__uint_as_float(r[(c & 3) * 8 + j]), __uint_as_float(r[(c & 3) * 8 + j + 1])),
-                                  make_float2(alpha, alpha), make_float2(b[j], b[j + 1]));
-      v[j] = y.x; v[j + 1] = y.y;
-    }
-    pre[c] = pack8(v);
+    for (int j = 0; j < 8; ++j) o[j] = v[c4 * 8 + j];
+    pre[c] = pack8(o);
     *reinterpret_cast<uint4*>(myrow + ((c ^ (lane & 7)) << 4)) = pre[c];
   }
 }
-// ... then GELU of those bf16 values into the second box.
-__device__ __forceinline__ void epi_slab_gelu(const GemmParams& p, const uint4 (&pre)[8], unsigned char* buf, int lane) {
-  unsigned char* myrow = buf + lane * 128;
+// ... then the GELU of those bf16 values, in place, ...
+__device__ __forceinline__ void epi_slab_gelu(uint4 (&pre)[8]) {
 #pragma unroll
   for (int c = 0; c < 8; ++c) {
     float x[8]; unpack8(pre[c], x);
@@ -347,10 +354,32 @@ __device__ __forceinline__ void epi_slab_gelu(const GemmParams& p, const uint4 (
       const float2 y = gelu_fast2(make_float2(x[j], x[j + 1]));
       x[j] = y.x; x[j + 1] = y.y;
     }
-    *reinterpret_cast<uint4*>(myrow + ((c ^ (lane & 7)) << 4)) = pack8(x);
+    pre[c] = pack8(x);
   }
 }
+// ... and to a box.
+__device__ __forceinline__ void epi_slab_store(const uint4 (&v)[8], unsigned char* buf, int lane) {
+  unsigned char* myrow = buf + lane * 128;
+#pragma unroll
+  for (int c = 0; c < 8; ++c) *reinterpret_cast<uint4*>(myrow + ((c ^ (lane & 7)) << 4)) = v[c];
+}
 
+
+// A whole slab; BIAS_GELU writes the pre-activation to `buf` and the activation to `buf + SLAB_BYTES`.
+template <int EPI>
+__device__ __forceinline__ void epi_slab_bf16(const GemmParams& p, const uint32_t (&r0)[32], const uint32_t (&r1)[32],
+                                              unsigned char* buf, int col0, float alpha, int lane) {
+  if (EPI == EPI_BIAS_GELU) {
+    uint4 pre[8];
+    epi_half_pre<0>(p, r0, buf, col0, alpha, lane, pre);
+    epi_half_pre<1>(p, r1, buf, col0, alpha, lane, pre);
+    epi_slab_gelu(pre);
+    epi_slab_store(pre, buf + SLAB_BYTES, lane);
+    return;
+  }
+  epi_half_bf16<EPI, 0>(p, r0, buf, col0, alpha, lane);
+  epi_half_bf16<EPI, 1>(p, r1, buf, col0, alpha, lane);
+}
 
 // fp32 storage (tf32 kind): one box of 32 rows x 32 columns (this lane's row) from registers to the swizzled staging box; with an
 // auxiliary input the box holds it on entry, BIAS_GELU writes the activation to `act` and the pre-activation to `buf`.

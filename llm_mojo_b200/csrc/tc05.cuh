@@ -243,6 +243,7 @@ __host__ __device__ constexpr uint32_t make_idesc_mxfp8(uint32_t a_fmt, uint32_t
 }
 // Shared-memory descriptor of one scale-factor atom: 32 rows of 16 bytes, no swizzle (8-row core matrices 128 B apart).
 __device__ __forceinline__ uint64_t make_sf_desc(uint32_t smem_addr) { return make_smem_desc(smem_addr, 16, 128, 0); }
+
 // Copies 32 rows x 16 bytes of shared memory into 4 TMEM columns of all four lane quarters (row r -> lane r of each
 // quarter): exactly the placement the block-scaled MMA expects for the scales of 128 rows x 4 blocks when the
 // shared-memory image is the 128 x 4 scale atom (byte (r % 32) * 16 + (r / 32) * 4 + block).  One thread issues;
@@ -281,8 +282,10 @@ __device__ __forceinline__ void cluster_sync_all() {
 __device__ __forceinline__ uint32_t mapa_u32(uint32_t local_addr, uint32_t rank) {
   uint32_t r; asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local_addr), "r"(rank)); return r;
 }
+// For a hand-back of tensor memory (after tcgen05.wait::ld and tcgen05.fence::before_thread_sync): nothing that this thread wrote is to be seen
+// by the waiting CTA, and release at cluster scope would wait for all of it (1200 - 2500 cycles with stores and reductions in flight).
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+  asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
 __device__ __forceinline__ void tma_load_2d_pair(void* dst, const CUtensorMap* t, uint32_t leader_bar_cluster_addr, int c0, int c1) {
   asm volatile(
@@ -363,7 +366,7 @@ inline bool tmap_cache_lookup(const TmapKey& k, CUtensorMap* out, bool store) {
 }
 
 // 2-D row-major tensor [rows, cols] with row pitch ld (elements); box = [box_rows, box_cols];
-// 128-byte swizzle (box_cols * elem_bytes must be 128).
+// 128-byte swizzle (box_cols * elem_bytes must be 128) unless another is given.
 inline int make_tmap_2d(CUtensorMap* m, const void* ptr, CUtensorMapDataType dt, int elem_bytes, uint64_t rows,
                         uint64_t cols, uint64_t ld, uint32_t box_rows, uint32_t box_cols,
                         CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_128B) {

@@ -418,6 +418,8 @@ template <int KIND> struct KindTraits;
 template <> struct KindTraits<KIND_F16> { static constexpr int ESZ = 2, BKE = ROW_BYTES / ESZ; static constexpr CUtensorMapDataType DT = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16; };
 template <> struct KindTraits<KIND_TF32> { static constexpr int ESZ = 4, BKE = ROW_BYTES / ESZ; static constexpr CUtensorMapDataType DT = CU_TENSOR_MAP_DATA_TYPE_FLOAT32; };
 template <> struct KindTraits<KIND_F8F6F4> { static constexpr int ESZ = 1, BKE = ROW_BYTES / ESZ; static constexpr CUtensorMapDataType DT = CU_TENSOR_MAP_DATA_TYPE_UINT8; };
+template <> struct KindTraits<KIND_MXF8> { static constexpr int ESZ = 1, BKE = ROW_BYTES; static constexpr CUtensorMapDataType DT = CU_TENSOR_MAP_DATA_TYPE_UINT8; };
+template <> struct KindTraits<KIND_NVF4> { static constexpr int ESZ = 1, BKE = ROW_BYTES; static constexpr CUtensorMapDataType DT = CU_TENSOR_MAP_DATA_TYPE_UINT8; };
 }  // namespace lgemm
 using namespace lgemm;
 

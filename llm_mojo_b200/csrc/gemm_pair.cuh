@@ -1,4 +1,4 @@
-// The CTA-pair GEMM kernel and its launch; gemm.cu instantiates it.
+// The CTA-pair GEMM kernel and its launch; gemm.cu instantiates it for bf16, TF32 and fp8 operands, gemm_scaled.cu for block-scaled ones.
 #pragma once
 #include "gemm_common.cuh"
 
@@ -24,27 +24,51 @@ constexpr int SMEM2_TAIL = 512;                        // barriers, TMEM slot, a
 // bytes a cycle that an SM gets when all of them load.
 constexpr int EPI_WARPS = 8;
 constexpr int PAIR_THREADS = 32 * (4 + EPI_WARPS);
+//
+// Block-scaled operands (KIND_MXF8: e4m3 / e5m2 bytes, one ue8m0 scale per 32 values; KIND_NVF4: packed e2m1, one ue4m3 scale per 16), both
+// K-major: a stage's 128-byte rows hold 128 / 256 values of K and come with their scales, in the atoms of 512 bytes that gemm_scaled.cu
+// describes: those of this CTA's 128 rows of A (SF_A bytes) and those of all 256 rows of B, of which either CTA needs every one.  The
+// leader copies a stage's atoms to both CTAs' tensor memory (tcgen05.cp.cta_group::2) just ahead of the MMAs that use them.  Those 48
+// columns leave no room for two 256-column accumulators, so the two OVERLAP in one 64-column slab: accumulator 0 = [0, 256), accumulator 1
+// = [192, 448), scales from 448.  The epilogue of a tile reads that slab first and says so (`tover`); the next tile's MMAs start when
+// it is read and the tile before has been drained completely (`tempty`).
+template <int KIND, int EPI> struct PairCfg {
+  static constexpr bool SCALED = KIND == KIND_MXF8 || KIND == KIND_NVF4;
+  static constexpr int SF_A = KIND == KIND_NVF4 ? 2048 : KIND == KIND_MXF8 ? 512 : 0;     // scales of 128 rows x one stage
+  static constexpr int STAGES = EpiCfg<EPI>::STAGES - (SCALED ? 1 : 0);
+  static constexpr int SMEM = STAGES * (STAGE2_BYTES + 3 * SF_A) + 4 * EpiCfg<EPI>::WARP_STAGE + 1024 + SMEM2_TAIL;
+  static constexpr uint32_t ACC1_COL = SCALED ? 192 : BN;
+};
+constexpr uint32_t SFA_COL = 448, SFB_COL = 464;
+// the tensor maps of the scales: [row blocks of 128][atoms along K * 64] 8-byte words, boxes of one / two row blocks and one stage
+template <int KIND> struct ScaleMaps {};
+template <> struct ScaleMaps<KIND_MXF8> { CUtensorMap a, b; };
+template <> struct ScaleMaps<KIND_NVF4> { CUtensorMap a, b; };
 constexpr int FLAG_ROWS_READY = 6;                     // flag kind (layout of comm.cu: flags[kind][8 ranks])
 constexpr int FLAG_PARAM = 3;                          // owners announce the optimizer step their parameter shard holds
-template <int EPI> constexpr int smem2_bytes() { return EpiCfg<EPI>::STAGES * STAGE2_BYTES + 4 * EpiCfg<EPI>::WARP_STAGE + 1024 + SMEM2_TAIL; }
 
 template <int KIND, int EPI>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                 const __grid_constant__ CUtensorMap tmD, const __grid_constant__ CUtensorMap tmAux, const GemmParams p) {
+                 const __grid_constant__ CUtensorMap tmD, const __grid_constant__ CUtensorMap tmAux, const __grid_constant__ ScaleMaps<KIND> sfm,
+                 const GemmParams p) {
   using Cfg = EpiCfg<EPI>;
-  constexpr int NST = Cfg::STAGES;
+  using PCfg = PairCfg<KIND, EPI>;
+  constexpr bool SCALED = PCfg::SCALED;
+  constexpr int NST = PCfg::STAGES, SF_A = PCfg::SF_A;
   constexpr int WSB = Cfg::WARP_STAGE;
   constexpr int BKE = KindTraits<KIND>::BKE;            // elements of a swizzled row: K of a stage, and the columns of an MN-major chunk
   extern __shared__ unsigned char smem_raw[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   unsigned char* epi_stage = smem + NST * STAGE2_BYTES;
-  uint64_t* full_bar = reinterpret_cast<uint64_t*>(epi_stage + 4 * WSB);
+  unsigned char* sf_stage = epi_stage + 4 * WSB;       // [NST][A rows][B rows 0..127][B rows 128..255]
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(sf_stage + NST * 3 * SF_A);
   uint64_t* empty_bar = full_bar + NST;
   uint64_t* tfull_bar = empty_bar + NST;
   uint64_t* tempty_bar = tfull_bar + 2;
   uint64_t* aux_bar = tempty_bar + 2;                   // [8 warps][2 boxes]: auxiliary-input tiles landed
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(aux_bar + 16);
+  uint64_t* tover_bar = aux_bar + 16;                   // [2] block-scaled: the columns shared with the other accumulator are read
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tover_bar + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
@@ -53,11 +77,12 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < NST; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
-    for (int a = 0; a < 2; ++a) { mbar_init(&tfull_bar[a], 1); mbar_init(&tempty_bar[a], 2 * EPI_WARPS); }
+    for (int a = 0; a < 2; ++a) { mbar_init(&tfull_bar[a], 1); mbar_init(&tempty_bar[a], 2 * EPI_WARPS); mbar_init(&tover_bar[a], 8); }
     for (int a = 0; a < 16; ++a) mbar_init(&aux_bar[a], 1);
     *abort_flag = 0;
     fence_barrier_init();
     prefetch_tmap(&tmA); prefetch_tmap(&tmB);
+    if constexpr (SCALED) { prefetch_tmap(&sfm.a); prefetch_tmap(&sfm.b); }
     if (p.tma_epi) { prefetch_tmap(&tmD); prefetch_tmap(&tmAux); }
   }
   if (warp == 1) tmem_alloc_pair<512>(tmem_slot);
@@ -154,7 +179,12 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           const uint32_t lead_full = lead_full0 + stage * 8;
           const int k0 = kb * BKE;
           if (elect_one()) {
-            if (leader) mbar_expect_tx(&full_bar[stage], 2 * STAGE2_BYTES);     // bytes of both CTAs
+            if (leader) mbar_expect_tx(&full_bar[stage], 2 * (STAGE2_BYTES + 3 * SF_A));     // bytes of both CTAs
+            if constexpr (SCALED) {
+              unsigned char* sf = sf_stage + stage * 3 * SF_A;
+              tma_load_2d_pair(sf, &sfm.a, lead_full, kb * (SF_A / 8), m_blk * 2 + (int)cta);
+              tma_load_2d_pair(sf + SF_A, &sfm.b, lead_full, kb * (SF_A / 8), n_blk * 2);
+            }
             if (!p.a_mn) tma_load_2d_pair(sa, &tmA, lead_full, k0, m0);
             else if (p.a_3d) tma_load_3d_pair(sa, &tmA, lead_full, 0, k0, m0 / BKE);
             else {
@@ -187,6 +217,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       const uint64_t adesc0 = make_smem_desc(smem_u32(smem), p.a_lbo, p.a_sbo, p.a_layout);
       const uint64_t bdesc0 = make_smem_desc(smem_u32(smem) + A_STAGE, p.b_lbo, p.b_sbo, p.b_layout);
       const uint64_t a_inc = (uint64_t)(p.a_kstep >> 4), b_inc = (uint64_t)(p.b_kstep >> 4);
+      const uint64_t sf0 = SCALED ? make_sf_desc(smem_u32(sf_stage)) : 0;
       const uint32_t idesc = p.idesc;
       const uint32_t eb0 = mapa_u32(smem_u32(&empty_bar[0]), 0), eb1 = mapa_u32(smem_u32(&empty_bar[0]), 1);
       const uint32_t tb0 = mapa_u32(smem_u32(&tfull_bar[0]), 0), tb1 = mapa_u32(smem_u32(&tfull_bar[0]), 1);
@@ -196,17 +227,39 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         const int acc = it & 1;
         const uint32_t acc_phase = (it >> 1) & 1;
         if (!mbar_wait(&tempty_bar[acc], acc_phase ^ 1)) { ok = false; break; }
+        if (SCALED && it > 0 && !mbar_wait(&tover_bar[acc ^ 1], ((it - 1) >> 1) & 1)) { ok = false; break; }
         fence_after_sync();
-        const uint32_t d_tmem = tmem_base + acc * BN;
+        const uint32_t d_tmem = tmem_base + acc * PCfg::ACC1_COL;
         for (int kb = kb0; kb < kb1; ++kb) {
           if (!mbar_wait(&full_bar[stage], phase)) { ok = false; break; }
           fence_after_sync();
           const uint64_t adesc = adesc0 + (uint64_t)(stage * (STAGE2_BYTES >> 4));
           const uint64_t bdesc = bdesc0 + (uint64_t)(stage * (STAGE2_BYTES >> 4));
           if (elect_one()) {
-            umma_ss_pair<KIND>(d_tmem, adesc, bdesc, idesc, kb > kb0 ? 1u : 0u);
+            if constexpr (SCALED) {
+              // scales to tensor memory, then up to four MMAs (32 bytes of K per row each); the copies and MMAs of a thread run in order
+              constexpr int VALS = KIND == KIND_NVF4 ? 64 : 32, ATOMS = SF_A / 512;
+              const int nk = min(4, (p.K - kb * 4 * VALS + VALS - 1) / VALS);
+              const uint32_t sfa_t = tmem_base + SFA_COL, sfb_t = tmem_base + SFB_COL;
+              const uint64_t sfa = sf0 + (uint64_t)(stage * (3 * SF_A >> 4)), sfb = sfa + (uint64_t)(SF_A >> 4);
+              for (int k = 0; k < ATOMS && k < nk; ++k) {
+                tmem_cp_sf_pair(sfa_t + 4 * k, sfa + (uint64_t)(k * 32));
+                tmem_cp_sf_pair(sfb_t + 8 * k, sfb + (uint64_t)(k * 32));
+                tmem_cp_sf_pair(sfb_t + 8 * k + 4, sfb + (uint64_t)((SF_A >> 4) + k * 32));
+              }
+              for (int k = 0; k < nk; ++k) {
+                const uint32_t acc_in = kb > kb0 || k > 0 ? 1u : 0u;
+                if constexpr (KIND == KIND_NVF4)
+                  umma_nvfp4_pair(d_tmem, adesc + k * a_inc, bdesc + k * b_inc, idesc, sfa_t + 4 * k, sfb_t + 8 * k, acc_in);
+                else                                        // byte k of the atom's columns: in the descriptor and in the addresses
+                  umma_mxfp8_pair(d_tmem, adesc + k * a_inc, bdesc + k * b_inc, idesc | ((uint32_t)k << 29) | ((uint32_t)k << 4),
+                                  sfa_t | ((uint32_t)k << 30), sfb_t | ((uint32_t)k << 30), acc_in);
+              }
+            } else {
+              umma_ss_pair<KIND>(d_tmem, adesc, bdesc, idesc, kb > kb0 ? 1u : 0u);
 #pragma unroll
-            for (int k = 1; k < 4; ++k) umma_ss_pair<KIND>(d_tmem, adesc + k * a_inc, bdesc + k * b_inc, idesc, 1u);
+              for (int k = 1; k < 4; ++k) umma_ss_pair<KIND>(d_tmem, adesc + k * a_inc, bdesc + k * b_inc, idesc, 1u);
+            }
             umma_commit_pair(eb0 + stage * 8);            // stage free in both CTAs once these MMAs have read it
             umma_commit_pair(eb1 + stage * 8);
           }
@@ -337,7 +390,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       int m_blk, n_blk, kb0, kb1; unit_coords(cluster_id, m_blk, n_blk, kb0, kb1);
       for (int ls = 0; ls < 2; ++ls) aux_issue(m_blk * 2 * BM + band_off, n_blk * BN, ls);
     }
-    const uint32_t te0 = mapa_u32(smem_u32(&tempty_bar[0]), 0);
+    const uint32_t te0 = mapa_u32(smem_u32(&tempty_bar[0]), 0), to0 = mapa_u32(smem_u32(&tover_bar[0]), 0);
     const float alpha = p.alpha ? *p.alpha : 1.0f;
     int it = 0;
     for (int unit = cluster_id; unit < total_units && !*abort_flag; unit += num_clusters, ++it) {
@@ -349,23 +402,43 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       fence_after_sync();
       const int n0 = n_blk * BN;
       const int row0 = m_blk * 2 * BM + band_off;
-      const uint32_t tacc = tmem_base + ((uint32_t)(q * 32) << 16) + acc * BN;
+      const uint32_t tacc = tmem_base + ((uint32_t)(q * 32) << 16) + acc * PCfg::ACC1_COL;
       if (!tma_epi) {
         if (e < 4) epilogue_warp<EPI>(p, tacc, wstage, row0, n0, alpha, lane);
+        if (SCALED && e < 4) {
+          fence_before_sync();
+          __syncwarp();
+          if (lane == 0) mbar_arrive_cluster(to0 + acc * 8);
+        }
       } else {
         const int nunit = unit + num_clusters;
         const bool has_next = AUX && nunit < total_units;
         int nrow0 = 0, nn0 = 0;
         if (has_next) { int mb, nb, k0, k1; unit_coords(nunit, mb, nb, k0, k1); nrow0 = mb * 2 * BM + band_off; nn0 = nb * BN; }
         bool ok = true;
+        // block-scaled: the slab shared with the other accumulator goes first, the last of accumulator 0 and the first of accumulator 1
+        const bool over = SCALED && hcol == (acc ? 0 : 1);
+        const int flip = SCALED && hcol == 1 && acc == 0 ? 1 : 0;
 #pragma unroll 1
-        for (int ls = 0; ls < NBOX; ++ls) {
-          if (!slab_valid(row0, n0, ls)) break;            // warp-uniform
+        for (int i = 0; i < NBOX; ++i) {
+          const int ls = i ^ flip;
+          const bool valid = slab_valid(row0, n0, ls);     // warp-uniform
+          if (!SCALED && !valid) break;
           const int col0 = n0 + hcol * 128 + ls * BOXC;
           uint32_t r0[32], r1[32];
-          tmem_ld32(tacc + hcol * 128 + ls * BOXC, r0);
-          if (!F32_IO) tmem_ld32(tacc + hcol * 128 + ls * BOXC + 32, r1);
-          tmem_wait_ld();
+          if (valid) {
+            tmem_ld32(tacc + hcol * 128 + ls * BOXC, r0);
+            if (!F32_IO) tmem_ld32(tacc + hcol * 128 + ls * BOXC + 32, r1);
+            tmem_wait_ld();
+          }
+          if (SCALED) {
+            if (i == 0 && over) {
+              fence_before_sync();
+              __syncwarp();
+              if (lane == 0) mbar_arrive_cluster(to0 + acc * 8);
+            }
+            if (!valid) continue;
+          }
           unsigned char* buf;
           if (Cfg::F32_OUT) {
             // fp32 accumulate / store: the slab leaves as two boxes of 32 rows x 32 fp32 columns (128-byte rows, swizzled), which
@@ -449,7 +522,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
         if (!ok) { *abort_flag = 1; atomicExch(p.status, LLMB_ERR_TIMEOUT); break; }
         if (AUX && has_next) {                            // refill each buffer once its store has been read
           // (a unit at the right edge may have stored its last slab from buffer 0: then both stores must have been read)
-          if (lane == 0) { if (slab_valid(row0, n0, NBOX - 1)) bulk_wait_read<1>(); else bulk_wait_read<0>(); }
+          if (lane == 0) { if (slab_valid(row0, n0, NBOX - 1) && !flip) bulk_wait_read<1>(); else bulk_wait_read<0>(); }
           __syncwarp();
           aux_issue(nrow0, nn0, 0);
           if (lane == 0) bulk_wait_read<0>();
@@ -478,30 +551,31 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
 
 template <int KIND, int EPI>
 int launch_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td, const CUtensorMap& taux,
-                const GemmParams& p, int grid, cudaStream_t st) {
+                const ScaleMaps<KIND>& sfm, const GemmParams& p, int grid, cudaStream_t st) {
   static bool attr_done = false;
-  constexpr int SMEM = smem2_bytes<EPI>();
+  constexpr int SMEM = PairCfg<KIND, EPI>::SMEM;
   static_assert(SMEM <= 227 * 1024, "shared memory of a CTA");
   if (!attr_done) {
     cudaError_t e = cudaFuncSetAttribute(gemm_pair_kernel<KIND, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
     if (e != cudaSuccess) return (int)e;
     attr_done = true;
   }
-  return launch_pdl(gemm_pair_kernel<KIND, EPI>, grid, PAIR_THREADS, SMEM, st, ta, tb, td, taux, p);
+  return launch_pdl(gemm_pair_kernel<KIND, EPI>, grid, PAIR_THREADS, SMEM, st, ta, tb, td, taux, sfm, p);
 }
 // ... by the epilogue's number, on as many pairs as there are work units (256 x 256 tiles x parts of K), at most one per two SMs
 template <int KIND>
-int launch_pair_epi(int epi, const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td, const CUtensorMap& taux, const GemmParams& p, cudaStream_t st) {
+int launch_pair_epi(int epi, const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& td, const CUtensorMap& taux, const ScaleMaps<KIND>& sfm,
+                    const GemmParams& p, cudaStream_t st) {
   const long long units = (long long)ceil_div(p.M, 2 * BM) * p.n_tiles * p.splits;
   const int most = sm_count() / 2, grid = 2 * (int)(units < most ? units : most);
   switch (epi) {
-    case EPI_NONE: return launch_pair<KIND, EPI_NONE>(ta, tb, td, taux, p, grid, st);
-    case EPI_BIAS: return launch_pair<KIND, EPI_BIAS>(ta, tb, td, taux, p, grid, st);
-    case EPI_BIAS_GELU: return launch_pair<KIND, EPI_BIAS_GELU>(ta, tb, td, taux, p, grid, st);
-    case EPI_DGELU: return launch_pair<KIND, EPI_DGELU>(ta, tb, td, taux, p, grid, st);
-    case EPI_ACC_F32: return launch_pair<KIND, EPI_ACC_F32>(ta, tb, td, taux, p, grid, st);
-    case EPI_BIAS_RESID: return launch_pair<KIND, EPI_BIAS_RESID>(ta, tb, td, taux, p, grid, st);
-    case EPI_STORE_F32: return launch_pair<KIND, EPI_STORE_F32>(ta, tb, td, taux, p, grid, st);
+    case EPI_NONE: return launch_pair<KIND, EPI_NONE>(ta, tb, td, taux, sfm, p, grid, st);
+    case EPI_BIAS: return launch_pair<KIND, EPI_BIAS>(ta, tb, td, taux, sfm, p, grid, st);
+    case EPI_BIAS_GELU: return launch_pair<KIND, EPI_BIAS_GELU>(ta, tb, td, taux, sfm, p, grid, st);
+    case EPI_DGELU: return launch_pair<KIND, EPI_DGELU>(ta, tb, td, taux, sfm, p, grid, st);
+    case EPI_ACC_F32: return launch_pair<KIND, EPI_ACC_F32>(ta, tb, td, taux, sfm, p, grid, st);
+    case EPI_BIAS_RESID: return launch_pair<KIND, EPI_BIAS_RESID>(ta, tb, td, taux, sfm, p, grid, st);
+    case EPI_STORE_F32: return launch_pair<KIND, EPI_STORE_F32>(ta, tb, td, taux, sfm, p, grid, st);
   }
   return LLMB_ERR_BAD_ARG;
 }

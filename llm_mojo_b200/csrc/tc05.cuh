@@ -204,7 +204,7 @@ __host__ __device__ constexpr uint32_t make_idesc(uint32_t a_fmt, uint32_t b_fmt
   return (1u << 4) | (a_fmt << 7) | (b_fmt << 10) | (a_mn << 15) | (b_mn << 16) | ((N >> 3) << 17) | ((M >> 4) << 24);
 }
 
-enum { KIND_F16 = 0, KIND_TF32 = 1, KIND_F8F6F4 = 2 };
+enum { KIND_F16 = 0, KIND_TF32 = 1, KIND_F8F6F4 = 2, KIND_MXF8 = 3, KIND_NVF4 = 4 };
 // One lane of a converged warp (the same lane on every call).  Keeping the surrounding control flow
 // warp-uniform and predicating only the tcgen05 instruction lets the compiler hold descriptors and
 // addresses in uniform registers instead of rebuilding them inside a single-lane branch.
@@ -243,30 +243,6 @@ __host__ __device__ constexpr uint32_t make_idesc_mxfp8(uint32_t a_fmt, uint32_t
 }
 // Shared-memory descriptor of one scale-factor atom: 32 rows of 16 bytes, no swizzle (8-row core matrices 128 B apart).
 __device__ __forceinline__ uint64_t make_sf_desc(uint32_t smem_addr) { return make_smem_desc(smem_addr, 16, 128, 0); }
-
-// Copies 32 rows x 16 bytes of shared memory into 4 TMEM columns of all four lane quarters (row r -> lane r of each
-// quarter): exactly the placement the block-scaled MMA expects for the scales of 128 rows x 4 blocks when the
-// shared-memory image is the 128 x 4 scale atom (byte (r % 32) * 16 + (r / 32) * 4 + block).  One thread issues;
-// the copy is ordered with this thread's earlier and later tcgen05.mma / tcgen05.cp.
-__device__ __forceinline__ void tmem_cp_sf(uint32_t taddr, uint64_t sdesc) {
-  asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;" ::"r"(taddr), "l"(sdesc) : "memory");
-}
-// D[tmem] (+)= (A * sfa) (B * sfb)^T, M = 128, K = 32 fp8 values per row, one scale per row: byte `id` of the TMEM columns at
-// sfa / sfb, where id is given both in the top two bits of the address and in the descriptor's scale id.
-__device__ __forceinline__ void umma_mxfp8(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t sfa,
-                                           uint32_t sfb, uint32_t accumulate) {
-  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-               "tcgen05.mma.cta_group::1.kind::mxf8f6f4.block_scale [%0], %1, %2, %3, [%5], [%6], p;\n\t}"
-               ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(sfa), "r"(sfb) : "memory");
-}
-// D[tmem] (+)= (A * sfa) (B * sfb)^T, M = 128, K = 64 e2m1 values per row; sfa / sfb: TMEM column addresses.
-__device__ __forceinline__ void umma_nvfp4(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t sfa,
-                                           uint32_t sfb, uint32_t accumulate) {
-  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-               "tcgen05.mma.cta_group::1.kind::mxf4nvf4.block_scale.scale_vec::4X [%0], %1, %2, %3, [%5], [%6], p;\n\t}"
-               ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(sfa), "r"(sfb) : "memory");
-}
-
 
 // ------------------------------------------------------------------ CTA-pair (cta_group::2) forms
 // Two CTAs of a cluster of 2 run one 256-row MMA: each CTA stages its 128 rows of A and its
@@ -324,6 +300,29 @@ __device__ __forceinline__ void umma_ss_pair(uint32_t tmem_d, uint64_t adesc, ui
     asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
                  "tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}"
                  ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
+}
+
+// Block-scaled forms.  Copies 32 rows x 16 bytes of shared memory into 4 TMEM columns of all four lane quarters (row r -> lane r of each
+// quarter), in both CTAs from their own shared memory at the descriptor's offset: exactly the placement the block-scaled MMA expects
+// for the scales of 128 rows x 4 blocks when the shared-memory image is the 128 x 4 scale atom (byte (r % 32) * 16 + (r / 32) * 4 + block).
+// One thread issues; the copy is ordered with this thread's earlier and later tcgen05.mma / tcgen05.cp.
+__device__ __forceinline__ void tmem_cp_sf_pair(uint32_t taddr, uint64_t sdesc) {
+  asm volatile("tcgen05.cp.cta_group::2.32x128b.warpx4 [%0], %1;" ::"r"(taddr), "l"(sdesc) : "memory");
+}
+// D[tmem] (+)= (A * sfa) (B * sfb)^T, M = 256, K = 32 fp8 values per row, one scale per row: byte `id` of the TMEM columns at
+// sfa / sfb, where id is given both in the top two bits of the address and in the descriptor's scale id.
+__device__ __forceinline__ void umma_mxfp8_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t sfa,
+                                                uint32_t sfb, uint32_t accumulate) {
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+               "tcgen05.mma.cta_group::2.kind::mxf8f6f4.block_scale [%0], %1, %2, %3, [%5], [%6], p;\n\t}"
+               ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(sfa), "r"(sfb) : "memory");
+}
+// D[tmem] (+)= (A * sfa) (B * sfb)^T, M = 256, K = 64 e2m1 values per row; sfa / sfb: TMEM column addresses.
+__device__ __forceinline__ void umma_nvfp4_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t sfa,
+                                                uint32_t sfb, uint32_t accumulate) {
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+               "tcgen05.mma.cta_group::2.kind::mxf4nvf4.block_scale.scale_vec::4X [%0], %1, %2, %3, [%5], [%6], p;\n\t}"
+               ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(sfa), "r"(sfb) : "memory");
 }
 
 // ------------------------------------------------------------------ host: tensor maps

@@ -563,7 +563,7 @@ def matmul_bwd_fp4(dinp, dweight, dbias, dout, inp, weight, *, gelu_pre=None, rh
                       aux=gelu_pre.view(rows, C) if gelu_pre is not None else None)
         qx = Fp4Operand(x, False, True, rht=rht, other1=qd.ts1, factor1=(1.0 / 16.0) if rht else 1.0)
         _gemm_fp4(dweight.view(OC, C), qd.q1, qd.sf1, qx.q1, qx.sf1, rows, qx.alpha1, epi=EPI_ACC_F32,
-                  splits=_splits_for(OC, C, rows, tile=128, tile_n=256, bk=256, units=148))
+                  splits=_splits_for(OC, C, rows, bk=256))
         if dbias is not None:
             dbias_reduce(dbias, d)
         return
@@ -579,7 +579,7 @@ def matmul_bwd_fp4(dinp, dweight, dbias, dout, inp, weight, *, gelu_pre=None, rh
         qd, sd, tsd = _qp(d, 0, 1, rht=usable_rht, sr=sr, seed=seed, stream_id=NVFP4_SR_STREAM + 3, step=step)
         qx, sx, tsx = _qp(x, 0, 1, rht=usable_rht)
         gemm_nvfp4(dweight.view(OC, C), qd, sd, qx, sx, rows, epi=EPI_ACC_F32,
-                   splits=_splits_for(OC, C, rows, tile=128, tile_n=256, bk=256, units=148),
+                   splits=_splits_for(OC, C, rows, bk=256),
                    alpha=tsd * tsx * ((1.0 / 16.0) if usable_rht else 1.0))
         if dbias is not None:
             dbias_reduce(dbias, d)
@@ -743,7 +743,7 @@ def matmul_bwd_fp8_block(dinp, dweight, dbias, dout, inp, weight, *, gelu_pre=No
         else:
             qx, sx = fp8_block_quant(x, 1, E4M3, transpose=True)
         gemm_mxfp8(dweight.view(OC, C), qd, sd, qx, sx, a_fmt=E5M2, b_fmt=E4M3, epi=EPI_ACC_F32,
-                   splits=_splits_for(OC, C, rows, tile=128, tile_n=256, bk=128, units=148))
+                   splits=_splits_for(OC, C, rows, bk=128))
         if dbias is not None:
             dbias_reduce(dbias, d)
         return

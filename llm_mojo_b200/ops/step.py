@@ -153,7 +153,7 @@ def backward(m, first: bool) -> bool:
             s.kept = m.step_kept.data_ptr()              # of this micro-step's forward pass
             if m.step_kept_stream != stream():           # it is let go below, while this stream may still have to read it
                 m.step_kept.record_stream(torch.cuda.current_stream())
-        lp = lambda n, k: _splits_for(n, k, rows, tile=128, tile_n=256, bk=128 if s.lowp == FP8B else 256, units=148)
+        lp = lambda n, k: _splits_for(n, k, rows, bk=128 if s.lowp == FP8B else 256)
         s.lp_splits_qkv, s.lp_splits_att, s.lp_splits_fc, s.lp_splits_proj = lp(3 * C, C), lp(C, C), lp(4 * C, C), lp(C, 4 * C)
     s.vocab_bits = max(1, (Vp - 1).bit_length())
     enc = scratch("encoder_bwd", L.llmb_encoder_bwd_scratch_bytes(rows, C), dev)

@@ -524,6 +524,48 @@ def test_native_mxfp8_gemm_matches_product_of_fake_quantised_operands(M, N, K):
 
 
 @gpu
+@pytest.mark.parametrize("kind,M,N,K", [("nvfp4", 2696, 2056, 320), ("nvfp4", 136, 264, 1600), ("nvfp4", 96, 72, 32), ("nvfp4", 5120, 2560, 576),
+                                        ("mxfp8", 2688, 2176, 384), ("mxfp8", 128, 128, 640), ("mxfp8", 5248, 2560, 256)])
+def test_block_scaled_gemm_tiles_and_epilogues(kind, M, N, K):
+    """Rows and columns that end inside a pair tile, its second 128-row block missing, K that ends inside a stage, several tiles per pair
+    (overlapping accumulators), with every epilogue, against the fp32 product of the dequantised operands.  bf16 results: half a unit in the
+    last place of 2^-8 (2e-3) and of the pre-activations before it; fp32 ones: sums of up to 1600 exact products, 2^-24 each."""
+    from llm_mojo_b200 import ops
+    if kind == "nvfp4":
+        da, qa, sa, db, qb, sb, alpha = _nvfp4_operands(M, N, K, seed=5)
+        run = lambda D, **k: ops.gemm_nvfp4(D, qa, sa, qb, sb, K, alpha=alpha, **k)
+        base = (da.float() @ db.float().t()) * alpha
+    else:
+        g = torch.Generator().manual_seed(6)
+        a, b = torch.randn(M, K, generator=g).bfloat16().cuda(), (torch.randn(N, K, generator=g) * 0.05).bfloat16().cuda()
+        (qa, sa), (qb, sb) = lowp.fp8_block_quant(a, 0, lowp.E5M2), lowp.fp8_block_quant(b, 2, lowp.E4M3)
+        run = lambda D, **k: ops.gemm_mxfp8(D, qa, sa, qb, sb, a_fmt=lowp.E5M2, b_fmt=lowp.E4M3, **k)
+        base = lowp.fp8_block_fake_quant(a, 0, lowp.E5M2).float() @ lowp.fp8_block_fake_quant(b, 2, lowp.E4M3).float().t()
+    err = lambda got, want: ((got.float() - want).norm() / want.norm()).item()
+    bias, aux = torch.randn(N, device="cuda").bfloat16(), torch.randn(M, N, device="cuda").bfloat16()
+    out, pre = torch.empty(M, N, dtype=torch.bfloat16, device="cuda"), torch.empty(M, N, dtype=torch.bfloat16, device="cuda")
+    run(out)
+    assert err(out, base) < 4e-3
+    run(out, epi=ops.EPI_BIAS, bias=bias)
+    assert err(out, base + bias.float()) < 4e-3
+    run(out, epi=ops.EPI_BIAS_GELU, bias=bias, aux=pre)
+    assert err(pre, base + bias.float()) < 4e-3
+    assert err(out, torch.nn.functional.gelu(pre.float(), approximate="tanh")) < 4e-3
+    run(out, epi=ops.EPI_BIAS_RESID, bias=bias, aux=aux)
+    assert err(out, base + bias.float() + aux.float()) < 4e-3
+    run(out, epi=ops.EPI_DGELU, aux=aux)
+    x = aux.float().requires_grad_()
+    torch.nn.functional.gelu(x, approximate="tanh").sum().backward()
+    assert err(out, base * x.grad) < 4e-3
+    f32 = torch.full((M, N), 2.0, device="cuda")
+    run(f32, epi=ops.EPI_STORE_F32)
+    assert err(f32, base) < 1e-5
+    run(f32, epi=ops.EPI_ACC_F32, splits=3)
+    assert err(f32, 2 * base) < 1e-5
+    assert int(ops.status_word(torch.device("cuda", 0)).item()) == 0
+
+
+@gpu
 def test_fp8_block_linear_native_matches_fake_quant_path(monkeypatch):
     rows, C, OC = 512, 256, 384
     g = torch.Generator().manual_seed(4)

@@ -11,7 +11,7 @@
 #define LLMB_API extern "C" __attribute__((visibility("default")))
 
 // Counts the changes of the entry points' arguments; the Python side (ABI in ops/_lib.py) refuses a library with another number.
-#define LLMB_ABI 1
+#define LLMB_ABI 2
 
 // dtype codes shared with the Python side
 enum { LLMB_F32 = 0, LLMB_BF16 = 1 };

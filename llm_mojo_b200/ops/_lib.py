@@ -65,11 +65,8 @@ _SIGS = {
     "llmb_amax_state_floats": [],
     "llmb_amax_update": [c_p, c_p, c_f, c_f, c_p],
     "llmb_quantize_fp8": [c_p, c_p, c_p, c_ll, c_int, c_int, c_p],
-    "llmb_quantize_fp8_delayed": [c_p, c_p, c_p, c_p, c_ll, c_int, c_f, c_f, c_int, c_p],
     "llmb_fp8_block_quant_dual": [c_p, c_p, c_p, c_p, c_p, c_int, c_int, c_int, c_p],
-    "llmb_fp8_prepare": [c_p, c_p, c_f, c_f, c_p, c_p, c_f, c_f, c_p, c_p, c_p, c_p, c_p, c_p, c_p],
-    "llmb_fp8_push": [c_p, c_p, c_p, c_p, c_p],
-    "llmb_quantize_fp8_amax": [c_p, c_p, c_p, c_p, c_ll, c_int, c_int, c_p],
+    "llmb_fp8_site_quant": [c_p, c_p, c_p, c_p, c_ll, c_f, c_p, c_p, c_p, c_p, c_ll, c_f, c_int, c_int, c_p, c_p, c_p, c_p, c_p],
     "llmb_dequantize_fp8": [c_p, c_p, c_p, c_ll, c_int, c_p],
     "llmb_nvfp4_tensor_scale": [c_p, c_p, c_p],
     "llmb_nvfp4_scale_bytes": [c_ll, c_ll, c_int],
@@ -108,7 +105,7 @@ def available() -> bool:
 
 
 # Counts the changes of the C entry points' arguments; LLMB_ABI in csrc/common.cuh is the library's side of it.
-ABI = 1
+ABI = 2
 
 
 def _declare(L) -> None:

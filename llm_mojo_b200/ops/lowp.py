@@ -56,6 +56,7 @@ class AmaxState:
         self.state[0] = 1.0
         self.state[1] = 1.0
         self.amax = torch.zeros(1, dtype=torch.float32, device=device)
+        self.work = torch.zeros(2, dtype=torch.int32, device=device)       # of ``llmb_fp8_site_quant``: zero between its launches
         self.host_step = 0
         self.static = False
 
@@ -200,13 +201,8 @@ def _q(name: str, x: torch.Tensor, state: AmaxState, buf: Optional[torch.Tensor]
     two-pass order of ``llmm/amax.mojo:425-565``)."""
     if buf is None:
         buf = scratch("fp8_" + name, x.numel(), x.device)[:x.numel()].view(x.shape)
-    vec = 8 if x.dtype == torch.bfloat16 else 4
-    if (FUSED_DELAYED and x.is_cuda and not state.static and state.host_step >= AMAX_HISTORY and x.is_contiguous()
-            and x.numel() % vec == 0 and x.dtype in (torch.bfloat16, torch.float32)):
-        check(lib().llmb_quantize_fp8_delayed(ptr(buf), ptr(x), ptr(state.state), ptr(state.amax), x.numel(), state.fmt,
-                                              FMT_MAX[state.fmt], state.margin_mult, dtype_code(x), stream()), "quantize_fp8_delayed")
-        _count(3)
-        state.host_step += 1
+    if _delayed_ready(state, x):
+        _site_quant((buf, x, state))
         return buf
     state.update_scale(x)
     quantize_fp8(buf, x, state.scale, state.fmt)
@@ -220,10 +216,18 @@ def _delayed_ready(state: AmaxState, x: torch.Tensor) -> bool:
             and x.numel() % vec == 0 and x.dtype in (torch.bfloat16, torch.float32))
 
 
-def _quant_amax(buf: torch.Tensor, x: torch.Tensor, state: AmaxState) -> None:
-    check(lib().llmb_quantize_fp8_amax(ptr(buf), ptr(x), ptr(state.state), ptr(state.amax), x.numel(), state.fmt, dtype_code(x),
-                                       stream()), "quantize_fp8_amax")
+def _site_quant(a, b=None, alpha1=None, other1=None, alpha2=None, other2=None) -> None:
+    """Quantises one or two operands ``(bytes, x, state)`` of a linear layer whose states are ``_delayed_ready``, in one launch;
+    ``alpha`` = 1/scale of ``a`` × 1/scale of the state ``other`` (``b``'s where that is None)."""
+    (qa, xa, sa), (qb, xb, sb) = a, b or (None, None, None)
+    check(lib().llmb_fp8_site_quant(ptr(qa), ptr(xa), ptr(sa.state), ptr(sa.work), xa.numel(), sa.margin_mult, ptr(qb), ptr(xb),
+                                    ptr(sb.state) if b else None, ptr(sb.work) if b else None, xb.numel() if b else 0, sb.margin_mult if b else 0.0,
+                                    sa.fmt, dtype_code(xa), ptr(alpha1), ptr(other1.state) if other1 else None, ptr(alpha2),
+                                    ptr(other2.state) if other2 else None, stream()), "fp8_site_quant")
     _count()
+    sa.host_step += 1
+    if b:
+        sb.host_step += 1
 
 
 def matmul_fwd_fp8(out, inp, weight, bias, site: LinearSite, *, pre_gelu=None, residual=None) -> None:
@@ -237,19 +241,9 @@ def matmul_fwd_fp8(out, inp, weight, bias, site: LinearSite, *, pre_gelu=None, r
             site.qx = torch.empty(x.shape, dtype=torch.uint8, device=x.device)
         if site.qw is None or site.qw.shape != weight.shape:
             site.qw = torch.empty(weight.shape, dtype=torch.uint8, device=x.device)
-        if _delayed_ready(site.inp, x) and _delayed_ready(site.weight, weight):
-            # both histories are full: one launch derives both scales and the GEMM's scale factor, one appends both amax values
-            si, sw = site.inp, site.weight
-            check(lib().llmb_fp8_prepare(ptr(si.state), ptr(si.amax), FMT_MAX[si.fmt], si.margin_mult, ptr(sw.state), ptr(sw.amax),
-                                         FMT_MAX[sw.fmt], sw.margin_mult, ptr(site.alpha), ptr(si.state), ptr(sw.state), None, None, None,
-                                         stream()), "fp8_prepare")
-            qx, qw = site.qx, site.qw
-            _quant_amax(qx, x, si)
-            _quant_amax(qw, weight, sw)
-            check(lib().llmb_fp8_push(ptr(si.state), ptr(si.amax), ptr(sw.state), ptr(sw.amax), stream()), "fp8_push")
-            _count(2)
-            si.host_step += 1
-            sw.host_step += 1
+        if _delayed_ready(site.inp, x) and _delayed_ready(site.weight, weight) and x.dtype == weight.dtype:
+            qx, qw = site.qx, site.qw                                     # both histories are full
+            _site_quant((qx, x, site.inp), (qw, weight, site.weight), site.alpha)
         else:
             qx = _q("x", x, site.inp, site.qx)
             qw = _q("w", weight, site.weight, site.qw)
@@ -292,15 +286,8 @@ def matmul_bwd_fp8(dinp, dweight, dbias, dout, inp, weight, site: LinearSite, *,
     site_fused = _delayed_ready(site.dout, d)
     if site_fused:
         # the d_output scale from its history and both GEMM scale factors (the input / weight scales of this step are final)
-        sd = site.dout
-        check(lib().llmb_fp8_prepare(ptr(sd.state), ptr(sd.amax), FMT_MAX[sd.fmt], sd.margin_mult, None, None, 0.0, 0.0, ptr(site.alpha),
-                                     ptr(sd.state), ptr(site.weight.state), ptr(site.alpha2), ptr(sd.state), ptr(site.inp.state), stream()),
-              "fp8_prepare")
         qd = scratch("fp8_d", d.numel(), d.device)[:d.numel()].view(d.shape)
-        _quant_amax(qd, d, sd)
-        check(lib().llmb_fp8_push(ptr(sd.state), ptr(sd.amax), None, None, stream()), "fp8_push")
-        _count(2)
-        sd.host_step += 1
+        _site_quant((qd, d, site.dout), None, site.alpha, site.weight, site.alpha2, site.inp)
     else:
         qd = _q("d", d, site.dout)
     if dinp is not None:

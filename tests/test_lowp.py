@@ -236,6 +236,56 @@ def test_fp8_block_dual_quantisation_equals_the_two_single_kernels(fmt):
 
 
 @gpu
+@pytest.mark.parametrize("fmt", [lowp.E4M3, lowp.E5M2])
+def test_fp8_block_dual_quantisation_at_the_ends_of_the_range(fmt):
+    """Block maxima whose scale comes from exponent bits (either side of 1.75, up to the largest) and those that go the general way: zeros,
+    denormals, magnitudes whose scale is denormal, infinity, NaN beside numbers and alone.  Bytes and scales equal the single kernels'."""
+    top = torch.finfo(torch.bfloat16)
+    peaks = [0.0, 1.0, 1.75, 1.7578125, 1.7421875, 448.0, 57344.0, 3e38, top.max, 1e-30, 2.0 ** -110, 2.0 ** -118, 2.0 ** -119, top.tiny, 1e-39,
+             float("inf"), float("nan"), -3.5, -1.7578125]
+    x = torch.rand(128 * 2, 128 * 2).mul(2).sub(1)
+    for i in range(256):
+        x[i] *= abs(peaks[i % len(peaks)])
+        x[i, (7 * i) % 256] = peaks[i % len(peaks)]
+    x[:, 200] = float("nan")
+    x[:, 17], x[:, 90] = 0.0, float("inf")
+    for y in (x, x.t().contiguous()):
+        y = y.bfloat16().cuda()
+        q0, s0, q1, s1 = lowp.fp8_block_quant_dual(y, fmt)
+        r0, t0 = lowp.fp8_block_quant(y, 0, fmt)
+        r1, t1 = lowp.fp8_block_quant(y, 1, fmt, transpose=True)
+        assert torch.equal(s0, t0) and torch.equal(s1, t1) and torch.equal(q0, r0) and torch.equal(q1, r1)
+
+
+@gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("na,nb", [(8, 0), (8, 24), (4096, 1 << 20), (1 << 20, 4104), (3 << 20, 2056), (5 << 20, (3 << 20) + 8)])
+def test_operands_of_a_site_in_one_launch_equal_one_by_one(na, nb, dtype):
+    """One vector, more vectors than threads, ends inside a thread's four, shares of the grid from one CTA to nearly all: bytes, states,
+    work words and scale factors against the two-pass order."""
+    a, b, c = (lowp.AmaxState("cuda", lowp.E4M3) for _ in range(3))
+    ra, rb = lowp.AmaxState("cuda", lowp.E4M3), lowp.AmaxState("cuda", lowp.E4M3)
+    for st in (a, b, ra, rb):
+        st.state[4:] = torch.linspace(0.5, 3.0, lowp.AMAX_HISTORY)
+        st.state[2] = torch.tensor([lowp.AMAX_HISTORY], dtype=torch.int32).view(torch.float32)[0]
+        st.host_step = lowp.AMAX_HISTORY
+    c.state[1] = 0.25
+    alpha1, alpha2 = torch.zeros(1, device="cuda"), torch.zeros(1, device="cuda")
+    for step in range(3):
+        xa, xb = (torch.randn(na) * 2).to(dtype).cuda(), (torch.randn(max(nb, 8)) * 9).to(dtype).cuda()
+        qa, qb = torch.empty(xa.shape, dtype=torch.uint8, device="cuda"), torch.empty(xb.shape, dtype=torch.uint8, device="cuda")
+        lowp._site_quant((qa, xa, a), (qb, xb, b) if nb else None, alpha1, None if nb else c, alpha2, c)
+        for q, x, one, two in ((qa, xa, a, ra), (qb, xb, b, rb))[:2 if nb else 1]:
+            two.update_scale(x)
+            want = torch.empty_like(q)
+            lowp.quantize_fp8(want, x, two.scale, lowp.E4M3)
+            assert torch.equal(q, want) and torch.equal(one.state, two.state) and not one.work.any()
+            assert one.host_step == two.host_step
+        assert alpha1.item() == (ra.scale_inv * (rb.scale_inv if nb else c.scale_inv)).item()
+        assert alpha2.item() == (ra.scale_inv * c.scale_inv).item()
+
+
+@gpu
 def test_fp8_block_linear_dual_path_is_bit_identical(monkeypatch):
     rows, C, OC = 256, 384, 512
     g = torch.Generator().manual_seed(2)

@@ -4,27 +4,38 @@
 // and the dQ / dK / dV products over stored [T,T] probabilities).  Here nothing of size T x T reaches HBM and the
 // scores are recomputed ONCE: a CTA owns a 128-key tile (K and V resident in shared memory, dK and dV accumulating
 // in TMEM) and walks the 128-row query blocks i that can see it.  Per block, with lanes = keys, columns = queries:
-//   S^T  = K Q_i^T          (tensor core, fp32 in TMEM)
-//   dP^T = V dO_i^T         (tensor core, fp32 in TMEM)
-//   P^T  = 2^(S^T * a - lse[q])          compute warps; packed bf16 into its own TMEM columns
+//   S^T  = K Q_i^T - lse / a    (tensor core, fp32 in TMEM)
+//   dP^T = V dO_i^T - D         (tensor core, fp32 in TMEM)
+//   P^T  = 2^(S^T * a)          compute warps; packed bf16 into its own TMEM columns
+//   dS^T = P^T * dP^T           compute warps; bf16 into a swizzled shared-memory tile [keys, queries]
 //   dV  += P^T dO_i         (A operand read from TMEM, dO_i as an MN-major shared-memory operand)
-//   dS^T = P^T * (dP^T - D[q])           compute warps; bf16 into a swizzled shared-memory tile [keys, queries]
 //   dK  += dS^T Q_i         (A K-major from that tile)
 //   dQ_i partial = dS K     (A MN-major from the SAME tile, B = the resident K tile as an MN-major operand)
-// Because P^T does not live in the columns of S^T, the issuer can start S^T(n+1) as soon as the compute warps hold
-// S^T(n) in registers (and dP^T(n+1) when they hold dP^T(n)): the scores of a block are in TMEM a whole block
-// before they are used, and no compute warp waits for a tcgen05.commit round trip in steady state.
+// A block is one chain - scores, compute warps, products - and the next block's scores are made beside it: as soon as the compute warps
+// hold S^T(n) and dP^T(n) in registers, those of n+1 are issued.  What the chain was spent on, and how that was cut (cycles per block of
+// about 6000, from clock traces of the roles):
+//   * -lse and -D differ from column to column, so every thread needed all of them: 32 vector loads a thread, 2000 cycles of the shared-memory
+//     pipe.  The tensor core adds them now, as one more K = 16 step of each score product: ones times rows that hold the values in
+//     three bf16 parts (24 bits, all of an fp32 value; attn_bwd3_prep_kernel writes them).
+//   * two phases of the compute warps (P^T, then dS^T) with twelve barrier round trips of 170 - 250 cycles: one phase with two waits.
+//   * one issuing warp, whose round trips came on top of 34 MMAs: one for the scores, one for the products.
+//   * reductions of the dQ partials in the way of the compute warps' stores: see there.
+//   * dK / dV stores that the dQ warpgroup waited for: warp 15 issues them.
+// Whole backward pass, us, before / now: B 64, T 1024, 12 heads 743 / 570; B 4 83 / 64; B 7, T 777 101 / 80; B 6, T 2048, 16 heads 339 / 238.
+// What bounds a block now (3200 cycles): the chain of 64 exponentials a thread at two warps per scheduler (1600), stores and barriers,
+// products (1700, beside them), TMEM loads.
 // The dQ partials of the key tiles are summed in an fp32 buffer by vector reductions (`red.global.add.v4.f32`, 16
 // per thread and block, laid out so that a warp's 32 lanes hit 512 consecutive bytes); a small second kernel scales
 // and rounds that buffer into the dQ part of dqkv and leaves it zeroed for the next call.  dK and dV are produced
 // by exactly one CTA each in a fixed order and leave through a staging tile as TMA stores.
 //
 // Roles of the 512 threads:
-//   warps 0..3 / 4..7   compute warpgroups: one thread per key row, query columns 0..63 / 64..127 of the block
+//   warps 0..7          compute: one thread per key row and 64 of the block's queries
 //   warps 8..11         dQ warpgroup: TMEM -> reductions per block, and the dK / dV epilogue per tile
 //   warp 12             TMA producer: K, V per tile (two buffers), Q_i, dO_i and the row statistics per block (ring),
 //                       and L2 prefetches of the CTA's next tile
-//   warp 13             MMA issuer (one warp: several issuing warps measured slower)
+//   warps 13, 14        MMA issuers of the scores / of the products
+//   warp 15             dK and dV of a tile from the staging tile to memory
 // TMEM columns (512): S^T 0..127 | dP^T 128..255 | dV 256..319 | dK 320..383 | dQ 384..447 | P^T 448..511.
 // Every wait is bounded; a wait that runs out sets the status word and the role leaves its loop.
 #include <type_traits>
@@ -33,8 +44,12 @@
 namespace {
 constexpr int B3_NS = 3;                                   // ring depth in blocks: Q_i and dO_i, 16 KB each
 constexpr int B3_THREADS = 512;
-constexpr int B3_SMEM = 4 * T128 /*K,V x2*/ + B3_NS * 2 * T128 + 2 * T128 /*dS^T*/ + T128 /*epilogue staging*/ + B3_NS * 1024 /*-lse, -D*/ +
-                        1024 /*alignment*/ + 512 /*barriers*/;
+constexpr int B3_EXT = TILE * 32;                          // the statistics of a block as operand rows of 16 bf16
+constexpr int B3_ONE = TILE * 16;                          // 128 rows of 8 bf16, rows in a column of 8-row core matrices
+constexpr unsigned B3_PACE_NS = 90;                        // B 64, T 1024, us: none 616, 20 x 16 582, 100 x 8 570, 150 x 8 (longer than a block) 692
+constexpr int B3_SLACK = 768;                              // for aligning the base, which is aligned already
+constexpr int B3_SMEM = 4 * T128 /*K,V x2*/ + B3_NS * (2 * T128 + B3_EXT) + 2 * T128 /*dS^T*/ + T128 /*epilogue staging*/ + 3 * B3_ONE + 256 /*barriers*/ + B3_SLACK;
+static_assert(B3_SMEM <= 227 * 1024, "shared memory of a CTA");
 constexpr uint32_t IDESC_TS_MN = make_idesc(FMT_BF16, FMT_BF16, 0, 1, 128, 64);     // A K-major (TMEM or smem), B stored [K rows, 64]
 constexpr uint32_t IDESC_MN_MN = make_idesc(FMT_BF16, FMT_BF16, 1, 1, 128, 64);     // A stored [K rows, 128], B stored [K rows, 64]
 
@@ -42,7 +57,6 @@ constexpr uint32_t IDESC_MN_MN = make_idesc(FMT_BF16, FMT_BF16, 1, 1, 128, 64); 
 
 struct B3Params {
   void* dqkv;            // [B,T,3C] bf16
-  const float* stats;    // per (batch, head, 128-row tile): -lse[128] (log2 domain; -inf beyond T), -D[128]
   float* dq_acc;         // per (batch, head, tile): [16 column groups][128 rows][4] fp32, zero on entry
   float* dbias;          // optional fp32 [3C]
   int B, T, NH, C;
@@ -50,10 +64,17 @@ struct B3Params {
   int* status;
 };
 
-// D = rowsum(dO * O) and the packed row statistics of every 128-row tile.  Eight threads per row, 16 bytes of dO and O each,
-// so that a warp reads four whole 128-byte rows per instruction.
-__global__ void attn_bwd3_prep_kernel(float* __restrict__ stats, const float* __restrict__ lse, const __nv_bfloat16* __restrict__ dout,
-                                      const __nv_bfloat16* __restrict__ out, int B, int T, int NH, int C) {
+// D = rowsum(dO * O) and the statistics of every row as 16 bf16 values, an operand of the score products (see above): columns 0 .. 2 the parts
+// of -lse / scale, columns 8 .. 10 those of -D.  Three bf16 parts hold 24 bits, all of an fp32 value.  Eight threads per row, 16 bytes of dO and O
+// each, so that a warp reads four whole 128-byte rows per instruction.
+__device__ __forceinline__ uint4 parts3(float v) {
+  const __nv_bfloat16 hi = __float2bfloat16_rn(v);
+  const float h = __bfloat162float(hi), r1 = isinf(h) ? 0.f : v - h;                // (an infinite value is its first part)
+  const __nv_bfloat16 mid = __float2bfloat16_rn(r1), lo = __float2bfloat16_rn(r1 - __bfloat162float(mid));
+  return make_uint4((uint32_t)__bfloat16_as_ushort(hi) | (uint32_t)__bfloat16_as_ushort(mid) << 16, __bfloat16_as_ushort(lo), 0u, 0u);
+}
+__global__ void attn_bwd3_prep_kernel(uint4* __restrict__ stats, const float* __restrict__ lse, const __nv_bfloat16* __restrict__ dout,
+                                      const __nv_bfloat16* __restrict__ out, int B, int T, int NH, int C, float inv_scale_log2) {
   pdl_trigger();
   pdl_wait();
   const int n_t = ceil_div(T, TILE), Tp = n_t * TILE;
@@ -71,11 +92,8 @@ __global__ void attn_bwd3_prep_kernel(float* __restrict__ stats, const float* __
     for (int k = 0; k < 8; ++k) s += x.v[k] * y.v[k];
   }
   s += __shfl_xor_sync(0xffffffffu, s, 1); s += __shfl_xor_sync(0xffffffffu, s, 2); s += __shfl_xor_sync(0xffffffffu, s, 4);
-  if (part == 0) {
-    float* pk = stats + (bh * n_t + t / TILE) * 256 + (t % TILE);
-    pk[0] = t < T ? -lse[bh * T + t] : -INFINITY;
-    pk[128] = -s;
-  }
+  if (part == 0) stats[idx * 2] = parts3(t < T ? -lse[bh * T + t] * inv_scale_log2 : -1e6f);     // rows beyond T: 2^(-1e6 scale) = 0
+  if (part == 1) stats[idx * 2 + 1] = parts3(-s);
 }
 
 struct Tile3 { int w, t, g, bh, tile; bool sub, done; };    // work item, tiles / blocks consumed so far, current tile
@@ -125,34 +143,36 @@ __device__ __forceinline__ void red_add_v4(float* addr, float a, float b, float 
 
 __global__ void __launch_bounds__(B3_THREADS, 1) attn_bwd3_kernel(const __grid_constant__ CUtensorMap tmQKV,
                                                                   const __grid_constant__ CUtensorMap tmDO,
-                                                                  const __grid_constant__ CUtensorMap tmOUT, const B3Params p) {
+                                                                  const __grid_constant__ CUtensorMap tmOUT,
+                                                                  const __grid_constant__ CUtensorMap tmEXT, const B3Params p) {
   extern __shared__ unsigned char smem_raw[];
   unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  if (sm - smem_raw > B3_SLACK) {                           // the alignment slack this launch was given does not cover the base it got
+    pdl_wait();                                             // (the kernel after this one counts on it, on this path too)
+    if (threadIdx.x == 0) atomicExch(p.status, LLMB_ERR_BAD_ARG);
+    return;
+  }
   unsigned char* sKV = sm;                                  // buffer kb: K at kb*2*T128, V at +T128
   unsigned char* sST = sKV + 4 * T128;                      // ring: stage s holds Q_i at s*2*T128, dO_i at +T128
   unsigned char* sDS = sST + B3_NS * 2 * T128;              // dS^T: queries 0..63 at +0, 64..127 at +T128 ([128 keys][64] each)
-  unsigned char* sEP = sDS + 2 * T128;                      // staging tile of the dK / dV epilogue ([128 keys][64] bf16, swizzled)
-  float* sStat = reinterpret_cast<float*>(sEP + T128);      // per stage: -lse[128], -D[128]
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sStat + B3_NS * 256);
+  unsigned char* sEXT = sDS + 2 * T128;                     // per stage: the block's statistics, [128 queries][16] bf16, 32-byte swizzle
+  unsigned char* sEP = sEXT + B3_NS * B3_EXT;               // staging tile of the dK / dV epilogue ([128 keys][64] bf16, swizzled)
+  unsigned char* sONE = sEP + T128;                         // no swizzle: eight columns 1 1 1 0 0 0 0 0, eight of zeros, eight as the first
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sONE + 3 * B3_ONE);
   uint64_t* kv_full = bars;                                 // [2]
-  uint64_t* kv_empty = kv_full + 2;                         // [2] the tile's last reads of K and V are complete 
+  uint64_t* kv_empty = kv_full + 2;                         // [2] the tile's last reads of K and V are complete
   uint64_t* st_full = kv_empty + 2;                         // [NS]
   uint64_t* st_empty = st_full + B3_NS;                     // [NS] the block's reads of Q and dO are complete 
-  uint64_t* s_full = st_empty + B3_NS;                      // S^T is in TMEM
-  uint64_t* s_free = s_full + 1;                            // the compute warps hold S^T in registers (8 warps)
-  uint64_t* dp_full = s_free + 1;                           // dP^T is in TMEM
-  uint64_t* dp_free = dp_full + 1;                          // the compute warps hold dP^T in registers (8 warps)
-  uint64_t* p_full = dp_free + 1;                           // P^T is in TMEM (8 warps)
-  uint64_t* p_used = p_full + 1;                            // dV has read P^T
-  uint64_t* ds_full = p_used + 1;                           // dS^T is in shared memory (8 warps)
-  uint64_t* ds_free = ds_full + 1;                          // dK and dQ have read dS^T
+  uint64_t* s_full = st_empty + B3_NS;                      // S^T and dP^T of a block are in TMEM
+  uint64_t* s_free = s_full + 1;                            // ... and in the compute warps' registers (8 warps)
+  uint64_t* p_full = s_free + 1;                            // P^T is in TMEM and dS^T in shared memory (8 warps), the block before's dQ has left TMEM (4 warps)
+  uint64_t* ds_free = p_full + 1;                           // dV has read P^T, dK and dQ have read dS^T
   uint64_t* dq_full = ds_free + 1;                          // the block's dQ partial is in TMEM
-  uint64_t* dq_free = dq_full + 1;                          // ... and has left it (4 warps)
-  uint64_t* acc_full = dq_free + 1;                         // dK and dV of a tile are complete 
+  uint64_t* acc_full = dq_full + 1;                         // dK and dV of a tile are complete 
   uint64_t* acc_free = acc_full + 1;                        // ... and have left TMEM (4 warps)
-  uint64_t* ep_ready = acc_free + 1;                        // the epilogue's staging tile is written (4 warps)
-  uint64_t* ep_done = ep_ready + 1;                         // ... and its TMA stores have read it
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(ep_done + 1);
+  uint64_t* ep_ready = acc_free + 1;                        // the staging tile is written (4 warps)
+  uint64_t* ep_free = ep_ready + 1;                         // ... and its TMA stores have read it
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(ep_free + 1);
 
   const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
   const int n_t = ceil_div(p.T, TILE);
@@ -161,11 +181,14 @@ __global__ void __launch_bounds__(B3_THREADS, 1) attn_bwd3_kernel(const __grid_c
   if (tid == 0) {
     for (int i = 0; i < 2; ++i) { mbar_init(&kv_full[i], 1); mbar_init(&kv_empty[i], 1); }
     for (int i = 0; i < B3_NS; ++i) { mbar_init(&st_full[i], 1); mbar_init(&st_empty[i], 1); }
-    mbar_init(s_full, 1); mbar_init(s_free, 8); mbar_init(dp_full, 1); mbar_init(dp_free, 8);
-    mbar_init(p_full, 8); mbar_init(p_used, 1); mbar_init(ds_full, 8); mbar_init(ds_free, 1);
-    mbar_init(dq_full, 1); mbar_init(dq_free, 4); mbar_init(acc_full, 1); mbar_init(acc_free, 4); mbar_init(ep_ready, 4); mbar_init(ep_done, 1);
+    mbar_init(s_full, 1); mbar_init(s_free, 8); mbar_init(p_full, 12); mbar_init(ds_free, 1);
+    mbar_init(dq_full, 1); mbar_init(acc_full, 1); mbar_init(acc_free, 4); mbar_init(ep_ready, 4); mbar_init(ep_free, 1);
     fence_barrier_init();
-    prefetch_tmap(&tmQKV); prefetch_tmap(&tmDO); prefetch_tmap(&tmOUT);
+    prefetch_tmap(&tmQKV); prefetch_tmap(&tmDO); prefetch_tmap(&tmOUT); prefetch_tmap(&tmEXT);
+  }
+  if (tid < 3 * TILE) {
+    *reinterpret_cast<uint4*>(sONE + tid * 16) = tid / TILE == 1 ? make_uint4(0u, 0u, 0u, 0u) : make_uint4(0x3f803f80u, 0x3f80u, 0u, 0u);
+    fence_proxy_async();
   }
   if (warp == 13) tmem_alloc<512>(tmem_slot);
   fence_before_sync();
@@ -178,7 +201,7 @@ __global__ void __launch_bounds__(B3_THREADS, 1) attn_bwd3_kernel(const __grid_c
   pdl_wait();
 
   // Registers move from the dQ warpgroup and the producer / issuer warpgroup to the two compute warpgroups:
-  // 2 x 128 x 176 + 2 x 128 x 80 = 65536 = the registers of the launch (512 x 128).
+  // 128 x (2 x 176 + 2 x 80) = 65536 = the registers of the launch (512 x 128).
   if (warp >= 12) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 80;");
     if (warp == 12) {
@@ -206,10 +229,10 @@ __global__ void __launch_bounds__(B3_THREADS, 1) attn_bwd3_kernel(const __grid_c
           if (n >= B3_NS && !mbar_wait_sleep(&st_empty[st], ((n / B3_NS) + 1) & 1)) { B3_FAIL(); break; }
           if (elect_one()) {
             unsigned char* stg = sST + st * 2 * T128;
-            mbar_expect_tx(&st_full[st], 2 * T128 + 1024);
+            mbar_expect_tx(&st_full[st], 2 * T128 + B3_EXT);
             load128(stg, &tmQKV, &st_full[st], colQ, i * TILE, b);
             load128(stg + T128, &tmDO, &st_full[st], colQ, i * TILE, b);
-            bulk_load_1d(sStat + st * 256, p.stats + ((size_t)c.bh * n_t + i) * 256, 1024, &st_full[st]);
+            tma_load_2d(sEXT + st * B3_EXT, &tmEXT, &st_full[st], 0, (c.bh * n_t + i) * TILE);
             for (int k = 0; k < pf_per; ++k) {
               const int r = pf + 64 * k;
               if (r < nx0) {
@@ -227,77 +250,81 @@ __global__ void __launch_bounds__(B3_THREADS, 1) attn_bwd3_kernel(const __grid_c
         if (failed) break;
         tile3_next(c, nbt, n_t, n_items);
       }
-    } else if (warp == 13) {
-      // ------------------------------------------------------------ MMA issuer.  Per block n, in the order in which the compute warps'
-      // signals arrive: S^T(n+1) when they hold S^T(n) in registers, dV(n) when P^T(n) is written, dP^T(n+1) when they hold
-      // dP^T(n), dK(n) and dQ(n) when dS^T(n) is written - so the scores of a block are ready a whole block before their use.
+    } else if (warp < 15) {
+      // ------------------------------------------------------------ MMA issuers: warp 13 S^T and dP^T of block n + 1 as soon as the compute
+      // warps hold those of n in registers, warp 14 dV, dK and dQ of n when P^T and dS^T are written.
       const uint64_t k_kk0 = make_smem_desc(smem_u32(sKV), 16, 1024);                 // K / V as K-major A operands
       const uint64_t k_mn0 = make_smem_desc(smem_u32(sKV), 8192, 1024);               // K as an MN-major B operand
       const uint64_t q_kk0 = make_smem_desc(smem_u32(sST), 16, 1024);                 // Q_i / dO_i as K-major B operands
       const uint64_t q_mn0 = make_smem_desc(smem_u32(sST), 8192, 1024);               // Q_i / dO_i as MN-major B operands
       const uint64_t ds_kk = make_smem_desc(smem_u32(sDS), 16, 1024);                 // dS^T as a K-major A operand (K = queries)
       const uint64_t ds_mn = make_smem_desc(smem_u32(sDS), T128, 1024);               // dS^T as an MN-major A operand (M = queries)
-      Blk3 nx = blk3_begin(n_t, n_items), it = nx;                                    // block n+1 (scores), block n (accumulating products)
-      auto scores_s = [&]() {                                                         // S^T of block nx
-        const int n = nx.n, st = n % B3_NS, kb = nx.c.t & 1;
-        if (nx.ib == 0 && !mbar_wait(&kv_full[kb], (nx.c.t >> 1) & 1)) { B3_FAIL(); return; }
+      const uint64_t ext0 = make_smem_desc(smem_u32(sEXT), 16, 256, 6);               // 32-byte swizzle
+      const uint64_t one0 = make_smem_desc(smem_u32(sONE), B3_ONE, 128, 0);           // no swizzle: core matrices of 8 rows x 16 bytes, the next along K in the next column
+      // a block in one word: 4 * (tiles before its tile) + 2 * (last of its tile) + (first of its tile), -1 when there is none left
+      auto info = [](const Blk3& b) { return b.c.done ? -1 : b.c.t * 4 + (b.ib + 1 == b.nbt ? 2 : 0) + (b.ib == 0 ? 1 : 0); };
+      auto scores = [&](int n, int what) {                                            // S^T and dP^T of block n
+        const int st = n % B3_NS, t = what >> 2, kb = t & 1;
+        if ((what & 1) && !mbar_wait(&kv_full[kb], (t >> 1) & 1)) { B3_FAIL(); return; }
         if (!mbar_wait(&st_full[st], (n / B3_NS) & 1)) { B3_FAIL(); return; }
         if (n >= 1 && !mbar_wait(s_free, (n - 1) & 1)) { B3_FAIL(); return; }
         fence_after_sync();
         const uint64_t kd = k_kk0 + (uint64_t)((kb * 2 * T128) >> 4), qd = q_kk0 + (uint64_t)((st * 2 * T128) >> 4);
+        const uint64_t ext = ext0 + (uint64_t)((st * B3_EXT) >> 4);
         if (elect_one()) {
+          umma_ss<KIND_F16>(tS, one0, ext, IDESC_S_128x128, 0u);                       // -lse / scale in every row
 #pragma unroll
-          for (int ks = 0; ks < HS / 16; ++ks) umma_ss<KIND_F16>(tS, kd + 2 * ks, qd + 2 * ks, IDESC_S_128x128, ks > 0 ? 1u : 0u);
+          for (int ks = 0; ks < HS / 16; ++ks) umma_ss<KIND_F16>(tS, kd + 2 * ks, qd + 2 * ks, IDESC_S_128x128, 1u);
+          umma_ss<KIND_F16>(tDP, one0 + (B3_ONE >> 4), ext, IDESC_S_128x128, 0u);      // -D
+#pragma unroll
+          for (int ks = 0; ks < HS / 16; ++ks) umma_ss<KIND_F16>(tDP, kd + (T128 >> 4) + 2 * ks, qd + (T128 >> 4) + 2 * ks, IDESC_S_128x128, 1u);
           umma_commit(s_full);
         }
         __syncwarp();
       };
-      auto scores_dp = [&]() {                                                        // dP^T of block nx, then nx moves on
-        const int n = nx.n, st = n % B3_NS, kb = nx.c.t & 1;
-        if (n >= 1 && !mbar_wait(dp_free, (n - 1) & 1)) { B3_FAIL(); return; }
+      auto products = [&](int n, int what) {                                          // dV += P^T dO, dK += dS^T Q, dQ = dS K of block n
+        const int st = n % B3_NS, t = what >> 2, kb = t & 1;
+        const bool first = what & 1, last = what & 2;
+        if (!mbar_wait(p_full, n & 1)) { B3_FAIL(); return; }
+        if (first && t >= 1 && !mbar_wait(acc_free, (t - 1) & 1)) { B3_FAIL(); return; }
         fence_after_sync();
-        const uint64_t vd = k_kk0 + (uint64_t)((kb * 2 * T128 + T128) >> 4), dod = q_kk0 + (uint64_t)((st * 2 * T128 + T128) >> 4);
-        if (elect_one()) {
-#pragma unroll
-          for (int ks = 0; ks < HS / 16; ++ks) umma_ss<KIND_F16>(tDP, vd + 2 * ks, dod + 2 * ks, IDESC_S_128x128, ks > 0 ? 1u : 0u);
-          umma_commit(dp_full);
-        }
-        __syncwarp();
-        blk3_next(nx, n_t, n_items);
-      };
-      if (!nx.c.done) { scores_s(); if (!failed) scores_dp(); }                       // block 0
-      while (!it.c.done && !failed) {
-        const int n = it.n, st = n % B3_NS, kb = it.c.t & 1;
-        const bool first = it.ib == 0, last = it.ib + 1 == it.nbt;
-        if (!nx.c.done) { scores_s(); if (failed) break; }                            // waits for s_free(n)
-        if (!mbar_wait(p_full, n & 1)) { B3_FAIL(); break; }
-        if (first && it.c.t >= 1 && !mbar_wait(acc_free, (it.c.t - 1) & 1)) { B3_FAIL(); break; }
-        fence_after_sync();
-        const uint64_t do_mn = q_mn0 + (uint64_t)((st * 2 * T128 + T128) >> 4), q_mn = q_mn0 + (uint64_t)((st * 2 * T128) >> 4);
-        if (elect_one()) {
-#pragma unroll
-          for (int ks = 0; ks < TILE / 16; ++ks) umma_ts(tDV, tP + ks * 8, do_mn + 128 * ks, IDESC_TS_MN, (ks > 0 || !first) ? 1u : 0u);   // dV += P^T dO
-          umma_commit(p_used);                                                        // the compute warps may write P^T(n+1)
-        }
-        __syncwarp();
-        if (!nx.c.done) { scores_dp(); if (failed) break; }                           // waits for dp_free(n)
-        if (!mbar_wait(ds_full, n & 1)) { B3_FAIL(); break; }
-        if (n >= 1 && !mbar_wait(dq_free, (n - 1) & 1)) { B3_FAIL(); break; }
-        fence_after_sync();
+        const uint64_t q_mn = q_mn0 + (uint64_t)((st * 2 * T128) >> 4), do_mn = q_mn + (T128 >> 4);
         const uint64_t kmn = k_mn0 + (uint64_t)((kb * 2 * T128) >> 4);
         if (elect_one()) {
 #pragma unroll
-          for (int ks = 0; ks < TILE / 16; ++ks)                                                                                          // dK += dS^T Q
+          for (int ks = 0; ks < TILE / 16; ++ks) umma_ts(tDV, tP + ks * 8, do_mn + 128 * ks, IDESC_TS_MN, (ks > 0 || !first) ? 1u : 0u);
+#pragma unroll
+          for (int ks = 0; ks < TILE / 16; ++ks)
             umma_ss<KIND_F16>(tDK, ds_kk + (ks < 4 ? 2 * ks : (T128 >> 4) + 2 * (ks - 4)), q_mn + 128 * ks, IDESC_TS_MN, (ks > 0 || !first) ? 1u : 0u);
 #pragma unroll
-          for (int ks = 0; ks < TILE / 16; ++ks) umma_ss<KIND_F16>(tDQ, ds_mn + 128 * ks, kmn + 128 * ks, IDESC_MN_MN, ks > 0 ? 1u : 0u);  // dQ = dS K
+          for (int ks = 0; ks < TILE / 16; ++ks) umma_ss<KIND_F16>(tDQ, ds_mn + 128 * ks, kmn + 128 * ks, IDESC_MN_MN, ks > 0 ? 1u : 0u);
           umma_commit(dq_full);
           umma_commit(ds_free);
           umma_commit(&st_empty[st]);
           if (last) { umma_commit(acc_full); umma_commit(&kv_empty[kb]); }
         }
         __syncwarp();
-        blk3_next(it, n_t, n_items);
+      };
+      for (Blk3 it = blk3_begin(n_t, n_items); !it.c.done && !failed; blk3_next(it, n_t, n_items)) {
+        if (warp == 13) scores(it.n, info(it)); else products(it.n, info(it));
+      }
+    } else {
+      // ------------------------------------------------------------ warp 15: dV, then dK of every tile from the staging tile to memory
+      Tile3 c{(int)blockIdx.x, 0, 0, 0, 0, false, false};
+      for (tile3_seek(c, n_t, n_items); !c.done && !failed; tile3_next(c, n_t - c.tile, n_t, n_items)) {
+        const int b = c.bh / p.NH, h = c.bh % p.NH, k0 = c.tile * TILE;
+        for (int mat = 0; mat < 2 && !failed; ++mat) {
+          if (!mbar_wait_sleep(ep_ready, mat)) { B3_FAIL(); break; }                   // two phases a tile
+          if (elect_one()) {
+            const int col = (mat ? 1 : 2) * p.C + h * HS;
+            tma_store_3d(&tmOUT, sEP, col, k0, b);
+            tma_store_3d(&tmOUT, sEP + T64, col, k0 + 64, b);
+            bulk_commit();
+            bulk_wait_read<0>();
+            mbar_arrive(ep_free);
+          }
+          __syncwarp();
+        }
       }
     }
   } else if (warp >= 8) {
@@ -305,34 +332,35 @@ __global__ void __launch_bounds__(B3_THREADS, 1) attn_bwd3_kernel(const __grid_c
     asm volatile("setmaxnreg.dec.sync.aligned.u32 80;");
     const int row = (warp & 3) * 32 + lane;
     const uint32_t lane_addr = (uint32_t)((warp & 3) * 32) << 16;
-    int ne = 0;                                             // epilogue rounds so far
+    int ne = 0;                                             // staging tiles written so far
+    if (lane == 0) mbar_arrive(p_full);                     // nothing to drain before the first block's dQ
     for (Blk3 it = blk3_begin(n_t, n_items); !it.c.done && !failed; blk3_next(it, n_t, n_items)) {
       const int n = it.n, i = it.c.tile + it.ib;
       if (!mbar_wait_sleep(dq_full, n & 1)) { B3_FAIL(); break; }
       fence_after_sync();
       float* dst = p.dq_acc + ((size_t)it.c.bh * n_t + i) * (TILE * HS) + row * 4;
-#pragma unroll 1
-      for (int half = 0; half < 2; ++half) {
-        uint32_t r[32];
-        tmem_ld32(tDQ + lane_addr + half * 32, r);
-        tmem_wait_ld();
-        if (half == 1) {
-          fence_before_sync();
-          __syncwarp();
-          if (lane == 0) mbar_arrive(dq_free);
-        }
+      uint32_t r0[32], r1[32];
+      tmem_ld32(tDQ + lane_addr, r0); tmem_ld32(tDQ + lane_addr + 32, r1);
+      tmem_wait_ld();
+      fence_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(p_full);
+      // Sixteen reductions at a stretch keep the load / store pipe busy for 1400 cycles, and the commit that starts them also lets the compute
+      // warps store dS^T(n+1), which then took 1000 cycles instead of 250.  So they go out two at a time, with a pause, inside a tile.
 #pragma unroll
-        for (int c = 0; c < 8; ++c)
-          red_add_v4(dst + (half * 8 + c) * (TILE * 4), __uint_as_float(r[4 * c]), __uint_as_float(r[4 * c + 1]), __uint_as_float(r[4 * c + 2]),
-                     __uint_as_float(r[4 * c + 3]));
+      for (int c = 0; c < 16; ++c) {
+        const uint32_t (&r)[32] = c < 8 ? r0 : r1;
+        red_add_v4(dst + c * (TILE * 4), __uint_as_float(r[4 * (c & 7)]), __uint_as_float(r[4 * (c & 7) + 1]), __uint_as_float(r[4 * (c & 7) + 2]),
+                   __uint_as_float(r[4 * (c & 7) + 3]));
+        if (c % 2 == 1 && it.ib + 1 < it.nbt) __nanosleep(B3_PACE_NS);
       }
       if (it.ib + 1 < it.nbt) continue;
-      // The tile's dV and dK: rounded rows go through a swizzled staging tile and leave as TMA stores (whole 128-byte
-      // rows; rows beyond T are clipped by the tensor map).  Per-thread stores of 16 bytes at a row stride of 3C would
-      // keep this warpgroup busy for longer than a whole block takes.
+      // The tile's dV and dK: rounded rows go through a swizzled staging tile and leave as TMA stores that warp 15 issues (whole 128-byte
+      // rows; rows beyond T are clipped by the tensor map).  Per-thread stores of 16 bytes at a row stride of 3C would keep this
+      // warpgroup busy for longer than a whole block takes.
       if (!mbar_wait_sleep(acc_full, it.c.t & 1)) { B3_FAIL(); break; }
       fence_after_sync();
-      const int b = it.c.bh / p.NH, h = it.c.bh % p.NH, k0 = it.c.tile * TILE, kj = k0 + row;
+      const int h = it.c.bh % p.NH, kj = it.c.tile * TILE + row;
 #pragma unroll 1
       for (int mat = 0; mat < 2; ++mat) {                   // 0: dV, 1: dK
         const float sc = mat ? p.scale : 1.0f;              // dS^T was stored without the 1/sqrt(HS) factor
@@ -349,28 +377,23 @@ __global__ void __launch_bounds__(B3_THREADS, 1) attn_bwd3_kernel(const __grid_c
           float v[32];
 #pragma unroll
           for (int x = 0; x < 32; ++x) v[x] = kj < p.T ? __uint_as_float(r[x]) * sc : 0.f;
-          store_row32(sEP, row, half * 32, v);
+          uint4 q[4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            q[j] = make_uint4(pack_bf16x2(v[8 * j], v[8 * j + 1]), pack_bf16x2(v[8 * j + 2], v[8 * j + 3]),
+                                         pack_bf16x2(v[8 * j + 4], v[8 * j + 5]), pack_bf16x2(v[8 * j + 6], v[8 * j + 7]));
           if (p.dbias) {                                    // qkv bias gradient, dK and dV parts: column sums of this warp's 32 rows
             const float cs = warp_colsum32(v, lane);
             atomicAdd(p.dbias + (mat ? 1 : 2) * p.C + h * HS + half * 32 + lane, cs);
           }
+          if (half == 0 && ne >= 1 && !mbar_wait_sleep(ep_free, (ne - 1) & 1)) { B3_FAIL(); break; }   // the stores before have read the tile
+#pragma unroll
+          for (int j = 0; j < 4; ++j) *reinterpret_cast<uint4*>(sEP + sw128(row, half * 4 + j)) = q[j];
         }
+        if (failed) break;
         fence_proxy_async();
         __syncwarp();
         if (lane == 0) mbar_arrive(ep_ready);
-        if (warp == 8) {
-          if (!mbar_wait_sleep(ep_ready, ne & 1)) { B3_FAIL(); break; }
-          if (elect_one()) {
-            const int col = (mat ? 1 : 2) * p.C + h * HS;
-            tma_store_3d(&tmOUT, sEP, col, k0, b);
-            tma_store_3d(&tmOUT, sEP + T64, col, k0 + 64, b);
-            bulk_commit();
-            bulk_wait_read<0>();
-            mbar_arrive(ep_done);
-          }
-          __syncwarp();
-        }
-        if (!mbar_wait_sleep(ep_done, ne & 1)) { B3_FAIL(); break; }      // the staging tile may be rewritten
         ++ne;
       }
     }
@@ -383,86 +406,61 @@ __global__ void __launch_bounds__(B3_THREADS, 1) attn_bwd3_kernel(const __grid_c
     const uint32_t tSh = tS + lane_addr + hq * 64, tDPh = tDP + lane_addr + hq * 64, tPh = tP + lane_addr + hq * 32;
     const float2 sc2 = make_float2(p.scale_log2, p.scale_log2);
     for (Blk3 it = blk3_begin(n_t, n_items); !it.c.done && !failed; blk3_next(it, n_t, n_items)) {
-      const int n = it.n, st = n % B3_NS;
-      const float* stat = sStat + st * 256 + hq * 64;
-      if (!mbar_wait_sleep(&st_full[st], (n / B3_NS) & 1)) { B3_FAIL(); break; }      // acquire the block's row statistics
+      const int n = it.n;
       if (!mbar_wait_sleep(s_full, n & 1)) { B3_FAIL(); break; }
       fence_after_sync();
-      uint32_t s[64];
+      uint32_t s[64], d[64];
       {
-        uint32_t (&q0)[32] = *reinterpret_cast<uint32_t (*)[32]>(&s[0]);
-        uint32_t (&q1)[32] = *reinterpret_cast<uint32_t (*)[32]>(&s[32]);
-        tmem_ld32(tSh, q0); tmem_ld32(tSh + 32, q1);
+        uint32_t (&s0)[32] = *reinterpret_cast<uint32_t (*)[32]>(&s[0]);
+        uint32_t (&s1)[32] = *reinterpret_cast<uint32_t (*)[32]>(&s[32]);
+        uint32_t (&d0)[32] = *reinterpret_cast<uint32_t (*)[32]>(&d[0]);
+        uint32_t (&d1)[32] = *reinterpret_cast<uint32_t (*)[32]>(&d[32]);
+        tmem_ld32(tSh, s0); tmem_ld32(tDPh, d0); tmem_ld32(tSh + 32, s1); tmem_ld32(tDPh + 32, d1);
       }
       tmem_wait_ld();
       fence_before_sync();
       __syncwarp();
-      if (lane == 0) mbar_arrive(s_free);                   // S^T(n+1) may be issued now
+      if (lane == 0) mbar_arrive(s_free);              // the scores of block n+1 may be issued now
+      uint32_t pk[32], dk[32];
       {
-        uint32_t pk[32];
-        const float4* nl4 = reinterpret_cast<const float4*>(stat);
-        auto p_phase = [&](auto diag) {
+        auto work = [&](auto diag) {
           const int lim = row - hq * 64;                    // diagonal block: local query columns x < lim see nothing of this key
+          auto exps = [&](int c) {
 #pragma unroll
-          for (int x = 0; x < 16; ++x) {
-            const float4 l = nl4[x];
-            const float2 t01 = __ffma2_rn(make_float2(__uint_as_float(s[4 * x]), __uint_as_float(s[4 * x + 1])), sc2, make_float2(l.x, l.y));
-            const float2 t23 = __ffma2_rn(make_float2(__uint_as_float(s[4 * x + 2]), __uint_as_float(s[4 * x + 3])), sc2, make_float2(l.z, l.w));
-            float e0 = ex2_approx(t01.x), e1 = ex2_approx(t01.y), e2 = ex2_approx(t23.x), e3 = ex2_approx(t23.y);
-            if (decltype(diag)::value) {
-              e0 = 4 * x < lim ? 0.f : e0; e1 = 4 * x + 1 < lim ? 0.f : e1;
-              e2 = 4 * x + 2 < lim ? 0.f : e2; e3 = 4 * x + 3 < lim ? 0.f : e3;
+            for (int k = 0; k < 8; k += 2) {
+              const float2 t = __fmul2_rn(make_float2(__uint_as_float(s[8 * c + k]), __uint_as_float(s[8 * c + k + 1])), sc2);
+              float e0 = ex2_approx(t.x), e1 = ex2_approx(t.y);
+              if (decltype(diag)::value) { e0 = 8 * c + k < lim ? 0.f : e0; e1 = 8 * c + k + 1 < lim ? 0.f : e1; }
+              s[8 * c + k] = __float_as_uint(e0); s[8 * c + k + 1] = __float_as_uint(e1);
             }
-            s[4 * x] = __float_as_uint(e0); s[4 * x + 1] = __float_as_uint(e1);
-            s[4 * x + 2] = __float_as_uint(e2); s[4 * x + 3] = __float_as_uint(e3);
-            pk[2 * x] = pack_bf16x2(e0, e1); pk[2 * x + 1] = pack_bf16x2(e2, e3);
+          };
+          exps(0);
+#pragma unroll
+          for (int c = 0; c < 8; ++c) {                     // a chunk's products beside the next chunk's exponentials
+            if (c + 1 < 8) exps(c + 1);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+              const float2 e = make_float2(__uint_as_float(s[8 * c + 2 * k]), __uint_as_float(s[8 * c + 2 * k + 1]));
+              const float2 r = __fmul2_rn(e, make_float2(__uint_as_float(d[8 * c + 2 * k]), __uint_as_float(d[8 * c + 2 * k + 1])));
+              pk[4 * c + k] = pack_bf16x2(e.x, e.y); dk[4 * c + k] = pack_bf16x2(r.x, r.y);
+            }
           }
         };
-        if (it.ib == 0) p_phase(std::true_type{}); else p_phase(std::false_type{});
-        if (n >= 1 && !mbar_wait_sleep(p_used, (n - 1) & 1)) { B3_FAIL(); break; }   // dV has read P^T(n-1)
-        fence_after_sync();
-        tmem_st32(tPh, pk);
+        if (it.ib == 0) work(std::true_type{}); else work(std::false_type{});
+#pragma unroll
+        for (int j = 0; j < 32; ++j) asm volatile("" : "+r"(pk[j]), "+r"(dk[j]));        // packed before the wait, not after it
       }
+      if (n >= 1 && !mbar_wait_sleep(ds_free, (n - 1) & 1)) { B3_FAIL(); break; }   // the products of block n-1 have read P^T and dS^T
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        *reinterpret_cast<uint4*>(sDS + hq * T128 + sw128(row, j)) = make_uint4(dk[4 * j], dk[4 * j + 1], dk[4 * j + 2], dk[4 * j + 3]);
+      fence_after_sync();
+      tmem_st32(tPh, pk);
+      fence_proxy_async();
       tmem_wait_st();
       fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive(p_full);
-      if (!mbar_wait_sleep(dp_full, n & 1)) { B3_FAIL(); break; }
-      fence_after_sync();
-      uint32_t d[64];
-      {
-        uint32_t (&q0)[32] = *reinterpret_cast<uint32_t (*)[32]>(&d[0]);
-        uint32_t (&q1)[32] = *reinterpret_cast<uint32_t (*)[32]>(&d[32]);
-        tmem_ld32(tDPh, q0); tmem_ld32(tDPh + 32, q1);
-      }
-      tmem_wait_ld();
-      fence_before_sync();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(dp_free);                  // dP^T(n+1) may be issued now
-      {
-        const float4* nd4 = reinterpret_cast<const float4*>(stat + 128);
-#pragma unroll
-        for (int x = 0; x < 16; ++x) {
-          const float4 nd = nd4[x];
-          const float2 a01 = __fadd2_rn(make_float2(__uint_as_float(d[4 * x]), __uint_as_float(d[4 * x + 1])), make_float2(nd.x, nd.y));
-          const float2 a23 = __fadd2_rn(make_float2(__uint_as_float(d[4 * x + 2]), __uint_as_float(d[4 * x + 3])), make_float2(nd.z, nd.w));
-          const float2 r01 = __fmul2_rn(make_float2(__uint_as_float(s[4 * x]), __uint_as_float(s[4 * x + 1])), a01);
-          const float2 r23 = __fmul2_rn(make_float2(__uint_as_float(s[4 * x + 2]), __uint_as_float(s[4 * x + 3])), a23);
-          s[4 * x] = __float_as_uint(r01.x); s[4 * x + 1] = __float_as_uint(r01.y);
-          s[4 * x + 2] = __float_as_uint(r23.x); s[4 * x + 3] = __float_as_uint(r23.y);
-        }
-      }
-      if (n >= 1 && !mbar_wait_sleep(ds_free, (n - 1) & 1)) { B3_FAIL(); break; }   // dK and dQ of block n-1 have read the tile
-      {
-        const float (&v0)[32] = *reinterpret_cast<const float (*)[32]>(&s[0]);
-        const float (&v1)[32] = *reinterpret_cast<const float (*)[32]>(&s[32]);
-        store_row32(sDS + hq * T128, row, 0, v0);
-        store_row32(sDS + hq * T128, row, 32, v1);
-      }
-      fence_proxy_async();
-      fence_before_sync();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(ds_full);
     }
   }
   fence_before_sync();
@@ -521,7 +519,7 @@ __global__ void __launch_bounds__(128) attn_bwd3_dq_kernel(__nv_bfloat16* __rest
 }  // namespace
 
 // Sizes (in floats) of the two scratch buffers of llmb_attention_bwd_fused.
-LLMB_API long long llmb_attention_bwd_fused_stats_floats(int B, int T, int NH) { return (long long)B * NH * ceil_div(T, TILE) * 256; }
+LLMB_API long long llmb_attention_bwd_fused_stats_floats(int B, int T, int NH) { return (long long)B * NH * ceil_div(T, TILE) * (B3_EXT / 4); }
 LLMB_API long long llmb_attention_bwd_fused_acc_floats(int B, int T, int NH) { return (long long)B * NH * ceil_div(T, TILE) * (TILE * HS); }
 
 // dqkv [B,T,3C] bf16 (fully overwritten) from dout [B,T,C], qkv [B,T,3C], out [B,T,C] (bf16) and the forward's lse [B,NH,T]
@@ -536,7 +534,10 @@ LLMB_API int llmb_attention_bwd_fused(void* dqkv, float* dbias, float* stats, fl
   rc = make_qkv_map(&td, dout, B, T, C); if (rc) return 1000 + rc;
   CUtensorMap to;
   rc = make_qkv_map(&to, dqkv, B, T, 3 * C); if (rc) return 1000 + rc;
-  B3Params p{}; p.dqkv = dqkv; p.stats = stats; p.dq_acc = dq_acc; p.dbias = dbias;
+  CUtensorMap tx;
+  rc = make_tmap_2d(&tx, stats, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)B * NH * ceil_div(T, TILE) * TILE, 16, 16, TILE, 16, CU_TENSOR_MAP_SWIZZLE_32B);
+  if (rc) return 1000 + rc;
+  B3Params p{}; p.dqkv = dqkv; p.dq_acc = dq_acc; p.dbias = dbias;
   p.B = B; p.T = T; p.NH = NH; p.C = C; p.scale = 0.125f; p.scale_log2 = 0.125f * 1.4426950408889634f; p.status = status;
   static bool attr = false;
   if (!attr) {
@@ -545,10 +546,11 @@ LLMB_API int llmb_attention_bwd_fused(void* dqkv, float* dbias, float* stats, fl
   }
   const int n_t = ceil_div(T, TILE);
   const long long rows = (long long)B * NH * n_t * TILE;
-  launch_pdl(attn_bwd3_prep_kernel, (unsigned)ceil_div_ll(rows * 8, 256), 256, 0, st, stats, lse, (const __nv_bfloat16*)dout, (const __nv_bfloat16*)out, B, T, NH, C);
+  launch_pdl(attn_bwd3_prep_kernel, (unsigned)ceil_div_ll(rows * 8, 256), 256, 0, st, (uint4*)stats, lse, (const __nv_bfloat16*)dout, (const __nv_bfloat16*)out, B, T, NH, C,
+             1.0f / p.scale_log2);
   const long long n_items = (long long)((n_t + 1) / 2) * B * NH;
   const int grid = (int)(n_items < sm_count() ? n_items : sm_count());          // persistent: one CTA per SM
-  launch_pdl(attn_bwd3_kernel, grid, B3_THREADS, B3_SMEM, st, tq, td, to, p);
+  launch_pdl(attn_bwd3_kernel, grid, B3_THREADS, B3_SMEM, st, tq, td, to, tx, p);
   launch_pdl(attn_bwd3_dq_kernel, (unsigned)(B * NH * n_t), 128, 0, st, (__nv_bfloat16*)dqkv, dbias, dq_acc, T, NH, C, p.scale);
   return (int)cudaGetLastError();
 }

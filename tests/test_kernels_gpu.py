@@ -385,6 +385,32 @@ def test_unfused_softmax_bwd_and_crossentropy():
     close(ops.softmax_bwd(dprobs, probs, V), ops.softmax_bwd(dprobs_c, probs_c, V), 1e-5, 1e-4, "softmax bwd", strict=True)
 
 
+@pytest.mark.parametrize("B,T,NH,scale", [(40, 100, 12, 1.0), (41, 128, 12, 1.0), (30, 200, 12, 1.0), (20, 300, 12, 1.0), (13, 520, 8, 1.0), (3, 129, 2, 6.0),
+                                          (5, 1024, 4, 4.0)])
+def test_fused_attention_backward_walks_short_tiles_and_large_statistics(B, T, NH, scale):
+    """CTAs that walk several items of one block (K and V buffers handed on block by block), of two and three tiles (a middle tile alone),
+    rows beyond T in every item; scores so large that the log-sum-exp, which reaches the products in three bf16 parts, is hundreds.
+    Oracle: the op with autograd in fp64.  Tolerance: P and dS are rounded to bf16 (2^-9 of a row's largest, relative to a column of up to
+    T of them) as are the inputs' gradients; the norm of the error stays below 2^-7 of the norm.  With large scores also D = sum(dO * O) counts, taken
+    from the rounded output: 2^-9 of |dP| in rows whose one probability near 1 leaves dP - D as the difference of nearly equal numbers; twice the
+    bound covers a dS half the size of dP."""
+    C, tol = NH * 64, 2 ** -7 if scale == 1.0 else 2 ** -6
+    qkv, dout = rnd(B, T, 3 * C, scale=scale).to(DEV), rnd(B, T, C, seed=1).to(DEV)
+    leaf = qkv.double().requires_grad_(True)
+    q, k, v = (t.view(B, T, NH, 64).transpose(1, 2) for t in leaf.split(C, dim=2))
+    sc = (q @ k.transpose(-1, -2) / 8.0).masked_fill(~torch.ones(T, T, dtype=torch.bool, device=DEV).tril(), float("-inf"))
+    r_out = (torch.softmax(sc, dim=-1) @ v).transpose(1, 2).reshape(B, T, C)
+    r_lse = (torch.logsumexp(sc, dim=-1) * math.log2(math.e)).float().detach().contiguous()
+    r_out.backward(dout.double())
+    dqkv = torch.full((B, T, 3 * C), float("nan"), dtype=torch.bfloat16, device=DEV)
+    ops.attention_bwd(dqkv, dout, qkv, r_out.detach().bfloat16(), r_lse, NH)
+    torch.cuda.synchronize()
+    status_ok()
+    for i, nm in enumerate(("dq", "dk", "dv")):
+        got, want = dqkv[..., i * C:(i + 1) * C].double(), leaf.grad[..., i * C:(i + 1) * C]
+        assert ((got - want).norm() / want.norm()).item() < tol, nm
+
+
 @pytest.mark.parametrize("bwd", ["fused", "split"])
 def test_attention_persistent_loops_large(bwd, monkeypatch):
     """B=16, NH=12, T=1024: 768 work items on at most 148 CTAs, so every persistent CTA walks several items per

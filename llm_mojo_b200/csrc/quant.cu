@@ -693,8 +693,8 @@ __device__ __forceinline__ unsigned block_umax(unsigned m, unsigned* red) {     
   return m;
 }
 
-// partial[0 .. gridDim): raw bits of max|x| (NaN sorts above infinity); partial[NVA_GRID .. +gridDim): of the transform along the rows
-template <bool PLAIN, bool RHT>
+// partial[0 .. gridDim): raw bits of max|x| (NaN sorts above infinity), with PLAIN; partial[NVA_GRID .. +gridDim): of the transform along the rows
+template <bool PLAIN>
 __global__ void __launch_bounds__(256) nvfp4_amax_kernel(unsigned* __restrict__ partial, const __nv_bfloat16* __restrict__ x, int rows, int cols) {
   pdl_trigger();
   pdl_wait();
@@ -716,20 +716,44 @@ __global__ void __launch_bounds__(256) nvfp4_amax_kernel(unsigned* __restrict__ 
         m0 = __vmaxu2(m0, t);
       }
     }
-    if (RHT) {
 #pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        float2 b[16];
+    for (int half = 0; half < 2; ++half) {
+      float2 b[16];
 #pragma unroll
-        for (int k = 0; k < 16; ++k) b[k] = bf16x2_f(half ? u[k].y : u[k].x);
-        rht16x2(b);
+      for (int k = 0; k < 16; ++k) b[k] = bf16x2_f(half ? u[k].y : u[k].x);
+      rht16x2(b);
 #pragma unroll
-        for (int k = 0; k < 16; ++k) m1 = max(m1, max(__float_as_uint(b[k].x) & 0x7fffffffu, __float_as_uint(b[k].y) & 0x7fffffffu));
-      }
+      for (int k = 0; k < 16; ++k) m1 = max(m1, max(__float_as_uint(b[k].x) & 0x7fffffffu, __float_as_uint(b[k].y) & 0x7fffffffu));
     }
   }
   if (PLAIN) { const unsigned m = block_umax(max(m0 & 0xffffu, m0 >> 16) << 16, red); if (threadIdx.x == 0) partial[blockIdx.x] = m; }
-  if (RHT) { const unsigned m = block_umax(m1, red); if (threadIdx.x == 0) partial[NVA_GRID + blockIdx.x] = m; }
+  const unsigned m = block_umax(m1, red);
+  if (threadIdx.x == 0) partial[NVA_GRID + blockIdx.x] = m;
+}
+
+// max|x| alone needs no rows: 16-byte loads, four in flight per thread, on packed pairs (a training step with NVFP4, 48 layers of C 1600 on
+// 4 x 1024 tokens, takes 264 of these: 55.96 -> 55.66 ms against the kernel above, which walks the tiles).
+__global__ void __launch_bounds__(256) nvfp4_amax_flat_kernel(unsigned* __restrict__ partial, const uint4* __restrict__ x, long long nvec) {
+  pdl_trigger();
+  pdl_wait();
+  __shared__ unsigned red[8];
+  constexpr int U = 4;
+  unsigned m = 0;
+  const long long stride = (long long)gridDim.x * 256;
+  auto take = [&](const uint4& u) {                       // 16-bit magnitudes order like the values
+    m = __vmaxu2(m, __vmaxu2(__vmaxu2(u.x & 0x7fff7fffu, u.y & 0x7fff7fffu), __vmaxu2(u.z & 0x7fff7fffu, u.w & 0x7fff7fffu)));
+  };
+  long long i = (long long)blockIdx.x * 256 + threadIdx.x;
+  for (; i + (U - 1) * stride < nvec; i += U * stride) {
+    uint4 u[U];
+#pragma unroll
+    for (int k = 0; k < U; ++k) u[k] = x[i + k * stride];
+#pragma unroll
+    for (int k = 0; k < U; ++k) take(u[k]);
+  }
+  for (; i < nvec; i += stride) take(x[i]);
+  m = block_umax(max(m & 0xffffu, m >> 16) << 16, red);
+  if (threadIdx.x == 0) partial[blockIdx.x] = m;
 }
 
 struct NvAlpha { float* out; const float* other; float factor; };       // *out = factor * this operand's tensor scale * *other
@@ -913,9 +937,9 @@ LLMB_API int llmb_nvfp4_operand(void* q0, void* sf0, void* q1, void* sf1, float*
   p.alpha0 = {alpha_other0 ? ws + 2 : nullptr, alpha_other0, factor0};
   p.alpha1 = {alpha_other1 ? ws + 3 : nullptr, alpha_other1, factor1};
   unsigned* part = reinterpret_cast<unsigned*>(ws + 4);
-  int rc = plain && tr ? launch_pdl(nvfp4_amax_kernel<true, true>, p.nparts, 256, 0, st, part, p.x, rows, cols)
-           : plain     ? launch_pdl(nvfp4_amax_kernel<true, false>, p.nparts, 256, 0, st, part, p.x, rows, cols)
-                       : launch_pdl(nvfp4_amax_kernel<false, true>, p.nparts, 256, 0, st, part, p.x, rows, cols);
+  int rc = plain && tr ? launch_pdl(nvfp4_amax_kernel<true>, p.nparts, 256, 0, st, part, p.x, rows, cols)
+           : plain     ? launch_pdl(nvfp4_amax_flat_kernel, p.nparts, 256, 0, st, part, (const uint4*)x, (long long)rows * cols / 8)
+                       : launch_pdl(nvfp4_amax_kernel<false>, p.nparts, 256, 0, st, part, p.x, rows, cols);
   if (rc) return rc;
   const long long tiles = (long long)ceil_div(rows, 128) * ceil_div(cols, 128);
   if (tiles > 0x7fffffffLL) return LLMB_ERR_BAD_ARG;

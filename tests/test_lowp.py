@@ -616,6 +616,21 @@ def test_block_scaled_gemm_tiles_and_epilogues(kind, M, N, K):
 
 
 @gpu
+@pytest.mark.parametrize("rows,cols", [(16, 16), (16, 48), (128, 4096 + 16), (4096, 1600), (2064, 4112)])
+def test_nvfp4_operand_tensor_scale_finds_the_maximum_anywhere(rows, cols):
+    """One vector, less than a CTA, and whole and ragged rounds of the unrolled loop: the maximum as the first, last, middle and a late
+    value, of either sign and either half of a packed pair, gives exactly the tensor scale max|x| / (448 * 6) in fp32."""
+    n = rows * cols
+    x = (torch.rand(rows, cols, generator=torch.Generator().manual_seed(rows)) - 0.5).bfloat16().cuda()
+    want = torch.tensor(37.5, device="cuda") / torch.tensor(448.0 * 6.0, device="cuda")
+    for at, v in ((0, 37.5), (n - 1, -37.5), (n // 2, -37.5), (n - 8, 37.5), (n - n // 3, 37.5)):
+        y = x.clone()
+        y.view(-1)[at] = v
+        op = lowp.Fp4Operand(y, True, False)
+        assert torch.equal(op.buf[:4].view(torch.float32)[0], want), at
+
+
+@gpu
 def test_fp8_block_linear_native_matches_fake_quant_path(monkeypatch):
     rows, C, OC = 512, 256, 384
     g = torch.Generator().manual_seed(4)

@@ -33,26 +33,28 @@ bool pair_mode() {
 struct Tile { int bn, cl, splits; };
 thread_local int g_force_bn = 0, g_force_cl = 1;          // test hook (llmb_gemm_force_tile): 0 = the rule decides
 
-// The configuration with the smallest estimated time, in microseconds on a B200: a fixed part (launch, set-up, epilogue) plus a cost per
-// 128-byte k-block, the same for operands stored along K or along the rows; more 128-row CTAs than SMs run side by side at the cost of each
-// other's k-blocks; a further round of pair tiles costs its epilogue if that is longer than its k-loop.  Clusters only while they fit in
-// one round: beyond it they were 1.5 - 4 times slower than one CTA per tile.  The constants are a fit over every configuration forced on
-// the twelve products of a layer, 13 sizes in bf16 (M 64 ... 12288, C 384 ... 1600) and 6 in TF32 (launches from a graph); the rule is then 0.7 %
-// slower than the best configuration on average, at worst 15 % (M 512, C 768, K 3072, input gradient: 64 x 2 CTAs 10.0, 64 x 4 8.8 us).
-// With a surcharge on operands stored along the rows, from when their loads had one, it was 1.9 % and up to 44 %: TF32 M 1024, C 768, N 3072
-// with GELU 31.8 / 22.0; bf16 M 8192, C 384 C x C input gradient 7.2 / 5.9, M 2048, K 3072 18.3 / 15.8, M 1024 weight gradient 10.3 / 9.0.
-// From M 4096 on the pair kernel is the fastest but for C x C at C up to 768.
+// The configuration with the smallest estimated time, in microseconds on a B200 from linear fits over M = 64 ... 5439, K and N =
+// 384 ... 5120 (the fits are within 15 %; the small kernel must win by 5 %): a fixed part (launch, set-up, epilogue) plus a cost per
+// 128-byte k-block, bounded by what one SM can fetch (24 / 32 KB per k-block) in the small kernel and by the 256-row MMAs in the pair
+// kernel; MN-major operands cost more per k-block; more CTAs than SMs run side by side at the cost of each other's k-blocks; a
+// further round of pair tiles costs its epilogue if that is longer than its k-loop.  Clusters only while they fit in one round:
+// beyond it they were 1.5 - 4 times slower than one CTA per tile.  Measured, bias + residual: M 64, K 3072, N 768: pair 22.4 us,
+// 128 x 128 17.8, 64 x 4 CTAs 8.7; M 776, K 1024, N 1024: 14.3 / 10.7 / (64 x 1) 8.8; M 4096, K 768, N 3072: 27.1 / 50.6 / 44.8.
+// Beyond the fits, every configuration forced on the seven products of a layer at M up to 16384 and C 768, 1024, 1600: from M 4096 on the
+// pair kernel is the fastest but for two products (M 5439, C 1600, input gradients: 128 x 128 11 - 13 % less) and the rule takes it;
+// elsewhere it is off by 10 - 19 % at three of the 42 products below that (M 776: C x C at C 1600 17.0 against 14.3 us).
 // splits: parts of K in the pair kernel; most: the most that this kernel's CTAs may cut it into.
-Tile pick_tile(int kind, int epi, int M, int N, int kb_total, int splits, int most) {
+Tile pick_tile(int kind, int epi, int M, int N, int kb_total, int splits, int most, int a_mn, int b_mn) {
   if (g_force_bn) return {kind == KIND_F8F6F4 && g_force_bn == 64 ? 128 : g_force_bn, g_force_cl, splits};
   if (!pair_mode()) return {128, 1, splits};
   const bool aux = epi == EPI_BIAS_GELU || epi == EPI_DGELU || epi == EPI_BIAS_RESID, acc = epi == EPI_ACC_F32;
   const int sms = sm_count();
-  const float f32 = kind == KIND_TF32 ? 1.3f : 0.0f;
+  const float mn = a_mn ? 1.8f : b_mn ? 1.4f : 1.0f, f32 = kind == KIND_TF32 ? 2.0f : 0.0f;
   const long long pt = (long long)ceil_div(M, 256) * ceil_div(N, 256) * splits;
   const int rounds = (int)((pt + sms / 2 - 1) / (sms / 2));
-  const float pair_kb = 0.31f * ceil_div(kb_total, splits), pair_epi = (aux ? 6.3f : 5.5f) + f32;
-  float best = (aux ? 7.8f : acc ? 6.7f : 4.7f) + f32 + pair_kb + (rounds - 1) * (pair_kb > pair_epi ? pair_kb : pair_epi);
+  const float pair_kb = 0.285f * ceil_div(kb_total, splits) * (a_mn ? 1.4f : b_mn ? 1.12f : 1.0f);
+  const float pair_epi = aux ? 6.0f + f32 : 4.8f;
+  float best = 0.95f * ((aux ? 9.3f : acc ? 8.0f : 6.7f) + f32 + pair_kb + (rounds - 1) * (pair_kb > pair_epi ? pair_kb : pair_epi));
   Tile t{256, 1, splits};
   for (int bn = 64; bn <= 128; bn += 64) {
     if (bn == 64 && kind == KIND_F8F6F4) continue;        // an fp8 row of an MN-major operand is 128 columns
@@ -63,15 +65,15 @@ Tile pick_tile(int kind, int epi, int M, int N, int kb_total, int splits, int mo
       if (acc)                                            // one round of CTAs, at least four k-blocks each, no more parts than allowed
         while (sp < most && tiles * (sp + 1) <= sms && kb_total / (sp + 1) >= 4) ++sp;
       const float per_sm = (float)(tiles * cl * sp) / sms;
-      // one to two CTAs per SM: the second CTA of an SM overlaps the first one's epilogue, and the kernels before and after overlap the short
-      // tail.  M 776, us, pair / 128 x 128: K 1024, N 4096 with GELU (224 CTAs) 13.6 / 12.7.  Not with an auxiliary input: bias + residual, M 4096, N 768
-      // (192), K 768 11.2 / 16.4; dGELU, M 2048, K 768, N 3072 (384) 14.8 / 23.1; nor where parts of K are added, M N 1600, K 4096 (169) 25.4 /
-      // 29.6, nor with the fp32 GELU, TF32 M 1024, K 768, N 3072 (192) 22.0 / 31.8.
-      const bool gelu = epi == EPI_BIAS_GELU && kind != KIND_TF32;
-      const bool beside = per_sm > 1.f && per_sm <= 2.f && !acc && (!aux || gelu);
+      // one to two CTAs per SM and operands stored along K: the second CTA of an SM overlaps the first one's epilogue, and the kernels
+      // before and after overlap the short tail.  M 776, us, pair / 128 x 128: K 1024, N 3072 (168 CTAs) 14.6 / 12.8, N 4096 with GELU
+      // (224) 17.1 / 15.6; K 1600, N 4800 (266) 28.9 / 20.9.  Not with an auxiliary input, which the pair kernel works in with 16
+      // warps: bias + residual, M 4096, N 768 (192), K 768 13.0 / 18.4, K 3072 25.4 / 37.5; dGELU, M 776, N 3072 (168) 13.0 / 18.7, N 4096
+      // (224) 15.2 / 23.2 (a backward product, whose weights lie along N, is out by that already).
+      const bool beside = per_sm > 1.f && per_sm <= 2.f && !a_mn && !b_mn && epi != EPI_BIAS_RESID && epi != EPI_DGELU;
       const float w = per_sm <= 1.f ? 1.f : beside ? per_sm : 0.5f * (per_sm + ceilf(per_sm));
-      const float fixed = (cl == 1 ? (bn == 64 ? 3.3f : 4.1f) : cl == 2 ? 4.65f : 5.3f) + (aux ? (bn == 64 ? 0.35f : gelu ? 1.5f : 2.1f) : 0.f) + f32;
-      const float est = fixed + w * ceil_div(kb_total, cl * sp) * (bn == 64 ? 0.215f : 0.25f) + (w - 1.f) * (!aux ? 0.45f : beside ? 1.0f : 2.1f) * (bn / 64);
+      const float fixed = (cl == 1 ? (bn == 64 ? 4.2f : 5.0f) : cl == 2 ? 5.6f : 6.2f) + (aux ? (bn == 64 ? 0.3f : 1.2f) : 0.f) + f32;
+      const float est = fixed + w * ceil_div(kb_total, cl * sp) * 0.24f * mn + (w - 1.f) * (!aux ? 0.7f : beside ? 1.0f : 3.0f) * (bn / 64);
       if (est < best) { best = est; t = {bn, cl, sp}; }
     }
   }
@@ -137,7 +139,7 @@ int gemm_dispatch(void* D, const void* A, const void* B, const void* bias, void*
   const int most = parts(splits, kb_total);
   if (epi != EPI_ACC_F32) splits = 1;
   Tile tile{256, 1, splits};
-  if (p.tma_epi && !keep_pair && p.g.W <= 1 && p.pull.nseg == 0 && p.pull.nwait == 0) tile = pick_tile(KIND, epi, M, N, kb_total, splits, most);
+  if (p.tma_epi && !keep_pair && p.g.W <= 1 && p.pull.nseg == 0 && p.pull.nwait == 0) tile = pick_tile(KIND, epi, M, N, kb_total, splits, most, a_mn, b_mn);
   while (tile.cl > 1 && tile.cl > kb_total) tile.cl >>= 1;
   splits = tile.splits;
   const bool pair = tile.bn == 256;
@@ -219,7 +221,7 @@ LLMB_API int llmb_gemm(void* D, const void* A, const void* B, const void* bias, 
 LLMB_API int llmb_gemm_dw_splits(int kind, int M, int N, int K, int splits) {
   const int kb = ceil_div(K, kind == 0 ? 64 : 32);
   const int most = parts(splits, kb);
-  return pick_tile(kind == 0 ? KIND_F16 : KIND_TF32, EPI_ACC_F32, M, N, kb, splits, most).splits;
+  return pick_tile(kind == 0 ? KIND_F16 : KIND_TF32, EPI_ACC_F32, M, N, kb, splits, most, 1, 1).splits;
 }
 
 // Arms the calling thread's NEXT llmb_gemm call to gather its A matrix from W ranks (see GatherArgs): A must be the

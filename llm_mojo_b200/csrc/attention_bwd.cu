@@ -16,7 +16,8 @@
 // about 6000, from clock traces of the roles):
 //   * -lse and -D differ from column to column, so every thread needed all of them: 32 vector loads a thread, 2000 cycles of the shared-memory
 //     pipe.  The tensor core adds them now, as one more K = 16 step of each score product: ones times rows that hold the values in
-//     three bf16 parts (24 bits, all of an fp32 value; attn_bwd3_prep_kernel writes them).
+//     three bf16 parts (24 bits, all of an fp32 value; attn_bwd3_prep_kernel writes them).  Each product reads its own statistic only:
+//     a shared row whose other half meets zeros would carry an infinity or NaN from one product into the other (0 * inf).
 //   * two phases of the compute warps (P^T, then dS^T) with twelve barrier round trips of 170 - 250 cycles: one phase with two waits.
 //   * one issuing warp, whose round trips came on top of 34 MMAs: one for the scores, one for the products.
 //   * reductions of the dQ partials in the way of the compute warps' stores: see there.
@@ -44,11 +45,11 @@
 namespace {
 constexpr int B3_NS = 3;                                   // ring depth in blocks: Q_i and dO_i, 16 KB each
 constexpr int B3_THREADS = 512;
-constexpr int B3_EXT = TILE * 32;                          // the statistics of a block as operand rows of 16 bf16
-constexpr int B3_ONE = TILE * 16;                          // 128 rows of 8 bf16, rows in a column of 8-row core matrices
+constexpr int B3_COL = TILE * 16;                          // 128 rows of 8 bf16: a column of core matrices of 8 rows x 16 bytes (no swizzle)
+constexpr int B3_EXT = 2 * B3_COL;                         // the statistics of a block: a column of -lse / scale, one of -D
 constexpr unsigned B3_PACE_NS = 90;                        // B 64, T 1024, us: none 616, 20 x 16 582, 100 x 8 570, 150 x 8 (longer than a block) 692
-constexpr int B3_SLACK = 768;                              // for aligning the base, which is aligned already
-constexpr int B3_SMEM = 4 * T128 /*K,V x2*/ + B3_NS * (2 * T128 + B3_EXT) + 2 * T128 /*dS^T*/ + T128 /*epilogue staging*/ + 3 * B3_ONE + 256 /*barriers*/ + B3_SLACK;
+constexpr int B3_SMEM = 4 * T128 /*K,V x2*/ + B3_NS * (2 * T128 + B3_EXT) + 2 * T128 /*dS^T*/ + T128 /*epilogue staging*/ + 2 * B3_COL + 256 /*barriers*/ +
+                        1024 /*alignment*/;
 static_assert(B3_SMEM <= 227 * 1024, "shared memory of a CTA");
 constexpr uint32_t IDESC_TS_MN = make_idesc(FMT_BF16, FMT_BF16, 0, 1, 128, 64);     // A K-major (TMEM or smem), B stored [K rows, 64]
 constexpr uint32_t IDESC_MN_MN = make_idesc(FMT_BF16, FMT_BF16, 1, 1, 128, 64);     // A stored [K rows, 128], B stored [K rows, 64]
@@ -56,7 +57,7 @@ constexpr uint32_t IDESC_MN_MN = make_idesc(FMT_BF16, FMT_BF16, 1, 1, 128, 64); 
 #define B3_FAIL() do { atomicExch(p.status, LLMB_ERR_TIMEOUT); failed = true; } while (0)
 
 struct B3Params {
-  void* dqkv;            // [B,T,3C] bf16
+  const uint4* stats;    // per (batch, head, 128-row tile): the column of -lse / scale, then that of -D, 16 bytes a row
   float* dq_acc;         // per (batch, head, tile): [16 column groups][128 rows][4] fp32, zero on entry
   float* dbias;          // optional fp32 [3C]
   int B, T, NH, C;
@@ -64,9 +65,8 @@ struct B3Params {
   int* status;
 };
 
-// D = rowsum(dO * O) and the statistics of every row as 16 bf16 values, an operand of the score products (see above): columns 0 .. 2 the parts
-// of -lse / scale, columns 8 .. 10 those of -D.  Three bf16 parts hold 24 bits, all of an fp32 value.  Eight threads per row, 16 bytes of dO and O
-// each, so that a warp reads four whole 128-byte rows per instruction.
+// D = rowsum(dO * O) and the statistics of every row as operands of the score products (see above): three bf16 parts, 24 bits, all of an fp32
+// value.  Eight threads per row, 16 bytes of dO and O each, so that a warp reads four whole 128-byte rows per instruction.
 __device__ __forceinline__ uint4 parts3(float v) {
   const __nv_bfloat16 hi = __float2bfloat16_rn(v);
   const float h = __bfloat162float(hi), r1 = isinf(h) ? 0.f : v - h;                // (an infinite value is its first part)
@@ -92,8 +92,9 @@ __global__ void attn_bwd3_prep_kernel(uint4* __restrict__ stats, const float* __
     for (int k = 0; k < 8; ++k) s += x.v[k] * y.v[k];
   }
   s += __shfl_xor_sync(0xffffffffu, s, 1); s += __shfl_xor_sync(0xffffffffu, s, 2); s += __shfl_xor_sync(0xffffffffu, s, 4);
-  if (part == 0) stats[idx * 2] = parts3(t < T ? -lse[bh * T + t] * inv_scale_log2 : -1e6f);     // rows beyond T: 2^(-1e6 scale) = 0
-  if (part == 1) stats[idx * 2 + 1] = parts3(-s);
+  uint4* st = stats + idx / TILE * (2 * TILE) + idx % TILE;
+  if (part == 0) st[0] = parts3(t < T ? -lse[bh * T + t] * inv_scale_log2 : -1e6f);     // rows beyond T: 2^(-1e6 scale) = 0
+  if (part == 1) st[TILE] = parts3(-s);
 }
 
 struct Tile3 { int w, t, g, bh, tile; bool sub, done; };    // work item, tiles / blocks consumed so far, current tile
@@ -143,22 +144,16 @@ __device__ __forceinline__ void red_add_v4(float* addr, float a, float b, float 
 
 __global__ void __launch_bounds__(B3_THREADS, 1) attn_bwd3_kernel(const __grid_constant__ CUtensorMap tmQKV,
                                                                   const __grid_constant__ CUtensorMap tmDO,
-                                                                  const __grid_constant__ CUtensorMap tmOUT,
-                                                                  const __grid_constant__ CUtensorMap tmEXT, const B3Params p) {
+                                                                  const __grid_constant__ CUtensorMap tmOUT, const B3Params p) {
   extern __shared__ unsigned char smem_raw[];
   unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  if (sm - smem_raw > B3_SLACK) {                           // the alignment slack this launch was given does not cover the base it got
-    pdl_wait();                                             // (the kernel after this one counts on it, on this path too)
-    if (threadIdx.x == 0) atomicExch(p.status, LLMB_ERR_BAD_ARG);
-    return;
-  }
   unsigned char* sKV = sm;                                  // buffer kb: K at kb*2*T128, V at +T128
   unsigned char* sST = sKV + 4 * T128;                      // ring: stage s holds Q_i at s*2*T128, dO_i at +T128
   unsigned char* sDS = sST + B3_NS * 2 * T128;              // dS^T: queries 0..63 at +0, 64..127 at +T128 ([128 keys][64] each)
-  unsigned char* sEXT = sDS + 2 * T128;                     // per stage: the block's statistics, [128 queries][16] bf16, 32-byte swizzle
+  unsigned char* sEXT = sDS + 2 * T128;                     // per stage: the block's statistics, two columns
   unsigned char* sEP = sEXT + B3_NS * B3_EXT;               // staging tile of the dK / dV epilogue ([128 keys][64] bf16, swizzled)
-  unsigned char* sONE = sEP + T128;                         // no swizzle: eight columns 1 1 1 0 0 0 0 0, eight of zeros, eight as the first
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sONE + 3 * B3_ONE);
+  unsigned char* sONE = sEP + T128;                         // a column of rows 1 1 1 0 0 0 0 0, then one of zeros: the second half of K on either side
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sONE + 2 * B3_COL);
   uint64_t* kv_full = bars;                                 // [2]
   uint64_t* kv_empty = kv_full + 2;                         // [2] the tile's last reads of K and V are complete
   uint64_t* st_full = kv_empty + 2;                         // [NS]
@@ -184,10 +179,10 @@ __global__ void __launch_bounds__(B3_THREADS, 1) attn_bwd3_kernel(const __grid_c
     mbar_init(s_full, 1); mbar_init(s_free, 8); mbar_init(p_full, 12); mbar_init(ds_free, 1);
     mbar_init(dq_full, 1); mbar_init(acc_full, 1); mbar_init(acc_free, 4); mbar_init(ep_ready, 4); mbar_init(ep_free, 1);
     fence_barrier_init();
-    prefetch_tmap(&tmQKV); prefetch_tmap(&tmDO); prefetch_tmap(&tmOUT); prefetch_tmap(&tmEXT);
+    prefetch_tmap(&tmQKV); prefetch_tmap(&tmDO); prefetch_tmap(&tmOUT);
   }
-  if (tid < 3 * TILE) {
-    *reinterpret_cast<uint4*>(sONE + tid * 16) = tid / TILE == 1 ? make_uint4(0u, 0u, 0u, 0u) : make_uint4(0x3f803f80u, 0x3f80u, 0u, 0u);
+  if (tid < 2 * TILE) {
+    *reinterpret_cast<uint4*>(sONE + tid * 16) = tid < TILE ? make_uint4(0x3f803f80u, 0x3f80u, 0u, 0u) : make_uint4(0u, 0u, 0u, 0u);
     fence_proxy_async();
   }
   if (warp == 13) tmem_alloc<512>(tmem_slot);
@@ -232,7 +227,7 @@ __global__ void __launch_bounds__(B3_THREADS, 1) attn_bwd3_kernel(const __grid_c
             mbar_expect_tx(&st_full[st], 2 * T128 + B3_EXT);
             load128(stg, &tmQKV, &st_full[st], colQ, i * TILE, b);
             load128(stg + T128, &tmDO, &st_full[st], colQ, i * TILE, b);
-            tma_load_2d(sEXT + st * B3_EXT, &tmEXT, &st_full[st], 0, (c.bh * n_t + i) * TILE);
+            bulk_load_1d(sEXT + st * B3_EXT, p.stats + ((size_t)c.bh * n_t + i) * (2 * TILE), B3_EXT, &st_full[st]);
             for (int k = 0; k < pf_per; ++k) {
               const int r = pf + 64 * k;
               if (r < nx0) {
@@ -259,8 +254,12 @@ __global__ void __launch_bounds__(B3_THREADS, 1) attn_bwd3_kernel(const __grid_c
       const uint64_t q_mn0 = make_smem_desc(smem_u32(sST), 8192, 1024);               // Q_i / dO_i as MN-major B operands
       const uint64_t ds_kk = make_smem_desc(smem_u32(sDS), 16, 1024);                 // dS^T as a K-major A operand (K = queries)
       const uint64_t ds_mn = make_smem_desc(smem_u32(sDS), T128, 1024);               // dS^T as an MN-major A operand (M = queries)
-      const uint64_t ext0 = make_smem_desc(smem_u32(sEXT), 16, 256, 6);               // 32-byte swizzle
-      const uint64_t one0 = make_smem_desc(smem_u32(sONE), B3_ONE, 128, 0);           // no swizzle: core matrices of 8 rows x 16 bytes, the next along K in the next column
+      // the statistics' step: ones / a statistic in the first eight values of K, zeros (the same column) in the others
+      const uint64_t one0 = make_smem_desc(smem_u32(sONE), B3_COL, 128, 0);
+      auto stat_desc = [&](int st, int col) {
+        const uint32_t at = smem_u32(sEXT) + st * B3_EXT + col * B3_COL;
+        return make_smem_desc(at, smem_u32(sONE) + B3_COL - at, 128, 0);
+      };
       // a block in one word: 4 * (tiles before its tile) + 2 * (last of its tile) + (first of its tile), -1 when there is none left
       auto info = [](const Blk3& b) { return b.c.done ? -1 : b.c.t * 4 + (b.ib + 1 == b.nbt ? 2 : 0) + (b.ib == 0 ? 1 : 0); };
       auto scores = [&](int n, int what) {                                            // S^T and dP^T of block n
@@ -270,12 +269,12 @@ __global__ void __launch_bounds__(B3_THREADS, 1) attn_bwd3_kernel(const __grid_c
         if (n >= 1 && !mbar_wait(s_free, (n - 1) & 1)) { B3_FAIL(); return; }
         fence_after_sync();
         const uint64_t kd = k_kk0 + (uint64_t)((kb * 2 * T128) >> 4), qd = q_kk0 + (uint64_t)((st * 2 * T128) >> 4);
-        const uint64_t ext = ext0 + (uint64_t)((st * B3_EXT) >> 4);
+        const uint64_t nlse = stat_desc(st, 0), nd = stat_desc(st, 1);
         if (elect_one()) {
-          umma_ss<KIND_F16>(tS, one0, ext, IDESC_S_128x128, 0u);                       // -lse / scale in every row
+          umma_ss<KIND_F16>(tS, one0, nlse, IDESC_S_128x128, 0u);                      // -lse / scale in every row
 #pragma unroll
           for (int ks = 0; ks < HS / 16; ++ks) umma_ss<KIND_F16>(tS, kd + 2 * ks, qd + 2 * ks, IDESC_S_128x128, 1u);
-          umma_ss<KIND_F16>(tDP, one0 + (B3_ONE >> 4), ext, IDESC_S_128x128, 0u);      // -D
+          umma_ss<KIND_F16>(tDP, one0, nd, IDESC_S_128x128, 0u);                       // -D
 #pragma unroll
           for (int ks = 0; ks < HS / 16; ++ks) umma_ss<KIND_F16>(tDP, kd + (T128 >> 4) + 2 * ks, qd + (T128 >> 4) + 2 * ks, IDESC_S_128x128, 1u);
           umma_commit(s_full);
@@ -523,9 +522,9 @@ LLMB_API long long llmb_attention_bwd_fused_stats_floats(int B, int T, int NH) {
 LLMB_API long long llmb_attention_bwd_fused_acc_floats(int B, int T, int NH) { return (long long)B * NH * ceil_div(T, TILE) * (TILE * HS); }
 
 // dqkv [B,T,3C] bf16 (fully overwritten) from dout [B,T,C], qkv [B,T,3C], out [B,T,C] (bf16) and the forward's lse [B,NH,T]
-// (log2 domain); C = NH*64.  `stats`: fp32 scratch of ..._stats_floats elements.  `dq_acc`: fp32 scratch of ..._acc_floats
-// elements, 16-byte aligned, which must be ZERO on entry and is zero again when the call has completed without an error in
-// the status word.  dbias (optional, fp32 [3C]) += column sums of dqkv, by atomic adds.
+// (log2 domain); C = NH*64.  `stats` (..._stats_floats elements) and `dq_acc` (..._acc_floats): fp32 scratch, 16-byte aligned; `dq_acc` must be
+// ZERO on entry and is zero again when the call has completed without an error in the status word.  dbias (optional, fp32 [3C]) +=
+// column sums of dqkv, by atomic adds.
 LLMB_API int llmb_attention_bwd_fused(void* dqkv, float* dbias, float* stats, float* dq_acc, const void* dout, const void* qkv, const void* out,
                                       const float* lse, int B, int T, int NH, int* status, cudaStream_t st) {
   const int C = NH * HS;
@@ -534,10 +533,8 @@ LLMB_API int llmb_attention_bwd_fused(void* dqkv, float* dbias, float* stats, fl
   rc = make_qkv_map(&td, dout, B, T, C); if (rc) return 1000 + rc;
   CUtensorMap to;
   rc = make_qkv_map(&to, dqkv, B, T, 3 * C); if (rc) return 1000 + rc;
-  CUtensorMap tx;
-  rc = make_tmap_2d(&tx, stats, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)B * NH * ceil_div(T, TILE) * TILE, 16, 16, TILE, 16, CU_TENSOR_MAP_SWIZZLE_32B);
-  if (rc) return 1000 + rc;
-  B3Params p{}; p.dqkv = dqkv; p.dq_acc = dq_acc; p.dbias = dbias;
+  if (reinterpret_cast<uintptr_t>(stats) & 15) return LLMB_ERR_BAD_ARG;
+  B3Params p{}; p.stats = (const uint4*)stats; p.dq_acc = dq_acc; p.dbias = dbias;
   p.B = B; p.T = T; p.NH = NH; p.C = C; p.scale = 0.125f; p.scale_log2 = 0.125f * 1.4426950408889634f; p.status = status;
   static bool attr = false;
   if (!attr) {
@@ -550,7 +547,7 @@ LLMB_API int llmb_attention_bwd_fused(void* dqkv, float* dbias, float* stats, fl
              1.0f / p.scale_log2);
   const long long n_items = (long long)((n_t + 1) / 2) * B * NH;
   const int grid = (int)(n_items < sm_count() ? n_items : sm_count());          // persistent: one CTA per SM
-  launch_pdl(attn_bwd3_kernel, grid, B3_THREADS, B3_SMEM, st, tq, td, to, tx, p);
+  launch_pdl(attn_bwd3_kernel, grid, B3_THREADS, B3_SMEM, st, tq, td, to, p);
   launch_pdl(attn_bwd3_dq_kernel, (unsigned)(B * NH * n_t), 128, 0, st, (__nv_bfloat16*)dqkv, dbias, dq_acc, T, NH, C, p.scale);
   return (int)cudaGetLastError();
 }

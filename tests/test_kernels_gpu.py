@@ -411,6 +411,46 @@ def test_fused_attention_backward_walks_short_tiles_and_large_statistics(B, T, N
         assert ((got - want).norm() / want.norm()).item() < tol, nm
 
 
+@pytest.mark.parametrize("stat,value", [("D", float("inf")), ("D", float("nan")), ("lse", float("inf"))])
+def test_fused_attention_backward_keeps_a_non_finite_statistic_in_its_own_product(stat, value):
+    """Row 200 of one head.  An infinite or NaN D (from the stored output) reaches dS, so dQ of that row and dK of the keys of its tile (zero
+    probabilities times it) and of those before; P and with it dV do not depend on D.  An infinite log-sum-exp makes the row's probabilities zero: the gradients of a row without an output
+    gradient.  dK and dV are summed in a fixed order, so what does not depend on the statistic has the same bits."""
+    B, T, NH, b, t, h = 2, 300, 2, 1, 200, 1
+    C = NH * 64
+    qkv, dout = rnd(B, T, 3 * C).to(DEV), rnd(B, T, C, seed=1).to(DEV)
+    out, lse = torch.empty(B, T, C, dtype=torch.bfloat16, device=DEV), torch.empty(B, NH, T, device=DEV)
+    ops.attention_fwd(out, lse, qkv, NH)
+
+    def grads(o, l, do):
+        g = torch.full((B, T, 3 * C), float("nan"), dtype=torch.bfloat16, device=DEV)
+        ops.attention_bwd(g, do, qkv, o, l, NH)
+        status_ok()
+        return g.view(B, T, 3, NH, 64)
+    if stat == "D":
+        want = grads(out, lse, dout)
+        out2 = out.clone()
+        out2[b, t, h * 64 + 5] = value
+        got = grads(out2, lse, dout)
+        assert torch.equal(got[:, :, 2], want[:, :, 2])                                # dV
+        assert not got[b, t, 0, h].isfinite().any() and not got[b, :t + 1, 1, h].isfinite().any()
+        keep = torch.ones(B, T, NH, dtype=torch.bool, device=DEV)
+        keep[b, :256, h] = False
+        assert torch.equal(got[:, :, 1][keep], want[:, :, 1][keep])                    # dK of the other heads and of later tiles
+        keep[b, :, h] = True
+        keep[b, t, h] = False
+        assert got[:, :, 0][keep].isfinite().all()                                     # dQ of all other rows
+    else:
+        dout2 = dout.clone()
+        dout2[b, t, h * 64:(h + 1) * 64] = 0.0
+        want = grads(out, lse, dout2)
+        lse2 = lse.clone()
+        lse2[b, h, t] = value
+        got = grads(out, lse2, dout)
+        assert torch.equal(got[:, :, 1:], want[:, :, 1:])
+        assert not got[b, t, 0, h].any() and got.isfinite().all()
+
+
 @pytest.mark.parametrize("bwd", ["fused", "split"])
 def test_attention_persistent_loops_large(bwd, monkeypatch):
     """B=16, NH=12, T=1024: 768 work items on at most 148 CTAs, so every persistent CTA walks several items per

@@ -127,13 +127,17 @@ int gemm_dispatch(void* D, const void* A, const void* B, const void* bias, void*
   if (tma_epi_on < 0) { const char* e = getenv("LLMB_GEMM_TMA_EPI"); tma_epi_on = (e && e[0] == '0') ? 0 : 1; }
   CUtensorMap ta, tb, td, taux;
   p.tma_epi = 0;
-  if (tma_epi_on && (ldd * osz) % 16 == 0 && (!needs_aux || (aux && (reinterpret_cast<uintptr_t>(aux) & 15) == 0 && (ldaux * osz) % 16 == 0))) {
+  const bool tma_layout = tma_epi_on && (ldd * osz) % 16 == 0 && (!needs_aux || (aux && (reinterpret_cast<uintptr_t>(aux) & 15) == 0 && (ldaux * osz) % 16 == 0));
+  const bool reg_layout = register_epilogue_takes(epi, KIND == KIND_TF32, M, bias, aux, ldd, ldaux);
+  if (!tma_layout && !reg_layout) return LLMB_ERR_BAD_ARG;
+  if (tma_layout) {
     const CUtensorMapDataType odt = out_f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
     const uint32_t box_cols = out_f32 ? 32 : 64;
     int ok = make_tmap_2d(&td, D, odt, osz, (uint64_t)M, (uint64_t)N, (uint64_t)ldd, 32, box_cols) == 0;
     if (ok && needs_aux) ok = make_tmap_2d(&taux, aux, odt, osz, (uint64_t)M, (uint64_t)N, (uint64_t)ldaux, 32, box_cols) == 0;
     p.tma_epi = ok;
   }
+  if (!p.tma_epi && !reg_layout) return LLMB_ERR_BAD_ARG;
   if (p.colsum && !p.tma_epi) return LLMB_ERR_BAD_ARG;    // the column sums are taken in the TMA epilogue only
   const int kb_total = ceil_div(K, BKE);
   const int most = parts(splits, kb_total);

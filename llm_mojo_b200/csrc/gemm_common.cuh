@@ -156,6 +156,16 @@ __device__ __forceinline__ void epi4(const GemmParams& p, float (&v)[4], int row
   *reinterpret_cast<uint2*>(dp) = o;
 }
 
+// What epi4's 16-byte (fp32) and 8-byte (bf16) accesses need of a layout that has no tensor map; D is 16-byte aligned and N % 8 == 0 in any
+// case, and the pitch of a single row is not used.  A dispatch that would fall back to it with anything else refuses the call.
+inline bool register_epilogue_takes(int epi, bool io_f32, int M, const void* bias, const void* aux, long long ldd, long long ldaux) {
+  const bool needs_aux = epi == EPI_BIAS_GELU || epi == EPI_DGELU || epi == EPI_BIAS_RESID;
+  const bool needs_bias = epi == EPI_BIAS || epi == EPI_BIAS_GELU || epi == EPI_BIAS_RESID;
+  const uintptr_t mask = io_f32 ? 15 : 7;
+  return (M == 1 || ldd % 4 == 0) && (!needs_aux || (aux && (reinterpret_cast<uintptr_t>(aux) & mask) == 0 && (M == 1 || ldaux % 4 == 0))) &&
+         (!needs_bias || (reinterpret_cast<uintptr_t>(bias) & mask) == 0);
+}
+
 // One epilogue warp drains its 32 rows x NCOLS columns of accumulator `tacc` (TMEM address incl. lane quarter).
 template <int EPI, int NCOLS = BN>
 __device__ __forceinline__ void epilogue_warp(const GemmParams& p, uint32_t tacc, unsigned char* stage, int row_base, int n0,

@@ -22,6 +22,12 @@ int gemm_block_scaled(void* D, const void* A, const void* B, const void* sfa, co
   if (M <= 0 || N <= 0 || K <= 0 || K % 32 || N % 8) return LLMB_ERR_BAD_ARG;
   if ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(B) | reinterpret_cast<uintptr_t>(D) |
        reinterpret_cast<uintptr_t>(sfa) | reinterpret_cast<uintptr_t>(sfb)) & 15) return LLMB_ERR_BAD_ARG;
+  // outputs (and bf16 auxiliary tensors) travel by TMA when their layout allows a tensor map
+  const bool needs_aux = epi == EPI_BIAS_GELU || epi == EPI_DGELU || epi == EPI_BIAS_RESID, out_f32 = epi == EPI_ACC_F32 || epi == EPI_STORE_F32;
+  const int osz = out_f32 ? 4 : 2;
+  const bool tma_layout = (ldd * osz) % 16 == 0 && (!needs_aux || (aux && (reinterpret_cast<uintptr_t>(aux) & 15) == 0 && (ldaux * 2) % 16 == 0));
+  const bool reg_layout = register_epilogue_takes(epi, false, M, bias, aux, ldd, ldaux);
+  if (!tma_layout && !reg_layout) return LLMB_ERR_BAD_ARG;
   CUtensorMap ta, tb;
   int rc = make_tmap_2d(&ta, A, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, (uint64_t)M, (uint64_t)(K / EPB), (uint64_t)(K / EPB), BM, ROW_BYTES);
   if (rc) return 1000 + rc;
@@ -48,17 +54,15 @@ int gemm_block_scaled(void* D, const void* A, const void* B, const void* sfa, co
   p.status = status;
   p.bias_vec = (reinterpret_cast<uintptr_t>(bias) & 15) == 0;
   p.idesc = KIND == KIND_MXF8 ? make_idesc_mxfp8((uint32_t)a_fmt, (uint32_t)b_fmt, 2 * BM, BN) : make_idesc_nvfp4(2 * BM, BN);
-  // outputs (and bf16 auxiliary tensors) travel by TMA when their layout allows a tensor map
   CUtensorMap td = ta, taux = ta;
-  const bool needs_aux = epi == EPI_BIAS_GELU || epi == EPI_DGELU || epi == EPI_BIAS_RESID, out_f32 = epi == EPI_ACC_F32 || epi == EPI_STORE_F32;
-  const int osz = out_f32 ? 4 : 2;
-  if ((ldd * osz) % 16 == 0 && (!needs_aux || (aux && (reinterpret_cast<uintptr_t>(aux) & 15) == 0 && (ldaux * 2) % 16 == 0))) {
+  if (tma_layout) {
     int ok = make_tmap_2d(&td, D, out_f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, osz, (uint64_t)M, (uint64_t)N,
                           (uint64_t)ldd, 32, out_f32 ? 32 : 64) == 0;
     if (ok && needs_aux)
       ok = make_tmap_2d(&taux, aux, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)M, (uint64_t)N, (uint64_t)ldaux, 32, 64) == 0;
     p.tma_epi = ok;
   }
+  if (!p.tma_epi && !reg_layout) return LLMB_ERR_BAD_ARG;
   return launch_pair_epi<KIND>(epi, ta, tb, td, taux, sfm, p, st);
 }
 }  // namespace

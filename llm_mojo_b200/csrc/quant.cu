@@ -509,7 +509,7 @@ __global__ void __launch_bounds__(512) fp8_site_quant_kernel(const Fp8Site a) {
     if (lane == 0) {
       const int step = __float_as_int(e.state[2]);
       e.state[0] = sc; e.state[1] = inv[w];
-      e.state[4 + step % AMAX_HISTORY] = __uint_as_float(atomicExch(&e.work[0], 0u));
+      e.state[3] = e.state[4 + step % AMAX_HISTORY] = __uint_as_float(atomicExch(&e.work[0], 0u));
       e.state[2] = __int_as_float(step + 1);
     }
   }
@@ -522,8 +522,8 @@ __global__ void __launch_bounds__(512) fp8_site_quant_kernel(const Fp8Site a) {
 }  // namespace
 
 // The operands of one linear layer whose histories are full (the caller checks that: state[2] >= the history length): out = fp8(x * scale)
-// saturated, state[0..1] = scale and 1 / scale from the history, max|x| appended to the history.  Operand b is optional (b_x null).  work: two zeroed
-// words per operand, zero again afterwards.  alpha1 / alpha2 (either may be null) = 1 / scale of a * other[1], with the state `other` of an operand
+// saturated, state[0..1] = scale and 1 / scale from the history, state[3] = max|x|, which is appended to the history.  Operand b is optional (b_x
+// null).  work: two zeroed words per operand, zero again afterwards.  alpha1 / alpha2 (either may be null) = 1 / scale of a * other[1], with the state `other` of an operand
 // whose scale is final, or of b where it is null.  n: multiples of the vector width (8 for bf16, 4 for fp32).
 LLMB_API int llmb_fp8_site_quant(void* a_out, const void* a_x, float* a_state, void* a_work, long long a_n, float a_margin, void* b_out, const void* b_x,
                                  float* b_state, void* b_work, long long b_n, float b_margin, int fmt, int dtype, float* alpha1, const float* other1,

@@ -55,7 +55,7 @@ class AmaxState:
         self.state = torch.zeros(4 + AMAX_HISTORY, dtype=torch.float32, device=device)
         self.state[0] = 1.0
         self.state[1] = 1.0
-        self.amax = torch.zeros(1, dtype=torch.float32, device=device)
+        self.amax = self.state[3:4]                                        # max|x| of the last operand
         self.work = torch.zeros(2, dtype=torch.int32, device=device)       # of ``llmb_fp8_site_quant``: zero between its launches
         self.host_step = 0
         self.static = False

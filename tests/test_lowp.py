@@ -286,6 +286,17 @@ def test_operands_of_a_site_in_one_launch_equal_one_by_one(na, nb, dtype):
 
 
 @gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_delayed_scaling_keeps_the_last_maximum(dtype):
+    """``amax`` is max|x| of the last operand, also once the history is full and one launch does everything."""
+    st = lowp.AmaxState("cuda", lowp.E4M3)
+    for step in range(lowp.AMAX_HISTORY + 3):
+        x = (torch.randn(64, 24) * (1 + step % 5)).to(dtype).cuda()
+        lowp._q("t", x, st, torch.empty(64, 24, dtype=torch.uint8, device="cuda"))
+        assert st.amax.item() == x.abs().max().item(), step
+
+
+@gpu
 def test_fp8_block_linear_dual_path_is_bit_identical(monkeypatch):
     rows, C, OC = 256, 384, 512
     g = torch.Generator().manual_seed(2)

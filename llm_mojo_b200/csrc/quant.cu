@@ -524,16 +524,17 @@ __global__ void __launch_bounds__(512) fp8_site_quant_kernel(const Fp8Site a) {
 // The operands of one linear layer whose histories are full (the caller checks that: state[2] >= the history length): out = fp8(x * scale)
 // saturated, state[0..1] = scale and 1 / scale from the history, state[3] = max|x|, which is appended to the history.  Operand b is optional (b_x
 // null).  work: two zeroed words per operand, zero again afterwards.  alpha1 / alpha2 (either may be null) = 1 / scale of a * other[1], with the state `other` of an operand
-// whose scale is final, or of b where it is null.  n: multiples of the vector width (8 for bf16, 4 for fp32).
+// whose scale is final, or of b where it is null.  n: multiples of the vector width (8 for bf16, 4 for fp32); a may
+// be empty, its maximum is zero then.
 LLMB_API int llmb_fp8_site_quant(void* a_out, const void* a_x, float* a_state, void* a_work, long long a_n, float a_margin, void* b_out, const void* b_x,
                                  float* b_state, void* b_work, long long b_n, float b_margin, int fmt, int dtype, float* alpha1, const float* other1,
                                  float* alpha2, const float* other2, cudaStream_t st) {
   const int N = dtype == LLMB_BF16 ? 8 : 4;
-  if (a_n <= 0 || a_n % N || (b_x && (b_n <= 0 || b_n % N)) || fmt < 0 || fmt > 1) return LLMB_ERR_BAD_ARG;
+  if (a_n < 0 || a_n % N || (b_x && (b_n <= 0 || b_n % N)) || fmt < 0 || fmt > 1) return LLMB_ERR_BAD_ARG;
   if (!b_x && ((alpha1 && !other1) || (alpha2 && !other2))) return LLMB_ERR_BAD_ARG;
   const float fmt_max = fmt == 0 ? 448.0f : 57344.0f;
   // four vectors a thread; what is more goes round on four CTAs per SM, shared by the operands' sizes
-  const long long wa = ceil_div_ll(a_n / N, 512 * 4), wb = b_x ? ceil_div_ll(b_n / N, 512 * 4) : 0, most = (long long)sm_count() * 4;
+  const long long wa = a_n ? ceil_div_ll(a_n / N, 512 * 4) : 1, wb = b_x ? ceil_div_ll(b_n / N, 512 * 4) : 0, most = (long long)sm_count() * 4;
   long long ba = wa, bb = wb;
   if (wa + wb > most) {
     ba = wa * most / (wa + wb);

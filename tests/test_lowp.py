@@ -297,6 +297,21 @@ def test_delayed_scaling_keeps_the_last_maximum(dtype):
 
 
 @gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_delayed_scaling_takes_an_empty_operand(dtype):
+    """Its maximum is zero, before and after the history is full."""
+    st = lowp.AmaxState("cuda", lowp.E4M3)
+    x, q = torch.ones(64, 24, dtype=dtype, device="cuda"), torch.empty(64, 24, dtype=torch.uint8, device="cuda")
+    for step in range(lowp.AMAX_HISTORY + 3):
+        lowp._q("t", x[:0] if step == 5 else x, st, q[:0] if step == 5 else q)
+    lowp._q("t", x[:0], st, q[:0])
+    want = torch.ones(lowp.AMAX_HISTORY, device="cuda")
+    want[5] = want[(lowp.AMAX_HISTORY + 3) % lowp.AMAX_HISTORY] = 0.0
+    assert torch.equal(st.state[4:], want) and st.amax.item() == 0.0 and not st.work.any()
+    assert st.host_step == lowp.AMAX_HISTORY + 4 and st.state[2:3].view(torch.int32).item() == lowp.AMAX_HISTORY + 4
+
+
+@gpu
 def test_fp8_block_linear_dual_path_is_bit_identical(monkeypatch):
     rows, C, OC = 256, 384, 512
     g = torch.Generator().manual_seed(2)

@@ -247,14 +247,6 @@ __device__ __forceinline__ uint4 bias8(const GemmParams& p, const __nv_bfloat16*
   u.z = __ldg(h + 4) | (uint32_t)__ldg(h + 5) << 16; u.w = __ldg(h + 6) | (uint32_t)__ldg(h + 7) << 16;
   return u;
 }
-// The bias of a 64-column slab into L1 while the warp has nothing else to do (a lane reads two values; the L2 latency of the first use was
-// 700 cycles of every tile).
-__device__ __forceinline__ void bias_prefetch(const GemmParams& p, int col0, int lane) {
-  const __nv_bfloat16* bias = reinterpret_cast<const __nv_bfloat16*>(p.bias);
-  const int col = col0 + 2 * lane;
-  unsigned short v;
-  if (bias && col < p.N) asm volatile("ld.global.nc.u16 %0, [%1];" : "=h"(v) : "l"(bias + col));
-}
 // alpha * accumulator + bias of 32 columns (this lane's row)
 template <bool BIAS>
 __device__ __forceinline__ void epi_affine32(const GemmParams& p, const uint32_t (&r)[32], int col0, float alpha, float (&v)[32]) {

@@ -16,7 +16,7 @@ constexpr int SMEM2_TAIL = 512;                        // barriers, TMEM slot, a
 // What a tile's epilogue costs its warps beside the arithmetic, and what was done about it (cycles per tile and warp at K = 768, where a tile's
 // MMAs take 6144; clock traces): the hand-back of the accumulator released at cluster scope, which waited for every store and reduction in
 // flight (1200 - 2500; relaxed now, see mbar_arrive_cluster); five integer divisions for the tile's place (500); the bias from L2 (700 a
-// slab, read into L1 while the MMAs run now); with an auxiliary input one box per warp, whose load, work and store took turns (two boxes now,
+// slab in which its loads took turns; the four of 32 columns go out together now); with an auxiliary input one box per warp, whose load, work and store took turns (two boxes now,
 // each loaded again as soon as it has left); column sums before the store of the box (after it now).  Sixteen epilogue warps hid some of
 // that behind one another, at 96 registers and with four of them contending for a scheduler; with it gone eight are faster: M 16384, C
 // 768, us, before / 16 / 8 warps: bias + GELU, N 3072 81.6 / 79.0 / 71.0, dGELU + column sums, N 3072 85.0 / 76.5 / 78.4; M 65536: 324 / 304 - 313 / 265 -
@@ -367,7 +367,6 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     // outputs, layouts without a tensor map) keeps four working warps with all four slabs of a band each.
     // An fp32-storage problem (tf32) moves its 128 columns as four 32-column boxes through the same buffers.
     constexpr bool F32_IO = KIND == KIND_TF32 && !Cfg::F32_OUT, AUX = Cfg::AUX_IN;
-    constexpr bool BF16_BIAS = (EPI == EPI_BIAS || EPI == EPI_BIAS_GELU || EPI == EPI_BIAS_RESID) && !F32_IO;
     constexpr int NBOX = F32_IO ? 4 : 2, BOXC = F32_IO ? 32 : 64;
     const int q = warp & 3, e = warp - 2, hcol = e >> 2;
     const bool tma_epi = p.tma_epi;                       // warp-uniform
@@ -397,7 +396,6 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       int m_blk, n_blk, kb0, kb1; unit_coords(unit, m_blk, n_blk, kb0, kb1);
       const int acc = it & 1;
       const uint32_t acc_phase = (it >> 1) & 1;
-      if (BF16_BIAS) { bias_prefetch(p, n_blk * BN + hcol * 128, lane); bias_prefetch(p, n_blk * BN + hcol * 128 + 64, lane); }
       if (!mbar_wait(&tfull_bar[acc], acc_phase)) { *abort_flag = 1; atomicExch(p.status, LLMB_ERR_TIMEOUT); break; }
       fence_after_sync();
       const int n0 = n_blk * BN;

@@ -98,10 +98,6 @@ gemm_small_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     for (int b = 0; b < nbox; ++b) tma_load_2d(aux_w + b * SLAB_BYTES, &tmAux, &aux_bar[warp], n0 + b * BOX_COLS, row0);
   }
   __syncwarp();
-  // bias lines into L1 beside the main loop, by the warps that have no loop to start: the epilogue's first read of them was an L2 round trip
-  // that nothing hides
-  if ((EPI == EPI_BIAS || EPI == EPI_BIAS_GELU || EPI == EPI_BIAS_RESID) && !Cfg::F32_IO && warp >= 2 && (warp - 2) * 64 < BN_)
-    bias_prefetch(p, n0 + (warp - 2) * 64, lane);
 
   if (warp == 0) {
     int stage = 0; uint32_t phase = 0;

@@ -28,17 +28,6 @@ __global__ void __launch_bounds__(256) ln_fwd_kernel(T* __restrict__ out, float*
   constexpr int per_lane = PER_LANE;            // 16-byte vectors per lane: the row lives in registers
   int row = blockIdx.x * (blockDim.x / 32) + wid;
   if (row >= rows) return;
-  // gamma and beta into L1 beside the row's loads: used at the end only, they were another L2 round trip of every row (with the bias of the
-  // small GEMMs: a generated token at C 1024, context 776, 1980 -> 1968 us; rows that fill the chip are unchanged)
-#pragma unroll
-  for (int i = 0; i < PER_LANE; ++i) {
-    const int vc = i * 32 + lane;
-    uint32_t v;
-    if (vc < nvec) {
-      asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(v) : "l"(w + vc * N));
-      asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(v) : "l"(b + vc * N));
-    }
-  }
   float x[PER_LANE][N];
   float sum = 0.f;
 #pragma unroll

@@ -52,6 +52,34 @@ def test_dependent_launches_wait_on_every_path(name, body):
     assert waits and not bad, (name, bad)
 
 
+def unused_loads(text):
+    """Inline loads none of whose results is read in the rest of the block they stand in."""
+    bad = []
+    for m in re.finditer(r'asm(?:\s+volatile)?\s*\("ld[^;]*?;"\s*:([^:;]*):[^;]*;', text):
+        rest, depth = "", 0
+        for ch in text[m.end():]:
+            depth += {"{": 1, "}": -1}.get(ch, 0)
+            if depth < 0:
+                break
+            rest += ch
+        rest = re.sub(r'"=\w"\(\w+\)', "", rest)
+        if not any(re.search(rf"\b{v}\b", rest) for v in re.findall(r'"=\w"\((\w+)', m.group(1))):
+            bad.append(m.group(0))
+    return bad
+
+
+@pytest.mark.parametrize("path", sorted(glob.glob(os.path.join(CSRC, "*.cu")) + glob.glob(os.path.join(CSRC, "*.cuh"))), ids=os.path.basename)
+def test_the_result_of_an_inline_load_is_read(path):
+    """The assembler drops a plain load whose result nothing reads, volatile or not: it is no prefetch."""
+    assert not unused_loads(re.sub(r"//[^\n]*", "", open(path).read()))
+
+
+def test_the_check_sees_a_load_without_a_reader():
+    load = 'asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(v) : "l"(p));'
+    assert len(unused_loads("{ uint32_t v; if (a) { " + load + load + " } }")) == 2
+    assert not unused_loads("{ uint32_t v; " + load + " return v; }")
+
+
 def test_the_check_sees_an_exit_without_a_wait():
     assert exits_without_wait("int a; if (a) { b(); return; } pdl_wait(); c();") == (True, [" b(); return; "])
     assert exits_without_wait("if (a) { pdl_wait(); return; } auto f = [&](int x) { return x; }; pdl_wait();") == (True, [])

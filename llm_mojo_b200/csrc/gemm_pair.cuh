@@ -237,17 +237,25 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
           const uint64_t bdesc = bdesc0 + (uint64_t)(stage * (STAGE2_BYTES >> 4));
           if (elect_one()) {
             if constexpr (SCALED) {
-              // scales to tensor memory, then up to four MMAs (32 bytes of K per row each); the copies and MMAs of a thread run in order
+              // Up to four MMAs (32 bytes of K per row each), the scales of each on their way to tensor memory beside the MMA before it; the
+              // copies and MMAs of a thread run in order.  Unrolled: a loop over the copies and then one over the MMAs, with trip counts known
+              // at run time, took 930 cycles per NVFP4 k-block where the MMAs take 512, and products of few tiles were slower than the single-CTA
+              // kernel before this one.  us, that kernel / the loops / now: NVFP4 4096 x 768 x 3072 9.63 / 10.53 / 8.80, 128 x 1600 x 6400
+              // 14.4 / 15.3 / 11.5, 8192 x 1600 x 6400 55.2 / 54.0 / 39.5; MXFP8 128 x 1280 x 5120 with residual 21.1 / 19.9 / 18.4.
               constexpr int VALS = KIND == KIND_NVF4 ? 64 : 32, ATOMS = SF_A / 512;
               const int nk = min(4, (p.K - kb * 4 * VALS + VALS - 1) / VALS);
               const uint32_t sfa_t = tmem_base + SFA_COL, sfb_t = tmem_base + SFB_COL;
               const uint64_t sfa = sf0 + (uint64_t)(stage * (3 * SF_A >> 4)), sfb = sfa + (uint64_t)(SF_A >> 4);
-              for (int k = 0; k < ATOMS && k < nk; ++k) {
+              auto scales = [&](int k) {
                 tmem_cp_sf_pair(sfa_t + 4 * k, sfa + (uint64_t)(k * 32));
                 tmem_cp_sf_pair(sfb_t + 8 * k, sfb + (uint64_t)(k * 32));
                 tmem_cp_sf_pair(sfb_t + 8 * k + 4, sfb + (uint64_t)((SF_A >> 4) + k * 32));
-              }
-              for (int k = 0; k < nk; ++k) {
+              };
+              scales(0);
+#pragma unroll
+              for (int k = 0; k < 4; ++k) {
+                if (k + 1 < ATOMS && k + 1 < nk) scales(k + 1);
+                if (k >= nk) continue;
                 const uint32_t acc_in = kb > kb0 || k > 0 ? 1u : 0u;
                 if constexpr (KIND == KIND_NVF4)
                   umma_nvfp4_pair(d_tmem, adesc + k * a_inc, bdesc + k * b_inc, idesc, sfa_t + 4 * k, sfb_t + 8 * k, acc_in);

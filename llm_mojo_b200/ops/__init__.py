@@ -267,16 +267,15 @@ def _tc_kind(t: torch.Tensor):
 
 
 @functools.lru_cache(maxsize=4096)
-def _splits_for(M: int, N: int, K: int, *, tile: int = 256, tile_n: int = 0, bk: int = 64, units: int = 74) -> int:
-    """Split-K factor for the dW GEMMs (by default 256x256 tiles on 74 CTA pairs, 64 values of K per stage; 128 and 256 of them
+def _splits_for(M: int, N: int, K: int, *, bk: int = 64) -> int:
+    """Split-K factor for the dW GEMMs (256x256 tiles on 74 CTA pairs, ``bk`` values of K per stage: 64 of bf16, 128 and 256
     in block-scaled FP8 and NVFP4): the number of splits that minimises waves x (k-blocks per
     unit + a fixed per-unit cost for the prologue and the fp32 red.add epilogue)."""
-    tile_n = tile_n or tile
-    tiles = max(1, ((M + tile - 1) // tile) * ((N + tile_n - 1) // tile_n))
+    tiles = max(1, ((M + 255) // 256) * ((N + 255) // 256))
     kb = (K + bk - 1) // bk
     best, best_cost = 1, None
     for s in range(1, max(1, min(16, kb // 8)) + 1):
-        waves = -(-tiles * s // units)
+        waves = -(-tiles * s // 74)
         cost = waves * (kb / s + 24.0)
         if best_cost is None or cost < best_cost - 1e-9:
             best, best_cost = s, cost

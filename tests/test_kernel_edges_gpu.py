@@ -163,7 +163,7 @@ def test_gemm_fp8_tile_configurations(bn, cl, force_tile):
 # columns in the last 256-wide tile: its first warps' halves hold 1, 2, 3 (and 4, then 1) boxes of 32 columns; 1 and 2 slabs of 64
 @pytest.mark.parametrize("N", [288, 320, 352, 416])
 @pytest.mark.parametrize("epi", ["residual", "dgelu"])
-@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])      # 16 warps with one box each / 8 warps with two buffers for four boxes
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])      # 8 warps with two boxes each / two buffers for four boxes
 def test_gemm_residual_right_edge_many_tiles(dtype, epi, N, force_tile):
     """Several tiles per CTA pair, the right edge leaving part of a warp's boxes: a buffer is refilled with the next tile's auxiliary
     input, which must wait for the store that still reads it."""

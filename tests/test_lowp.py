@@ -153,10 +153,11 @@ def test_native_path_switches_and_split_k_choice(monkeypatch):
     assert lowp.fp8_block_native()
     monkeypatch.setenv("LLMM_FP8B_NATIVE", "0")
     assert not lowp.fp8_block_native()
-    # wgrad of a 124M layer on 128x256 tiles: 6 x 12 = 72 tiles, two splits fill the 148 CTAs once
-    assert ops._splits_for(768, 3072, 65536, tile=128, tile_n=256, bk=256, units=148) == 2
-    # a 768 x 768 wgrad has 18 tiles: eight splits
-    assert ops._splits_for(768, 768, 65536, tile=128, tile_n=256, bk=256, units=148) == 8
+    # NVFP4 wgrad of a 124M layer on 256x256 tiles: 3 x 12 = 36 tiles, two splits fill the 74 CTA pairs once; a 768 x 768 one has nine tiles: eight splits
+    assert ops._splits_for(768, 3072, 65536, bk=256) == 2 and ops._splits_for(768, 768, 65536, bk=256) == 8
+    # 4096 rows: MXFP8 at C 1280, 25 tiles and 32 k-blocks in two parts, 75 and 100 tiles in one; NVFP4 at C 1600 has 16 k-blocks only, one part
+    assert [ops._splits_for(n * 1280, 1280, 4096, bk=128) for n in (1, 3, 4)] == [2, 1, 1]
+    assert [ops._splits_for(n * 1600, 1600, 4096, bk=256) for n in (1, 3, 4)] == [1, 1, 1]
     assert 1 <= ops._splits_for(768, 768, 65536) <= 16
 
 

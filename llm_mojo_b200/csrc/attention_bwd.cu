@@ -22,7 +22,7 @@
 //   * one issuing warp, whose round trips came on top of 34 MMAs: one for the scores, one for the products.
 //   * reductions of the dQ partials in the way of the compute warps' stores: see there.
 //   * dK / dV stores that the dQ warpgroup waited for: warp 15 issues them.
-// Whole backward pass, us, before / now: B 64, T 1024, 12 heads 743 / 570; B 4 83 / 64; B 7, T 777 101 / 80; B 6, T 2048, 16 heads 339 / 238.
+// Whole backward pass, us, before / now: B 64, T 1024, 12 heads 743 / 570 - 602; B 4 83 / 61; B 7, T 777 101 / 75; B 6, T 2048, 16 heads 339 / 238 - 247.
 // What bounds a block now (3200 cycles): the chain of 64 exponentials a thread at two warps per scheduler (1600), stores and barriers,
 // products (1700, beside them), TMEM loads.
 // The dQ partials of the key tiles are summed in an fp32 buffer by vector reductions (`red.global.add.v4.f32`, 16
@@ -47,7 +47,10 @@ constexpr int B3_NS = 3;                                   // ring depth in bloc
 constexpr int B3_THREADS = 512;
 constexpr int B3_COL = TILE * 16;                          // 128 rows of 8 bf16: a column of core matrices of 8 rows x 16 bytes (no swizzle)
 constexpr int B3_EXT = 2 * B3_COL;                         // the statistics of a block: a column of -lse / scale, one of -D
-constexpr unsigned B3_PACE_NS = 90;                        // B 64, T 1024, us: none 616, 20 x 16 582, 100 x 8 570, 150 x 8 (longer than a block) 692
+// A pause after every second reduction.  __nanosleep counts in steps: 90 and 120 ns give the same time, 150 falls into the next step, and eight of
+// those with the reductions' own 1400 cycles outlast a block of 3200.  Whole backward, 12 heads, us, none / 45 / 90 / 120 / 150 ns: B 64, T 1024 620 / 611 /
+// 602 / 604 / 652; B 4 65.5 / 61.9 / 60.5 / 60.5 / 67.9; B 7, T 777 81.6 / 77.4 / 75.2 / 75.2 / 84.7; B 2, T 1024 35.2 / 33.5 / 32.8 / 32.8 / 36.7.
+constexpr unsigned B3_PACE_NS = 90;
 constexpr int B3_SMEM = 4 * T128 /*K,V x2*/ + B3_NS * (2 * T128 + B3_EXT) + 2 * T128 /*dS^T*/ + T128 /*epilogue staging*/ + 2 * B3_COL + 256 /*barriers*/ +
                         1024 /*alignment*/;
 static_assert(B3_SMEM <= 227 * 1024, "shared memory of a CTA");

@@ -34,15 +34,17 @@ struct Tile { int bn, cl, splits; };
 thread_local int g_force_bn = 0, g_force_cl = 1;          // test hook (llmb_gemm_force_tile): 0 = the rule decides
 
 // The configuration with the smallest estimated time, in microseconds on a B200 from linear fits over M = 64 ... 5439, K and N =
-// 384 ... 5120 (the fits are within 15 %; the small kernel must win by 5 %): a fixed part (launch, set-up, epilogue) plus a cost per
+// 384 ... 5120 (the small kernel must win by 5 %): a fixed part (launch, set-up, epilogue) plus a cost per
 // 128-byte k-block, bounded by what one SM can fetch (24 / 32 KB per k-block) in the small kernel and by the 256-row MMAs in the pair
 // kernel; MN-major operands cost more per k-block; more CTAs than SMs run side by side at the cost of each other's k-blocks; a
 // further round of pair tiles costs its epilogue if that is longer than its k-loop.  Clusters only while they fit in one round:
-// beyond it they were 1.5 - 4 times slower than one CTA per tile.  Measured, bias + residual: M 64, K 3072, N 768: pair 22.4 us,
-// 128 x 128 17.8, 64 x 4 CTAs 8.7; M 776, K 1024, N 1024: 14.3 / 10.7 / (64 x 1) 8.8; M 4096, K 768, N 3072: 27.1 / 50.6 / 44.8.
-// Beyond the fits, every configuration forced on the seven products of a layer at M up to 16384 and C 768, 1024, 1600: from M 4096 on the
-// pair kernel is the fastest but for two products (M 5439, C 1600, input gradients: 128 x 128 11 - 13 % less) and the rule takes it;
-// elsewhere it is off by 10 - 19 % at three of the 42 products below that (M 776: C x C at C 1600 17.0 against 14.3 us).
+// beyond it they are 1.5 - 4 times slower than one CTA per tile.
+// The constants were fitted to kernels whose epilogues took longer and whose loads of MN-major operands did cost more, which those of today
+// no longer do.  With the kernels as they are the choice is 1.9 % slower than the best configuration on average over 19 sizes, at worst 44 % (TF32 M
+// 1024, C 768, N 3072 with GELU, 31.8 against 22.0 us; M 8192, C 384 C x C input gradient 7.2 / 5.9).  A new fit (0.7 %, 15 %) was not kept: forward
+// passes of one row at C 384 with 656 and more tokens became 3 - 9 % slower.  Now, us, launches from a graph, pair / 128 x 128 / best 64-column
+// form: bias + residual, M 64, K 3072, N 768 19.8 / 15.8 / (4 CTAs) 7.7, M 776, K 1024, N 1024 10.9 / 8.7 / (1) 7.4, M 776, K 1600, N 1600 14.2 / 11.7 /
+// (1) 12.4; bias + GELU, M 4096, K 768, N 3072 21.4 / 30.9 / (1) 45.5; the rule takes the fastest of the three each time.
 // splits: parts of K in the pair kernel; most: the most that this kernel's CTAs may cut it into.
 Tile pick_tile(int kind, int epi, int M, int N, int kb_total, int splits, int most, int a_mn, int b_mn) {
   if (g_force_bn) return {kind == KIND_F8F6F4 && g_force_bn == 64 ? 128 : g_force_bn, g_force_cl, splits};
@@ -66,10 +68,10 @@ Tile pick_tile(int kind, int epi, int M, int N, int kb_total, int splits, int mo
         while (sp < most && tiles * (sp + 1) <= sms && kb_total / (sp + 1) >= 4) ++sp;
       const float per_sm = (float)(tiles * cl * sp) / sms;
       // one to two CTAs per SM and operands stored along K: the second CTA of an SM overlaps the first one's epilogue, and the kernels
-      // before and after overlap the short tail.  M 776, us, pair / 128 x 128: K 1024, N 3072 (168 CTAs) 14.6 / 12.8, N 4096 with GELU
-      // (224) 17.1 / 15.6; K 1600, N 4800 (266) 28.9 / 20.9.  Not with an auxiliary input, which the pair kernel works in with 16
-      // warps: bias + residual, M 4096, N 768 (192), K 768 13.0 / 18.4, K 3072 25.4 / 37.5; dGELU, M 776, N 3072 (168) 13.0 / 18.7, N 4096
-      // (224) 15.2 / 23.2 (a backward product, whose weights lie along N, is out by that already).
+      // before and after overlap the short tail.  M 776, us, pair / 128 x 128: K 1024, N 3072 (168 CTAs) 11.4 / 10.7, N 4096 with GELU
+      // (224) 13.5 / 12.5; K 1600, N 4800 (266) 20.1 / 14.9.  Not with an auxiliary input: bias + residual, M 4096, N 768 (192), K 768
+      // 11.0 / 16.1, K 3072 21.9 / 33.9; dGELU, M 776, K 1024, N 3072 (168) 12.2 / 17.2, N 4096 (224) 12.5 / 17.5 (a backward product,
+      // whose weights lie along N, is out by that already).
       const bool beside = per_sm > 1.f && per_sm <= 2.f && !a_mn && !b_mn && epi != EPI_BIAS_RESID && epi != EPI_DGELU;
       const float w = per_sm <= 1.f ? 1.f : beside ? per_sm : 0.5f * (per_sm + ceilf(per_sm));
       const float fixed = (cl == 1 ? (bn == 64 ? 4.2f : 5.0f) : cl == 2 ? 5.6f : 6.2f) + (aux ? (bn == 64 ? 0.3f : 1.2f) : 0.f) + f32;

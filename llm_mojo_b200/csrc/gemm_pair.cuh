@@ -16,11 +16,11 @@ constexpr int SMEM2_TAIL = 512;                        // barriers, TMEM slot, a
 // What a tile's epilogue costs its warps beside the arithmetic, and what was done about it (cycles per tile and warp at K = 768, where a tile's
 // MMAs take 6144; clock traces): the hand-back of the accumulator released at cluster scope, which waited for every store and reduction in
 // flight (1200 - 2500; relaxed now, see mbar_arrive_cluster); five integer divisions for the tile's place (500); the bias from L2 (700 a
-// slab in which its loads took turns; the four of 32 columns go out together now); with an auxiliary input one box per warp, whose load, work and store took turns (two boxes now,
-// each loaded again as soon as it has left); column sums before the store of the box (after it now).  Sixteen epilogue warps hid some of
-// that behind one another, at 96 registers and with four of them contending for a scheduler; with it gone eight are faster: M 16384, C
-// 768, us, before / 16 / 8 warps: bias + GELU, N 3072 81.6 / 79.0 / 71.0, dGELU + column sums, N 3072 85.0 / 76.5 / 78.4; M 65536: 324 / 304 - 313 / 265 -
-// 275.  What bounds a tile now is what it moves: 390 KB of operands and 128 KB of auxiliary input and results per CTA at the 60 - 70
+// slab in which its loads took turns; the four of 32 columns go out together now); with an auxiliary input one box per warp, whose load,
+// work and store took turns (two boxes now, each loaded again as soon as it has left); column sums before the store of the box (after it now).  Sixteen epilogue warps hid some of
+// that behind one another, at 96 registers and with four of them contending for a scheduler; with it gone eight are faster with two outputs,
+// nearly as fast with an auxiliary input, and one form serves both.  C 768, N 3072, us, before / 16 / 8 warps: bias + GELU, M 16384 81.6 / 79.0 / 71.0, M
+// 65536 324 / 304 - 313 / 265 - 275; dGELU + column sums, M 16384 85.0 / 76.5 / 78.4.  What bounds a tile now is what it moves: 390 KB of operands and 128 KB of auxiliary input and results per CTA at the 60 - 70
 // bytes a cycle that an SM gets when all of them load.
 constexpr int EPI_WARPS = 8;
 constexpr int PAIR_THREADS = 32 * (4 + EPI_WARPS);

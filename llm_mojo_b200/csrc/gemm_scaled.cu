@@ -7,8 +7,9 @@
 //
 // What bounds these products is the operands' way from L2: 512 cycles of MMAs eat 32 KB per CTA of a 256 x 256 pair tile, 64 bytes a
 // cycle and SM of the 68 - 86 there are; a 128 x 256 tile of one CTA needs 96.  The eight products of a layer, us, 128 x 256 tiles on
-// single CTAs (whose fp32 results went through registers of four warps) / pairs: MXFP8 M 4096, C 1280 249 / 229, M 16384, C 768 347 /
-// 319; NVFP4 M 4096, C 1600 237 / 230; up to M 1152 all the same.
+// single CTAs (whose fp32 results went through registers of four warps) / pairs: MXFP8 M 128, C 1280 98.9 / 88.5, M 4096, C 1280 246 /
+// 206, M 8192, C 768 194 / 175; NVFP4 M 128, C 1600 94.4 / 80.2, M 4096, C 1600 234 / 193.  Single ones that stay slower than on single CTAs, for
+// the cluster's set-up: MXFP8 dGELU M 2048, K 384, N 1536 7.8 / 8.3, M 1024, K 768, N 3072 8.9 / 9.3; weight gradient 3072 x 768 of 2048 rows 9.3 / 9.9.
 #include "gemm_pair.cuh"
 
 namespace {

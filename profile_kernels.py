@@ -6,6 +6,7 @@
     python profile_kernels.py small       # layer GEMMs of 776 rows (d24 sampling): 128-row tiles, one CTA each or a cluster per contraction
     python profile_kernels.py f32attn     # fp32 attention forward + backward, B=8 T=1024 NH=12
     python profile_kernels.py nvfp4       # NVFP4 operands (maxima, both orientations) and block-scaled GEMMs, 8192 x 1600 x 6400
+    python profile_kernels.py fp8b        # block-scaled FP8 operands (both orientations) and GEMMs, 8192 x 1280 x 5120
     python profile_kernels.py lmhead      # LM-head GEMM on 8192 rows + fused softmax/cross-entropy
     python profile_kernels.py layernorm   # LayerNorm forward + backward on 65536 x 768
     python profile_kernels.py fusedpull   # a layer GEMM that pulls its own weight (four emulated owners) with its copier warps
@@ -187,7 +188,23 @@ def case_nvfp4(reps):
         lowp.matmul_bwd_fp4(dinp, dw, None, d, x, w, seed=1, step=i)
 
 
-CASES = {"small": case_small, "f32attn": case_f32attn, "nvfp4": case_nvfp4, "fusedgather": case_fusedgather, "fusedpull": case_fusedpull, "attn": case_attn, "gemm": case_gemm, "lmhead": case_lmhead, "layernorm": case_layernorm}
+def case_fp8b(reps):
+    """Block-scaled FP8 linear layer pieces: quantisation in both orientations, native block-scaled GEMMs."""
+    from llm_mojo_b200.ops import lowp
+    rows, C, OC = 8192, 1280, 5120
+    x = torch.randn(rows, C, device="cuda").bfloat16()
+    w = (torch.randn(OC, C, device="cuda") * 0.02).bfloat16()
+    d = torch.randn(rows, OC, device="cuda").bfloat16()
+    b = torch.zeros(OC, device="cuda", dtype=torch.bfloat16)
+    out, pre = torch.empty(rows, OC, device="cuda", dtype=torch.bfloat16), torch.empty(rows, OC, device="cuda", dtype=torch.bfloat16)
+    dinp = torch.empty(rows, C, device="cuda", dtype=torch.bfloat16)
+    dw = torch.zeros(OC, C, device="cuda")
+    for _ in range(reps):
+        lowp.matmul_fwd_fp8_block(out, x, w, b, pre_gelu=pre)
+        lowp.matmul_bwd_fp8_block(dinp, dw, None, d, x, w)
+
+
+CASES = {"fp8b": case_fp8b, "small": case_small, "f32attn": case_f32attn, "nvfp4": case_nvfp4, "fusedgather": case_fusedgather, "fusedpull": case_fusedpull, "attn": case_attn, "gemm": case_gemm, "lmhead": case_lmhead, "layernorm": case_layernorm}
 
 if __name__ == "__main__":
     ap = argparse.ArgumentParser(description=__doc__, formatter_class=argparse.RawDescriptionHelpFormatter)
